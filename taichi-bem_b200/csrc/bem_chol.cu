@@ -37,7 +37,6 @@ namespace {
 constexpr int CH_IB = 64;   // diagonal sub-block
 constexpr int CH_SP = 256;  // sub-panel width of the panel factorisation
 constexpr int CH_NB_DEFAULT = 1024;  // panel width (columns per trailing update; measured 510 / 410 / 384 ms for 256 / 512 / 1024 on the 30722-unknown normal matrix)
-constexpr int CH_LD = CH_IB + 1;
 
 struct cd {
     double re, im;
@@ -61,87 +60,121 @@ __device__ __forceinline__ void st_c(double* A, int64_t idx, cd v) {
 // read and written), and Linv = L^{-1} (64 x 64, identity beyond nb) into
 // inv.  A non-positive or non-finite pivot sets *info to 1 + its global
 // column (the first one wins) and is replaced by 1 so the kernel finishes.
+//
+// One CTA on the factorisation's serial chain, so what counts is the latency
+// of a column.  Both triangles live in registers (thread (ty, tx) of a 16 x 16
+// grid holds the entries (ty + 16 a, tx + 16 b) of the block and of the
+// inverse) and one elimination runs on both: with the unscaled column m_i =
+// M[i][j], pivot d and the unscaled row x_c = X[j][c],
+//   M[i][c] -= m_i conj(m_c) / d  (i >= c > j),   X[i][c] -= m_i x_c / d  (i > j),
+// so the square roots stay off the chain (L[i][j] = m_i / sqrt(d_j), X[i][c]
+// / sqrt(d_i), taken at the end) and a column costs one CTA barrier: its
+// owners publish the column and the row in one of two shared buffers, the
+// others read them while those of the next column are filled.  Blocks that
+// the column does not reach are skipped (whole 16 x 16 blocks, so a warp does
+// not diverge on it).  Measured (64 x 64 complex, B200): 26 us a block in a factorisation
+// against 110 us with the block and the inverse in shared memory, three
+// barriers a column, and the inverse built by rows afterwards.
 template <bool C>
 __global__ void __launch_bounds__(256) chol64_kernel(double* A, int64_t lda, int nb, double* inv, int32_t* info,
                                                      int col0) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    cd* M = reinterpret_cast<cd*>(smem_raw);  // [64][CH_LD]
-    cd* X = M + CH_IB * CH_LD;                // [64][64] inverse being built
-    __shared__ double s_d;
+    __shared__ cd s_col[2][CH_IB];
+    __shared__ cd s_row[2][CH_IB];
+    __shared__ double s_piv[CH_IB];
     const int tid = threadIdx.x;
-    for (int e = tid; e < CH_IB * CH_IB; e += blockDim.x) {
-        const int r = e / CH_IB, c = e - r * CH_IB;
-        cd v{r == c ? 1.0 : 0.0, 0.0};
-        if (r < nb && c < nb && c <= r) v = ld_c<C>(A, (int64_t)r * lda + c);
-        M[r * CH_LD + c] = v;
-    }
-    __syncthreads();
-    for (int j = 0; j < nb; ++j) {
-        if (tid == 0) {
-            double d = M[j * CH_LD + j].re;
-            if (!(d > 0.0) || !isfinite(d)) {
-                atomicCAS(info, 0, col0 + j + 1);
-                d = 1.0;
+    const int tx = tid & 15, ty = tid >> 4;
+    cd M[4][4], X[4][4];
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+            const int r = ty + 16 * a, c = tx + 16 * b;
+            X[a][b] = cd{r == c ? 1.0 : 0.0, 0.0};
+            M[a][b] = X[a][b];
+            if (r < nb && c <= r) M[a][b] = ld_c<C>(A, (int64_t)r * lda + c);
+        }
+#pragma unroll
+    for (int jb = 0; jb < 4; ++jb) {
+        for (int jj = 0; jj < 16; ++jj) {
+            const int j = 16 * jb + jj;
+            cd* col = s_col[j & 1];
+            cd* row = s_row[j & 1];
+            if (tx == jj) {
+#pragma unroll
+                for (int a = jb; a < 4; ++a) col[ty + 16 * a] = M[a][jb];
             }
-            d = sqrt(d);
-            M[j * CH_LD + j] = cd{d, 0.0};
-            s_d = 1.0 / d;
-        }
-        __syncthreads();
-        const double rd = s_d;
-        for (int i = j + 1 + tid; i < nb; i += blockDim.x) {
-            cd v = M[i * CH_LD + j];
-            M[i * CH_LD + j] = cd{v.re * rd, v.im * rd};
-        }
-        __syncthreads();
-        // rank-1 update of the trailing lower triangle: row i = j + 1 + tid % 64,
-        // columns j + 1 + tid / 64, + 4, ... up to i
-        {
-            const int i = j + 1 + (tid & 63);
-            if (i < nb) {
-                const cd a = M[i * CH_LD + j];
-                for (int c = j + 1 + (tid >> 6); c <= i; c += 4) {
-                    const cd b = M[c * CH_LD + j];
-                    // M[i][c] -= a conj(b)
-                    cd v = M[i * CH_LD + c];
-                    v.re -= a.re * b.re + a.im * b.im;
-                    v.im -= a.im * b.re - a.re * b.im;
-                    M[i * CH_LD + c] = v;
-                }
-            }
-        }
-        __syncthreads();
-    }
-    for (int e = tid; e < nb * nb; e += blockDim.x) {
-        const int r = e / nb, c = e - r * nb;
-        if (c <= r) st_c<C>(A, (int64_t)r * lda + c, M[r * CH_LD + c]);
-    }
-    // X = L^{-1} (lower), row by row: X[r][c] = (delta_rc - sum_{c<=q<r} L[r][q] X[q][c]) / L[r][r];
-    // four threads per column split the sum over q and combine by shuffles
-    {
-        const int c = tid >> 2, part = tid & 3;
-        for (int r = 0; r < CH_IB; ++r) {
-            cd v{0.0, 0.0};
-            if (r > c)
-                for (int q = c + part; q < r; q += 4) {
-                    const cd l = M[r * CH_LD + q], x = X[q * CH_IB + c];
-                    v.re -= l.re * x.re - l.im * x.im;
-                    v.im -= l.re * x.im + l.im * x.re;
-                }
-            v.re += __shfl_xor_sync(0xffffffffu, v.re, 1);
-            v.im += __shfl_xor_sync(0xffffffffu, v.im, 1);
-            v.re += __shfl_xor_sync(0xffffffffu, v.re, 2);
-            v.im += __shfl_xor_sync(0xffffffffu, v.im, 2);
-            if (part == 0) {
-                if (r == c) v = cd{1.0, 0.0};
-                if (r < c) v = cd{0.0, 0.0};
-                const double d = M[r * CH_LD + r].re;  // real positive (identity padding beyond nb)
-                X[r * CH_IB + c] = cd{v.re / d, v.im / d};
+            if (ty == jj) {
+#pragma unroll
+                for (int b = 0; b <= jb; ++b) row[tx + 16 * b] = X[jb][b];
             }
             __syncthreads();
+            double d = col[j].re;
+            if (!(d > 0.0) || !isfinite(d)) {
+                if (tid == 0 && j < nb) atomicCAS(info, 0, col0 + j + 1);
+                d = 1.0;
+            }
+            if (tid == 0) s_piv[j] = d;
+            const double rd = 1.0 / d;
+            cd mi[4];  // m_i / d of this thread's rows below j (0 elsewhere)
+#pragma unroll
+            for (int a = jb; a < 4; ++a) {
+                const bool below = ty + 16 * a > j;
+                const cd v = col[ty + 16 * a];
+                mi[a] = cd{below ? v.re * rd : 0.0, C && below ? v.im * rd : 0.0};
+            }
+#pragma unroll
+            for (int b = jb; b < 4; ++b) {
+                const bool right = tx + 16 * b > j;
+                cd v = col[tx + 16 * b];
+                if (!right) v = cd{0.0, 0.0};
+#pragma unroll
+                for (int a = b; a < 4; ++a) {
+                    // M -= (m_i / d) conj(m_c)
+                    M[a][b].re -= mi[a].re * v.re;
+                    if (C) {
+                        M[a][b].re -= mi[a].im * v.im;
+                        M[a][b].im -= mi[a].im * v.re;
+                        M[a][b].im += mi[a].re * v.im;
+                    }
+                }
+            }
+#pragma unroll
+            for (int b = 0; b <= jb; ++b) {
+                const cd v = row[tx + 16 * b];  // zero right of the diagonal
+#pragma unroll
+                for (int a = jb; a < 4; ++a) {
+                    X[a][b].re -= mi[a].re * v.re;
+                    if (C) {
+                        X[a][b].re += mi[a].im * v.im;
+                        X[a][b].im -= mi[a].re * v.im;
+                        X[a][b].im -= mi[a].im * v.re;
+                    }
+                }
+            }
         }
     }
-    for (int e = tid; e < CH_IB * CH_IB; e += blockDim.x) st_c<C>(inv, e, X[e]);
+    __syncthreads();
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+        const int c = tx + 16 * b;
+        const double sc = sqrt(s_piv[c]), rc = 1.0 / sc;
+#pragma unroll
+        for (int a = b; a < 4; ++a) {
+            const int r = ty + 16 * a;
+            if (r < nb && c <= r)
+                st_c<C>(A, (int64_t)r * lda + c, r == c ? cd{sc, 0.0} : cd{M[a][b].re * rc, M[a][b].im * rc});
+        }
+    }
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+        const int r = ty + 16 * a;
+        const double rc = 1.0 / sqrt(s_piv[r]);
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+            const int c = tx + 16 * b;
+            st_c<C>(inv, r * CH_IB + c, cd{X[a][b].re * rc, X[a][b].im * rc});
+        }
+    }
 }
 
 // General FP64 tensor-core product  C += alpha A op(B)  (m x n, K = k),
@@ -370,11 +403,6 @@ int chol_t(bem_ctx* ctx, double* A, int64_t n, int64_t lda, bool tensor_cores, i
     double* tmp = inv + inv_d;
     double* dg = tmp + tmp_d;
     if (int rc = bem_check_cuda(ctx, cudaMemsetAsync(info, 0, sizeof(int32_t), s), "chol info")) return rc;
-    const size_t smem = sizeof(cd) * (CH_IB * CH_LD + CH_IB * CH_IB);
-    if (int rc = bem_check_cuda(ctx, cudaFuncSetAttribute(chol64_kernel<C>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                          (int)smem),
-                                "chol64 smem"))
-        return rc;
     auto at = [&](int64_t r, int64_t c) { return A + W * (r * lda + c); };
     const int nbw = ctx->tune[BEM_TUNE_CHOL_NB] > 0 ? ctx->tune[BEM_TUNE_CHOL_NB] : CH_NB_DEFAULT;
     for (int64_t k0 = 0; k0 < n; k0 += nbw) {
@@ -386,7 +414,7 @@ int chol_t(bem_ctx* ctx, double* A, int64_t n, int64_t lda, bool tensor_cores, i
         const int64_t sb = std::min<int64_t>(CH_SP, k0 + kb - s0);
         for (int64_t j0 = s0; j0 < s0 + sb; j0 += CH_IB) {
             const int jb = (int)std::min<int64_t>(CH_IB, s0 + sb - j0);
-            chol64_kernel<C><<<1, 256, smem, s>>>(at(j0, j0), lda, jb, inv, info, (int)j0);
+            chol64_kernel<C><<<1, 256, 0, s>>>(at(j0, j0), lda, jb, inv, info, (int)j0);
             ctx->launches++;
             if (int rc = bem_check_cuda(ctx, cudaGetLastError(), "chol64_kernel")) return rc;
             if (X)
