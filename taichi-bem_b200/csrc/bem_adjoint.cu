@@ -20,6 +20,7 @@
 // vertex), so the same quadrature integrates them.  All in FP64.
 #include <cuda_runtime.h>
 
+#include "bem_farfield.cuh"
 #include "bem_internal.cuh"
 #include "bem_quadrature.cuh"
 
@@ -97,7 +98,7 @@ __device__ __forceinline__ void adj_point(PairMoments& M, const double d[3], dou
                                           const double by[3], double uy, double sgn, const double nj[3],
                                           double invJj) {
     const double r2 = d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
-    const double rinv = rsqrt(r2);
+    const double rinv = dev_rsqrt(r2);
     const double rinv2 = rinv * rinv;
     double g[3];
     if (OP == BEM_OP_V) {

@@ -1637,6 +1637,13 @@ int bem_launch_assemble_parts(bem_ctx* ctx, const bem_op_desc* op, const bem_spa
     fa.y = (double*)y;
     fa.conj_x = conj_x;
 
+    if (!near_only) {
+        // FP64: the kernel that evaluates an unordered pair once, where it has the bases
+        const int rc = bem_launch_far64(ctx, op, test, trial, mode, out, ld, scale, out_t, scale_t, x, y, conj_x, s);
+        if (rc < 0) return rc;
+        if (rc == BEM_OK) fa.skip_far = 1;
+    }
+
     NearArgs na;
     na.n_near = ctx->n_near;
     na.near = ctx->near;

@@ -32,8 +32,23 @@ __device__ __forceinline__ void dev_r_rinv(float r2, float& r, float& rinv) {
     rinv = fmaf(0.5f * y0, e, y0);
     r = fmaf(0.5f * p, e, p);
 }
+// FP64: the hardware's approximate reciprocal square root (about 20 bits; the
+// low word of its result is zero, so its square is exact) and one step of the
+// third-order iteration y (1 + e/2 + 3 e^2/8), e = 1 - r2 y^2, whose remainder
+// 5 e^3/16 is below 2^-58: five FP64 operations, against about ten and a range
+// check in the library's rsqrt.  0 and infinity keep the approximation's
+// infinity and 0, as the library's do.
+__device__ __forceinline__ double dev_rsqrt(double r2) {
+    double y0;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y0) : "d"(r2));
+    const double e = fma(-r2, y0 * y0, 1.0);
+    const double y = fma(y0 * e, fma(0.375, e, 0.5), y0);
+    // exponent field 0 or all ones: the iteration has no finite value there
+    const bool special = (unsigned)(__double2hiint(y0) - 0x00100000) >= 0x7fe00000u;
+    return special ? y0 : y;
+}
 __device__ __forceinline__ void dev_r_rinv(double r2, double& r, double& rinv) {
-    rinv = rsqrt(r2);
+    rinv = dev_rsqrt(r2);
     r = r2 * rinv;
 }
 
@@ -134,7 +149,71 @@ __device__ __forceinline__ void dev_sincos_phase(float x, bool small, float* s, 
     else
         dev_sincos(x, s, c);
 }
-__device__ __forceinline__ void dev_sincos(double x, double* s, double* c) { sincos(x, s, c); }
+
+// FP64 sine and cosine on |y| <= 0.3 (SHORT) or |y| <= pi/4: Taylor
+// polynomials whose first dropped terms are below 2.7e-17 (y^13) and 5.5e-19
+// (y^14), or 4.7e-17 (y^17) and 2.1e-18 (y^18).
+template <bool SHORT>
+__device__ __forceinline__ void dev_sincos_poly64(double y, double* s, double* c) {
+    const double y2 = y * y;
+    double ps, pc;
+    if (SHORT) {
+        ps = fma(y2, -1.0 / 39916800.0, 1.0 / 362880.0);
+        pc = fma(y2, 1.0 / 479001600.0, -1.0 / 3628800.0);
+    } else {
+        ps = fma(y2, -1.0 / 1307674368000.0, 1.0 / 6227020800.0);
+        ps = fma(y2, ps, -1.0 / 39916800.0);
+        ps = fma(y2, ps, 1.0 / 362880.0);
+        pc = fma(y2, 1.0 / 20922789888000.0, -1.0 / 87178291200.0);
+        pc = fma(y2, pc, 1.0 / 479001600.0);
+        pc = fma(y2, pc, -1.0 / 3628800.0);
+    }
+    ps = fma(y2, ps, -1.0 / 5040.0);
+    ps = fma(y2, ps, 1.0 / 120.0);
+    ps = fma(y2, ps, -1.0 / 6.0);
+    *s = fma(y * y2, ps, y);
+    pc = fma(y2, pc, 1.0 / 40320.0);
+    pc = fma(y2, pc, -1.0 / 720.0);
+    pc = fma(y2, pc, 1.0 / 24.0);
+    pc = fma(y2, pc, -0.5);
+    *c = fma(y2, pc, 1.0);
+}
+__device__ __noinline__ void dev_sincos_any(double x, double* s, double* c) { sincos(x, s, c); }
+// Any FP64 phase.  Up to 1e5 (a wavenumber of 1e5 on a unit mesh): reduction
+// by n pi/2 with pi/2 split in two doubles (n pi/2_hi enters by one FMA, the
+// remainder is good to 2^-54), the polynomials above and the quadrant; beyond,
+// and for infinities and NaN, the library's sincos.  About 24 FP64 operations
+// against about 40; the library's large-argument path is kept out of line.
+__device__ __forceinline__ void dev_sincos(double x, double* s, double* c) {
+    if (!(fabs(x) <= 1e5)) {
+        double a, b;
+        dev_sincos_any(x, &a, &b);
+        *s = a;
+        *c = b;
+        return;
+    }
+    // rint by the 1.5 2^52 shift; the integer sits in the low word
+    const double t = fma(x, 0.63661977236758134308, 6755399441055744.0);
+    const int q = __double2loint(t);
+    const double fn = t - 6755399441055744.0;
+    double y = fma(-fn, 1.57079632679489661923, x);
+    y = fma(-fn, 6.12323399573676603587e-17, y);
+    double sy, cy;
+    dev_sincos_poly64<false>(y, &sy, &cy);
+    const double ss = (q & 1) ? cy : sy, cc = (q & 1) ? sy : cy;
+    *s = (q & 2) ? -ss : ss;
+    *c = ((q + 1) & 2) ? -cc : cc;
+}
+// The phase of a pair frame, bounded on the host: PH 2 <= 0.3, 1 <= pi/4, 0 any
+template <int PH>
+__device__ __forceinline__ void dev_sincos_ph(double y, double* s, double* c) {
+    if (PH == 2)
+        dev_sincos_poly64<true>(y, s, c);
+    else if (PH == 1)
+        dev_sincos_poly64<false>(y, s, c);
+    else
+        dev_sincos(y, s, c);
+}
 
 struct cxd {
     double re, im;

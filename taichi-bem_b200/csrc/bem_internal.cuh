@@ -106,6 +106,11 @@ int bem_launch_assemble(bem_ctx* ctx, const bem_op_desc* op, const bem_space* te
 int bem_launch_assemble_parts(bem_ctx* ctx, const bem_op_desc* op, const bem_space* test, const bem_space* trial,
                               int mode, void* out, int64_t ld, double scale, void* out_t, double scale_t,
                               const void* x, void* y, int conj_x, cudaStream_t s, bool near_only);
+// FP64 far pairs of one operator, each unordered pair evaluated once
+// (bem_far64.cu); 1 where the general far_kernel has to run.
+int bem_launch_far64(bem_ctx* ctx, const bem_op_desc* op, const bem_space* test, const bem_space* trial, int mode,
+                     void* out, int64_t ld, double scale, void* out_t, double scale_t, const void* x, void* y,
+                     int conj_x, cudaStream_t s);
 // One operator at nk Helmholtz wavenumbers (bem_kbatch.cu): far pairs in
 // k-batched launches, near pairs per wavenumber.
 int bem_launch_assemble_batch(bem_ctx* ctx, const bem_op_desc* op, const bem_space* test, const bem_space* trial,
