@@ -94,3 +94,69 @@ def test_unordered_pairs_over_partial_lists(engine, op, nbx, nby, k):
     yd = torch.zeros(n, dtype=out.dtype, device="cuda")
     engine.apply(desc, td, rd, torch.as_tensor(x, device="cuda"), yd, scale=-0.5, conj_x=helm)
     assert np.abs(yd.cpu().numpy() - y).max() < 1e-12 * np.abs(y).max()
+
+
+# ---- partial-pivoting LU --------------------------------------------------------------
+_EPS = {"float64": 2.3e-16, "complex128": 2.3e-16, "float32": 1.2e-7, "complex64": 1.2e-7}
+
+
+def _swapped(A, piv):
+    A = A.copy()
+    for i, p in enumerate(piv):
+        A[[i, p]] = A[[p, i]]
+    return A
+
+
+@pytest.mark.parametrize("dtype", list(_EPS))
+@pytest.mark.parametrize("n", [1, 2, 7, 8, 9, 63, 64, 65, 72, 127, 130, 257, 513, 700, 1089])
+def test_lu_panel_sizes(engine, n, dtype):
+    """P A = L U with |re| + |im| pivoting (so |l| <= sqrt 2), over the
+    cluster sizes of the panel (1 to 16 CTAs), partial panels and partial
+    sub-blocks.  |P A - L U| is at most about n eps |L||U| entrywise; a random
+    matrix's growth keeps |L||U| below about sqrt(n) max|A| n^(2/3), and
+    rounding errors add like sqrt(n): 4 n eps max|U|."""
+    cplx = dtype.startswith("complex")
+    A = _gaussian((n, n), cplx, n)
+    LU = torch.as_tensor(A, device="cuda").to(getattr(torch, dtype)).contiguous()
+    A = LU.cpu().numpy().astype(np.complex128 if cplx else np.float64)
+    piv, info = engine.lu_factor(LU)
+    assert int(info.item()) == 0
+    F = LU.cpu().numpy().astype(A.dtype)
+    piv = piv.cpu().numpy()
+    assert ((piv >= np.arange(n)) & (piv < n)).all()
+    low, up = np.tril(F, -1) + np.eye(n), np.triu(F)
+    assert np.abs(low).max() <= 1.4143 and np.isfinite(F).all()
+    # a lower precision's product of the factors runs on the tensor cores in split TF32
+    tol = 4 * max(n, 8) * _EPS[dtype] * np.abs(up).max()
+    assert np.abs(_swapped(A, piv) - low @ up).max() < tol
+
+
+def test_lu_pivots_match_the_textbook(engine):
+    """The pivot sequence of a matrix with ties and exact zeros: the lowest
+    row of the largest |re| + |im|."""
+    rng = np.random.default_rng(5)
+    A = rng.integers(-3, 4, (150, 150)).astype(np.float64)
+    ref, want = A.copy(), []
+    for j in range(40):  # the steps whose values stay exact enough to tie only where the integers do
+        p = j + int(np.argmax(np.abs(ref[j:, j])))
+        want.append(p)
+        ref[[j, p]] = ref[[p, j]]
+        ref[j + 1:, j] /= ref[j, j]
+        ref[j + 1:, j + 1:] -= np.outer(ref[j + 1:, j], ref[j, j + 1:])
+    piv, _ = engine.lu_factor(torch.as_tensor(A, device="cuda"))
+    assert list(piv.cpu().numpy()[:4]) == want[:4]
+
+
+@pytest.mark.parametrize("col", [0, 5, 70])
+def test_lu_zero_and_nan_columns(engine, col):
+    """A zero column sets info to 1 + that column; a NaN never becomes a
+    pivot while a finite candidate is left."""
+    A = np.eye(140) * 3.0
+    A[col, col] = 0.0
+    _, info = engine.lu_factor(torch.as_tensor(A, device="cuda"))
+    assert int(info.item()) == col + 1
+    A = np.eye(140) * 3.0
+    A[col, col] = np.nan
+    A[col + 3, col] = 1.0
+    piv, _ = engine.lu_factor(torch.as_tensor(A, device="cuda"))
+    assert int(piv[col].item()) == col + 3
