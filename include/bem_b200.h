@@ -339,7 +339,7 @@ int bem_lu_solve_tiled(bem_ctx* ctx, int dtype, const void* LU, int64_t n, int64
  * device synchronisation is not acceptable -- and that therefore cannot create
  * a bem_ctx workspace.  It takes no context and performs no allocation: its
  * scratch is a file-scope device array sized for n <= BEM_STATIC_SOLVE_MAX_N
- * (about 0.65 MB, held by every GPU that loads the library until the process
+ * (about 1.7 MB, held by every GPU that loads the library until the process
  * exits); larger n is rejected with BEM_ERR_INVALID.  The first call on a
  * device looks up the array's device address (cudaGetSymbolAddress) with that
  * device current and caches it per device ordinal, i.e. for the runtime's

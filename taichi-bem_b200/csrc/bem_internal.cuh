@@ -88,6 +88,11 @@ int bem_big_ws(bem_ctx* ctx, size_t bytes, void** out);
 // Explicit inverses of the 64 x 64 diagonal tiles of a tile-LU factor into
 // dinv (bem_tilelu.cu); dtype BEM_F64/C128/F32/C64.
 int bem_tile_inverses(bem_ctx* ctx, int dtype, const void* A, int64_t n, int64_t lda, void* dinv, cudaStream_t s);
+// x = U^{-1} L^{-1} b for nrhs (already permuted) right-hand sides, vs doubles
+// apart, with a partial-pivoting factor and its tiles' inverses; y is scratch,
+// err (zeroed by the caller) receives BEM_ERR_TIMEOUT (bem_tilelu.cu).
+int bem_lu_tri_solve(bem_ctx* ctx, int dtype, const void* LU, int64_t n, int64_t lda, const void* dinv, const double* b,
+                     double* y, double* x, int nrhs, int64_t vs, int32_t* err, cudaStream_t s);
 // Asynchronous preconditioner step of the refinement (bem_tilelu.cu).
 int bem_tiled_precond_async(bem_ctx* ctx, int dtype, const void* LU, int64_t n, int64_t lda, const int32_t* piv,
                             const void* dinv, const double* r, double** out, const int* skip, cudaStream_t s);

@@ -733,155 +733,46 @@ __global__ void __launch_bounds__(TRSM_COLS* TRSM_ROWS) trsm_kernel(T* A, int64_
     }
 }
 
-// perm[i] = original row that ends up at row i after the LAPACK swap sequence
-// (sequential by nature; run in shared memory by one thread)
-__global__ void piv_to_perm_kernel(const int32_t* piv, int32_t* perm, int n) {
-    extern __shared__ int32_t sp[];
-    for (int i = threadIdx.x; i < n; i += blockDim.x) sp[i] = i;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int i = 0; i < n; ++i) {
-            int p = piv[i];
-            if (p != i && p >= 0 && p < n) {
-                int t = sp[i];
-                sp[i] = sp[p];
-                sp[p] = t;
-            }
+// perm[i] = original row that ends up at row i after the LAPACK swap sequence.
+// The swaps are sequential, but a row's path through them is not: each thread
+// follows one row (its position moves when a swap names it), with the swap
+// targets read in tiles from shared memory.  n threads of n compares, 38 us at
+// 3000 against 122 us with the sequence run by one thread.
+constexpr int PERM_TILE = 2048;
+__global__ void __launch_bounds__(256) piv_to_perm_kernel(const int32_t* piv, int32_t* perm, int n) {
+    __shared__ int32_t sp[PERM_TILE];
+    const int row = blockIdx.x * blockDim.x + threadIdx.x;
+    int pos = row;
+    for (int i0 = 0; i0 < n; i0 += PERM_TILE) {
+        const int m = min(PERM_TILE, n - i0);
+        __syncthreads();
+        for (int i = threadIdx.x; i < m; i += blockDim.x) {
+            const int p = piv[i0 + i];
+            sp[i] = p >= 0 && p < n ? p : i0 + i;
+        }
+        __syncthreads();
+        for (int i = 0; i < m; ++i) {
+            const int a = i0 + i, p = sp[i];
+            pos = pos == a ? p : (pos == p ? a : pos);
         }
     }
-    __syncthreads();
-    for (int i = threadIdx.x; i < n; i += blockDim.x) perm[i] = sp[i];
+    if (row < n) perm[pos] = row;
 }
 
-// ----------------------------------------------------------------------------
-// triangular solves: x = U^{-1} L^{-1} P b, one cooperative launch.
-// Vectors are FP64 (real or complex) whatever the factor storage type.
-// ----------------------------------------------------------------------------
-constexpr int TRSV_NB = 64;
-
-template <typename T, bool C>
-__global__ void __launch_bounds__(256) lu_solve_kernel(const T* LU, int64_t lda, int n, const int32_t* perm,
-                                                        const double* b, double* x, double* tmp, int64_t nrhs,
-                                                        int64_t ldb, GridBar* bar, int32_t* flag) {
-    using E = El<T, C>;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    E* sL = reinterpret_cast<E*>(smem_raw);                                  // [TRSV_NB][TRSV_NB]
-    double* sx = reinterpret_cast<double*>(sL + TRSV_NB * TRSV_NB);          // [TRSV_NB][8][2]
-    const unsigned nblk = gridDim.x;
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const int gwarp = blockIdx.x * (blockDim.x >> 5) + wid;
-    const int nwarp_total = nblk * (blockDim.x >> 5);
-    const int W = C ? 2 : 1;
-    // y = P b  (x is the work vector)
-    for (int64_t idx = blockIdx.x * blockDim.x + threadIdx.x; idx < (int64_t)n * nrhs;
-         idx += (int64_t)nblk * blockDim.x) {
-        int i = (int)(idx / nrhs), c = (int)(idx % nrhs);
-        int src = perm[i];
-        for (int w = 0; w < W; ++w) x[W * ((int64_t)i * ldb + c) + w] = b[W * ((int64_t)src * ldb + c) + w];
-    }
-    if (!grid_barrier(bar, nblk, flag)) return;
-    const int nblocks_r = (n + TRSV_NB - 1) / TRSV_NB;
-
-    // Diagonal block solve on CTA 0: the block of LU and the x segment are
-    // staged in shared memory, one warp per right-hand side.
-    auto diag_solve = [&](int r0, int r1, bool lower) {
-        const int m = r1 - r0;
-        for (int e = threadIdx.x; e < m * m; e += blockDim.x) {
-            int r = e / m, q = e - r * m;
-            sL[r * TRSV_NB + q] = ld<T, C>(LU, (int64_t)(r0 + r) * lda + r0 + q);
-        }
-        for (int e = threadIdx.x; e < m * nrhs; e += blockDim.x) {
-            int r = e / (int)nrhs, c = e - r * (int)nrhs;
-            sx[(r * 8 + c) * 2] = __ldcg(&x[W * ((int64_t)(r0 + r) * ldb + c)]);
-            sx[(r * 8 + c) * 2 + 1] = C ? __ldcg(&x[W * ((int64_t)(r0 + r) * ldb + c) + 1]) : 0.0;
-        }
-        __syncthreads();
-        if (wid < nrhs) {
-            const int c = wid;
-            for (int t = 0; t < m; ++t) {
-                const int r = lower ? t : m - 1 - t;
-                double sr = 0.0, si = 0.0;
-                const int q0 = lower ? 0 : r + 1, q1 = lower ? r : m;
-                for (int q = q0 + lane; q < q1; q += 32) {
-                    E l = sL[r * TRSV_NB + q];
-                    double xr = sx[(q * 8 + c) * 2], xi = sx[(q * 8 + c) * 2 + 1];
-                    sr += (double)l.re * xr - (C ? (double)l.im * xi : 0.0);
-                    if (C) si += (double)l.re * xi + (double)l.im * xr;
-                }
-                for (int o = 16; o > 0; o >>= 1) {
-                    sr += __shfl_xor_sync(0xffffffffu, sr, o);
-                    if (C) si += __shfl_xor_sync(0xffffffffu, si, o);
-                }
-                if (lane == 0) {
-                    double vr = sx[(r * 8 + c) * 2] - sr, vi = sx[(r * 8 + c) * 2 + 1] - si;
-                    if (!lower) {
-                        E d = sL[r * TRSV_NB + r];
-                        if (C) {
-                            double dr = d.re, di = d.im, den = dr * dr + di * di;
-                            double tr = (vr * dr + vi * di) / den;
-                            vi = (vi * dr - vr * di) / den;
-                            vr = tr;
-                        } else {
-                            vr = vr / (double)d.re;
-                        }
-                    }
-                    sx[(r * 8 + c) * 2] = vr;
-                    sx[(r * 8 + c) * 2 + 1] = vi;
-                }
-                __syncwarp();
-            }
-        }
-        __syncthreads();
-        for (int e = threadIdx.x; e < m * nrhs; e += blockDim.x) {
-            int r = e / (int)nrhs, c = e - r * (int)nrhs;
-            x[W * ((int64_t)(r0 + r) * ldb + c)] = sx[(r * 8 + c) * 2];
-            if (C) x[W * ((int64_t)(r0 + r) * ldb + c) + 1] = sx[(r * 8 + c) * 2 + 1];
-        }
-    };
-    // rows [i0, i1) (distributed over all warps): x[i] -= LU[i, r0:r1] x[r0:r1]
-    auto update = [&](int i0, int i1, int r0, int r1) {
-        for (int i = i0 + gwarp; i < i1; i += nwarp_total) {
-            for (int c = 0; c < nrhs; ++c) {
-                double sr = 0.0, si = 0.0;
-                for (int q = r0 + lane; q < r1; q += 32) {
-                    E l = ld<T, C>(LU, (int64_t)i * lda + q);
-                    double xr = __ldcg(&x[W * ((int64_t)q * ldb + c)]);
-                    double xi = C ? __ldcg(&x[W * ((int64_t)q * ldb + c) + 1]) : 0.0;
-                    sr += (double)l.re * xr - (C ? (double)l.im * xi : 0.0);
-                    if (C) si += (double)l.re * xi + (double)l.im * xr;
-                }
-                for (int o = 16; o > 0; o >>= 1) {
-                    sr += __shfl_xor_sync(0xffffffffu, sr, o);
-                    if (C) si += __shfl_xor_sync(0xffffffffu, si, o);
-                }
-                if (lane == 0) {
-                    x[W * ((int64_t)i * ldb + c)] = __ldcg(&x[W * ((int64_t)i * ldb + c)]) - sr;
-                    if (C) x[W * ((int64_t)i * ldb + c) + 1] = __ldcg(&x[W * ((int64_t)i * ldb + c) + 1]) - si;
-                }
-            }
-        }
-    };
-    // forward: L y = P b (unit diagonal)
-    for (int kb = 0; kb < nblocks_r; ++kb) {
-        const int r0 = kb * TRSV_NB, r1 = min(n, r0 + TRSV_NB);
-        if (blockIdx.x == 0) diag_solve(r0, r1, true);
-        if (!grid_barrier(bar, nblk, flag)) return;
-        if (r1 < n) {
-            update(r1, n, r0, r1);
-            if (!grid_barrier(bar, nblk, flag)) return;
-        }
-    }
-    // backward: U x = y
-    for (int kb = nblocks_r - 1; kb >= 0; --kb) {
-        const int r0 = kb * TRSV_NB, r1 = min(n, r0 + TRSV_NB);
-        if (blockIdx.x == 0) diag_solve(r0, r1, false);
-        if (!grid_barrier(bar, nblk, flag)) return;
-        if (r0 > 0) {
-            update(0, r0, r0, r1);
-            if (!grid_barrier(bar, nblk, flag)) return;
-        }
-    }
-    (void)tmp;
+// right-hand sides of the triangular solve, each contiguous and permuted, and back
+__global__ void gather_rhs_kernel(const double* b, int64_t ldb, const int32_t* perm, double* out, int64_t vs, int n,
+                                  int nrhs, int W) {
+    const int64_t id = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (id >= (int64_t)n * nrhs) return;
+    const int i = (int)(id / nrhs), c = (int)(id % nrhs);
+    const int64_t src = W * ((int64_t)perm[i] * ldb + c);
+    for (int w = 0; w < W; ++w) out[c * vs + (int64_t)W * i + w] = b[src + w];
+}
+__global__ void scatter_rhs_kernel(const double* x, int64_t vs, double* b, int64_t ldb, int n, int nrhs, int W) {
+    const int64_t id = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (id >= (int64_t)n * nrhs) return;
+    const int i = (int)(id / nrhs), c = (int)(id % nrhs);
+    for (int w = 0; w < W; ++w) b[W * ((int64_t)i * ldb + c) + w] = x[c * vs + (int64_t)W * i + w];
 }
 
 // y = alpha A x + beta y, A stored as T (real/complex), x/y FP64
@@ -1033,24 +924,18 @@ struct LinWs {
     GridBar* bar;
     PivSlot* slots;  // [2][PANEL_MAXB]
     void* rowbuf;    // [2][PANEL_MAXB+1][LU_NB] panel-row copies (16 B per element)
-    int32_t* perm;
-    double* vec;     // scratch vectors for the triangular solves
 };
 
-int linws(bem_ctx* ctx, int64_t n, int64_t nvec_doubles, LinWs* w) {
-    size_t off_bar = 0;
-    size_t off_slots = 256;
-    size_t off_rows = off_slots + sizeof(PivSlot) * 2 * PANEL_MAXB;
-    size_t off_perm = off_rows + 16 * (size_t)2 * (PANEL_MAXB + 1) * LU_NB;
-    size_t off_vec = (off_perm + sizeof(int32_t) * (size_t)n + 255) & ~size_t(255);
-    size_t total = off_vec + sizeof(double) * (size_t)nvec_doubles;
-    if (int rc = bem_ws_reserve(ctx, total)) return rc;
+// at_least: bytes the workspace has to have for a later call too
+int linws(bem_ctx* ctx, size_t at_least, LinWs* w) {
+    const size_t off_slots = 256;
+    const size_t off_rows = off_slots + sizeof(PivSlot) * 2 * PANEL_MAXB;
+    const size_t total = off_rows + 16 * (size_t)2 * (PANEL_MAXB + 1) * LU_NB;
+    if (int rc = bem_ws_reserve(ctx, std::max(total, at_least))) return rc;
     char* base = (char*)ctx->ws;
-    w->bar = (GridBar*)(base + off_bar);
+    w->bar = (GridBar*)base;
     w->slots = (PivSlot*)(base + off_slots);
     w->rowbuf = (void*)(base + off_rows);
-    w->perm = (int32_t*)(base + off_perm);
-    w->vec = (double*)(base + off_vec);
     return BEM_OK;
 }
 
@@ -1120,10 +1005,25 @@ int lu_panel_cluster(bem_ctx* ctx, T* A, int64_t lda, int n, int k0, int nb, int
     return chunk <= 256 ? go(lu_panel_cluster_kernel<T, C, 256>, 256) : go(lu_panel_cluster_kernel<T, C, 512>, 512);
 }
 
+// Workspace of lu_solve: permutation, the inverses of the diagonal tiles,
+// three sets of nrhs vectors vs doubles apart.
+struct SolveLayout {
+    size_t off_dinv, off_vec, total;
+    int64_t vs;
+    SolveLayout(size_t elem, int W, int64_t n, int64_t nrhs) {
+        auto up = [](size_t v) { return (v + 255) & ~size_t(255); };
+        off_dinv = up(sizeof(int32_t) * (size_t)n);
+        off_vec = off_dinv + up(2 * elem * (size_t)bem_lu_dinv_elems(n));
+        vs = (int64_t)(up(sizeof(double) * W * (size_t)n) / sizeof(double));
+        total = off_vec + 3 * sizeof(double) * (size_t)(nrhs * vs);
+    }
+};
+
 template <typename T, bool C>
 int lu_factor_t(bem_ctx* ctx, T* A, int64_t n, int64_t lda, int32_t* piv, int32_t* info, cudaStream_t s) {
+    // one growth of the workspace for the factorisation and a solve with it
     LinWs w;
-    if (int rc = linws(ctx, n, 0, &w)) return rc;
+    if (int rc = linws(ctx, SolveLayout(sizeof(T), C ? 2 : 1, n, 1).total, &w)) return rc;
     cudaMemsetAsync(w.bar, 0, sizeof(GridBar), s);
     cudaMemsetAsync(info, 0, sizeof(int32_t), s);
     cudaMemsetAsync(ctx->flags + 2, 0, sizeof(int32_t), s);
@@ -1185,35 +1085,28 @@ template <typename T, bool C>
 int lu_solve_t(bem_ctx* ctx, const T* LU, int64_t n, int64_t lda, const int32_t* piv, double* b, int64_t nrhs,
                int64_t ldb, cudaStream_t s) {
     if (nrhs < 1 || nrhs > 8) return bem_fail(ctx, BEM_ERR_INVALID, "lu_solve supports 1..8 right-hand sides");
-    const int W = C ? 2 : 1;
-    LinWs w;
-    if (int rc = linws(ctx, n, (int64_t)W * n * ldb, &w)) return rc;
-    cudaMemsetAsync(w.bar, 0, sizeof(GridBar), s);
-    cudaMemsetAsync(ctx->flags + 2, 0, sizeof(int32_t), s);
     if ((size_t)n * sizeof(int32_t) > 200 * 1024) return bem_fail(ctx, BEM_ERR_INVALID, "lu_solve: n > 51200");
-    cudaFuncSetAttribute(piv_to_perm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)(n * sizeof(int32_t)));
-    piv_to_perm_kernel<<<1, 256, n * sizeof(int32_t), s>>>(piv, w.perm, (int)n);
-    ctx->launches++;
-    const int threads = 256;
-    const size_t smem = sizeof(El<T, C>) * TRSV_NB * TRSV_NB + sizeof(double) * TRSV_NB * 8 * 2;
-    cudaFuncSetAttribute(lu_solve_kernel<T, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    int nblk = coop_blocks(ctx, (const void*)lu_solve_kernel<T, C>, threads, smem, ctx->num_sms);
-    if (nblk < 1) return bem_fail(ctx, BEM_ERR_CUDA, "lu_solve_kernel cannot be made co-resident");
-    int ni = (int)n;
-    double* xw = w.vec;
-    double* tmp = nullptr;
+    const int W = C ? 2 : 1;
+    const SolveLayout lay(sizeof(T), W, n, nrhs);
+    if (int rc = bem_ws_reserve(ctx, lay.total)) return rc;
+    const int64_t vs = lay.vs;
+    char* base = (char*)ctx->ws;
+    int32_t* perm = (int32_t*)base;
+    void* dinv = base + lay.off_dinv;
+    double* vb = (double*)(base + lay.off_vec);
+    double *vy = vb + nrhs * vs, *vx = vy + nrhs * vs;
     int32_t* flag = ctx->flags + 2;
-    const double* bc = b;
-    void* args[] = {(void*)&LU, &lda, &ni, &w.perm, &bc, &xw, &tmp, &nrhs, &ldb, &w.bar, &flag};
-    if (int rc = bem_check_cuda(ctx, cudaLaunchCooperativeKernel((const void*)lu_solve_kernel<T, C>, nblk, threads,
-                                                                args, smem, s),
-                                "lu_solve_kernel"))
-        return rc;
+    cudaMemsetAsync(flag, 0, sizeof(int32_t), s);
+    const int dtype = sizeof(T) == 8 ? (C ? BEM_C128 : BEM_F64) : (C ? BEM_C64 : BEM_F32);
+    piv_to_perm_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(piv, perm, (int)n);
+    const unsigned blocks = (unsigned)((n * nrhs + 255) / 256);
+    gather_rhs_kernel<<<blocks, 256, 0, s>>>(b, ldb, perm, vb, vs, (int)n, (int)nrhs, W);
+    ctx->launches += 2;
+    if (int rc = bem_tile_inverses(ctx, dtype, LU, n, lda, dinv, s)) return rc;
+    if (int rc = bem_lu_tri_solve(ctx, dtype, LU, n, lda, dinv, vb, vy, vx, (int)nrhs, vs, flag, s)) return rc;
+    scatter_rhs_kernel<<<blocks, 256, 0, s>>>(vx, vs, b, ldb, (int)n, (int)nrhs, W);
     ctx->launches++;
-    if (int rc = bem_check_cuda(ctx, cudaMemcpyAsync(b, xw, sizeof(double) * W * n * ldb, cudaMemcpyDeviceToDevice, s),
-                                "lu_solve copy"))
-        return rc;
+    if (int rc = bem_check_cuda(ctx, cudaGetLastError(), "lu_solve")) return rc;
     return check_flag(ctx, s, "lu_solve");
 }
 

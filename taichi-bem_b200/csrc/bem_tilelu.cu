@@ -17,13 +17,14 @@
 // consumes this factor corrects the difference (and reports non-convergence).
 //
 // Solve: a persistent kernel in which CTA b owns block rows b, b+P, b+2P...;
-// block row k accumulates L_kj x_j for every finished j < k (ready flags,
-// acquire/release, bounded waits), applies Linv_k, publishes x_k and its flag.
-// Each CTA handles its block rows in increasing order and all CTAs are
-// co-resident (cooperative launch), so every wait ends.
+// block row k accumulates L_kj x_j for every finished j < k (each value is its
+// own ready flag; bounded waits), applies Linv_k and publishes x_k.  Each CTA
+// handles its block rows in increasing order and all CTAs are co-resident
+// (cooperative launch), so every wait ends.
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "bem_gemm.cuh"
 #include "bem_internal.cuh"
@@ -519,255 +520,365 @@ __global__ void __launch_bounds__(256) tile_apply_kernel(T* A, int64_t lda, int 
 // --------------------------------------------------------------------------
 // barrier-free triangular solves
 // --------------------------------------------------------------------------
-__device__ __forceinline__ int ld_acquire_i(const int* p) {
-    int v;
-    asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+// "Not written yet": a signalling NaN, which no arithmetic produces (results
+// that are NaN are quiet) and which the permutation kernels below fill the
+// solution vectors with.  A value is its own ready flag.
+constexpr unsigned long long PENDING = 0x7ff4deadbeef0001ull;
+
+__device__ __forceinline__ double ld_vol(const double* p) {
+    double v;
+    asm volatile("ld.volatile.global.f64 %0, [%1];" : "=d"(v) : "l"(p) : "memory");
     return v;
 }
-__device__ __forceinline__ void st_release_i(int* p, int v) {
-    asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+__device__ __forceinline__ void st_vol(double* p, double v) {
+    asm volatile("st.volatile.global.f64 [%0], %1;" ::"l"(p), "d"(v) : "memory");
 }
+__device__ __forceinline__ bool pending(double v) { return __double_as_longlong(v) == (long long)PENDING; }
 
-// Waits (bounded) until flags[j] == epoch.  Returns false on timeout / failure.
-__device__ __forceinline__ bool wait_flag(const int* flags, int j, int epoch, int32_t* err) {
-    __shared__ int s_ok;
-    if (threadIdx.x == 0) {
-        int ok = 1;
-        unsigned it = 0;
-        while (ld_acquire_i(flags + j) != epoch) {
-            if (++it > FLAG_SPIN_CAP) {
-                atomicExch(err, BEM_ERR_TIMEOUT);
-                ok = 0;
-                break;
-            }
-            if ((it & 63u) == 0u && *(volatile int32_t*)err != 0) {
-                ok = 0;
-                break;
-            }
-            if (it > 256u) __nanosleep(64);
-        }
-        s_ok = ok;
-    }
-    __syncthreads();
-    return s_ok != 0;
-}
-
-// Warp-level bounded wait for a ready flag: lane 0 spins with acquire loads,
-// the warp barrier that follows orders the other lanes' reads after it.
-__device__ __forceinline__ bool warp_wait_flag(const int* flags, int j, int epoch, int32_t* err) {
-    int ok = 1;
-    if ((threadIdx.x & 31) == 0) {
-        unsigned it = 0;
-        while (ld_acquire_i(flags + j) != epoch) {
-            if (++it > FLAG_SPIN_CAP) {
-                atomicExch(err, BEM_ERR_TIMEOUT);
-                ok = 0;
-                break;
-            }
-            if ((it & 63u) == 0u && *(volatile int32_t*)err != 0) {
-                ok = 0;
-                break;
-            }
-            if (it > 256u) __nanosleep(64);
-        }
-    }
-    ok = __shfl_sync(0xffffffffu, ok, 0);
-    __syncwarp();
-    return ok != 0;
-}
-
-// x (FP64, real or complex interleaved, one right-hand side) overwritten by
-// U^{-1} L^{-1} x; the input must already be permuted (x = P b).
-// Block row k, per pass (forward with L, backward with U):
-//   * the block of the last dependency (L_k,k-1 or U_k,k+1) and the diagonal
-//     inverse (Linv_k or Uinv_k) are prefetched into shared memory;
-//   * every other finished block j is streamed from memory: warp w owns rows
-//     w, w+8, ... and keeps per-lane partial sums of L_kj x_j (in the factor's
-//     precision), two blocks per iteration, no CTA barrier, one cross-lane
-//     reduction at the end;
-//   * once the last dependency's flag is set only two GEMVs out of shared
-//     memory remain on the critical path; x_k is then published with a
-//     release store of its flag.
+// x = U^{-1} L^{-1} b for NR right-hand sides (FP64, real or complex
+// interleaved, vs doubles apart; b already permuted), y the intermediate;
+// y and x are PENDING on entry.  Persistent: CTA b owns block rows b, b + P,
+// ... of each pass (forward with L into y, backward with U into x), all CTAs
+// are co-resident (cooperative launch) and wait only for rows earlier in the
+// pass's order, so every wait ends; the waits are bounded all the same.
+//
+// What bounds it is the chain of 2 n / 64 block rows, each waiting for the one
+// before; the factor's bytes stream beside it.  So per hop there is one trip
+// through L2 and nothing else: the consumer polls the 64 values themselves (no
+// fence, flag and second read), the block of that last dependency, the
+// diagonal inverse (and, REF, the diagonal block) are already in shared
+// memory, and the blocks of the earlier dependencies are loaded into registers
+// before their values are waited for.  Measured (B200, one right-hand side,
+// against a ready flag per block row and the loads after it): complex FP64
+// 2999 rows 228 against 505 us, 7682 rows 612 against 1510 us; complex FP32
+// 5120 rows 334 against 543 us.  With REF, against one CTA solving each
+// diagonal block between grid barriers: 2999 complex, three right-hand sides,
+// 0.84 against 5.2 ms.
+//
+// Sums over the streamed blocks are held in ACC: the factor's own type for the
+// preconditioners (as the products of an FP32 factor are), FP64 with REF.  REF
+// (the solves of a partial-pivoting factor): the explicit inverse is corrected
+// once against the diagonal block itself, y0 = D a, y = y0 + D (a - T y0) in
+// FP64, which brings its backward error to that of substitution.
 constexpr int SOLVE_LD = LU_T + 4;  // padded row stride of the staged blocks
-constexpr size_t solve_smem_bytes(size_t elem) { return 2 * elem * LU_T * SOLVE_LD; }
+constexpr size_t solve_smem_bytes(size_t elem, bool ref) { return (ref ? 3 : 2) * elem * LU_T * SOLVE_LD; }
 
-template <typename T, bool C>
-__global__ void __launch_bounds__(256) tile_solve_kernel(const T* LU, int64_t lda, int n, const CE<T>* dinv,
-                                                         double* x, int* flags, int epoch, int32_t* err,
-                                                         const int* skip) {
+template <typename T, bool C, int NR, bool REF>
+__global__ void __launch_bounds__(256) tri_solve_kernel(const T* LU, int64_t lda, int n, const CE<T>* dinv,
+                                                        const double* b, double* y, double* x, int64_t vs,
+                                                        int vec, int32_t* err, const int* skip) {
     // skip != NULL: a device word set by the asynchronous refinement once it
     // has converged; the later, already queued solves return at once
     if (skip != nullptr && *skip != 0) return;
+    using ACC = typename std::conditional<REF, double, T>::type;
     constexpr int RW = LU_T / 8;  // rows per warp in the streamed part
+    constexpr int W = C ? 2 : 1;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     CE<T>* sB = reinterpret_cast<CE<T>*>(smem_raw);  // [LU_T][SOLVE_LD] last dependency block
     CE<T>* sD = sB + LU_T * SOLVE_LD;                 // [LU_T][SOLVE_LD] diagonal inverse
-    __shared__ double s_acc[LU_T][2];
-    __shared__ double s_x[LU_T][2];
+    CE<T>* sT = sD + LU_T * SOLVE_LD;                 // REF: [LU_T][SOLVE_LD] diagonal block
+    __shared__ double s_acc[LU_T][NR][2];
+    __shared__ double s_x[LU_T][NR][2];
+    __shared__ double s_r[REF ? LU_T : 1][NR][2];
     __shared__ int s_abort;
+    __shared__ int s_zero[2];  // REF: last row of the diagonal block with a zero pivot, -1 = none; by row parity
     const int nbk = (n + LU_T - 1) / LU_T;
     const int P = gridDim.x;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const int gr = tid >> 2, gq = tid & 3;  // GEMV mapping: row gr, columns gq + 4i
-    const int W = C ? 2 : 1;
-    if (tid == 0) s_abort = 0;
+    if (tid == 0) {
+        s_abort = 0;
+        s_zero[0] = s_zero[1] = -1;
+    }
+    int par = 0;
     __syncthreads();
+    // element i of the row at p (aligned: one access per complex element)
+    auto elem = [&](const T* p, int i) -> CE<T> {
+        if (C && vec) {
+            if constexpr (sizeof(T) == 8) {
+                const double2 v = *reinterpret_cast<const double2*>(p + 2 * i);
+                return CE<T>{(T)v.x, (T)v.y};
+            } else {
+                const float2 v = *reinterpret_cast<const float2*>(p + 2 * i);
+                return CE<T>{(T)v.x, (T)v.y};
+            }
+        }
+        return ldE<T, C>(p, i);
+    };
+    // One warp: value c of every right-hand side of v into (re, im), 0 for c >= lim;
+    // waits (bounded) until all of the warp's are written.
+    auto fetch = [&](const double* v, int base, int c0_, int lim, double (*re)[NR], double (*im)[NR], int cols) -> bool {
+        unsigned it = 0;
+        for (;;) {
+            bool ready = true;
+            for (int h = 0; h < cols; ++h) {
+                const int c = c0_ + 32 * h;
+#pragma unroll
+                for (int r = 0; r < NR; ++r) {
+                    double a = 0.0, d = 0.0;
+                    if (c < lim) {
+                        a = ld_vol(v + r * vs + (int64_t)W * (base + c));
+                        if (C) d = ld_vol(v + r * vs + (int64_t)W * (base + c) + 1);
+                        ready = ready && !pending(a) && !pending(d);
+                    }
+                    re[h][r] = a;
+                    im[h][r] = d;
+                }
+            }
+            if (__all_sync(0xffffffffu, ready)) return true;
+            // lane 0 polls one value; the others wait for it
+            int ok = 1;
+            if (lane == 0) {
+                while (pending(ld_vol(v + (int64_t)W * base))) {
+                    if (++it > FLAG_SPIN_CAP) {
+                        atomicExch(err, BEM_ERR_TIMEOUT);
+                        ok = 0;
+                        break;
+                    }
+                    if ((it & 63u) == 0u && *(volatile int32_t*)err != 0) {
+                        ok = 0;
+                        break;
+                    }
+                    if (it > 256u) __nanosleep(32);
+                }
+                if (++it > FLAG_SPIN_CAP) {
+                    atomicExch(err, BEM_ERR_TIMEOUT);
+                    ok = 0;
+                }
+            }
+            if (!__shfl_sync(0xffffffffu, ok, 0)) return false;
+        }
+    };
     for (int pass = 0; pass < 2; ++pass) {
         const bool fwd = pass == 0;
+        const double* src = fwd ? b : y;
+        double* dst = fwd ? y : x;
         for (int t = blockIdx.x; t < nbk; t += P) {
             const int k = fwd ? t : nbk - 1 - t;
             const int r0 = k * LU_T, m = min(LU_T, n - r0);
             const int ndep = fwd ? k : nbk - 1 - k;
             const int jc = ndep > 0 ? (fwd ? k - 1 : k + 1) : -1;  // critical (last) dependency
-            // prefetch: diagonal inverse and the critical block
-            const CE<T>* Dk = dinv + (size_t)k * 2 * LU_T * LU_T + (fwd ? 0 : LU_T * LU_T);
-            for (int e = tid; e < LU_T * LU_T; e += blockDim.x) {
-                const int r = e / LU_T, c = e - r * LU_T;
-                sD[r * SOLVE_LD + c] = Dk[e];
-                CE<T> v = CE<T>{T(0), T(0)};
-                if (jc >= 0) {
-                    const int c0 = jc * LU_T;
-                    if (r < m && c0 + c < n) v = ldE<T, C>(LU, (int64_t)(r0 + r) * lda + c0 + c);
-                }
-                sB[r * SOLVE_LD + c] = v;
-            }
-            // streamed dependencies
-            T acc_re[RW], acc_im[RW];
-#pragma unroll
-            for (int i = 0; i < RW; ++i) acc_re[i] = acc_im[i] = T(0);
-            auto accum = [&](int j) {
-                const int c0 = j * LU_T, mj = min(LU_T, n - c0);
-                T xr0 = T(0), xi0 = T(0), xr1 = T(0), xi1 = T(0);
-                if (lane < mj) {
-                    xr0 = (T)__ldcg(&x[W * (c0 + lane)]);
-                    if (C) xi0 = (T)__ldcg(&x[W * (c0 + lane) + 1]);
-                }
-                if (lane + 32 < mj) {
-                    xr1 = (T)__ldcg(&x[W * (c0 + lane + 32)]);
-                    if (C) xi1 = (T)__ldcg(&x[W * (c0 + lane + 32) + 1]);
-                }
-                // all 2 RW loads of the block first, so that they are in flight
-                // together, then the products (entries outside the block are zero)
-                CE<T> la[RW], lb[RW];
+            const int nstream = ndep > 0 ? ndep - 1 : 0;           // the others
+            auto block = [&](int d) { return fwd ? d : nbk - 1 - d; };
+            // the streamed block d: row wid + 8i, columns lane and lane + 32 of each warp
+            CE<T> la[RW], lb[RW];
+            auto load = [&](int d) {
+                const int c0 = block(d) * LU_T, mj = min(LU_T, n - c0);
 #pragma unroll
                 for (int i = 0; i < RW; ++i) {
                     const int r = wid + 8 * i;
                     const T* row = LU + W * ((int64_t)(r0 + r) * lda + c0);
-                    la[i] = (r < m && lane < mj) ? ldE<T, C>(row, lane) : CE<T>{T(0), T(0)};
-                    lb[i] = (r < m && lane + 32 < mj) ? ldE<T, C>(row, lane + 32) : CE<T>{T(0), T(0)};
-                }
-#pragma unroll
-                for (int i = 0; i < RW; ++i) {
-                    acc_re[i] += la[i].re * xr0 - la[i].im * xi0;
-                    acc_im[i] += la[i].re * xi0 + la[i].im * xr0;
-                    acc_re[i] += lb[i].re * xr1 - lb[i].im * xi1;
-                    acc_im[i] += lb[i].re * xi1 + lb[i].im * xr1;
+                    la[i] = (r < m && lane < mj) ? elem(row, lane) : CE<T>{T(0), T(0)};
+                    lb[i] = (r < m && lane + 32 < mj) ? elem(row, lane + 32) : CE<T>{T(0), T(0)};
                 }
             };
-            const int nstream = ndep > 0 ? ndep - 1 : 0;  // all but the critical one
-            bool ok = true;
-            int d = 0;
-            for (; d + 1 < nstream && ok; d += 2) {
-                const int j0 = fwd ? d : nbk - 1 - d, j1 = fwd ? d + 1 : nbk - 2 - d;
-                ok = warp_wait_flag(flags, pass * nbk + j0, epoch, err) &&
-                     warp_wait_flag(flags, pass * nbk + j1, epoch, err);
-                if (ok) {
-                    accum(j0);
-                    accum(j1);
+            if (nstream > 0) load(0);
+            // stage the diagonal inverse, the critical block and the diagonal block
+            const CE<T>* Dk = dinv + (size_t)k * 2 * LU_T * LU_T + (fwd ? 0 : LU_T * LU_T);
+            for (int e = tid; e < LU_T * LU_T; e += blockDim.x) {
+                const int r = e / LU_T, c = e - r * LU_T;
+                sD[r * SOLVE_LD + c] = Dk[e];
+                const T* row = LU + W * ((int64_t)(r0 + r) * lda);
+                CE<T> v = CE<T>{T(0), T(0)};
+                if (jc >= 0) {
+                    const int c0 = jc * LU_T;
+                    if (r < m && c0 + c < n) v = elem(row + (int64_t)W * c0, c);
+                }
+                sB[r * SOLVE_LD + c] = v;
+                if constexpr (REF) {
+                    CE<T> d = CE<T>{r == c ? T(1) : T(0), T(0)};
+                    if (r < m && c < m && (fwd ? c < r : c >= r)) {
+                        d = elem(row + (int64_t)W * r0, c);
+                        if (r == c && d.re == T(0) && d.im == T(0)) atomicMax(&s_zero[par], r);
+                    }
+                    sT[r * SOLVE_LD + c] = d;
                 }
             }
-            if (ok && d < nstream) {
-                const int j0 = fwd ? d : nbk - 1 - d;
-                ok = warp_wait_flag(flags, pass * nbk + j0, epoch, err);
-                if (ok) accum(j0);
+            ACC acc_re[RW][NR], acc_im[RW][NR];
+#pragma unroll
+            for (int i = 0; i < RW; ++i)
+#pragma unroll
+                for (int r = 0; r < NR; ++r) acc_re[i][r] = acc_im[i][r] = ACC(0);
+            bool ok = true;
+            for (int d = 0; d < nstream && ok; ++d) {
+                const int c0 = block(d) * LU_T;
+                double xr[2][NR], xi[2][NR];
+                ok = fetch(dst, c0, lane, min(LU_T, n - c0), xr, xi, 2);
+                if (!ok) break;
+#pragma unroll
+                for (int i = 0; i < RW; ++i)
+#pragma unroll
+                    for (int r = 0; r < NR; ++r) {
+                        const ACC x0 = (ACC)xr[0][r], z0 = (ACC)xi[0][r], x1 = (ACC)xr[1][r], z1 = (ACC)xi[1][r];
+                        acc_re[i][r] += (ACC)la[i].re * x0;
+                        acc_re[i][r] += (ACC)lb[i].re * x1;
+                        if (C) {
+                            acc_re[i][r] -= (ACC)la[i].im * z0;
+                            acc_im[i][r] += (ACC)la[i].re * z0;
+                            acc_im[i][r] += (ACC)la[i].im * x0;
+                            acc_re[i][r] -= (ACC)lb[i].im * z1;
+                            acc_im[i][r] += (ACC)lb[i].re * z1;
+                            acc_im[i][r] += (ACC)lb[i].im * x1;
+                        }
+                    }
+                if (d + 1 < nstream) load(d + 1);
             }
+            // this row's right-hand side (the forward pass's value in the backward one)
+            double br[2][NR], bi[2][NR];
+            if (ok) ok = fetch(src, r0, lane, m, br, bi, 2);
             if (!ok && lane == 0) s_abort = 1;
 #pragma unroll
-            for (int i = 0; i < RW; ++i) {
-                T sr = acc_re[i], si = acc_im[i];
+            for (int i = 0; i < RW; ++i)
 #pragma unroll
-                for (int o = 16; o > 0; o >>= 1) {
-                    sr += __shfl_xor_sync(0xffffffffu, sr, o);
-                    si += __shfl_xor_sync(0xffffffffu, si, o);
-                }
-                const int r = wid + 8 * i;
-                if (lane == 0) {
-                    double br = 0.0, bi = 0.0;
-                    if (r < m) {
-                        br = __ldcg(&x[W * (r0 + r)]) - (double)sr;
-                        bi = C ? __ldcg(&x[W * (r0 + r) + 1]) - (double)si : 0.0;
+                for (int r = 0; r < NR; ++r) {
+                    ACC sr = acc_re[i][r], si = acc_im[i][r];
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1) {
+                        sr += __shfl_xor_sync(0xffffffffu, sr, o);
+                        if (C) si += __shfl_xor_sync(0xffffffffu, si, o);
                     }
-                    s_acc[r][0] = br;
-                    s_acc[r][1] = bi;
+                    const int q = wid + 8 * i;  // value q sits in lane q % 32, half q / 32
+                    if (lane == (q & 31)) {
+                        s_acc[q][r][0] = ((i < RW / 2) ? br[0][r] : br[1][r]) - (double)sr;
+                        s_acc[q][r][1] = C ? ((i < RW / 2) ? bi[0][r] : bi[1][r]) - (double)si : 0.0;
+                    }
                 }
-            }
             __syncthreads();
             if (s_abort) return;
-            // critical dependency out of shared memory
-            if (jc >= 0) {
-                if (!wait_flag(flags, pass * nbk + jc, epoch, err)) return;
-                const int c0 = jc * LU_T, mj = min(LU_T, n - c0);
-                if (tid < LU_T) {
-                    s_x[tid][0] = tid < mj ? __ldcg(&x[W * (c0 + tid)]) : 0.0;
-                    s_x[tid][1] = (C && tid < mj) ? __ldcg(&x[W * (c0 + tid) + 1]) : 0.0;
-                }
-                __syncthreads();
-                T sr = T(0), si = T(0);
+            if (REF && tid == 0) s_zero[par ^ 1] = -1;  // the previous row's reads are done, the next row's writes not begun
+            // (row gr of S) . v, in A, in all four lanes of the row
+            auto gemv = [&](auto zero, const CE<T>* S, const double (*v)[NR][2], double (*out)[2]) {
+                using A = decltype(zero);
+                A sr[NR], si[NR];
+#pragma unroll
+                for (int r = 0; r < NR; ++r) sr[r] = si[r] = A(0);
 #pragma unroll
                 for (int i = 0; i < LU_T / 4; ++i) {
                     const int c = gq + 4 * i;
-                    const CE<T> l = sB[gr * SOLVE_LD + c];
-                    const T xr = (T)s_x[c][0], xi = (T)s_x[c][1];
-                    sr += l.re * xr - l.im * xi;
-                    si += l.re * xi + l.im * xr;
+                    const CE<T> l = S[gr * SOLVE_LD + c];
+#pragma unroll
+                    for (int r = 0; r < NR; ++r) {
+                        const A vr = (A)v[c][r][0], vi = (A)v[c][r][1];
+                        sr[r] += (A)l.re * vr;
+                        if (C) {
+                            sr[r] -= (A)l.im * vi;
+                            si[r] += (A)l.re * vi;
+                            si[r] += (A)l.im * vr;
+                        }
+                    }
                 }
-                sr += __shfl_xor_sync(0xffffffffu, sr, 1);
-                si += __shfl_xor_sync(0xffffffffu, si, 1);
-                sr += __shfl_xor_sync(0xffffffffu, sr, 2);
-                si += __shfl_xor_sync(0xffffffffu, si, 2);
-                if (gq == 0 && gr < m) {
-                    s_acc[gr][0] -= (double)sr;
-                    s_acc[gr][1] -= (double)si;
+#pragma unroll
+                for (int r = 0; r < NR; ++r) {
+                    sr[r] += __shfl_xor_sync(0xffffffffu, sr[r], 1);
+                    sr[r] += __shfl_xor_sync(0xffffffffu, sr[r], 2);
+                    if (C) {
+                        si[r] += __shfl_xor_sync(0xffffffffu, si[r], 1);
+                        si[r] += __shfl_xor_sync(0xffffffffu, si[r], 2);
+                    }
+                    out[r][0] = (double)sr[r];
+                    out[r][1] = (double)si[r];
+                }
+            };
+            double o[NR][2];
+            // critical dependency out of shared memory
+            if (jc >= 0) {
+                if (wid < 2) {
+                    const int c0 = jc * LU_T;
+                    double xr[1][NR], xi[1][NR];
+                    if (!fetch(dst, c0, 32 * wid + lane, min(LU_T, n - c0), xr, xi, 1)) s_abort = 1;
+#pragma unroll
+                    for (int r = 0; r < NR; ++r) {
+                        s_x[32 * wid + lane][r][0] = xr[0][r];
+                        s_x[32 * wid + lane][r][1] = xi[0][r];
+                    }
                 }
                 __syncthreads();
-            }
-            // y = inverse(diagonal block) * acc, in FP64
-            double yr = 0.0, yi = 0.0;
+                if (s_abort) return;
+                gemv(ACC(0), sB, s_x, o);
+                if (gq == 0 && gr < m)
 #pragma unroll
-            for (int i = 0; i < LU_T / 4; ++i) {
-                const int c = gq + 4 * i;
-                const CE<T> dd = sD[gr * SOLVE_LD + c];
-                yr += (double)dd.re * s_acc[c][0] - (double)dd.im * s_acc[c][1];
-                yi += (double)dd.re * s_acc[c][1] + (double)dd.im * s_acc[c][0];
+                    for (int r = 0; r < NR; ++r) {
+                        s_acc[gr][r][0] -= o[r][0];
+                        s_acc[gr][r][1] -= o[r][1];
+                    }
+                __syncthreads();
             }
-            yr += __shfl_xor_sync(0xffffffffu, yr, 1);
-            yi += __shfl_xor_sync(0xffffffffu, yi, 1);
-            yr += __shfl_xor_sync(0xffffffffu, yr, 2);
-            yi += __shfl_xor_sync(0xffffffffu, yi, 2);
-            if (gq == 0 && gr < m) {
-                x[W * (r0 + gr)] = yr;
-                if (C) x[W * (r0 + gr) + 1] = yi;
+            // inverse(diagonal block) * acc, in FP64
+            gemv(0.0, sD, s_acc, o);
+            if constexpr (REF) {
+                if (gq == 0)
+#pragma unroll
+                    for (int r = 0; r < NR; ++r) {
+                        s_x[gr][r][0] = o[r][0];
+                        s_x[gr][r][1] = o[r][1];
+                    }
+                __syncthreads();
+                double q[NR][2];
+                gemv(0.0, sT, s_x, q);
+                if (gq == 0)
+#pragma unroll
+                    for (int r = 0; r < NR; ++r) {
+                        s_r[gr][r][0] = s_acc[gr][r][0] - q[r][0];
+                        s_r[gr][r][1] = s_acc[gr][r][1] - q[r][1];
+                    }
+                __syncthreads();
+                gemv(0.0, sD, s_r, q);
+#pragma unroll
+                for (int r = 0; r < NR; ++r) {
+                    o[r][0] += q[r][0];
+                    o[r][1] += q[r][1];
+                    // a zero pivot divides by zero, as substitution would, and the rows above
+                    // it depend on that value (the inverse holds 0 there)
+                    if (gr <= s_zero[par]) o[r][0] = o[r][1] = (gr == s_zero[par] && !C ? s_r[gr][r][0] : 0.0) / 0.0;
+                }
             }
-            __threadfence();
+            if (gq == 0 && gr < m)
+#pragma unroll
+                for (int r = 0; r < NR; ++r) {
+                    st_vol(dst + r * vs + (int64_t)W * (r0 + gr), o[r][0]);
+                    if (C) st_vol(dst + r * vs + (int64_t)W * (r0 + gr) + 1, o[r][1]);
+                }
             __syncthreads();
-            if (tid == 0) st_release_i(flags + pass * nbk + k, epoch);
-        }
-        // the backward pass of block k needs x_k from the forward pass: every
-        // block row's forward flag is checked before its value is read below
-        if (fwd) {
-            for (int t = blockIdx.x; t < nbk; t += P) {
-                const int k = nbk - 1 - t;
-                if (!wait_flag(flags, k, epoch, err)) return;
-            }
+            par ^= 1;
         }
     }
 }
 
-__global__ void permute_kernel(const double* b, const int32_t* perm, double* x, int n, int W) {
+__global__ void permute_kernel(const double* b, const int32_t* perm, double* out, int n, int W, const int* skip) {
+    if (skip != nullptr && *skip != 0) return;
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     int s = perm[i];
-    for (int w = 0; w < W; ++w) x[W * i + w] = b[W * s + w];
+    for (int w = 0; w < W; ++w) out[W * i + w] = b[W * s + w];
+}
+
+// y and x start out not written
+__global__ void pending_kernel(double* y, double* x, int64_t nd, const int* skip) {
+    if (skip != nullptr && *skip != 0) return;
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i >= nd) return;
+    y[i] = x[i] = __longlong_as_double((long long)PENDING);
+}
+
+// Queues the triangular solve of NR permuted right-hand sides b (vs doubles
+// apart) into x; y is scratch.  err receives BEM_ERR_TIMEOUT if a wait runs out.
+template <typename T, bool C, int NR, bool REF>
+cudaError_t queue_tri_solve(int sms, const T* LU, int64_t n, int64_t lda, const CE<T>* dinv, const double* b, double* y,
+                            double* x, int64_t vs, int32_t* err, const int* skip, cudaStream_t s) {
+    const int nbk = (int)((n + LU_T - 1) / LU_T);
+    const int64_t nd = NR == 1 ? (C ? 2 : 1) * n : NR * vs;
+    pending_kernel<<<(unsigned)((nd + 255) / 256), 256, 0, s>>>(y, x, nd, skip);
+    const size_t smem = solve_smem_bytes(sizeof(CE<T>), REF);
+    const void* fn = (const void*)tri_solve_kernel<T, C, NR, REF>;
+    if (cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) return e;
+    int per_sm = 0;
+    if (cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tri_solve_kernel<T, C, NR, REF>, 256, smem))
+        return e;
+    const int P = std::max(1, std::min(nbk, std::min(per_sm * sms, sms)));
+    int ni = (int)n;
+    int vec = ((uintptr_t)LU % sizeof(CE<T>)) == 0 ? 1 : 0;
+    void* args[] = {(void*)&LU, &lda, &ni, (void*)&dinv, (void*)&b, &y, &x, &vs, &vec, &err, (void*)&skip};
+    return cudaLaunchCooperativeKernel(fn, P, 256, args, smem, s);
 }
 
 // Row permutation of the tile-pivoted factor: every swap of diagonal tile k
@@ -867,45 +978,54 @@ int factor_t(bem_ctx* ctx, T* A, int64_t n, int64_t lda, int32_t* piv, CE<T>* di
     return bem_check_cuda(ctx, cudaGetLastError(), "tiled lu");
 }
 
+// Scratch of a tiled solve in the context workspace: the row permutation and
+// three vectors (permuted right-hand side, intermediate, solution).
+struct SolveWs {
+    int32_t* perm;
+    double *b, *y, *x;
+};
+
+int solve_ws(bem_ctx* ctx, int64_t n, int W, SolveWs* w) {
+    if ((size_t)n * sizeof(int32_t) > 200 * 1024) return bem_fail(ctx, BEM_ERR_INVALID, "tiled solve: n > 51200");
+    const size_t off = ((size_t)n * 4 + 255) & ~size_t(255);
+    const size_t vec = (sizeof(double) * W * (size_t)n + 255) & ~size_t(255);
+    if (int rc = bem_ws_reserve(ctx, off + 3 * vec)) return rc;
+    char* base = (char*)ctx->ws;
+    w->perm = (int32_t*)base;
+    w->b = (double*)(base + off);
+    w->y = (double*)(base + off + vec);
+    w->x = (double*)(base + off + 2 * vec);
+    return BEM_OK;
+}
+
+// One solve queued on the stream: out receives the scratch vector that holds
+// the solution; skipped on the device when skip != NULL and *skip != 0.
+template <typename T, bool C>
+int queue_solve(bem_ctx* ctx, const T* LU, int64_t n, int64_t lda, const int32_t* piv, const CE<T>* dinv,
+                const double* r, double** out, const int* skip, cudaStream_t s) {
+    const int W = C ? 2 : 1;
+    SolveWs w;
+    if (int rc = solve_ws(ctx, n, W, &w)) return rc;
+    const unsigned ptiles = (unsigned)((n + LU_T - 1) / LU_T);
+    tile_piv_to_perm_kernel<<<(ptiles + 127) / 128, 128, 0, s>>>(piv, w.perm, (int)n);
+    permute_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(r, w.perm, w.b, (int)n, W, skip);
+    if (int rc = bem_check_cuda(ctx, queue_tri_solve<T, C, 1, false>(ctx->num_sms, LU, n, lda, dinv, w.b, w.y, w.x, 0,
+                                                                     ctx->flags + 3, skip, s),
+                                "tri_solve_kernel"))
+        return rc;
+    ctx->launches += 4;
+    *out = w.x;
+    return bem_check_cuda(ctx, cudaGetLastError(), "tiled solve");
+}
+
 template <typename T, bool C>
 int solve_t(bem_ctx* ctx, const T* LU, int64_t n, int64_t lda, const int32_t* piv, const CE<T>* dinv, double* b,
             cudaStream_t s) {
     const int W = C ? 2 : 1;
-    const int nbk = (int)((n + LU_T - 1) / LU_T);
-    // workspace: perm [n], flags [2*nbk], x [W*n]
-    size_t off_flags = ((size_t)n * 4 + 255) & ~size_t(255);
-    size_t off_x = off_flags + (((size_t)2 * nbk * 4 + 255) & ~size_t(255));
-    size_t total = off_x + sizeof(double) * W * (size_t)n;
-    if (int rc = bem_ws_reserve(ctx, total)) return rc;
-    char* base = (char*)ctx->ws;
-    int32_t* perm = (int32_t*)base;
-    int* flags = (int*)(base + off_flags);
-    double* x = (double*)(base + off_x);
-    if ((size_t)n * sizeof(int32_t) > 200 * 1024) return bem_fail(ctx, BEM_ERR_INVALID, "tiled solve: n > 51200");
-    const unsigned ptiles = (unsigned)((n + LU_T - 1) / LU_T);
-    tile_piv_to_perm_kernel<<<(ptiles + 127) / 128, 128, 0, s>>>(piv, perm, (int)n);
-    permute_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(b, perm, x, (int)n, W);
-    cudaMemsetAsync(flags, 0, sizeof(int) * 2 * nbk, s);
-    cudaMemsetAsync(ctx->flags + 3, 0, sizeof(int32_t), s);
-    ctx->launches += 2;
-    const size_t ssmem = solve_smem_bytes(sizeof(CE<T>));
-    if (int rc = bem_check_cuda(ctx, cudaFuncSetAttribute(tile_solve_kernel<T, C>,
-                                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ssmem),
-                                "tile_solve_kernel smem"))
-        return rc;
-    int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tile_solve_kernel<T, C>, 256, ssmem);
-    int P = std::max(1, std::min(nbk, per_sm * ctx->num_sms));
-    P = std::min(P, ctx->num_sms);
-    int ni = (int)n, epoch = 1;
     int32_t* err = ctx->flags + 3;
-    const int* no_skip = nullptr;
-    void* args[] = {(void*)&LU, &lda, &ni, (void*)&dinv, &x, &flags, &epoch, &err, (void*)&no_skip};
-    if (int rc = bem_check_cuda(ctx, cudaLaunchCooperativeKernel((const void*)tile_solve_kernel<T, C>, P, 256, args,
-                                                                ssmem, s),
-                                "tile_solve_kernel"))
-        return rc;
-    ctx->launches++;
+    cudaMemsetAsync(err, 0, sizeof(int32_t), s);
+    double* x = nullptr;
+    if (int rc = queue_solve<T, C>(ctx, LU, n, lda, piv, dinv, b, &x, nullptr, s)) return rc;
     if (int rc = bem_check_cuda(ctx, cudaMemcpyAsync(b, x, sizeof(double) * W * n, cudaMemcpyDeviceToDevice, s),
                                 "tiled solve copy"))
         return rc;
@@ -914,7 +1034,7 @@ int solve_t(bem_ctx* ctx, const T* LU, int64_t n, int64_t lda, const int32_t* pi
     cudaMemcpyAsync(&e[1], ctx->flags + 4, sizeof(int32_t), cudaMemcpyDeviceToHost, s);
     if (int rc = bem_check_cuda(ctx, cudaStreamSynchronize(s), "tiled solve")) return rc;
     if (int rc = bem_take_factor_error(ctx, e[1], s)) return rc;
-    if (e[0] != 0) return bem_fail(ctx, BEM_ERR_TIMEOUT, "tiled solve: a ready-flag wait hit its iteration cap");
+    if (e[0] != 0) return bem_fail(ctx, BEM_ERR_TIMEOUT, "tiled solve: a wait hit its iteration cap");
     return BEM_OK;
 }
 
@@ -923,52 +1043,29 @@ int solve_t(bem_ctx* ctx, const T* LU, int64_t n, int64_t lda, const int32_t* pi
 // workspace (*out), queued without synchronisation and skipped on the device
 // when *skip != 0.  The caller resets ctx->flags[3] once before its loop and
 // reads it after its final synchronisation.
-__global__ void permute_if_kernel(const double* b, const int32_t* perm, double* x, int n, int W, const int* skip) {
-    if (*skip != 0) return;
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    int s = perm[i];
-    for (int w = 0; w < W; ++w) x[W * i + w] = b[W * s + w];
-}
-
 template <typename T, bool C>
 int precond_t(bem_ctx* ctx, const T* LU, int64_t n, int64_t lda, const int32_t* piv, const CE<T>* dinv,
               const double* r, double** out, const int* skip, cudaStream_t s) {
-    const int W = C ? 2 : 1;
-    const int nbk = (int)((n + LU_T - 1) / LU_T);
-    size_t off_flags = ((size_t)n * 4 + 255) & ~size_t(255);
-    size_t off_x = off_flags + (((size_t)2 * nbk * 4 + 255) & ~size_t(255));
-    size_t total = off_x + sizeof(double) * W * (size_t)n;
-    if (int rc = bem_ws_reserve(ctx, total)) return rc;
-    char* base = (char*)ctx->ws;
-    int32_t* perm = (int32_t*)base;
-    int* flags = (int*)(base + off_flags);
-    double* x = (double*)(base + off_x);
-    if ((size_t)n * sizeof(int32_t) > 200 * 1024) return bem_fail(ctx, BEM_ERR_INVALID, "tiled solve: n > 51200");
-    const unsigned ptiles = (unsigned)((n + LU_T - 1) / LU_T);
-    tile_piv_to_perm_kernel<<<(ptiles + 127) / 128, 128, 0, s>>>(piv, perm, (int)n);
-    permute_if_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(r, perm, x, (int)n, W, skip);
-    cudaMemsetAsync(flags, 0, sizeof(int) * 2 * nbk, s);
-    ctx->launches += 2;
-    const size_t ssmem = solve_smem_bytes(sizeof(CE<T>));
-    if (int rc = bem_check_cuda(ctx, cudaFuncSetAttribute(tile_solve_kernel<T, C>,
-                                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ssmem),
-                                "tile_solve_kernel smem"))
-        return rc;
-    int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tile_solve_kernel<T, C>, 256, ssmem);
-    int P = std::max(1, std::min(nbk, per_sm * ctx->num_sms));
-    P = std::min(P, ctx->num_sms);
-    int ni = (int)n, epoch = 1;
-    int32_t* err = ctx->flags + 3;
-    void* args[] = {(void*)&LU, &lda, &ni, (void*)&dinv, &x, &flags, &epoch, &err, (void*)&skip};
-    if (int rc = bem_check_cuda(ctx, cudaLaunchCooperativeKernel((const void*)tile_solve_kernel<T, C>, P, 256, args,
-                                                                ssmem, s),
-                                "tile_solve_kernel"))
-        return rc;
-    ctx->launches++;
-    *out = x;
-    return BEM_OK;
+    return queue_solve<T, C>(ctx, LU, n, lda, piv, dinv, r, out, skip, s);
+}
+
+// x = U^{-1} L^{-1} b for nrhs permuted right-hand sides (vs doubles apart), the
+// diagonal inverses refined against the diagonal blocks; two at a time.
+template <typename T, bool C>
+int lu_tri_t(bem_ctx* ctx, const T* LU, int64_t n, int64_t lda, const CE<T>* dinv, const double* b, double* y, double* x,
+             int nrhs, int64_t vs, int32_t* err, cudaStream_t s) {
+    for (int c = 0; c < nrhs;) {
+        const int m = nrhs - c >= 2 ? 2 : 1;
+        const cudaError_t e =
+            m == 2 ? queue_tri_solve<T, C, 2, true>(ctx->num_sms, LU, n, lda, dinv, b + c * vs, y + c * vs, x + c * vs, vs,
+                                                    err, nullptr, s)
+                   : queue_tri_solve<T, C, 1, true>(ctx->num_sms, LU, n, lda, dinv, b + c * vs, y + c * vs, x + c * vs, vs,
+                                                    err, nullptr, s);
+        if (int rc = bem_check_cuda(ctx, e, "tri_solve_kernel")) return rc;
+        ctx->launches += 2;
+        c += m;
+    }
+    return bem_check_cuda(ctx, cudaGetLastError(), "lu_solve");
 }
 
 }  // namespace
@@ -1039,6 +1136,17 @@ int bem_tile_inverses(bem_ctx* ctx, int dtype, const void* A, int64_t n, int64_t
     }
 }
 
+int bem_lu_tri_solve(bem_ctx* ctx, int dtype, const void* LU, int64_t n, int64_t lda, const void* dinv, const double* b,
+                     double* y, double* x, int nrhs, int64_t vs, int32_t* err, cudaStream_t s) {
+    switch (dtype) {
+        case BEM_F64: return lu_tri_t<double, false>(ctx, (const double*)LU, n, lda, (const CE<double>*)dinv, b, y, x, nrhs, vs, err, s);
+        case BEM_C128: return lu_tri_t<double, true>(ctx, (const double*)LU, n, lda, (const CE<double>*)dinv, b, y, x, nrhs, vs, err, s);
+        case BEM_F32: return lu_tri_t<float, false>(ctx, (const float*)LU, n, lda, (const CE<float>*)dinv, b, y, x, nrhs, vs, err, s);
+        case BEM_C64: return lu_tri_t<float, true>(ctx, (const float*)LU, n, lda, (const CE<float>*)dinv, b, y, x, nrhs, vs, err, s);
+        default: return bem_fail(ctx, BEM_ERR_INVALID, "lu_solve: unknown dtype");
+    }
+}
+
 int bem_tiled_precond_async(bem_ctx* ctx, int dtype, const void* LU, int64_t n, int64_t lda, const int32_t* piv,
                             const void* dinv, const double* r, double** out, const int* skip, cudaStream_t s) {
     switch (dtype) {
@@ -1053,7 +1161,7 @@ int bem_tiled_precond_async(bem_ctx* ctx, int dtype, const void* LU, int64_t n, 
 // ----------------------------------------------------------------------------
 // Allocation-free variant of bem_lu_solve_tiled.
 //
-// Its scratch (row permutation, ready flags, error word, work vector) lives in
+// Its scratch (row permutation, error word, three work vectors) lives in
 // one file-scope __device__ array instead of a context workspace, so the call
 // needs no bem_ctx and performs no device allocation.  The array is sized for
 // n <= BEM_STATIC_SOLVE_MAX_N and is held by every GPU that loads this library
@@ -1066,12 +1174,12 @@ int bem_tiled_precond_async(bem_ctx* ctx, int dtype, const void* LU, int64_t n, 
 namespace {
 
 constexpr int64_t kStaticSolveMaxN = BEM_STATIC_SOLVE_MAX_N;
-constexpr int kStaticSolveMaxTiles = (int)((kStaticSolveMaxN + LU_T - 1) / LU_T);
 
 struct StaticSolveScratch {
     int32_t perm[kStaticSolveMaxN];
-    int flags[2 * kStaticSolveMaxTiles];
     int32_t err[4];
+    double b[2 * kStaticSolveMaxN];
+    double y[2 * kStaticSolveMaxN];
     double x[2 * kStaticSolveMaxN];
 };
 
@@ -1114,37 +1222,17 @@ int solve_static_t(const T* LU, int64_t n, int64_t lda, const int32_t* piv, cons
     int dev = 0, sms = 1;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    int32_t* perm = sc->perm;
-    int* flags = sc->flags;
     int32_t* err = sc->err;
-    double* x = sc->x;
-    tile_piv_to_perm_kernel<<<(unsigned)((nbk + 127) / 128), 128, 0, s>>>(piv, perm, (int)n);
-    permute_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(b, perm, x, (int)n, W);
+    tile_piv_to_perm_kernel<<<(unsigned)((nbk + 127) / 128), 128, 0, s>>>(piv, sc->perm, (int)n);
+    permute_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(b, sc->perm, sc->b, (int)n, W, nullptr);
     if (cudaGetLastError() != cudaSuccess) return BEM_ERR_CUDA;
-    // the array keeps the previous call's contents: the flags and the error
-    // word must start at zero
-    if (cudaMemsetAsync(flags, 0, sizeof(int) * 2 * nbk, s) != cudaSuccess ||
-        cudaMemsetAsync(err, 0, sizeof(int32_t), s) != cudaSuccess) {
+    // the array keeps the previous call's contents: the error word must start at zero
+    if (cudaMemsetAsync(err, 0, sizeof(int32_t), s) != cudaSuccess ||
+        queue_tri_solve<T, C, 1, false>(sms, LU, n, lda, dinv, sc->b, sc->y, sc->x, 0, err, nullptr, s) != cudaSuccess) {
         cudaGetLastError();
         return BEM_ERR_CUDA;
     }
-    const size_t ssmem = solve_smem_bytes(sizeof(CE<T>));
-    if (cudaFuncSetAttribute(tile_solve_kernel<T, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ssmem) !=
-        cudaSuccess) {
-        cudaGetLastError();
-        return BEM_ERR_CUDA;
-    }
-    int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tile_solve_kernel<T, C>, 256, ssmem);
-    int P = std::max(1, std::min(nbk, std::min(per_sm * sms, sms)));
-    int ni = (int)n, epoch = 1;
-    const int* no_skip = nullptr;
-    void* args[] = {(void*)&LU, &lda, &ni, (void*)&dinv, &x, &flags, &epoch, &err, (void*)&no_skip};
-    if (cudaLaunchCooperativeKernel((const void*)tile_solve_kernel<T, C>, P, 256, args, ssmem, s) != cudaSuccess) {
-        cudaGetLastError();
-        return BEM_ERR_CUDA;
-    }
-    if (cudaMemcpyAsync(b, x, sizeof(double) * W * n, cudaMemcpyDeviceToDevice, s) != cudaSuccess) {
+    if (cudaMemcpyAsync(b, sc->x, sizeof(double) * W * n, cudaMemcpyDeviceToDevice, s) != cudaSuccess) {
         cudaGetLastError();
         return BEM_ERR_CUDA;
     }
