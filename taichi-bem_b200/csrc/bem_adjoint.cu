@@ -137,7 +137,7 @@ struct AdjArgs {
     const double* area;
     const double4* pts;   // FP64 separate-rule points (offset, weight with 2A)
     const double* phi64;  // [Q2*3] barycentric weights of the separate-rule points
-    int Q2;
+    int Q2, ti;           // points per panel, test panels per CTA (separate pairs)
     int64_t n_near;
     const int4* near;
     const int32_t* test_local;
@@ -181,83 +181,241 @@ __device__ __forceinline__ void pair_grads(const PairMoments& M, double cw, cons
     }
 }
 
-// ---- separate pairs: CTA = ADJ_TI test panels (shared memory) x ADJ_THREADS trial panels ----
+// ---- separate pairs: CTA = a.ti test panels (shared memory) x ADJ_THREADS trial panels ----
+//
+// As in the FP64 assembly, both orders of a pair come from one evaluation (the
+// order with the smaller test panel does it when the reversed one is in the
+// call too).  With t = w/r^3, the trial density u_j(y) and lam_i of the pair,
+// and u_i(x), lam_j of the reversed one,
+//   V   cw = lam_i u_j + lam_j u_i,   d/dd = -cw t d;
+//   K   A = lam_i u_j(y), B = lam_j u_i(x):
+//       d/dd = t (A n_j - B n_i) - 3 t/r^2 (A d.n_j - B d.n_i) d,
+// and K's J_i, J_j, N_i and N_j parts.  The sums over the test points carry
+// (total, phi_1, phi_2) moments of t, of B t and of the vector along d; hats of
+// the trial side, n_j, n_i and lam_i u_j(y) are constant over them and enter
+// once per trial point.  Bound: FP64 issue, 27 (V) and 50 (K) instructions a
+// point pair for both orders, two thirds of the FP64 pipe at 168 and 252
+// registers (capping K at 168 measured the same).  5120 panels, GaussQR 4
+// (B200): V 8.0 and K 14.3 ms, against 22 and 33 ms per ordered pair with the
+// hats of both sides applied at every point.
 template <int OP>
 __global__ void __launch_bounds__(ADJ_THREADS) adj_far_kernel(AdjArgs a) {
+    constexpr bool K = OP == BEM_OP_K;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    double4* sx = reinterpret_cast<double4*>(smem_raw);   // [ADJ_TI][Q2]
-    double* sphi = reinterpret_cast<double*>(sx + ADJ_TI * a.Q2);  // [Q2*3]
+    double4* sx = reinterpret_cast<double4*>(smem_raw);             // [ti][Q2]
+    double2* sp = reinterpret_cast<double2*>(sx + a.ti * a.Q2);    // [Q2] phi_1, phi_2
+    double* su = reinterpret_cast<double*>(sp + a.Q2);             // K: [ti][Q2] u_i at the test points
     __shared__ int s_gi[ADJ_TI];
+    __shared__ int s_ri[ADJ_TI];  // index of the test panel in the trial list, -1 = absent
     __shared__ int s_tri[ADJ_TI][3];
     __shared__ double s_lam[ADJ_TI];
+    __shared__ double s_u[ADJ_TI][3];  // trial data of the test panel (the reversed pair's density)
     const int Q2 = a.Q2;
     const int lj = blockIdx.x * ADJ_THREADS + threadIdx.x;
-    const int li0 = blockIdx.y * ADJ_TI;
+    const int li0 = blockIdx.y * a.ti;
     const int lane = threadIdx.x & 31;
-    for (int idx = threadIdx.x; idx < Q2 * 3; idx += ADJ_THREADS) sphi[idx] = a.phi64[idx];
-    if (threadIdx.x < ADJ_TI) {
-        const int li = li0 + threadIdx.x;
+    // trial coefficient (V, P0 data: the same at every vertex) or nodal data of trial-list entry l
+    auto trial_data = [&](int l, double u[3]) {
+        u[0] = u[1] = u[2] = 0.0;
+        if (l < 0) return;
+        for (int b = 0; b < a.nby; ++b) {
+            const int col = a.trial_dof[l * a.nby + b];
+            u[b] = col >= 0 ? a.u[col] : 0.0;
+        }
+    };
+    for (int q = threadIdx.x; q < Q2; q += ADJ_THREADS) sp[q] = make_double2(a.phi64[3 * q + 1], a.phi64[3 * q + 2]);
+    if (threadIdx.x < a.ti) {
+        const int t = threadIdx.x, li = li0 + t;
         const int gi = li < a.n_test ? a.test_panels[li] : -1;
-        s_gi[threadIdx.x] = gi;
+        s_gi[t] = gi;
+        s_ri[t] = gi >= 0 ? a.trial_local[gi] : -1;
         const int row = li < a.n_test ? a.test_dof[li] : -1;
-        s_lam[threadIdx.x] = row >= 0 ? a.lam[row] : 0.0;
-        for (int c = 0; c < 3; ++c) s_tri[threadIdx.x][c] = gi >= 0 ? a.tris[3 * gi + c] : -1;
+        s_lam[t] = row >= 0 ? a.lam[row] : 0.0;
+        double u[3];
+        trial_data(s_ri[t], u);
+        for (int c = 0; c < 3; ++c) {
+            s_u[t][c] = u[c];
+            s_tri[t][c] = gi >= 0 ? a.tris[3 * gi + c] : -1;
+        }
     }
     __syncthreads();
-    for (int idx = threadIdx.x; idx < ADJ_TI * Q2; idx += ADJ_THREADS) {
+    for (int idx = threadIdx.x; idx < a.ti * Q2; idx += ADJ_THREADS) {
         const int t = idx / Q2, q = idx - t * Q2;
-        if (s_gi[t] >= 0) sx[idx] = a.pts[(size_t)s_gi[t] * Q2 + q];
+        if (s_gi[t] < 0) continue;
+        sx[idx] = a.pts[(size_t)s_gi[t] * Q2 + q];
+        // the hats in the order of the general rule: beta . u
+        if (K) {
+            const double p1 = sp[q].x, p2 = sp[q].y;
+            su[idx] = (1.0 - p1 - p2) * s_u[t][0] + p1 * s_u[t][1] + p2 * s_u[t][2];
+        }
     }
     __syncthreads();
 
     const bool valid_j = lj < a.n_trial;
     const int gj = valid_j ? a.trial_panels[lj] : 0;
+    const int rj = valid_j ? a.test_local[gj] : -1;  // index of the trial panel in the test list
     int tri_j[3];
     for (int c = 0; c < 3; ++c) tri_j[c] = a.tris[3 * gj + c];
-    double vj[3][3], nj[3];
-    load_tri(a, gj, vj, nj);
-    const double Jj = 2.0 * a.area[gj];
-    double cj[3];
-    for (int c = 0; c < 3; ++c) cj[c] = a.centroid[3 * gj + c];
-    // trial coefficient (V) or nodal data of the trial panel (K)
-    double uj[3] = {0.0, 0.0, 0.0};
-    if (valid_j)
-        for (int b = 0; b < a.nby; ++b) {
-            const int col = a.trial_dof[lj * a.nby + b];
-            uj[b] = col >= 0 ? a.u[col] : 0.0;
-        }
+    const double nj[3] = {a.normal[3 * gj], a.normal[3 * gj + 1], a.normal[3 * gj + 2]};
+    const double cj[3] = {a.centroid[3 * gj], a.centroid[3 * gj + 1], a.centroid[3 * gj + 2]};
+    double uj[3];
+    trial_data(valid_j ? lj : -1, uj);
+    double lamj = 0.0;
+    if (rj >= 0) {
+        const int row = a.test_dof[rj];
+        lamj = row >= 0 ? a.lam[row] : 0.0;
+    }
     double gyacc[3][3] = {{0.0}};
     const double4* ptsj = a.pts + (size_t)gj * Q2;
 
-    for (int t = 0; t < ADJ_TI; ++t) {
+    for (int t = 0; t < a.ti; ++t) {
         const int gi = s_gi[t];
-        if (gi < 0) break;
-        const bool sep = valid_j && s_lam[t] != 0.0 && (bem_relation(s_tri[t], tri_j, gi == gj) == REL_SEPARATE);
+        if (gi < 0) break;  // uniform across the CTA
+        const bool both = s_ri[t] >= 0 && rj >= 0;
+        const double lami = s_lam[t], lamb = both ? lamj : 0.0;
+        const bool live = valid_j && !(both && gi > gj) && (lami != 0.0 || lamb != 0.0) &&
+                          bem_relation(s_tri[t], tri_j, gi == gj) == REL_SEPARATE;
         double gx[3][3] = {{0.0}};
-        if (sep) {
-            double vi[3][3], ni[3];
-            load_tri(a, gi, vi, ni);
-            const double Ji = 2.0 * a.area[gi];
-            double D[3];
-            for (int c = 0; c < 3; ++c) D[c] = a.centroid[3 * gi + c] - cj[c];
-            PairMoments M;
-            M.zero();
+        if (live) {
+            double ni[3], D[3];
+            for (int c = 0; c < 3; ++c) {
+                ni[c] = a.normal[3 * gi + c];
+                D[c] = a.centroid[3 * gi + c] - cj[c];
+            }
+            const double4* sxt = sx + t * Q2;
+            const double* sut = su + t * Q2;
+            // vector sums along d: [hat moment (total, phi_1, phi_2)][component], x and y side
+            double X[3][3] = {{0.0}}, Y[3][3] = {{0.0}};
+            double S0 = 0.0;                                          // V: sum w/r
+            double xa[3] = {0.0}, ya[3] = {0.0};                      // K: moments of A t (along n_j)
+            double xb[3] = {0.0}, yb3[3] = {0.0};                     // K: moments of B t (along -n_i)
+            double sij = 0.0, sji = 0.0, Nj[3] = {0.0}, Ni[3] = {0.0};  // K: J_i, J_j, N_j and N_i parts
+            const double Dnj = D[0] * nj[0] + D[1] * nj[1] + D[2] * nj[2];
+            const double Dni = D[0] * ni[0] + D[1] * ni[1] + D[2] * ni[2];
             for (int b = 0; b < Q2; ++b) {
                 const double4 yb = ptsj[b];
-                const double by[3] = {sphi[3 * b], sphi[3 * b + 1], sphi[3 * b + 2]};
-                const double ub = OP == BEM_OP_V ? 1.0 : by[0] * uj[0] + by[1] * uj[1] + by[2] * uj[2];
+                const double e0 = D[0] - yb.x, e1 = D[1] - yb.y, e2 = D[2] - yb.z;
+                const double2 pb = sp[b];
+                double A = 0.0, dni = 0.0, lamdni = 0.0;
+                if (K) {
+                    A = lami * ((1.0 - pb.x - pb.y) * uj[0] + pb.x * uj[1] + pb.y * uj[2]);
+                    dni = Dni - (yb.x * ni[0] + yb.y * ni[1] + yb.z * ni[2]);
+                    lamdni = lamb * dni;
+                }
+                double v[3][3] = {{0.0}};  // [moment][component]
+                double s0 = 0.0, ta[3] = {0.0}, tb[3] = {0.0}, tdn = 0.0, td[3] = {0.0}, tbd[3] = {0.0};
+#pragma unroll 4
                 for (int q = 0; q < Q2; ++q) {
-                    const double4 xa = sx[t * Q2 + q];
-                    const double d[3] = {D[0] + xa.x - yb.x, D[1] + xa.y - yb.y, D[2] + xa.z - yb.z};
-                    const double bx[3] = {sphi[3 * q], sphi[3 * q + 1], sphi[3 * q + 2]};
-                    adj_point<OP>(M, d, xa.w * yb.w, bx, by, ub, 1.0, nj, 1.0 / Jj);
+                    const double4 xp = sxt[q];
+                    const double2 ph = sp[q];
+                    const double dx = xp.x + e0, dy = xp.y + e1, dz = xp.z + e2;
+                    const double rinv = dev_rsqrt(fma(dx, dx, fma(dy, dy, dz * dz)));
+                    const double rinv2 = rinv * rinv;
+                    const double h = xp.w * rinv;
+                    const double w3 = h * rinv2;  // w / r^3
+                    double c;
+                    if (!K) {
+                        s0 += h;
+                        c = w3;
+                    } else {
+                        const double ui = sut[q];
+                        const double dnj = fma(xp.x, nj[0], fma(xp.y, nj[1], fma(xp.z, nj[2], Dnj)));
+                        const double B = w3 * ui;  // without lam_j
+                        // A d.n_j - B d.n_i, with lam_j
+                        const double e = fma(A, dnj, -(lamdni * ui));
+                        c = (w3 * rinv2) * e;
+                        ta[0] += w3;
+                        ta[1] = fma(ph.x, w3, ta[1]);
+                        ta[2] = fma(ph.y, w3, ta[2]);
+                        tb[0] += B;
+                        tb[1] = fma(ph.x, B, tb[1]);
+                        tb[2] = fma(ph.y, B, tb[2]);
+                        tdn = fma(w3, dnj, tdn);
+                        td[0] = fma(w3, dx, td[0]);
+                        td[1] = fma(w3, dy, td[1]);
+                        td[2] = fma(w3, dz, td[2]);
+                        tbd[0] = fma(B, dx, tbd[0]);
+                        tbd[1] = fma(B, dy, tbd[1]);
+                        tbd[2] = fma(B, dz, tbd[2]);
+                    }
+                    const double vx = c * dx, vy = c * dy, vz = c * dz;
+                    v[0][0] += vx;
+                    v[0][1] += vy;
+                    v[0][2] += vz;
+                    v[1][0] = fma(ph.x, vx, v[1][0]);
+                    v[1][1] = fma(ph.x, vy, v[1][1]);
+                    v[1][2] = fma(ph.x, vz, v[1][2]);
+                    v[2][0] = fma(ph.y, vx, v[2][0]);
+                    v[2][1] = fma(ph.y, vy, v[2][1]);
+                    v[2][2] = fma(ph.y, vz, v[2][2]);
+                }
+                const double w = yb.w;
+                const double wp[3] = {w, w * pb.x, w * pb.y};
+#pragma unroll
+                for (int m = 0; m < 3; ++m)
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) {
+                        X[m][c] = fma(w, v[m][c], X[m][c]);
+                        Y[m][c] = fma(wp[m], v[0][c], Y[m][c]);
+                    }
+                if (!K) {
+                    S0 = fma(w, s0, S0);
+                } else {
+                    const double wA = w * A, wB = w * lamb;
+                    sij = fma(wA, tdn, sij);
+                    sji = fma(-wB * dni, tb[0], sji);
+#pragma unroll
+                    for (int m = 0; m < 3; ++m) {
+                        xa[m] = fma(wA, ta[m], xa[m]);
+                        ya[m] = fma(wp[m] * A, ta[0], ya[m]);
+                        xb[m] = fma(wB, tb[m], xb[m]);
+                        yb3[m] = fma(wp[m] * lamb, tb[0], yb3[m]);
+                        Nj[m] = fma(wA, td[m], Nj[m]);
+                        Ni[m] = fma(-wB, tbd[m], Ni[m]);
+                    }
                 }
             }
-            const double cw = s_lam[t] * (OP == BEM_OP_V ? uj[0] : 1.0);
-            double gy[3][3];
-            pair_grads<OP>(M, cw, vi, ni, Ji, vj, nj, Jj, gx, gy);
-            for (int b = 0; b < 3; ++b)
-                for (int c = 0; c < 3; ++c) gyacc[b][c] += gy[b][c];
+            // hats from the moments, and the vertices' gradients
+            double vi[3][3], vj[3][3], n_[3];
+            load_tri(a, gi, vi, n_);
+            load_tri(a, gj, vj, n_);
+            const double Ji = 2.0 * a.area[gi], Jj = 2.0 * a.area[gj];
+            double cw = BEM_INV4PI;
+            if (!K) cw *= lami * uj[0] + lamb * s_u[t][0];
+            const double along = K ? -3.0 : -1.0;
+#pragma unroll
+            for (int h = 0; h < 3; ++h) {
+                double jg[3], hj[3], tx[3], ty[3];
+                jac_grad(vi, ni, h, jg);
+                jac_grad(vj, nj, h, hj);
+                if (!K) {
+                    for (int c = 0; c < 3; ++c) {
+                        tx[c] = jg[c] / Ji * S0;
+                        ty[c] = hj[c] / Jj * S0;
+                    }
+                } else {
+                    double g1[3], g2[3];
+                    normal_grad(vi, Ni, h, g1);
+                    normal_grad(vj, Nj, h, g2);
+                    for (int c = 0; c < 3; ++c) {
+                        tx[c] = jg[c] / Ji * sij + g1[c] / Ji;
+                        ty[c] = hj[c] / Jj * sji + g2[c] / Jj;
+                    }
+                    const double hxa = h == 0 ? xa[0] - xa[1] - xa[2] : xa[h], hya = h == 0 ? ya[0] - ya[1] - ya[2] : ya[h];
+                    const double hxb = h == 0 ? xb[0] - xb[1] - xb[2] : xb[h],
+                                 hyb = h == 0 ? yb3[0] - yb3[1] - yb3[2] : yb3[h];
+                    for (int c = 0; c < 3; ++c) {
+                        tx[c] += hxa * nj[c] - hxb * ni[c];
+                        ty[c] -= hya * nj[c] - hyb * ni[c];
+                    }
+                }
+                for (int c = 0; c < 3; ++c) {
+                    const double hx = h == 0 ? X[0][c] - X[1][c] - X[2][c] : X[h][c];
+                    const double hy = h == 0 ? Y[0][c] - Y[1][c] - Y[2][c] : Y[h][c];
+                    gx[h][c] = cw * (tx[c] + along * hx);
+                    gyacc[h][c] += cw * (ty[c] - along * hy);
+                }
+            }
         }
         // test-vertex gradients: reduce over the warp's trial panels
         for (int b = 0; b < 3; ++b)
@@ -386,8 +544,12 @@ int bem_launch_adjoint(bem_ctx* ctx, const bem_op_desc* op, const bem_space* tes
     a.lam = lam;
     a.u = u;
     a.grad = grad;
-    const size_t smem = sizeof(double4) * ADJ_TI * ctx->Q2 + sizeof(double) * 3 * ctx->Q2;
-    const dim3 fgrid((unsigned)((a.n_trial + ADJ_THREADS - 1) / ADJ_THREADS), (unsigned)((a.n_test + ADJ_TI - 1) / ADJ_TI));
+    // as in bem_launch_far64: fewer test panels per CTA where the call has too few CTAs for some waves
+    a.ti = ADJ_TI;
+    const int64_t cols = (a.n_trial + ADJ_THREADS - 1) / ADJ_THREADS;
+    while (a.ti > 1 && cols * ((a.n_test + a.ti - 1) / a.ti) < 16 * (int64_t)ctx->num_sms) a.ti /= 2;
+    const size_t smem = ((sizeof(double4) + sizeof(double)) * a.ti + sizeof(double2)) * ctx->Q2;
+    const dim3 fgrid((unsigned)cols, (unsigned)((a.n_test + a.ti - 1) / a.ti));
     const unsigned nblocks = (unsigned)((a.n_near + 3) / 4);
     if (a.n_test > 0 && a.n_trial > 0) {
         if (op->op == BEM_OP_V) {
