@@ -471,8 +471,9 @@ __global__ void __launch_bounds__(128) adj_near_kernel(AdjArgs a) {
     }
     PairMoments M;
     M.zero();
-    auto add = [&](double r1x, double r2x, double r1y, double r2y, double wj, bool second, double px1, double px2,
-                   double py1, double py2) {
+    const bool twin = rel == REL_COINCIDE, quirk = a.quirk != 0;
+    const double invJj = 1.0 / Jj;
+    auto add = [&](double r1x, double r2x, double r1y, double r2y, double wj) {
         const double sx_[3] = {1.0 - r1x, r1x - r2x, r2x};
         const double sy_[3] = {1.0 - r1y, r1y - r2y, r2y};
         double d[3];
@@ -482,21 +483,26 @@ __global__ void __launch_bounds__(128) adj_near_kernel(AdjArgs a) {
         // barycentric weights per stored vertex
         const double bx[3] = {sx_[slotx[0]], sx_[slotx[1]], sx_[slotx[2]]};
         const double by[3] = {sy_[sloty[0]], sy_[sloty[1]], sy_[sloty[2]]};
-        double ub = 1.0;
+        // P1 data at the trial point; the swapped twin of a coincident point has the
+        // opposite normal derivative, with the data at the same point (quirk: the two
+        // cancel) or at the test point's parameters, and V's same value
+        double ub = 1.0, w = wj;
         if (OP == BEM_OP_K) {
-            // P1 data at the basis parameters of the trial side
-            const double pb[3] = {1.0 - py1, py1 - py2, py2};
-            ub = pb[sloty[0]] * uj[0] + pb[sloty[1]] * uj[1] + pb[sloty[2]] * uj[2];
+            ub = by[0] * uj[0] + by[1] * uj[1] + by[2] * uj[2];
+            if (twin)
+                ub -= quirk ? ub : sx_[sloty[0]] * uj[0] + sx_[sloty[1]] * uj[1] + sx_[sloty[2]] * uj[2];
+        } else if (twin) {
+            w = wj + wj;
         }
-        (void)px1;
-        (void)px2;
-        adj_point<OP>(M, d, wj, bx, by, ub, second ? -1.0 : 1.0, nj, 1.0 / Jj);
+        adj_point<OP>(M, d, w, bx, by, ub, 1.0, nj, invJj);
     };
+    NearDigits dg;
     const int Q = a.Q, Q4 = Q * Q * Q * Q;
+    dg.start(lane, Q);
     for (int p = lane; p < Q4; p += 32) {
-        const int iw = p % Q, iz = (p / Q) % Q, iy = (p / (Q * Q)) % Q, ix = p / (Q * Q * Q);
-        const double weight = (a.gw[ix] * a.gw[iy] * Ji) * (a.gw[iz] * a.gw[iw] * Jj);
-        near_points(rel, a.quirk != 0, a.gp[ix], a.gp[iy], a.gp[iz], a.gp[iw], weight, add);
+        const double weight = (a.gw[dg.ix] * a.gw[dg.iy] * Ji) * (a.gw[dg.iz] * a.gw[dg.iw] * Jj);
+        near_points(rel, a.gp[dg.ix], a.gp[dg.iy], a.gp[dg.iz], a.gp[dg.iw], weight, add);
+        dg.next(Q);
     }
     M.reduce();
     if (lane != 0) return;

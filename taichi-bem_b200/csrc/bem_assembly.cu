@@ -17,15 +17,13 @@
 //    formed in FP64, so the FP32 variant (mixed precision) keeps its relative
 //    accuracy for close pairs.
 //  * coincident / edge / vertex pairs (about 13 per panel on an icosphere)
-//    run in `near_kernel` in FP64: one warp per pair, lanes split the
-//    GaussQR^4 Sauter-Schwab points, warp-shuffle reduction.
+//    run in FP64 in bem_near.cu.
 //  * P0 rows/columns are written in place (each entry has one writer); P1
 //    entries receive contributions from several panel pairs and use FP64
 //    atomics, as the reference's Taichi `+=` does (hypersingular_layer_3d.py:500).
 #include <cuda_runtime.h>
 
 #include "bem_internal.cuh"
-#include "bem_quadrature.cuh"
 #include "bem_farfield.cuh"
 
 namespace {
@@ -215,7 +213,6 @@ struct FarArgs {
     const double* x;
     double* y;
     int conj_x;
-    int skip_far;  // 1: launch only the near-pair kernel (bem_launch_assemble_parts)
     int dk = 0;    // 1: the kernel's k-derivative (kval)
 };
 
@@ -462,212 +459,8 @@ __global__ void __launch_bounds__(FAR_THREADS) far_kernel(FarArgs a) {
     }
 }
 
-// ----------------------------------------------------------------------------
-// near field: coincident / edge / vertex pairs in FP64 (Sauter-Schwab maps of
-// single_layer_3d.py:178-367, identical in the other operators)
-// ----------------------------------------------------------------------------
-struct NearArgs {
-    int64_t n_near;
-    const int4* near;
-    const int32_t* test_local;
-    const int32_t* trial_local;
-    const int32_t* test_dof;
-    const int32_t* trial_dof;
-    const int32_t* tris;
-    const double* verts;
-    const double* area;
-    const double* normal;
-    const double* curl;
-    const double* gp;
-    const double* gw;
-    int Q;
-    double k, k2;
-    int quirk;
-    int mode;
-    double* out;
-    int64_t ld;
-    double scale;
-    double* out_t;
-    double scale_t;
-    const double* x;
-    double* y;
-    int conj_x;
-    int dk = 0;  // 1: the kernel's k-derivative (kval)
-};
-
-struct NearPanel {
-    double x1[3], x2[3], x3[3];
-    double n[3];
-    double area;
-    int slot[3];  // parameter slot of original vertex b
-};
-
-__device__ __forceinline__ void load_near_panel(NearPanel& P, const NearArgs& a, int g, int perm) {
-    int pm[3] = {perm & 3, (perm >> 2) & 3, (perm >> 4) & 3};
-    const int32_t* t = a.tris + 3 * g;
-    for (int c = 0; c < 3; ++c) {
-        P.x1[c] = a.verts[3 * t[pm[0]] + c];
-        P.x2[c] = a.verts[3 * t[pm[1]] + c];
-        P.x3[c] = a.verts[3 * t[pm[2]] + c];
-        P.n[c] = a.normal[3 * g + c];
-    }
-    P.area = a.area[g];
-    for (int s = 0; s < 3; ++s) P.slot[pm[s]] = s;
-}
-
 __device__ __forceinline__ double shape_slot(double r1, double r2, int s) {
     return s == 0 ? 1.0 - r1 : (s == 1 ? r1 - r2 : r2);
-}
-
-template <int OP, bool HELM, int NBX, int NBY>
-__global__ void __launch_bounds__(128) near_kernel(NearArgs a) {
-    constexpr bool W_OP = (OP == BEM_OP_W);
-    constexpr bool NEED_PHI = !(W_OP && !HELM);
-    const int lane = threadIdx.x & 31;
-    const int64_t pid = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (pid >= a.n_near) return;
-    const int4 e = a.near[pid];
-    const int gi = e.x, gj = e.y, rel = e.z;
-    const int li = a.test_local[gi], lj = a.trial_local[gj];
-    if (li < 0 || lj < 0) return;  // warp-uniform
-    const int permx = a.quirk ? (0 | (1 << 2) | (2 << 4)) : (e.w & 63);
-    const int permy = a.quirk ? (0 | (1 << 2) | (2 << 4)) : ((e.w >> 6) & 63);
-    NearPanel X, Y;
-    load_near_panel(X, a, gi, permx);
-    load_near_panel(Y, a, gj, permy);
-    const double* nKx = X.n;  // normal used by KP
-    const double* nKy = Y.n;  // normal used by K
-
-    double acc_re[NBX][NBY], acc_im[NBX][NBY], acc0_re = 0.0, acc0_im = 0.0;
-#pragma unroll
-    for (int bx = 0; bx < NBX; ++bx)
-#pragma unroll
-        for (int by = 0; by < NBY; ++by) acc_re[bx][by] = acc_im[bx][by] = 0.0;
-
-    int sx[NBX], sy[NBY];
-#pragma unroll
-    for (int bx = 0; bx < NBX; ++bx) sx[bx] = NBX == 1 ? -1 : X.slot[bx];
-#pragma unroll
-    for (int by = 0; by < NBY; ++by) sy[by] = NBY == 1 ? -1 : Y.slot[by];
-
-    const int Q = a.Q;
-    const int Q4 = Q * Q * Q * Q;
-    // One kernel evaluation at parameters (r1x,r2x) on X and (r1y,r2y) on Y,
-    // argument order `second` (the swapped coincide term), basis values taken
-    // at (px1,px2) for the test side and (py1,py2) for the trial side.
-    auto add = [&](double r1x, double r2x, double r1y, double r2y, double wj, bool second, double px1, double px2,
-                   double py1, double py2) {
-        double x[3], yv[3];
-        for (int c = 0; c < 3; ++c) {
-            x[c] = (1.0 - r1x) * X.x1[c] + (r1x - r2x) * X.x2[c] + r2x * X.x3[c];
-            yv[c] = (1.0 - r1y) * Y.x1[c] + (r1y - r2y) * Y.x2[c] + r2y * Y.x3[c];
-        }
-        double dx = x[0] - yv[0], dy = x[1] - yv[1], dz = x[2] - yv[2];
-        double re, im;
-        if (OP == BEM_OP_K) {
-            // first: grad_G_y(x, y, n_y); second: grad_G_y(y, x, n_y)
-            double sgn = second ? -1.0 : 1.0;
-            kval<BEM_OP_K, HELM, double>(sgn * dx, sgn * dy, sgn * dz, nKy[0], nKy[1], nKy[2], a.k, re, im, a.dk != 0);
-        } else if (OP == BEM_OP_KP) {
-            // first: grad_G_y(y, x, n_x); second: grad_G_y(x, y, n_x)
-            double sgn = second ? -1.0 : 1.0;
-            kval<BEM_OP_KP, HELM, double>(sgn * dx, sgn * dy, sgn * dz, nKx[0], nKx[1], nKx[2], a.k, re, im,
-                                          a.dk != 0);
-        } else {
-            kval<BEM_OP_V, HELM, double>(dx, dy, dz, 0.0, 0.0, 0.0, a.k, re, im, a.dk != 0);
-        }
-        re *= wj;
-        im *= wj;
-        if (W_OP) {
-            acc0_re += re;
-            acc0_im += im;
-        }
-        if (NEED_PHI) {
-#pragma unroll
-            for (int bx = 0; bx < NBX; ++bx) {
-                double phx = NBX == 1 ? 1.0 : shape_slot(px1, px2, sx[bx]);
-#pragma unroll
-                for (int by = 0; by < NBY; ++by) {
-                    double phy = NBY == 1 ? 1.0 : shape_slot(py1, py2, sy[by]);
-                    acc_re[bx][by] += re * phx * phy;
-                    acc_im[bx][by] += im * phx * phy;
-                }
-            }
-        }
-    };
-
-    for (int p = lane; p < Q4; p += 32) {
-        int iw = p % Q, iz = (p / Q) % Q, iy = (p / (Q * Q)) % Q, ix = p / (Q * Q * Q);
-        const double xsi = a.gp[ix], eta1 = a.gp[iy], eta2 = a.gp[iz], eta3 = a.gp[iw];
-        const double weight = (a.gw[ix] * a.gw[iy] * (X.area * 2.0)) * (a.gw[iz] * a.gw[iw] * (Y.area * 2.0));
-        near_points(rel, a.quirk != 0, xsi, eta1, eta2, eta3, weight, add);
-    }
-
-    // warp reduction of every moment
-    acc0_re = warp_sum(acc0_re);
-    acc0_im = warp_sum(acc0_im);
-#pragma unroll
-    for (int bx = 0; bx < NBX; ++bx)
-#pragma unroll
-        for (int by = 0; by < NBY; ++by) {
-            acc_re[bx][by] = warp_sum(acc_re[bx][by]);
-            acc_im[bx][by] = warp_sum(acc_im[bx][by]);
-        }
-    if (lane != 0) return;
-
-    const double nd = X.n[0] * Y.n[0] + X.n[1] * Y.n[1] + X.n[2] * Y.n[2];
-#pragma unroll
-    for (int bx = 0; bx < NBX; ++bx) {
-        const int row = a.test_dof[li * NBX + bx];
-        if (row < 0) continue;
-        double cr = 0.0, ci = 0.0;
-#pragma unroll
-        for (int by = 0; by < NBY; ++by) {
-            const int col = a.trial_dof[lj * NBY + by];
-            if (col < 0) continue;
-            double vr, vi;
-            if (W_OP) {
-                double cd = 0.0;
-                if (NBX == 3 && NBY == 3) {
-                    const double* cx = a.curl + 9 * gi + 3 * bx;
-                    const double* cy = a.curl + 9 * gj + 3 * by;
-                    cd = cx[0] * cy[0] + cx[1] * cy[1] + cx[2] * cy[2];
-                }
-                vr = acc0_re * cd;
-                vi = acc0_im * cd;
-                if (NEED_PHI) {
-                    vr -= a.k2 * nd * acc_re[bx][by];
-                    vi -= a.k2 * nd * acc_im[bx][by];
-                }
-            } else {
-                vr = acc_re[bx][by];
-                vi = acc_im[bx][by];
-            }
-            vr *= BEM_INV4PI;
-            vi *= BEM_INV4PI;
-            if (a.mode == 0) {
-                add_entry<HELM>(a.out, (int64_t)row * a.ld + col, a.scale * vr, a.scale * vi, true);
-                if (a.out_t) add_entry<HELM>(a.out_t, (int64_t)col * a.ld + row, a.scale_t * vr, a.scale_t * vi, true);
-            } else {
-                if (HELM) {
-                    double xr = a.x[2 * col], xi = a.x[2 * col + 1];
-                    if (a.conj_x) xi = -xi;
-                    cr += vr * xr - vi * xi;
-                    ci += vr * xi + vi * xr;
-                } else {
-                    cr += vr * a.x[col];
-                }
-            }
-        }
-        if (a.mode != 0) {
-            if (HELM) {
-                atomicAdd(a.y + 2 * row, a.scale * cr);
-                atomicAdd(a.y + 2 * row + 1, a.scale * ci);
-            } else {
-                atomicAdd(a.y + row, a.scale * cr);
-            }
-        }
-    }
 }
 
 // ----------------------------------------------------------------------------
@@ -730,121 +523,6 @@ __global__ void mass_kernel(MassArgs a) {
         } else {
             atomicAdd(a.y + row, a.scale * acc * a.x[col]);
         }
-    }
-}
-
-// Fused near field of the Dirichlet pass: V (P0 x P0, dense, `v`) and the
-// matrix-free K g (P0 rows, NBD data bases on the trial panel, `k`) of one
-// near pair from the same Sauter-Schwab points.  Each point's r, 1/r and
-// e^{ikr} serve both integrands; the values and their accumulation are those
-// of near_kernel<BEM_OP_V, HELM, 1, 1> and near_kernel<BEM_OP_K, HELM, 1, NBD>
-// (the swapped coincide term takes K's kernel with -d, as there).  One warp
-// per near pair.
-template <bool HELM, int NBD>
-__global__ void __launch_bounds__(128) near_vkg_kernel(NearArgs v, NearArgs k) {
-    const int lane = threadIdx.x & 31;
-    const int64_t pid = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (pid >= v.n_near) return;
-    const int4 e = v.near[pid];
-    const int gi = e.x, gj = e.y, rel = e.z;
-    const int li = v.test_local[gi], lj = v.trial_local[gj];
-    if (li < 0 || lj < 0) return;  // warp-uniform
-    const int permx = v.quirk ? (0 | (1 << 2) | (2 << 4)) : (e.w & 63);
-    const int permy = v.quirk ? (0 | (1 << 2) | (2 << 4)) : ((e.w >> 6) & 63);
-    NearPanel X, Y;
-    load_near_panel(X, v, gi, permx);
-    load_near_panel(Y, v, gj, permy);
-    int sy[NBD];
-#pragma unroll
-    for (int b = 0; b < NBD; ++b) sy[b] = NBD == 1 ? -1 : Y.slot[b];
-    double av_re = 0.0, av_im = 0.0, ak_re[NBD], ak_im[NBD];
-#pragma unroll
-    for (int b = 0; b < NBD; ++b) ak_re[b] = ak_im[b] = 0.0;
-    const double kk = v.k;
-    auto add = [&](double r1x, double r2x, double r1y, double r2y, double wj, bool second, double px1, double px2,
-                   double py1, double py2) {
-        double x[3], yv[3];
-        for (int c = 0; c < 3; ++c) {
-            x[c] = (1.0 - r1x) * X.x1[c] + (r1x - r2x) * X.x2[c] + r2x * X.x3[c];
-            yv[c] = (1.0 - r1y) * Y.x1[c] + (r1y - r2y) * Y.x2[c] + r2y * Y.x3[c];
-        }
-        const double dx = x[0] - yv[0], dy = x[1] - yv[1], dz = x[2] - yv[2];
-        const double r2 = dx * dx + dy * dy + dz * dz;
-        double r, rinv;
-        dev_r_rinv(r2, r, rinv);
-        // K: grad_G_y(x, y, n_y); the swapped coincide term grad_G_y(y, x, n_y)
-        const double dn = (second ? -1.0 : 1.0) * (dx * Y.n[0] + dy * Y.n[1] + dz * Y.n[2]);
-        const double t = dn * rinv * rinv * rinv;
-        double vre, vim, kre, kim;
-        if (HELM) {
-            const double kr = kk * r;
-            double sn, cs;
-            dev_sincos(kr, &sn, &cs);
-            vre = rinv * cs;
-            vim = rinv * sn;
-            kre = t * (cs + kr * sn);
-            kim = t * (sn - kr * cs);
-        } else {
-            vre = rinv;
-            vim = 0.0;
-            kre = t;
-            kim = 0.0;
-        }
-        av_re += vre * wj;
-        av_im += vim * wj;
-        (void)px1;
-        (void)px2;
-#pragma unroll
-        for (int b = 0; b < NBD; ++b) {
-            const double phy = NBD == 1 ? 1.0 : shape_slot(py1, py2, sy[b]);
-            ak_re[b] += (kre * wj) * phy;
-            ak_im[b] += (kim * wj) * phy;
-        }
-    };
-    const int Q = v.Q;
-    const int Q4 = Q * Q * Q * Q;
-    for (int p = lane; p < Q4; p += 32) {
-        int iw = p % Q, iz = (p / Q) % Q, iy = (p / (Q * Q)) % Q, ix = p / (Q * Q * Q);
-        const double xsi = v.gp[ix], eta1 = v.gp[iy], eta2 = v.gp[iz], eta3 = v.gp[iw];
-        const double weight = (v.gw[ix] * v.gw[iy] * (X.area * 2.0)) * (v.gw[iz] * v.gw[iw] * (Y.area * 2.0));
-        near_points(rel, v.quirk != 0, xsi, eta1, eta2, eta3, weight, add);
-    }
-    av_re = warp_sum(av_re);
-    av_im = warp_sum(av_im);
-#pragma unroll
-    for (int b = 0; b < NBD; ++b) {
-        ak_re[b] = warp_sum(ak_re[b]);
-        ak_im[b] = warp_sum(ak_im[b]);
-    }
-    if (lane != 0) return;
-    {
-        const int row = v.test_dof[li], col = v.trial_dof[lj];
-        if (row >= 0 && col >= 0)
-            add_entry<HELM>(v.out, (int64_t)row * v.ld + col, v.scale * BEM_INV4PI * av_re,
-                            v.scale * BEM_INV4PI * av_im, true);
-    }
-    const int row = k.test_dof[li];
-    if (row < 0) return;
-    double cr = 0.0, ci = 0.0;
-#pragma unroll
-    for (int b = 0; b < NBD; ++b) {
-        const int col = k.trial_dof[lj * NBD + b];
-        if (col < 0) continue;
-        const double vr = ak_re[b] * BEM_INV4PI, vi = ak_im[b] * BEM_INV4PI;
-        if (HELM) {
-            double xr = k.x[2 * col], xi = k.x[2 * col + 1];
-            if (k.conj_x) xi = -xi;
-            cr += vr * xr - vi * xi;
-            ci += vr * xi + vi * xr;
-        } else {
-            cr += vr * k.x[col];
-        }
-    }
-    if (HELM) {
-        atomicAdd(k.y + 2 * row, k.scale * cr);
-        atomicAdd(k.y + 2 * row + 1, k.scale * ci);
-    } else {
-        atomicAdd(k.y + row, k.scale * cr);
     }
 }
 
@@ -1524,45 +1202,33 @@ __global__ void __launch_bounds__(FAR_THREADS, 5) far_vkg_sym_x2_kernel(FarArgs 
 }
 
 template <int OP, bool HELM, int NBX, int NBY>
-int launch_op(bem_ctx* ctx, const FarArgs& fa, const NearArgs& na, bool fp32, cudaStream_t s) {
+int launch_far(bem_ctx* ctx, const FarArgs& fa, bool fp32, cudaStream_t s) {
     dim3 grid((fa.n_trial + FAR_THREADS - 1) / FAR_THREADS, (fa.n_test + FAR_TI - 1) / FAR_TI);
     if (grid.y > 65535) return bem_fail(ctx, BEM_ERR_INVALID, "too many test panels for one launch");
-    if (fa.n_test > 0 && fa.n_trial > 0 && !fa.skip_far) {
-        size_t smem;
-        if (fp32) {
-            smem = FAR_TI * fa.Q2 * sizeof(float4) + fa.Q2 * 3 * sizeof(float);
-            far_kernel<OP, HELM, NBX, NBY, float><<<grid, FAR_THREADS, smem, s>>>(fa);
-        } else {
-            smem = FAR_TI * fa.Q2 * sizeof(double4) + fa.Q2 * 3 * sizeof(double);
-            far_kernel<OP, HELM, NBX, NBY, double><<<grid, FAR_THREADS, smem, s>>>(fa);
-        }
-        ctx->launches++;
-        if (int rc = bem_check_cuda(ctx, cudaGetLastError(), "far_kernel launch")) return rc;
+    if (fa.n_test <= 0 || fa.n_trial <= 0) return BEM_OK;
+    if (fp32) {
+        const size_t smem = FAR_TI * fa.Q2 * sizeof(float4) + fa.Q2 * 3 * sizeof(float);
+        far_kernel<OP, HELM, NBX, NBY, float><<<grid, FAR_THREADS, smem, s>>>(fa);
+    } else {
+        const size_t smem = FAR_TI * fa.Q2 * sizeof(double4) + fa.Q2 * 3 * sizeof(double);
+        far_kernel<OP, HELM, NBX, NBY, double><<<grid, FAR_THREADS, smem, s>>>(fa);
     }
-    if (na.n_near > 0) {
-        int warps = 4;
-        int64_t blocks = (na.n_near + warps - 1) / warps;
-        near_kernel<OP, HELM, NBX, NBY><<<(unsigned)blocks, 32 * warps, 0, s>>>(na);
-        ctx->launches++;
-        if (int rc = bem_check_cuda(ctx, cudaGetLastError(), "near_kernel launch")) return rc;
-    }
-    return BEM_OK;
+    ctx->launches++;
+    return bem_check_cuda(ctx, cudaGetLastError(), "far_kernel launch");
 }
 
 template <int OP, bool HELM>
-int dispatch_nb(bem_ctx* ctx, int nbx, int nby, const FarArgs& fa, const NearArgs& na, bool fp32, cudaStream_t s) {
-    if (nbx == 1 && nby == 1) return launch_op<OP, HELM, 1, 1>(ctx, fa, na, fp32, s);
-    if (nbx == 1 && nby == 3) return launch_op<OP, HELM, 1, 3>(ctx, fa, na, fp32, s);
-    if (nbx == 3 && nby == 1) return launch_op<OP, HELM, 3, 1>(ctx, fa, na, fp32, s);
-    if (nbx == 3 && nby == 3) return launch_op<OP, HELM, 3, 3>(ctx, fa, na, fp32, s);
+int dispatch_nb(bem_ctx* ctx, int nbx, int nby, const FarArgs& fa, bool fp32, cudaStream_t s) {
+    if (nbx == 1 && nby == 1) return launch_far<OP, HELM, 1, 1>(ctx, fa, fp32, s);
+    if (nbx == 1 && nby == 3) return launch_far<OP, HELM, 1, 3>(ctx, fa, fp32, s);
+    if (nbx == 3 && nby == 1) return launch_far<OP, HELM, 3, 1>(ctx, fa, fp32, s);
+    if (nbx == 3 && nby == 3) return launch_far<OP, HELM, 3, 3>(ctx, fa, fp32, s);
     return bem_fail(ctx, BEM_ERR_INVALID, "nb must be 1 (P0) or 3 (P1)");
 }
 
 template <int OP>
-int dispatch_helm(bem_ctx* ctx, bool helm, int nbx, int nby, const FarArgs& fa, const NearArgs& na, bool fp32,
-                  cudaStream_t s) {
-    return helm ? dispatch_nb<OP, true>(ctx, nbx, nby, fa, na, fp32, s)
-                : dispatch_nb<OP, false>(ctx, nbx, nby, fa, na, fp32, s);
+int dispatch_helm(bem_ctx* ctx, bool helm, int nbx, int nby, const FarArgs& fa, bool fp32, cudaStream_t s) {
+    return helm ? dispatch_nb<OP, true>(ctx, nbx, nby, fa, fp32, s) : dispatch_nb<OP, false>(ctx, nbx, nby, fa, fp32, s);
 }
 
 }  // namespace
@@ -1595,92 +1261,53 @@ int bem_fill_local_map(bem_ctx* ctx, const bem_space* sp, int32_t* map, cudaStre
 int bem_launch_assemble(bem_ctx* ctx, const bem_op_desc* op, const bem_space* test, const bem_space* trial,
                         int mode, void* out, int64_t ld, double scale, void* out_t, double scale_t, const void* x,
                         void* y, int conj_x, cudaStream_t s) {
-    return bem_launch_assemble_parts(ctx, op, test, trial, mode, out, ld, scale, out_t, scale_t, x, y, conj_x, s,
-                                     false);
-}
-
-int bem_launch_assemble_parts(bem_ctx* ctx, const bem_op_desc* op, const bem_space* test, const bem_space* trial,
-                              int mode, void* out, int64_t ld, double scale, void* out_t, double scale_t,
-                              const void* x, void* y, int conj_x, cudaStream_t s, bool near_only) {
     if (int rc = bem_fill_local_map(ctx, test, ctx->test_local, s)) return rc;
     if (int rc = bem_fill_local_map(ctx, trial, ctx->trial_local, s)) return rc;
-    bool fp32 = op->precision == BEM_PREC_MIXED;
-    FarArgs fa{};
-    fa.skip_far = near_only ? 1 : 0;
-    fa.n_test = test->n_panels;
-    fa.n_trial = trial->n_panels;
-    fa.test_panels = test->panels;
-    fa.test_dof = test->dof;
-    fa.trial_panels = trial->panels;
-    fa.trial_dof = trial->dof;
-    fa.tris = ctx->tris;
-    fa.centroid = ctx->centroid;
-    fa.normal = ctx->normal;
-    fa.curl = ctx->curl;
-    fa.area = ctx->area;
-    fa.wcorr = ctx->wcorr32;
-    fa.small_phase = fp32 && op->kernel == BEM_KERNEL_HELMHOLTZ ? bem_phase_class(op->k * 2.0 * ctx->rho_max) : 0;
-    fa.pts = fp32 ? (const void*)ctx->pts32 : (const void*)ctx->pts64;
-    fa.phi = fp32 ? (const void*)ctx->phi32 : (const void*)ctx->phi64;
-    fa.phi64 = ctx->phi64;
-    fa.Q2 = ctx->Q2;
-    fa.k = op->k;
-    fa.k2 = op->k2;
-    fa.dk = op->deriv_k ? 1 : 0;
-    fa.mode = mode;
-    fa.out = (double*)out;
-    fa.ld = ld;
-    fa.scale = scale;
-    fa.out_t = (double*)out_t;
-    fa.scale_t = scale_t;
-    fa.x = (const double*)x;
-    fa.y = (double*)y;
-    fa.conj_x = conj_x;
-
-    if (!near_only) {
-        // FP64: the kernel that evaluates an unordered pair once, where it has the bases
-        const int rc = bem_launch_far64(ctx, op, test, trial, mode, out, ld, scale, out_t, scale_t, x, y, conj_x, s);
-        if (rc < 0) return rc;
-        if (rc == BEM_OK) fa.skip_far = 1;
+    const bool fp32 = op->precision == BEM_PREC_MIXED;
+    const bool helm = op->kernel == BEM_KERNEL_HELMHOLTZ;
+    // FP64: the kernel that evaluates an unordered pair once, where it has the bases
+    int rc = bem_launch_far64(ctx, op, test, trial, mode, out, ld, scale, out_t, scale_t, x, y, conj_x, s);
+    if (rc == 1) {
+        FarArgs fa{};
+        fa.n_test = test->n_panels;
+        fa.n_trial = trial->n_panels;
+        fa.test_panels = test->panels;
+        fa.test_dof = test->dof;
+        fa.trial_panels = trial->panels;
+        fa.trial_dof = trial->dof;
+        fa.tris = ctx->tris;
+        fa.centroid = ctx->centroid;
+        fa.normal = ctx->normal;
+        fa.curl = ctx->curl;
+        fa.area = ctx->area;
+        fa.wcorr = ctx->wcorr32;
+        fa.small_phase = fp32 && helm ? bem_phase_class(op->k * 2.0 * ctx->rho_max) : 0;
+        fa.pts = fp32 ? (const void*)ctx->pts32 : (const void*)ctx->pts64;
+        fa.phi = fp32 ? (const void*)ctx->phi32 : (const void*)ctx->phi64;
+        fa.phi64 = ctx->phi64;
+        fa.Q2 = ctx->Q2;
+        fa.k = op->k;
+        fa.k2 = op->k2;
+        fa.dk = op->deriv_k ? 1 : 0;
+        fa.mode = mode;
+        fa.out = (double*)out;
+        fa.ld = ld;
+        fa.scale = scale;
+        fa.out_t = (double*)out_t;
+        fa.scale_t = scale_t;
+        fa.x = (const double*)x;
+        fa.y = (double*)y;
+        fa.conj_x = conj_x;
+        switch (op->op) {
+            case BEM_OP_V: rc = dispatch_helm<BEM_OP_V>(ctx, helm, test->nb, trial->nb, fa, fp32, s); break;
+            case BEM_OP_K: rc = dispatch_helm<BEM_OP_K>(ctx, helm, test->nb, trial->nb, fa, fp32, s); break;
+            case BEM_OP_KP: rc = dispatch_helm<BEM_OP_KP>(ctx, helm, test->nb, trial->nb, fa, fp32, s); break;
+            case BEM_OP_W: rc = dispatch_helm<BEM_OP_W>(ctx, helm, test->nb, trial->nb, fa, fp32, s); break;
+            default: rc = bem_fail(ctx, BEM_ERR_INVALID, "unknown operator");
+        }
     }
-
-    NearArgs na;
-    na.n_near = ctx->n_near;
-    na.near = ctx->near;
-    na.test_local = ctx->test_local;
-    na.trial_local = ctx->trial_local;
-    na.test_dof = test->dof;
-    na.trial_dof = trial->dof;
-    na.tris = ctx->tris;
-    na.verts = ctx->verts;
-    na.area = ctx->area;
-    na.normal = ctx->normal;
-    na.curl = ctx->curl;
-    na.gp = ctx->gp;
-    na.gw = ctx->gw;
-    na.Q = ctx->Q;
-    na.k = op->k;
-    na.k2 = op->k2;
-    na.dk = op->deriv_k ? 1 : 0;
-    na.quirk = op->quirk;
-    na.mode = mode;
-    na.out = (double*)out;
-    na.ld = ld;
-    na.scale = scale;
-    na.out_t = (double*)out_t;
-    na.scale_t = scale_t;
-    na.x = (const double*)x;
-    na.y = (double*)y;
-    na.conj_x = conj_x;
-
-    bool helm = op->kernel == BEM_KERNEL_HELMHOLTZ;
-    switch (op->op) {
-        case BEM_OP_V: return dispatch_helm<BEM_OP_V>(ctx, helm, test->nb, trial->nb, fa, na, fp32, s);
-        case BEM_OP_K: return dispatch_helm<BEM_OP_K>(ctx, helm, test->nb, trial->nb, fa, na, fp32, s);
-        case BEM_OP_KP: return dispatch_helm<BEM_OP_KP>(ctx, helm, test->nb, trial->nb, fa, na, fp32, s);
-        case BEM_OP_W: return dispatch_helm<BEM_OP_W>(ctx, helm, test->nb, trial->nb, fa, na, fp32, s);
-        default: return bem_fail(ctx, BEM_ERR_INVALID, "unknown operator");
-    }
+    if (rc) return rc;
+    return bem_launch_near(ctx, op, test, trial, mode, out, ld, scale, out_t, scale_t, x, y, conj_x, s);
 }
 
 int bem_launch_dirichlet(bem_ctx* ctx, const bem_op_desc* op, const bem_space* test, const bem_space* trial,
@@ -1769,54 +1396,9 @@ int bem_launch_dirichlet(bem_ctx* ctx, const bem_op_desc* op, const bem_space* t
         ctx->launches++;
         if (int rc = bem_check_cuda(ctx, cudaGetLastError(), "far_vkg_kernel launch")) return rc;
     }
-    // near field: V dense and K g apply, FP64, with the operator's own kernels
-    NearArgs na{};
-    na.n_near = ctx->n_near;
-    na.near = ctx->near;
-    na.test_local = ctx->test_local;
-    na.trial_local = ctx->trial_local;
-    na.tris = ctx->tris;
-    na.verts = ctx->verts;
-    na.area = ctx->area;
-    na.normal = ctx->normal;
-    na.curl = ctx->curl;
-    na.gp = ctx->gp;
-    na.gw = ctx->gw;
-    na.Q = ctx->Q;
-    na.k = op->k;
-    na.k2 = op->k2;
-    na.quirk = op->quirk;
-    if (na.n_near > 0) {
-        const unsigned blocks = (unsigned)((na.n_near + 3) / 4);
-        NearArgs nv = na;
-        nv.test_dof = test->dof;
-        nv.trial_dof = trial->dof;
-        nv.mode = 0;
-        nv.out = (double*)out;
-        nv.ld = ld;
-        nv.scale = scale;
-        NearArgs nk = na;
-        nk.test_dof = rows->dof;
-        nk.trial_dof = data->dof;
-        nk.mode = 1;
-        nk.x = (const double*)g;
-        nk.y = (double*)y;
-        nk.scale = scale_k;
-        nk.conj_x = conj_g;
-        if (helm) {
-            if (data->nb == 3)
-                near_vkg_kernel<true, 3><<<blocks, 128, 0, sn>>>(nv, nk);
-            else
-                near_vkg_kernel<true, 1><<<blocks, 128, 0, sn>>>(nv, nk);
-        } else {
-            if (data->nb == 3)
-                near_vkg_kernel<false, 3><<<blocks, 128, 0, sn>>>(nv, nk);
-            else
-                near_vkg_kernel<false, 1><<<blocks, 128, 0, sn>>>(nv, nk);
-        }
-        ctx->launches++;
-        if (int rc = bem_check_cuda(ctx, cudaGetLastError(), "near_vkg_kernel launch")) return rc;
-    }
+    // near field: V dense and K g apply from the same FP64 points
+    if (int rc = bem_launch_near_dirichlet(ctx, op, test, trial, out, ld, scale, rows, data, g, y, scale_k, conj_g, sn))
+        return rc;
     if (side) {
         cudaEventRecord(ctx->ev_diag, ctx->aux);
         cudaStreamWaitEvent(s, ctx->ev_diag, 0);

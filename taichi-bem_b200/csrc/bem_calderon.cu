@@ -25,7 +25,7 @@
 // rescaled in FP64; the sums over the test points run in FP32, the sums over
 // the trial points in FP64.  FP64 (plain path) evaluates d = x - y directly.
 // Coincident / edge / vertex pairs are left to the FP64 Sauter-Schwab
-// kernels (bem_launch_assemble_parts, near only), which run on the side
+// kernel (bem_launch_near_calderon), which runs on the side
 // stream while the sweep runs.
 #include <cmath>
 
@@ -853,8 +853,8 @@ extern "C" int bem_assemble_calderon(bem_ctx* ctx, const bem_op_desc* op, int nk
     cudaStream_t s = (cudaStream_t)stream;
     const bool fp32 = op->precision == BEM_PREC_MIXED;
     const bool helm = op->kernel == BEM_KERNEL_HELMHOLTZ;
-    // near pairs: the FP64 Sauter-Schwab kernels of each operator, per
-    // wavenumber, on the high-priority side stream, concurrently with the far
+    // near pairs: every operator and wavenumber from the same FP64 Sauter-Schwab
+    // points, on the high-priority side stream, concurrently with the far
     // sweep (different pipes; they write other V entries, and every entry they
     // share with the sweep -- the P1 columns and rows -- is added atomically);
     // the caller's stream waits for both
@@ -862,24 +862,9 @@ extern "C" int bem_assemble_calderon(bem_ctx* ctx, const bem_op_desc* op, int nk
     if (int rc = bem_check_cuda(ctx, cudaEventRecord(ctx->ev_next, s), "calderon fork")) return rc;
     if (int rc = bem_check_cuda(ctx, cudaStreamWaitEvent(ctx->aux, ctx->ev_next, 0), "calderon fork")) return rc;
     const cudaStream_t sn = ctx->aux;
-    for (int w = 0; w < nk; ++w) {
-        bem_op_desc d = *op;
-        d.k = k[w];
-        d.k2 = k2[w];
-        const double c = coef[w];
-        d.op = BEM_OP_V;
-        if (int rc = bem_launch_assemble_parts(ctx, &d, neu, neu, 0, out[w], ld, -c, nullptr, 0.0, nullptr, nullptr, 0,
-                                               sn, true))
-            return rc;
-        d.op = BEM_OP_K;
-        if (int rc = bem_launch_assemble_parts(ctx, &d, neu, dir, 0, out[w], ld, c, out[w], -c, nullptr, nullptr, 0,
-                                               sn, true))
-            return rc;
-        d.op = BEM_OP_W;
-        if (int rc = bem_launch_assemble_parts(ctx, &d, dir, dir, 0, out[w], ld, -c, nullptr, 0.0, nullptr, nullptr, 0,
-                                               sn, true))
-            return rc;
-    }
+    if (int rc = bem_fill_local_map(ctx, neu, ctx->test_local, sn)) return rc;
+    if (int rc = bem_fill_local_map(ctx, neu, ctx->trial_local, sn)) return rc;
+    if (int rc = bem_launch_near_calderon(ctx, op, nk, k, k2, neu, dir, out, coef, ld, sn)) return rc;
     CalArgs a{};
     a.n = neu->n_panels;
     a.panels = neu->panels;

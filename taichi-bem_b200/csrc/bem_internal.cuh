@@ -106,11 +106,21 @@ int bem_lookahead_stream(bem_ctx* ctx);
 int bem_launch_assemble(bem_ctx* ctx, const bem_op_desc* op, const bem_space* test, const bem_space* trial,
                         int mode, void* out, int64_t ld, double scale, void* out_t, double scale_t, const void* x,
                         void* y, int conj_x, cudaStream_t s);
-// bem_launch_assemble restricted to the near-pair (coincident / edge / vertex)
-// kernel when near_only (the far pairs then come from a fused sweep).
-int bem_launch_assemble_parts(bem_ctx* ctx, const bem_op_desc* op, const bem_space* test, const bem_space* trial,
-                              int mode, void* out, int64_t ld, double scale, void* out_t, double scale_t,
-                              const void* x, void* y, int conj_x, cudaStream_t s, bool near_only);
+// Near pairs (bem_near.cu): one operator; one operator at nk Helmholtz
+// wavenumbers; the Dirichlet pass's V and K g; the Calderon blocks of up to two
+// wavenumbers.  The local maps have to be filled (bem_fill_local_map).
+int bem_launch_near(bem_ctx* ctx, const bem_op_desc* op, const bem_space* test, const bem_space* trial, int mode,
+                    void* out, int64_t ld, double scale, void* out_t, double scale_t, const void* x, void* y, int conj_x,
+                    cudaStream_t s);
+int bem_launch_near_batch(bem_ctx* ctx, const bem_op_desc* op, const bem_space* test, const bem_space* trial, int nk,
+                          const double* k, const double* k2, void* const* out, int64_t ld, const double* scale,
+                          void* const* out_t, const double* scale_t, cudaStream_t s);
+int bem_launch_near_dirichlet(bem_ctx* ctx, const bem_op_desc* op, const bem_space* test, const bem_space* trial,
+                              void* out, int64_t ld, double scale, const bem_space* rows, const bem_space* data,
+                              const void* g, void* y, double scale_k, int conj_g, cudaStream_t s);
+int bem_launch_near_calderon(bem_ctx* ctx, const bem_op_desc* op, int nk, const double* k, const double* k2,
+                             const bem_space* neu, const bem_space* dir, void* const* out, const double* coef, int64_t ld,
+                             cudaStream_t s);
 // FP64 far pairs of one operator, each unordered pair evaluated once
 // (bem_far64.cu); 1 where the general far_kernel has to run.
 int bem_launch_far64(bem_ctx* ctx, const bem_op_desc* op, const bem_space* test, const bem_space* trial, int mode,

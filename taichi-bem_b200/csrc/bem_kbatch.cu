@@ -15,7 +15,7 @@
 // points in shared memory, FP32 sums over the test points and FP64 sums over
 // the trial points in mixed precision (pair frame, bem_farfield.cuh), FP64
 // throughout on the plain path.  Coincident / edge / vertex pairs take the
-// FP64 Sauter-Schwab kernel once per wavenumber (bem_launch_assemble_parts).
+// FP64 Sauter-Schwab kernel, two wavenumbers per launch (bem_near.cu).
 #include <cmath>
 
 #include "bem_farfield.cuh"
@@ -390,14 +390,7 @@ int bem_launch_assemble_batch(bem_ctx* ctx, const bem_op_desc* op, const bem_spa
             if (rc) return rc;
         }
     }
-    for (int w = 0; w < nk; ++w) {
-        bem_op_desc ow = *op;
-        ow.k = k[w];
-        ow.k2 = k2[w];
-        void* ot = out_t ? out_t[w] : nullptr;
-        if (int rc = bem_launch_assemble_parts(ctx, &ow, test, trial, 0, out[w], ld, scale[w], ot,
-                                               ot ? scale_t[w] : 0.0, nullptr, nullptr, 0, s, true))
-            return rc;
-    }
-    return BEM_OK;
+    if (int rc = bem_fill_local_map(ctx, test, ctx->test_local, s)) return rc;
+    if (int rc = bem_fill_local_map(ctx, trial, ctx->trial_local, s)) return rc;
+    return bem_launch_near_batch(ctx, op, test, trial, nk, k, k2, out, ld, scale, out_t, scale_t, s);
 }

@@ -829,7 +829,10 @@ __global__ void __launch_bounds__(256) tri_solve_kernel(const T* LU, int64_t lda
                     o[r][1] += q[r][1];
                     // a zero pivot divides by zero, as substitution would, and the rows above
                     // it depend on that value (the inverse holds 0 there)
-                    if (gr <= s_zero[par]) o[r][0] = o[r][1] = (gr == s_zero[par] && !C ? s_r[gr][r][0] : 0.0) / 0.0;
+                    if (gr <= s_zero[par]) {
+                        const double zero = (double)sT[s_zero[par] * SOLVE_LD + s_zero[par]].re;
+                        o[r][0] = o[r][1] = (gr == s_zero[par] && !C ? s_r[gr][r][0] : zero) / zero;
+                    }
                 }
             }
             if (gq == 0 && gr < m)

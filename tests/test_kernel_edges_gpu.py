@@ -240,3 +240,45 @@ def test_adjoint_over_partial_lists(engine, op, nby):
         m[i, c] -= h
         fd = (form(p)[0] - form(m)[0]) / (2 * h)
         assert abs(fd - grad[i, c]) < 1e-6 * np.abs(grad).max()
+
+
+# ---- near pairs ------------------------------------------------------------------------------
+@pytest.mark.parametrize("quirk", [True, False])
+@pytest.mark.parametrize("Q", [1, 2, 3, 6])
+@pytest.mark.parametrize("op,nbx,nby", [("V", 1, 1), ("V", 3, 3), ("K", 1, 3), ("K", 3, 3), ("KP", 3, 1), ("W", 3, 3),
+                                        ("W", 1, 1)])
+def test_near_pairs_orders_and_batches(engine, op, nbx, nby, Q, quirk):
+    """Every point order whose Q^4 points fill part of a warp, a warp, and
+    several; one wavenumber and batches of two and three (one launch of two
+    and one of one), in each phase class.  On an icosphere of 20 panels most
+    pairs touch.  FP64 sums in another order than the oracle's: 1e-12 of the
+    largest entry."""
+    from bem_b200 import icosphere
+    from oracle import oracle as O
+    from bem_b200.engine import DeviceSpace
+    v, f = icosphere(0)
+    engine.set_mesh(v, f, Q)
+    code = getattr(O, "OP_" + op)
+    full = {1: (np.arange(len(f), dtype=np.int32), 1, np.arange(len(f), dtype=np.int32)),
+            3: (np.arange(len(f), dtype=np.int32), 3, f.reshape(-1).copy())}
+    ts, rs = full[nbx], full[nby]
+    td, rd = (DeviceSpace.from_numpy(*s, engine.device) for s in (ts, rs))
+    rows, cols = (len(f) if nb == 1 else len(v) for nb in (nbx, nby))
+
+    def ref(k):
+        out = np.zeros((rows, cols), np.complex128)
+        O.assemble(v, f, code, True, k, k * k, Q, quirk, ts, rs, out=out)
+        return out
+
+    ks = [0.05, 0.25, 3.0]
+    want = [ref(k) for k in ks]
+    for k, w in zip(ks, want):
+        out = torch.zeros(rows, cols, dtype=torch.complex128, device="cuda")
+        engine.assemble(engine.op_desc(code, True, k, k * k, quirk=quirk), td, rd, out)
+        assert np.abs(out.cpu().numpy() - w).max() < 1e-12 * np.abs(w).max()
+    for count in (2, 3):
+        outs = [torch.zeros(rows, cols, dtype=torch.complex128, device="cuda") for _ in range(count)]
+        engine.assemble_batch(engine.op_desc(code, True, quirk=quirk), td, rd, ks[:count], [k * k for k in ks[:count]],
+                              outs, [1.0] * count)
+        for o, w in zip(outs, want):
+            assert np.abs(o.cpu().numpy() - w).max() < 1e-12 * np.abs(w).max()
