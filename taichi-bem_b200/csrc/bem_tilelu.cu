@@ -6,8 +6,8 @@
 //            restricted to the block's rows;
 //   laswp  : the block's row swaps applied to the other columns;
 //   U12 = L11^{-1} A12 and L21 = A21 U11^{-1}: one CTA per 64-wide tile,
-//            substitution against the factored diagonal block, blocked by 8
-//            rows (columns), in shared memory (two CTA barriers per block);
+//            substitution against the factored diagonal block, the tile in
+//            registers (one CTA barrier per row or column);
 //   update : A22 -= L21 U12 (the trailing GEMM of bem_gemm.cuh).
 // After the last block, one launch forms the explicit inverses Linv_k (unit
 // lower) and Uinv_k (upper) of every diagonal block (`dinv`, used by the
@@ -69,194 +69,142 @@ __device__ __forceinline__ CE<T> cinv(CE<T> a) {
 // diagonal tile: GEPP inside the tile; explicit inverses of the factored tiles
 // --------------------------------------------------------------------------
 // Pivot key of a candidate: |re| + |im| as float bits (monotonic for
-// non-negative floats) above 63 - row, so that atomicMax picks the largest
-// magnitude and, among equal ones, the smallest row (the first maximum).  NaN
-// counts as 0.
+// non-negative floats), plus one so that 0 means "no candidate".  NaN counts
+// as 0.
 template <typename T>
-__device__ __forceinline__ unsigned long long pivot_key(CE<T> v, int r) {
+__device__ __forceinline__ unsigned pivot_key(CE<T> v) {
     float a = (float)(fabs(v.re) + fabs(v.im));
     if (!(a == a)) a = 0.0f;
-    return ((unsigned long long)__float_as_uint(a) << 32) | (unsigned)(LU_T - 1 - r);
+    return __float_as_uint(a) + 1u;
 }
 
 constexpr int DIAG_LD = LU_T + 1;  // padded row stride: column reads hit distinct banks
-constexpr int DIAG_PW = 8;         // panel width of the blocked factorisation
-constexpr size_t diag_smem_bytes(size_t elem) { return elem * LU_T * DIAG_LD; }
+constexpr int DIAG_PW = 8;         // row blocks of tile_inv_kernel
 // tile_inv_kernel: the factored block and the inverse being built
 constexpr size_t inv_smem_bytes(size_t elem) { return elem * (LU_T * DIAG_LD + LU_T * LU_T); }
 
 // One CTA of 256 threads factors the 64x64 diagonal tile (GEPP restricted to
-// the tile's rows).  Blocked by panels of
-// DIAG_PW columns:
-//   panel  : the 64 x DIAG_PW panel in registers (two elements per thread);
-//            per column a pivot max over packed keys (shuffles, then across
-//            the 8 warps), the pivot row exchanged through shared memory,
-//            multipliers shuffled within each row's four threads; two CTA
-//            barriers per column; the panel's row swaps are applied to the
-//            other columns once the panel is done;
-//   U12    : the panel's rows right of it, L11^{-1} applied by substitution
-//            (one thread per column);
-//   update : rank-DIAG_PW update of the trailing block, one column per thread
-//            with the column's U12 values held in registers.
-// The explicit inverses are formed later, by tile_inv_kernel.  Shared memory
-// (33 KB for complex FP32) leaves room for the trailing GEMM's CTAs on an SM.
+// the tile's rows).  The tile is on the factorisation's serial chain, so the
+// latency of a column is what it costs.  It stays in registers: thread (ty,
+// tx) of a 16 x 16 grid holds the entries (ty + 16 a, tx + 16 b).  Per column
+// two barriers: its owners publish the column; every warp finds the pivot
+// itself (lane l looks at rows l and l + 32; two warp reductions, largest |re|
+// + |im|, first position on ties); the pivot row's owners publish that row;
+// every thread updates its entries.  Rows do not move: a row carries its
+// position and is written to it at the end (the pivots are those of moved
+// rows).  Measured (complex FP32, B200): 34 us a tile alone on the GPU against
+// 48 us with the tile in shared memory, 8-column panels in registers and three
+// barriers a column.  The explicit inverses are formed later, by
+// tile_inv_kernel.
 template <typename T, bool C>
 __global__ void __launch_bounds__(256) tile_diag_kernel(T* A, int64_t lda, int n, int k0, int32_t* piv,
                                                         int32_t* info) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    CE<T>* S = reinterpret_cast<CE<T>*>(smem_raw);  // [LU_T][DIAG_LD]
-    __shared__ int s_zero_pivot;                    // first zero pivot of this tile (1-based), 0 = none
-    __shared__ unsigned long long s_wkey[8];        // per-warp pivot keys
-    __shared__ CE<T> s_rowj[DIAG_PW], s_rowp[DIAG_PW];
-    __shared__ int s_perm[DIAG_PW];                 // pivot rows of the current panel
+    __shared__ CE<T> s_col[2][LU_T];
+    __shared__ CE<T> s_row[LU_T];
+    __shared__ int s_pos[LU_T];
     const int m = min(LU_T, n - k0);
-    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    if (tid == 0) s_zero_pivot = 0;
-    for (int e = tid; e < LU_T * LU_T; e += blockDim.x) {
-        const int r = e / LU_T, c = e - r * LU_T;
-        CE<T> v = CE<T>{T(0), T(0)};
-        if (r < m && c < m) v = ldE<T, C>(A, (int64_t)(k0 + r) * lda + k0 + c);
-        S[r * DIAG_LD + c] = v;
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int tx = tid & 15, ty = tid >> 4;
+    CE<T> M[4][4];
+    int done = 0;  // bit a: row ty + 16 a is a pivot row already, or outside the matrix
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+        if (ty + 16 * a >= m) done |= 1 << a;
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+            const int r = ty + 16 * a, c = tx + 16 * b;
+            M[a][b] = r < m && c < m ? ldE<T, C>(A, (int64_t)(k0 + r) * lda + k0 + c) : CE<T>{T(0), T(0)};
+        }
+    }
+    // positions of rows lane and lane + 32, in every warp; LU_T = not a candidate any more
+    int pos0 = lane, pos1 = lane + 32;
+    bool free0 = lane < m, free1 = lane + 32 < m;
+    int zero = 0;  // 1 + first column whose pivot is zero
+#pragma unroll
+    for (int jb = 0; jb < 4; ++jb) {
+        const int je = min(16, m - 16 * jb);
+        for (int jj = 0; jj < je; ++jj) {
+            const int j = 16 * jb + jj;
+            CE<T>* col = s_col[j & 1];
+            if (tx == jj) {
+#pragma unroll
+                for (int a = 0; a < 4; ++a) col[ty + 16 * a] = M[a][jb];
+            }
+            __syncthreads();
+            const unsigned key0 = free0 ? pivot_key(col[lane]) : 0u, key1 = free1 ? pivot_key(col[lane + 32]) : 0u;
+            const unsigned best = __reduce_max_sync(0xffffffffu, key0 > key1 ? key0 : key1);
+            // first position, with the row it belongs to in the low bits
+            int cand = 0x7fffffff;
+            if (key0 == best && free0) cand = (pos0 << 6) | lane;
+            if (key1 == best && free1) cand = min(cand, (pos1 << 6) | (lane + 32));
+            cand = __reduce_min_sync(0xffffffffu, cand);
+            const int p = cand & 63, pp = cand >> 6;  // pivot row and its position
+            if (pos0 == j) pos0 = pp;
+            if (pos1 == j) pos1 = pp;
+            if (p == lane) {
+                pos0 = j;
+                free0 = false;
+            }
+            if (p == lane + 32) {
+                pos1 = j;
+                free1 = false;
+            }
+            if (ty == (p & 15)) {
+                // selects, not an index: the entries stay in registers
+                const int pa = p >> 4;
+                done |= 1 << pa;
+#pragma unroll
+                for (int b = 0; b < 4; ++b) {
+                    const CE<T> lo = (pa & 1) ? M[1][b] : M[0][b], hi = (pa & 1) ? M[3][b] : M[2][b];
+                    s_row[tx + 16 * b] = (pa & 2) ? hi : lo;
+                }
+            }
+            if (tid == 0) piv[k0 + j] = k0 + pp;
+            __syncthreads();
+            const CE<T> pv = s_row[j];
+            if (!(pv.re != T(0) || pv.im != T(0)) && zero == 0) zero = k0 + j + 1;
+            const CE<T> inv = cinv(pv);
+            CE<T> l[4];
+#pragma unroll
+            for (int a = 0; a < 4; ++a) {
+                l[a] = cmul(col[ty + 16 * a], inv);
+                if ((done >> a) & 1) l[a] = CE<T>{T(0), T(0)};
+            }
+            // no branches: l = 0 on finished rows, u = 0 left of and on the column
+#pragma unroll
+            for (int b = jb; b < 4; ++b) {
+                CE<T> u = s_row[tx + 16 * b];
+                if (b == jb && tx <= jj) u = CE<T>{T(0), T(0)};
+#pragma unroll
+                for (int a = 0; a < 4; ++a) {
+                    M[a][b].re -= l[a].re * u.re - (C ? l[a].im * u.im : T(0));
+                    if (C) M[a][b].im -= l[a].re * u.im + l[a].im * u.re;
+                }
+            }
+#pragma unroll
+            for (int a = 0; a < 4; ++a) {
+                const bool own = tx == jj && !((done >> a) & 1);
+                M[a][jb].re = own ? l[a].re : M[a][jb].re;
+                M[a][jb].im = own ? l[a].im : M[a][jb].im;
+            }
+        }
+    }
+    if (tid < 32) {
+        s_pos[lane] = pos0;
+        s_pos[lane + 32] = pos1;
     }
     __syncthreads();
-    // panel registers: thread t holds row pr = t >> 2, panel columns 2*pc, 2*pc+1 (pc = t & 3)
-    const int pr = tid >> 2, pc = tid & 3;
-    for (int j0 = 0; j0 < m; j0 += DIAG_PW) {
-        const int w = min(DIAG_PW, m - j0);
-        CE<T> e0 = S[pr * DIAG_LD + j0 + 2 * pc], e1 = S[pr * DIAG_LD + j0 + 2 * pc + 1];
-        for (int j = j0; j < j0 + w; ++j) {
-            const int jq = j - j0;  // panel column of j, held by threads with pc == jq / 2
-            // pivot: largest |re| + |im| in column j among rows j..m-1 (first one on ties):
-            // owners post keys, max over the warp's rows, then over the 8 warps
-            unsigned long long key = 0ull;
-            if (pc == (jq >> 1) && pr >= j && pr < m) key = pivot_key((jq & 1) ? e1 : e0, pr);
+    if (tid == 0 && zero != 0 && *info == 0) *info = zero;
 #pragma unroll
-            for (int o = 4; o < 32; o <<= 1) {
-                const unsigned long long ko = __shfl_xor_sync(0xffffffffu, key, o);
-                key = ko > key ? ko : key;
-            }
-            if (lane == (jq >> 1)) s_wkey[wid] = key;
-            __syncthreads();
-            unsigned long long best = s_wkey[0];
+    for (int a = 0; a < 4; ++a) {
+        const int r = ty + 16 * a;
+        if (r >= m) continue;
+        const int64_t row = (int64_t)(k0 + s_pos[r]) * lda + k0;
 #pragma unroll
-            for (int q = 1; q < 8; ++q) best = s_wkey[q] > best ? s_wkey[q] : best;
-            const int p = LU_T - 1 - (int)(best & 0xffffffffull);
-            const int prow = (p >= j && p < m) ? p : j;  // all-zero or NaN column: no swap
-            // exchange rows j and prow inside the panel; everyone reads the new pivot row
-            if (pr == j) {
-                s_rowj[2 * pc] = e0;
-                s_rowj[2 * pc + 1] = e1;
-            }
-            if (pr == prow) {
-                s_rowp[2 * pc] = e0;
-                s_rowp[2 * pc + 1] = e1;
-            }
-            __syncthreads();
-            if (prow != j) {
-                if (pr == j) {
-                    e0 = s_rowp[2 * pc];
-                    e1 = s_rowp[2 * pc + 1];
-                } else if (pr == prow) {
-                    e0 = s_rowj[2 * pc];
-                    e1 = s_rowj[2 * pc + 1];
-                }
-            }
-            const CE<T> pv = s_rowp[jq];
-            if (tid == 0) {
-                s_perm[jq] = prow;
-                piv[k0 + j] = k0 + prow;
-                if (!((double)pv.re != 0.0 || (double)pv.im != 0.0) && s_zero_pivot == 0) s_zero_pivot = k0 + j + 1;
-            }
-            // multiplier of row pr (held by the thread of column j), shared within the row's 4 lanes
-            CE<T> l = CE<T>{T(0), T(0)};
-            if (pc == (jq >> 1)) l = cmul((jq & 1) ? e1 : e0, cinv(pv));
-            const int src = (lane & ~3) | (jq >> 1);
-            l.re = __shfl_sync(0xffffffffu, l.re, src);
-            l.im = __shfl_sync(0xffffffffu, l.im, src);
-            if (pr > j && pr < m) {
-                const int c0 = j0 + 2 * pc, c1e = c0 + 1;
-                if (c0 == j) {
-                    e0 = l;
-                } else if (c0 > j && c0 < j0 + w) {
-                    const CE<T> u = s_rowp[2 * pc];
-                    e0.re -= l.re * u.re - l.im * u.im;
-                    e0.im -= l.re * u.im + l.im * u.re;
-                }
-                if (c1e == j) {
-                    e1 = l;
-                } else if (c1e > j && c1e < j0 + w) {
-                    const CE<T> u = s_rowp[2 * pc + 1];
-                    e1.re -= l.re * u.re - l.im * u.im;
-                    e1.im -= l.re * u.im + l.im * u.re;
-                }
-            }
-            __syncthreads();  // s_rowj / s_rowp / s_wkey are reused by the next column
-        }
-        // panel back to shared memory; the panel's swaps applied to the other columns
-        if (pr < m) {
-            if (2 * pc < w) S[pr * DIAG_LD + j0 + 2 * pc] = e0;
-            if (2 * pc + 1 < w) S[pr * DIAG_LD + j0 + 2 * pc + 1] = e1;
-        }
-        if (tid < LU_T && (tid < j0 || tid >= j0 + w)) {
-            for (int q = 0; q < w; ++q) {
-                const int ra = j0 + q, rb = s_perm[q];
-                if (rb != ra) {
-                    const CE<T> t = S[ra * DIAG_LD + tid];
-                    S[ra * DIAG_LD + tid] = S[rb * DIAG_LD + tid];
-                    S[rb * DIAG_LD + tid] = t;
-                }
-            }
-        }
-        __syncthreads();
-        const int c1 = j0 + w;  // first column right of the panel
-        if (c1 < m) {
-            // U12 = L11^{-1} A12: rows j0..c1-1, one thread per column
-            for (int c = c1 + tid; c < m; c += blockDim.x) {
-                CE<T> u[DIAG_PW];
-#pragma unroll
-                for (int i = 0; i < DIAG_PW; ++i) {
-                    if (i < w) {
-                        CE<T> v = S[(j0 + i) * DIAG_LD + c];
-#pragma unroll
-                        for (int q = 0; q < i; ++q) {
-                            const CE<T> l = S[(j0 + i) * DIAG_LD + j0 + q];
-                            v.re -= l.re * u[q].re - l.im * u[q].im;
-                            v.im -= l.re * u[q].im + l.im * u[q].re;
-                        }
-                        u[i] = v;
-                        S[(j0 + i) * DIAG_LD + c] = v;
-                    }
-                }
-            }
-            __syncthreads();
-            // A22 -= L21 U12: thread column c1 + (tid & 63), rows (tid >> 6) + 4k
-            const int cc = c1 + (tid & 63);
-            if (cc < m) {
-                CE<T> u[DIAG_PW];
-#pragma unroll
-                for (int q = 0; q < DIAG_PW; ++q)
-                    u[q] = q < w ? S[(j0 + q) * DIAG_LD + cc] : CE<T>{T(0), T(0)};
-                for (int r = c1 + (tid >> 6); r < m; r += 4) {
-                    CE<T> v = S[r * DIAG_LD + cc];
-#pragma unroll
-                    for (int q = 0; q < DIAG_PW; ++q) {
-                        const CE<T> l = S[r * DIAG_LD + j0 + q];
-                        v.re -= l.re * u[q].re - l.im * u[q].im;
-                        v.im -= l.re * u[q].im + l.im * u[q].re;
-                    }
-                    S[r * DIAG_LD + cc] = v;
-                }
-            }
-            __syncthreads();
-        }
-    }
-    if (tid == 0 && s_zero_pivot != 0 && *info == 0) *info = s_zero_pivot;
-    for (int e = tid; e < LU_T * LU_T; e += blockDim.x) {
-        const int r = e / LU_T, cc = e - r * LU_T;
-        if (r < m && cc < m) stE<T, C>(A, (int64_t)(k0 + r) * lda + k0 + cc, S[r * DIAG_LD + cc]);
+        for (int b = 0; b < 4; ++b)
+            if (tx + 16 * b < m) stE<T, C>(A, row + tx + 16 * b, M[a][b]);
     }
 }
-
 
 // Explicit inverses Linv (unit lower) and Uinv (upper) of every factored
 // diagonal block, one CTA per block (blockIdx.x = block), by block
@@ -381,140 +329,110 @@ __global__ void tile_laswp_kernel(T* A, int64_t lda, int n, int k0, int m, const
 // blockIdx.y = 0: U12 tile (rows k0.., 64 columns) <- L11^{-1} tile (unit lower)
 // blockIdx.y = 1: L21 tile (64 rows, columns k0..) <- tile U11^{-1} (upper)
 // Both run in one launch (they touch disjoint parts of A).  The factored
-// diagonal block and the tile are staged in shared memory and the
-// substitution is blocked by APPLY_B rows (mode 0) or columns (mode 1): the
-// block's own triangle is solved by one thread per column (row), sequentially
-// over the APPLY_B entries, then every thread applies the block's rank-APPLY_B
-// update to its entries below (right of) it -- two CTA barriers per block.
+// diagonal block is in shared memory, the tile in registers (thread (ty, tx) of
+// a 16 x 16 grid holds the entries (ty + 16 a, tx + 16 b)); the substitution
+// goes row by row (mode 0) or column by column (mode 1): the owners publish
+// the finished row (column) in one of two buffers, one barrier, and every
+// thread takes it off its entries below (right of) it.  Measured (complex FP32,
+// B200): 22 us a launch against 26 us in blocks of eight out of shared
+// memory, a block's triangle solved by one thread per column.
 constexpr int APPLY_LD = LU_T + 1;
-constexpr int APPLY_B = 8;
-constexpr size_t apply_smem_bytes(size_t elem) { return 2 * elem * LU_T * APPLY_LD; }
+constexpr size_t apply_smem_bytes(size_t elem) { return elem * LU_T * APPLY_LD; }
 
 template <typename T, bool C>
 __global__ void __launch_bounds__(256) tile_apply_kernel(T* A, int64_t lda, int n, int k0, int m) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    CE<T>* M = reinterpret_cast<CE<T>*>(smem_raw);  // [LU_T][APPLY_LD] factored diagonal block
-    CE<T>* X = M + LU_T * APPLY_LD;                 // [LU_T][APPLY_LD] the tile
+    CE<T>* D = reinterpret_cast<CE<T>*>(smem_raw);  // [LU_T][APPLY_LD] factored diagonal block
     __shared__ CE<T> s_rdiag[LU_T];
+    __shared__ CE<T> s_vec[2][LU_T];
     const int mode = blockIdx.y;
     const int base = k0 + m + blockIdx.x * LU_T;  // first column (mode 0) / row (mode 1) of the tile
     const int cnt = min(LU_T, n - base);
-    for (int e = threadIdx.x; e < LU_T * LU_T; e += blockDim.x) {
-        const int r = e / LU_T, c = e - r * LU_T;
-        CE<T> d = CE<T>{T(0), T(0)}, v = CE<T>{T(0), T(0)};
-        if (r < m && c < m) d = ldE<T, C>(A, (int64_t)(k0 + r) * lda + k0 + c);
-        if (mode == 0) {
-            if (r < m && c < cnt) v = ldE<T, C>(A, (int64_t)(k0 + r) * lda + base + c);
-        } else {
-            if (r < cnt && c < m) v = ldE<T, C>(A, (int64_t)(base + r) * lda + k0 + c);
+    const int tid = threadIdx.x;
+    const int tx = tid & 15, ty = tid >> 4;
+    const int rows = mode == 0 ? m : cnt, cols = mode == 0 ? cnt : m;
+    T* tile = A + (C ? 2 : 1) * (mode == 0 ? (int64_t)k0 * lda + base : (int64_t)base * lda + k0);
+    CE<T> X[4][4];
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+            const int r = ty + 16 * a, c = tx + 16 * b;
+            X[a][b] = r < rows && c < cols ? ldE<T, C>(tile, (int64_t)r * lda + c) : CE<T>{T(0), T(0)};
         }
-        M[r * APPLY_LD + c] = d;
-        X[r * APPLY_LD + c] = v;
-    }
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+            const int r = ty + 16 * a, c = tx + 16 * b;
+            const CE<T> d = r < m && c < m ? ldE<T, C>(A, (int64_t)(k0 + r) * lda + k0 + c) : CE<T>{T(0), T(0)};
+            D[r * APPLY_LD + c] = d;
+            if (r == c) s_rdiag[r] = r < m ? cinv(d) : CE<T>{T(0), T(0)};
+        }
     __syncthreads();
-    if (mode == 1 && threadIdx.x < LU_T)
-        s_rdiag[threadIdx.x] = threadIdx.x < m ? cinv(M[threadIdx.x * APPLY_LD + threadIdx.x]) : CE<T>{T(0), T(0)};
-    __syncthreads();
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    const int t = threadIdx.x;
-    for (int b0 = 0; b0 < m; b0 += APPLY_B) {
-        const int bw = min(APPLY_B, m - b0);
-        if (mode == 0) {
-            // rows b0..b0+bw-1: X_b <- L_bb^{-1} X_b, one thread per column
-            if (t < LU_T) {
-                CE<T> y[APPLY_B];
+    if (mode == 0) {
 #pragma unroll
-                for (int i = 0; i < APPLY_B; ++i) {
-                    if (i >= bw) break;
-                    CE<T> v = X[(b0 + i) * APPLY_LD + t];
+        for (int jb = 0; jb < 4; ++jb) {
+            const int je = min(16, m - 16 * jb);
+            for (int jj = 0; jj < je; ++jj) {
+                const int j = 16 * jb + jj;
+                CE<T>* v = s_vec[j & 1];
+                if (ty == jj) {
 #pragma unroll
-                    for (int q = 0; q < i; ++q) {
-                        const CE<T> l = M[(b0 + i) * APPLY_LD + b0 + q];
-                        v.re -= l.re * y[q].re - (C ? l.im * y[q].im : T(0));
-                        if (C) v.im -= l.re * y[q].im + l.im * y[q].re;
+                    for (int b = 0; b < 4; ++b) v[tx + 16 * b] = X[jb][b];
+                }
+                __syncthreads();
+#pragma unroll
+                for (int a = jb; a < 4; ++a) {
+                    const int r = ty + 16 * a;
+                    if (r <= j) continue;
+                    const CE<T> l = D[r * APPLY_LD + j];
+#pragma unroll
+                    for (int b = 0; b < 4; ++b) {
+                        const CE<T> u = v[tx + 16 * b];
+                        X[a][b].re -= l.re * u.re - (C ? l.im * u.im : T(0));
+                        if (C) X[a][b].im -= l.re * u.im + l.im * u.re;
                     }
-                    y[i] = v;
-                    X[(b0 + i) * APPLY_LD + t] = v;
                 }
             }
-            __syncthreads();
-            // rows below the block: X_r -= L_rb X_b
+        }
+    } else {
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int r = ty + 16 * i;
-                if (r < b0 + bw) continue;
-                CE<T> l[APPLY_B];
+        for (int jb = 0; jb < 4; ++jb) {
+            const int je = min(16, m - 16 * jb);
+            for (int jj = 0; jj < je; ++jj) {
+                const int j = 16 * jb + jj;
+                CE<T>* v = s_vec[j & 1];
+                if (tx == jj) {
 #pragma unroll
-                for (int q = 0; q < APPLY_B; ++q)
-                    l[q] = q < bw ? M[r * APPLY_LD + b0 + q] : CE<T>{T(0), T(0)};
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const int c = tx + 16 * j;
-                    CE<T> v = X[r * APPLY_LD + c];
-#pragma unroll
-                    for (int q = 0; q < APPLY_B; ++q) {
-                        if (q >= bw) break;
-                        const CE<T> u = X[(b0 + q) * APPLY_LD + c];
-                        v.re -= l[q].re * u.re - (C ? l[q].im * u.im : T(0));
-                        if (C) v.im -= l[q].re * u.im + l[q].im * u.re;
+                    for (int a = 0; a < 4; ++a) {
+                        X[a][jb] = cmul(X[a][jb], s_rdiag[j]);
+                        v[ty + 16 * a] = X[a][jb];
                     }
-                    X[r * APPLY_LD + c] = v;
+                }
+                __syncthreads();
+#pragma unroll
+                for (int b = jb; b < 4; ++b) {
+                    const int c = tx + 16 * b;
+                    if (c <= j) continue;
+                    const CE<T> u = D[j * APPLY_LD + c];
+#pragma unroll
+                    for (int a = 0; a < 4; ++a) {
+                        const CE<T> l = v[ty + 16 * a];
+                        X[a][b].re -= l.re * u.re - (C ? l.im * u.im : T(0));
+                        if (C) X[a][b].im -= l.re * u.im + l.im * u.re;
+                    }
                 }
             }
-            __syncthreads();
-        } else {
-            // columns b0..b0+bw-1: X_b <- X_b U_bb^{-1}, one thread per row
-            if (t < LU_T) {
-                CE<T> y[APPLY_B];
-#pragma unroll
-                for (int j = 0; j < APPLY_B; ++j) {
-                    if (j >= bw) break;
-                    CE<T> v = X[t * APPLY_LD + b0 + j];
-#pragma unroll
-                    for (int q = 0; q < j; ++q) {
-                        const CE<T> u = M[(b0 + q) * APPLY_LD + b0 + j];
-                        v.re -= y[q].re * u.re - (C ? y[q].im * u.im : T(0));
-                        if (C) v.im -= y[q].re * u.im + y[q].im * u.re;
-                    }
-                    y[j] = cmul(v, s_rdiag[b0 + j]);
-                    X[t * APPLY_LD + b0 + j] = y[j];
-                }
-            }
-            __syncthreads();
-            // columns right of the block: X_c -= X_b U_bc
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const int c = tx + 16 * j;
-                if (c < b0 + bw) continue;
-                CE<T> u[APPLY_B];
-#pragma unroll
-                for (int q = 0; q < APPLY_B; ++q)
-                    u[q] = q < bw ? M[(b0 + q) * APPLY_LD + c] : CE<T>{T(0), T(0)};
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const int r = ty + 16 * i;
-                    CE<T> v = X[r * APPLY_LD + c];
-#pragma unroll
-                    for (int q = 0; q < APPLY_B; ++q) {
-                        if (q >= bw) break;
-                        const CE<T> l = X[r * APPLY_LD + b0 + q];
-                        v.re -= l.re * u[q].re - (C ? l.im * u[q].im : T(0));
-                        if (C) v.im -= l.re * u[q].im + l.im * u[q].re;
-                    }
-                    X[r * APPLY_LD + c] = v;
-                }
-            }
-            __syncthreads();
         }
     }
-    for (int e = threadIdx.x; e < LU_T * LU_T; e += blockDim.x) {
-        const int r = e / LU_T, c = e - r * LU_T;
-        if (mode == 0) {
-            if (r < m && c < cnt) stE<T, C>(A, (int64_t)(k0 + r) * lda + base + c, X[r * APPLY_LD + c]);
-        } else {
-            if (r < cnt && c < m) stE<T, C>(A, (int64_t)(base + r) * lda + k0 + c, X[r * APPLY_LD + c]);
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+            const int r = ty + 16 * a, c = tx + 16 * b;
+            if (r < rows && c < cols) stE<T, C>(tile, (int64_t)r * lda + c, X[a][b]);
         }
-    }
 }
 
 // --------------------------------------------------------------------------
@@ -907,9 +825,7 @@ template <typename T, bool C>
 int factor_t(bem_ctx* ctx, T* A, int64_t n, int64_t lda, int32_t* piv, CE<T>* dinv, int32_t* info,
              cudaStream_t s) {
     cudaMemsetAsync(info, 0, sizeof(int32_t), s);
-    const size_t dsmem = diag_smem_bytes(sizeof(CE<T>));
     const size_t asmem = apply_smem_bytes(sizeof(CE<T>));
-    cudaFuncSetAttribute(tile_diag_kernel<T, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dsmem);
     const size_t ismem = inv_smem_bytes(sizeof(CE<T>));
     cudaFuncSetAttribute(tile_inv_kernel<T, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ismem);
     cudaFuncSetAttribute(tile_apply_kernel<T, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)asmem);
@@ -926,7 +842,7 @@ int factor_t(bem_ctx* ctx, T* A, int64_t n, int64_t lda, int32_t* piv, CE<T>* di
     auto diag_aside = [&](int64_t k0) {
         cudaEventRecord(ctx->ev_next, s);
         cudaStreamWaitEvent(ctx->aux, ctx->ev_next, 0);
-        tile_diag_kernel<T, C><<<1, 256, dsmem, ctx->aux>>>(A, lda, ni, (int)k0, piv, info);
+        tile_diag_kernel<T, C><<<1, 256, 0, ctx->aux>>>(A, lda, ni, (int)k0, piv, info);
         cudaEventRecord(ctx->ev_diag, ctx->aux);
         ctx->launches++;
     };
@@ -948,7 +864,7 @@ int factor_t(bem_ctx* ctx, T* A, int64_t n, int64_t lda, int32_t* piv, CE<T>* di
     // the read-modify-write traffic of the trailing GEMMs).  The update's first
     // tile column goes first so that the next pair's diagonal tile overlaps the
     // rest of it.
-    tile_diag_kernel<T, C><<<1, 256, dsmem, s>>>(A, lda, ni, 0, piv, info);
+    tile_diag_kernel<T, C><<<1, 256, 0, s>>>(A, lda, ni, 0, piv, info);
     ctx->launches++;
     bool on_aux = false;
     for (int64_t k0 = 0; k0 < n; k0 += 2 * LU_T) {

@@ -282,3 +282,43 @@ def test_near_pairs_orders_and_batches(engine, op, nbx, nby, Q, quirk):
                               outs, [1.0] * count)
         for o, w in zip(outs, want):
             assert np.abs(o.cpu().numpy() - w).max() < 1e-12 * np.abs(w).max()
+
+
+# ---- tile-pivoted LU -------------------------------------------------------------------------
+@pytest.mark.parametrize("dtype", ["float32", "complex64", "float64", "complex128"])
+@pytest.mark.parametrize("n", [1, 15, 16, 17, 63, 64, 65, 100, 128, 191, 330])
+def test_tile_lu_sizes(engine, n, dtype):
+    """P A = L U with row swaps inside each 64-row tile, |l| <= sqrt 2 inside
+    the diagonal tiles, and the tile's first pivot the largest |re| + |im| of
+    its first column.  A diagonally dominant random matrix keeps the factors
+    of the size of A: n eps max|A|, times 8 for the split TF32 products."""
+    cplx = dtype.startswith("complex")
+    A = _gaussian((n, n), cplx, n + 1) / np.sqrt(n) + 2.0 * np.eye(n)
+    LU = torch.as_tensor(A, device="cuda").to(getattr(torch, dtype)).contiguous()
+    A = LU.cpu().numpy().astype(np.complex128 if cplx else np.float64)
+    piv, _, info = engine.lu_factor_tiled(LU)
+    assert int(info.item()) == 0
+    F = LU.cpu().numpy().astype(A.dtype)
+    piv = piv.cpu().numpy()
+    tile = np.arange(n) // 64 * 64
+    assert ((piv >= np.arange(n)) & (piv < np.minimum(tile + 64, n))).all()
+    first = A[:64, 0]
+    assert piv[0] == int(np.argmax(np.abs(first.real) + np.abs(first.imag)))
+    low, up = np.tril(F, -1) + np.eye(n), np.triu(F)
+    for t in range(0, n, 64):
+        assert np.abs(low[t:t + 64, t:t + 64]).max() <= 1.4143
+    assert np.abs(_swapped(A, piv) - low @ up).max() < 8 * max(n, 16) * _EPS[dtype] * np.abs(A).max()
+
+
+@pytest.mark.parametrize("col", [0, 20, 63, 64, 90])
+def test_tile_lu_zero_and_nan_columns(engine, col):
+    A = torch.eye(100, dtype=torch.float32, device="cuda") * 2.0
+    A[col, col] = 0.0
+    _, _, info = engine.lu_factor_tiled(A)
+    assert int(info.item()) == col + 1
+    if col % 64 < 60 and col + 3 < 100:
+        A = torch.eye(100, dtype=torch.float32, device="cuda") * 2.0
+        A[col, col] = float("nan")
+        A[col + 3, col] = 1.0
+        piv, _, _ = engine.lu_factor_tiled(A)
+        assert int(piv[col].item()) == col + 3
