@@ -322,3 +322,43 @@ def test_tile_lu_zero_and_nan_columns(engine, col):
         A[col + 3, col] = 1.0
         piv, _, _ = engine.lu_factor_tiled(A)
         assert int(piv[col].item()) == col + 3
+
+
+# ---- FP64 tensor-core products --------------------------------------------------------------
+@pytest.mark.parametrize("cplx", [False, True])
+@pytest.mark.parametrize("conj_a,conj_b", [(False, False), (False, True), (True, False), (True, True)])
+@pytest.mark.parametrize("m,n,k", [(1, 1, 1), (63, 65, 7), (64, 64, 8), (130, 66, 33), (65, 129, 200), (70, 70, 1100)])
+def test_gemm_edges(engine, m, n, k, conj_a, conj_b, cplx):
+    """C += alpha op(A) op(B) with leading dimensions beyond the widths, tiles
+    and stages partly filled, fewer stages than the ring, split K (k = 1100):
+    k eps max|A| max|B| sqrt-ish sums, 1e-13 k of the result."""
+    dt = torch.complex128 if cplx else torch.float64
+
+    def padded(r, c, seed):
+        return torch.as_tensor(_gaussian((r, c + 3), cplx, seed), device="cuda", dtype=dt)[:, :c]
+
+    A, B, C = padded(*((k, m) if conj_a else (m, k)), 1), padded(*((n, k) if conj_b else (k, n)), 2), padded(m, n, 3)
+    opA, opB = (X.conj().T if c else X for X, c in ((A, conj_a), (B, conj_b)))
+    want = (C + 0.75 * opA @ opB).cpu().numpy()
+    engine.gemm(A, B, C, alpha=0.75, conj_a=conj_a, conj_b=conj_b)
+    assert np.abs(C.cpu().numpy() - want).max() < 1e-13 * max(k, 8) ** 0.5 * 10
+
+
+def test_gemm_on_unaligned_complex_operands(engine):
+    """Complex operands that start on an odd multiple of 8 bytes take 8-byte
+    copies."""
+    n = 70
+    raw = torch.zeros(2 * n * n + 1, dtype=torch.float64, device="cuda")
+    raw[1:] = torch.as_tensor(_gaussian((2 * n * n,), False, 4), device="cuda")
+    A = torch.as_tensor(_gaussian((n, n), True, 5), device="cuda")
+    C = torch.zeros(n, n, dtype=torch.complex128, device="cuda")
+    L = engine.lib
+    import ctypes
+    from bem_b200 import _lib
+    rc = L.bem_gemm(engine.ctx, _lib.C128, 0, 0, 0, n, n, n, 1.0, ctypes.c_void_p(raw.data_ptr() + 8), n,
+                    ctypes.c_void_p(A.data_ptr()), n, ctypes.c_void_p(C.data_ptr()), n,
+                    ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+    assert rc == 0
+    B = raw[1:].cpu().numpy().reshape(n, n, 2)
+    want = (B[..., 0] + 1j * B[..., 1]) @ A.cpu().numpy()
+    assert np.abs(C.cpu().numpy() - want).max() < 1e-12 * 10
