@@ -102,8 +102,9 @@ int64_t bem_launch_count(const bem_ctx* ctx);
  * autotuner (bem_b200/tuning.py) after timing the candidates on this GPU;
  * value 0 restores the built-in default.  Keys:
  *   BEM_TUNE_CALDERON_GROUP  form of the fused Calderon sweep: 1 scalar, one
- *                            wavenumber per launch; 2 scalar, both in one
- *                            launch (the default for two wavenumbers); 3 packed
+ *                            wavenumber per launch; 2 both in one launch, over
+ *                            lane pairs for Helmholtz (the default for two
+ *                            wavenumbers); 3 packed
  *                            FP32x2 over test points, one wavenumber per
  *                            launch (the default of a single-wavenumber mixed
  *                            Helmholtz sweep); 4 both wavenumbers packed into

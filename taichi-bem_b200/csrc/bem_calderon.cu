@@ -791,6 +791,250 @@ __global__ void __launch_bounds__(FAR_THREADS, SM ? 3 : 1) far_calderon_k2_kerne
     }
 }
 
+// Both wavenumbers of the Helmholtz sweep over the two lanes of a lane pair
+// (lane 2p: k[0], lane 2p + 1: k[1]) that share a trial panel.  With both in
+// one thread the 60 FP64 moments take 120 registers and two CTAs fill an SM;
+// one thread per wavenumber alone would evaluate the geometry twice.  Here each
+// lane evaluates the geometry of every second test point and the pair exchanges
+// it (five shuffles each way), so a lane does half the geometry, its own
+// wavenumber's phase, sine and cosine, and carries 30 moments.  FP32: a point
+// pair (q, q + 1) runs packed through the phase and the products, and the sums
+// take q, then q + 1, so every value and its rounding is that of
+// far_calderon_kernel<float, 2, true, PH>.  FP64: the phase relative to the
+// centroid distance, as in the other FP64 sweeps.  An odd Q^2 is padded by a
+// copy of the last point with weight 0 (it adds exact zeros).
+//   Assembly of both block systems, against both wavenumbers in one scalar
+// thread (60 moments): FP64 48.3 -> 33.7 ms (5120 panels, Q = 6, k = 5 / 7.5)
+// and 9.8 -> 8.8 ms (2070 panels); mixed 22.2 -> 21.4 and 5.2 -> 5.0 ms (one
+// launch per wavenumber: 52.0 ms FP64, 25.6 ms mixed).  The FP32 form issues 120 instructions per
+// warp and evaluation with the FMA pipe at 48 %: what is left are the FP64
+// moments, the exchange and the latency between them.  Four CTAs of the FP32
+// form per SM cost registers (22.3 ms); fetching the next points early did not
+// pay either (24 to 25 ms).
+template <typename T, int PH>
+__global__ void __launch_bounds__(FAR_THREADS, 3) far_calderon_pair_kernel(CalArgs a) {
+    using V4 = typename V4T<T>::type;
+    constexpr bool SPLIT = sizeof(T) == 4;
+    constexpr unsigned FULL = 0xffffffffu;
+    const int Q2 = a.Q2, QP = (Q2 + 1) / 2;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    V4* sx = reinterpret_cast<V4*>(smem_raw);              // [FAR_TI][2 QP] test points
+    V4* sp = reinterpret_cast<V4*>(sx + FAR_TI * 2 * QP);  // [QP] (phi_1, phi_1', phi_2, phi_2') of a point pair
+    __shared__ int s_gi[FAR_TI];
+    __shared__ int s_tri[FAR_TI][3];
+    __shared__ double s_cen[FAR_TI][3];
+    __shared__ double s_nrm[FAR_TI][3];
+
+    const int n = a.n;
+    const int j0 = blockIdx.x * (FAR_THREADS / 2);
+    const int li0 = blockIdx.y * FAR_TI;
+    if (j0 + FAR_THREADS / 2 - 1 <= li0) return;  // tile strictly below the diagonal
+    const int lj = j0 + (threadIdx.x >> 1), w = threadIdx.x & 1;
+    const int even = threadIdx.x & 30;  // the pair's first lane
+    const V4* pts = reinterpret_cast<const V4*>(a.pts);
+    {
+        const T* phi = reinterpret_cast<const T*>(a.phi);
+        for (int p = threadIdx.x; p < QP; p += FAR_THREADS) {
+            const int q1 = 2 * p + 1 < Q2 ? 2 * p + 1 : Q2 - 1;
+            V4 v;
+            v.x = phi[6 * p + 1];
+            v.y = phi[3 * q1 + 1];
+            v.z = phi[6 * p + 2];
+            v.w = phi[3 * q1 + 2];
+            sp[p] = v;
+        }
+    }
+    if (threadIdx.x < FAR_TI) {
+        const int li = li0 + threadIdx.x;
+        const int gi = li < n ? a.panels[li] : -1;
+        s_gi[threadIdx.x] = gi;
+        for (int c = 0; c < 3; ++c) {
+            s_tri[threadIdx.x][c] = gi >= 0 ? a.tris[3 * gi + c] : -1;
+            s_cen[threadIdx.x][c] = gi >= 0 ? a.centroid[3 * gi + c] : 0.0;
+            s_nrm[threadIdx.x][c] = gi >= 0 ? a.normal[3 * gi + c] : 0.0;
+        }
+    }
+    __syncthreads();
+    for (int idx = threadIdx.x; idx < FAR_TI * 2 * QP; idx += FAR_THREADS) {
+        const int t = idx / (2 * QP), q = idx - t * 2 * QP;
+        if (li0 + t >= n) continue;
+        V4 v = pts[(size_t)s_gi[t] * Q2 + (q < Q2 ? q : Q2 - 1)];
+        if (q >= Q2) v.w = T(0);
+        sx[idx] = v;
+    }
+    __syncthreads();
+
+    const bool valid_j = lj < n;
+    const int gj = valid_j ? a.panels[lj] : 0;
+    int tri_j[3];
+    double cen_j[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        tri_j[c] = a.tris[3 * gj + c];
+        cen_j[c] = a.centroid[3 * gj + c];
+    }
+    const double nj64[3] = {a.normal[3 * gj + 0], a.normal[3 * gj + 1], a.normal[3 * gj + 2]};
+    const V4* ptsj = pts + (size_t)gj * Q2;
+    const T kk = T(w ? a.k[1] : a.k[0]);
+
+    for (int t = 0; t < FAR_TI; ++t) {
+        const int li = li0 + t;
+        if (li >= n) break;  // uniform across the CTA
+        const int gi = s_gi[t];
+        const bool sep = valid_j && li < lj && (bem_relation(s_tri[t], tri_j, gi == gj) == REL_SEPARATE);
+        // the pairs of a warp go together (the exchange is a warp's); one that is
+        // not separate evaluates values that nobody reads
+        if (!__any_sync(FULL, sep)) continue;
+        const double Dx = s_cen[t][0] - cen_j[0], Dy = s_cen[t][1] - cen_j[1], Dz = s_cen[t][2] - cen_j[2];
+        const double ni64[3] = {s_nrm[t][0], s_nrm[t][1], s_nrm[t][2]};
+        const T dcx = T(Dx), dcy = T(Dy), dcz = T(Dz);
+        const T ux = T(2.0 * Dx), uy = T(2.0 * Dy), uz = T(2.0 * Dz);
+        const double R2d = Dx * Dx + Dy * Dy + Dz * Dz;
+        const T R2 = T(R2d);
+        const double Rd = sqrt(R2d);
+        const T Rf = T(Rd);
+        const double pf = SPLIT ? 4.0 * a.area[gi] * a.area[gj] * a.wcorr : 1.0;
+        const double phR = (w ? a.k[1] : a.k[0]) * Rd;  // FP64: the phase is relative to this very value
+        const T Dnj = T(Dx * nj64[0] + Dy * nj64[1] + Dz * nj64[2]);
+        const double Dni64 = Dx * ni64[0] + Dy * ni64[1] + Dz * ni64[2];
+        // FP32: n_j - n_i (x_a.n_j = x_a.(n_j - n_i)); FP64: n_j itself
+        const T mx = T(SPLIT ? nj64[0] - ni64[0] : nj64[0]), my = T(SPLIT ? nj64[1] - ni64[1] : nj64[1]),
+                mz = T(SPLIT ? nj64[2] - ni64[2] : nj64[2]);
+        const V4* sxt = sx + t * 2 * QP;
+
+        double Mr[15], Mi[15];  // moments as in far_calderon_kernel
+#pragma unroll
+        for (int m = 0; m < 15; ++m) Mr[m] = Mi[m] = 0.0;
+
+        for (int b = 0; b < Q2; ++b) {
+            const V4 yb = ptsj[b];
+            const T ex = dcx - yb.x, ey = dcy - yb.y, ez = dcz - yb.z;
+            const T wx = ux - yb.x, wy = uy - yb.y, wz = uz - yb.z;
+            T sr[7], si[7];
+#pragma unroll
+            for (int m = 0; m < 7; ++m) sr[m] = si[m] = T(0);
+#pragma unroll 2
+            for (int p = 0; p < QP; ++p) {
+                const V4 xa = sxt[2 * p + w];
+                const V4 pp = sp[p];
+                T r, rinv, ph;
+                if constexpr (SPLIT) {
+                    const T e_x = xa.x - yb.x, e_y = xa.y - yb.y, e_z = xa.z - yb.z;
+                    const T sq = e_x * (xa.x + wx) + e_y * (xa.y + wy) + e_z * (xa.z + wz);
+                    dev_r_rinv(R2 + sq, r, rinv);
+                    ph = __fdividef(sq, r + Rf);
+                } else {
+                    const T dx = xa.x + ex, dy = xa.y + ey, dz = xa.z + ez;
+                    dev_r_rinv(fma(dx, dx, fma(dy, dy, dz * dz)), r, rinv);
+                    ph = r;
+                }
+                const T dnj = fma(xa.x, mx, fma(xa.y, my, fma(xa.z, mz, Dnj)));
+                const T wr = xa.w * rinv;
+                const T wr3 = wr * (rinv * rinv);
+                const T tj = wr3 * dnj;
+                // geometry of both points of the pair
+                const T r0 = __shfl_sync(FULL, r, even), r1 = __shfl_sync(FULL, r, even + 1);
+                const T wr0 = __shfl_sync(FULL, wr, even), wr1 = __shfl_sync(FULL, wr, even + 1);
+                const T w30 = __shfl_sync(FULL, wr3, even), w31 = __shfl_sync(FULL, wr3, even + 1);
+                const T tj0 = __shfl_sync(FULL, tj, even), tj1 = __shfl_sync(FULL, tj, even + 1);
+                if constexpr (SPLIT) {
+                    const float ph0 = __shfl_sync(FULL, ph, even), ph1 = __shfl_sync(FULL, ph, even + 1);
+                    const float2 K2 = f2(kk), N2 = f2(-kk);
+                    const float2 y = fmul2(K2, make_float2(ph0, ph1)), rr = make_float2(r0, r1);
+                    float2 sn, cs;
+                    if (PH != 0) {
+                        dev_sincos_poly2<false>(y, sn, cs);
+                    } else {
+                        dev_sincos(y.x, &sn.x, &cs.x);
+                        dev_sincos(y.y, &sn.y, &cs.y);
+                    }
+                    const float2 wv = make_float2(wr0, wr1), w3 = make_float2(w30, w31);
+                    const float2 gr = fmul2(wv, cs), gm = fmul2(wv, sn);
+                    const float2 fr = ffma2(fmul2(K2, rr), sn, cs), fi = ffma2(fmul2(N2, rr), cs, sn);
+                    const float2 hr = fmul2(w3, fr), hi = fmul2(w3, fi);
+                    sr[0] = __fadd_rn(__fadd_rn(sr[0], gr.x), gr.y);
+                    si[0] = __fadd_rn(__fadd_rn(si[0], gm.x), gm.y);
+                    sr[1] = fmaf(pp.y, gr.y, fmaf(pp.x, gr.x, sr[1]));
+                    si[1] = fmaf(pp.y, gm.y, fmaf(pp.x, gm.x, si[1]));
+                    sr[2] = fmaf(pp.w, gr.y, fmaf(pp.z, gr.x, sr[2]));
+                    si[2] = fmaf(pp.w, gm.y, fmaf(pp.z, gm.x, si[2]));
+                    sr[3] = fmaf(tj1, fr.y, fmaf(tj0, fr.x, sr[3]));
+                    si[3] = fmaf(tj1, fi.y, fmaf(tj0, fi.x, si[3]));
+                    sr[4] = __fadd_rn(__fadd_rn(sr[4], hr.x), hr.y);
+                    si[4] = __fadd_rn(__fadd_rn(si[4], hi.x), hi.y);
+                    sr[5] = fmaf(pp.y, hr.y, fmaf(pp.x, hr.x, sr[5]));
+                    si[5] = fmaf(pp.y, hi.y, fmaf(pp.x, hi.x, si[5]));
+                    sr[6] = fmaf(pp.w, hr.y, fmaf(pp.z, hr.x, sr[6]));
+                    si[6] = fmaf(pp.w, hi.y, fmaf(pp.z, hi.x, si[6]));
+                } else {
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const T rh = h ? r1 : r0, wv = h ? wr1 : wr0, w3 = h ? w31 : w30, tv = h ? tj1 : tj0;
+                        const T p1 = h ? pp.y : pp.x, p2 = h ? pp.w : pp.z;
+                        double sn, cs;
+                        dev_sincos_ph<PH>(fma(kk, rh, -phR), &sn, &cs);
+                        const double kr = kk * rh;
+                        const double gr = wv * cs, gm = wv * sn;
+                        const double fr = fma(kr, sn, cs), fi = fma(-kr, cs, sn);
+                        const double hr = w3 * fr, hi = w3 * fi;
+                        sr[0] += gr;
+                        si[0] += gm;
+                        sr[1] = fma(p1, gr, sr[1]);
+                        si[1] = fma(p1, gm, si[1]);
+                        sr[2] = fma(p2, gr, sr[2]);
+                        si[2] = fma(p2, gm, si[2]);
+                        sr[3] = fma(tv, fr, sr[3]);
+                        si[3] = fma(tv, fi, si[3]);
+                        sr[4] += hr;
+                        si[4] += hi;
+                        sr[5] = fma(p1, hr, sr[5]);
+                        si[5] = fma(p1, hi, si[5]);
+                        sr[6] = fma(p2, hr, sr[6]);
+                        si[6] = fma(p2, hi, si[6]);
+                    }
+                }
+            }
+            const double wb = double(yb.w);
+            const double wb1 = wb * a.phi64[3 * b + 1], wb2 = wb * a.phi64[3 * b + 2];
+            // -d.n_i = -(D.n_i - y_b.n_i), constant over the test points
+            const double wbn =
+                wb * -(Dni64 - (double(yb.x) * ni64[0] + double(yb.y) * ni64[1] + double(yb.z) * ni64[2]));
+            auto add = [&](int m, double f, int s) {
+                Mr[m] += f * double(sr[s]);
+                Mi[m] += f * double(si[s]);
+            };
+            add(0, wb, 0);
+            add(1, wb, 3);
+            add(2, wb1, 3);
+            add(3, wb2, 3);
+            add(4, wbn, 4);
+            add(5, wbn, 5);
+            add(6, wbn, 6);
+            add(7, wb1, 0);
+            add(8, wb2, 0);
+            add(9, wb, 1);
+            add(10, wb1, 1);
+            add(11, wb2, 1);
+            add(12, wb, 2);
+            add(13, wb1, 2);
+            add(14, wb2, 2);
+        }
+        if (sep) calderon_epilogue<true>(a, w, li, lj, gi, gj, ni64, nj64, pf, Rd, Mr, Mi, true);
+        __syncwarp();
+    }
+}
+
+template <typename T, int PH>
+int launch_calderon_pair(bem_ctx* ctx, const CalArgs& a, cudaStream_t s) {
+    dim3 grid((a.n + FAR_THREADS / 2 - 1) / (FAR_THREADS / 2), (a.n + FAR_TI - 1) / FAR_TI);
+    if (grid.y > 65535) return bem_fail(ctx, BEM_ERR_INVALID, "calderon: too many panels for one launch");
+    const int QP = (a.Q2 + 1) / 2;
+    const size_t smem = (size_t)(FAR_TI * 2 * QP + QP) * sizeof(typename V4T<T>::type);
+    far_calderon_pair_kernel<T, PH><<<grid, FAR_THREADS, smem, s>>>(a);
+    ctx->launches++;
+    return bem_check_cuda(ctx, cudaGetLastError(), "far_calderon_pair_kernel launch");
+}
+
 template <int PH, bool SM>
 int launch_calderon_k2(bem_ctx* ctx, const CalArgs& a, cudaStream_t s) {
     dim3 grid((a.n + FAR_THREADS - 1) / FAR_THREADS, (a.n + FAR_TI - 1) / FAR_TI);
@@ -827,13 +1071,11 @@ int launch_calderon_x2(bem_ctx* ctx, const CalArgs& a, cudaStream_t s) {
     return bem_check_cuda(ctx, cudaGetLastError(), "far_calderon_x2_kernel launch");
 }
 
-template <int NK>
-int dispatch_calderon(bem_ctx* ctx, const CalArgs& a, bool fp32, bool helm, cudaStream_t s) {
-    if (!fp32)
-        return helm ? launch_calderon<double, NK, true, 0>(ctx, a, s) : launch_calderon<double, NK, false, 0>(ctx, a, s);
-    if (!helm) return launch_calderon<float, NK, false, 0>(ctx, a, s);
-    if (a.small_phase != 0) return launch_calderon<float, NK, true, 1>(ctx, a, s);
-    return launch_calderon<float, NK, true, 0>(ctx, a, s);
+// one launch for the first wavenumber in `a`
+int launch_calderon_one(bem_ctx* ctx, const CalArgs& a, bool fp32, bool helm, cudaStream_t s) {
+    if (!fp32) return helm ? launch_calderon<double, 1, true, 0>(ctx, a, s) : launch_calderon<double, 1, false, 0>(ctx, a, s);
+    if (!helm) return launch_calderon<float, 1, false, 0>(ctx, a, s);
+    return a.small_phase ? launch_calderon<float, 1, true, 1>(ctx, a, s) : launch_calderon<float, 1, true, 0>(ctx, a, s);
 }
 
 }  // namespace
@@ -893,11 +1135,10 @@ extern "C" int bem_assemble_calderon(bem_ctx* ctx, const bem_op_desc* op, int nk
         a.out[w] = (double*)out[w];
     }
     a.ld = ld;
-    // default with two wavenumbers: both in one scalar launch (measured on the
-    // 20480-panel transmission problem: FP64 1602 vs 1736 ms for one launch
-    // per wavenumber; mixed 656 ms, against 802 ms scalar and 750 ms packed
-    // FP32x2 per wavenumber); with one wavenumber the packed sweep is the
-    // mixed Helmholtz default
+    // default with two wavenumbers: both over lane pairs (Helmholtz; figures at
+    // far_calderon_pair_kernel) or in one scalar launch (Laplace); with one
+    // wavenumber the packed sweep is the mixed Helmholtz default (two of
+    // them on 20480 panels: 750 ms, against 802 ms scalar)
     int rc = BEM_OK;
     const int variant = ctx->tune[BEM_TUNE_CALDERON_GROUP];
     if (fp32 && helm && nk == 2 && variant == 4) {
@@ -921,8 +1162,17 @@ extern "C" int bem_assemble_calderon(bem_ctx* ctx, const bem_op_desc* op, int nk
             rc = phase_class == 2 ? launch_calderon_x2<2>(ctx, b, s)
                                   : (phase_class == 1 ? launch_calderon_x2<1>(ctx, b, s) : launch_calderon_x2<0>(ctx, b, s));
         }
+    } else if (helm && nk == 2 && variant != 1) {
+        // both wavenumbers over lane pairs
+        const int ph = fp32 ? a.small_phase : bem_phase_class(kmax * 2.0 * ctx->rho_max);
+        if (fp32)
+            rc = ph ? launch_calderon_pair<float, 1>(ctx, a, s) : launch_calderon_pair<float, 0>(ctx, a, s);
+        else
+            rc = ph == 2 ? launch_calderon_pair<double, 2>(ctx, a, s)
+                         : (ph == 1 ? launch_calderon_pair<double, 1>(ctx, a, s)
+                                    : launch_calderon_pair<double, 0>(ctx, a, s));
     } else if (nk == 2 && variant != 1) {
-        rc = dispatch_calderon<2>(ctx, a, fp32, helm, s);
+        rc = fp32 ? launch_calderon<float, 2, false, 0>(ctx, a, s) : launch_calderon<double, 2, false, 0>(ctx, a, s);
     } else {
         for (int w = 0; w < nk && !rc; ++w) {
             CalArgs b = a;
@@ -930,7 +1180,7 @@ extern "C" int bem_assemble_calderon(bem_ctx* ctx, const bem_op_desc* op, int nk
             b.k2[0] = a.k2[w];
             b.coef[0] = a.coef[w];
             b.out[0] = a.out[w];
-            rc = dispatch_calderon<1>(ctx, b, fp32, helm, s);
+            rc = launch_calderon_one(ctx, b, fp32, helm, s);
         }
     }
     // join: the caller's stream waits for the near-pair kernels

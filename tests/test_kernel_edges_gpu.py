@@ -362,3 +362,39 @@ def test_gemm_on_unaligned_complex_operands(engine):
     B = raw[1:].cpu().numpy().reshape(n, n, 2)
     want = (B[..., 0] + 1j * B[..., 1]) @ A.cpu().numpy()
     assert np.abs(C.cpu().numpy() - want).max() < 1e-12 * 10
+
+
+# ---- both wavenumbers of the Calderon sweep over lane pairs ---------------------------
+@pytest.mark.parametrize("ks", [(0.1, 0.05), (1.2, 0.4), (30.0, 45.0), (0.7, -0.3)])
+@pytest.mark.parametrize("Q", [1, 2, 3])
+def test_calderon_lane_pairs(engine, ks, Q):
+    """Odd and even numbers of points and the phase classes (<= 0.3, <= pi/4,
+    reduced), over a part of the panels in no order.  FP64 against one
+    launch per wavenumber, sums in another order: 1e-12 of the largest entry;
+    mixed: the same FP32 values and sums, the FP64 ones in another order
+    (atomics): 1e-12 too."""
+    from bem_b200 import _lib as L
+    from bem_b200 import icosphere
+    from bem_b200.engine import DeviceSpace
+    from oracle import oracle as O
+    v, f = icosphere(2)
+    engine.set_mesh(v, f, Q)
+    panels, _, dof = _partial_space(f, len(v), 1, 233, 5)
+    dof3 = f[panels].astype(np.int32)
+    dof3[np.random.default_rng(6).random(dof3.shape) < 0.03] = -1
+    dof3[dof3 >= 0] += len(f)
+    n = len(f) + len(v)
+    neu = DeviceSpace.from_numpy(panels, 1, dof, engine.device)
+    dirs = DeviceSpace.from_numpy(panels, 3, np.ascontiguousarray(dof3.reshape(-1)), engine.device)
+    for prec in (L.PREC_FP64, L.PREC_MIXED):
+        desc = engine.op_desc(O.OP_V, True, ks[0], ks[0] ** 2, precision=prec)
+        got = []
+        for form in (1, 0):
+            engine.set_tuning(L.TUNE_CALDERON_GROUP, form)
+            outs = [torch.zeros(n, n, dtype=torch.complex128, device="cuda") for _ in ks]
+            engine.assemble_calderon(desc, ks, [k * k for k in ks], neu, dirs, outs, (-1.0, 0.7))
+            got.append(outs)
+        engine.set_tuning(L.TUNE_CALDERON_GROUP, 0)
+        for want, out in zip(*got):
+            assert float(want.abs().max()) > 0
+            assert float((want - out).abs().max()) < 1e-12 * float(want.abs().max())
