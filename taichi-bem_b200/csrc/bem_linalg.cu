@@ -347,29 +347,34 @@ __global__ void __launch_bounds__(256) lu_panel_kernel(T* A, int64_t lda, int n,
 // PCL_SB columns of it in registers, and per column
 //   * each CTA reduces its pivot candidate (largest |re| + |im|, lowest
 //     position) and pushes value, position and the candidate's PCL_SB
-//     elements into every CTA's mailbox (distributed shared memory);
-//   * one cluster barrier; every CTA takes the best of the mailboxes and
-//     updates its rows' registers.
+//     elements into every CTA's mailbox (distributed shared memory, st.async
+//     counted by the mailbox's mbarrier: a CTA goes on when all candidates
+//     have arrived, without the round trip of a cluster barrier);
+//   * every CTA takes the best of the mailboxes and updates its rows'
+//     registers; the pivot row's CTA pushes the row's remaining elements.
+// A mailbox or U row is written again only by a CTA that has received a later
+// candidate of this one, which was sent after this one read the old contents.
 // Rows never move: a row carries its position, the row at the diagonal
 // position takes the pivot's, and the panel is written out by position (the
 // swap sequence in piv is that of moved rows).  After a sub-block the pivot
-// rows' remaining elements are pushed to every CTA, solved against the
-// sub-block's unit lower triangle and applied as one rank-PCL_SB update, so
-// shared memory is swept once per PCL_SB columns (FP64: on the FP64 tensor
+// rows' remaining elements are solved against the sub-block's unit lower
+// triangle and applied as one rank-PCL_SB update, so shared memory is swept once per PCL_SB columns (FP64: on the FP64 tensor
 // cores).  Measured (B200, a column step averaged over a whole factorisation):
-// 2999 complex rows 1.95 us against 6.0 us of the cooperative kernel below (a
-// grid barrier a column), 1280 real rows 1.73 against 5.8 us.
+// 2999 complex rows 1.62 us (6.0 us of the cooperative kernel below, a grid
+// barrier a column; 1.95 with a cluster barrier a column and the panel read
+// through registers), 1280 real rows 1.31 us (5.8; 1.73).
 // ----------------------------------------------------------------------------
 constexpr int PCL_SB = 8;
 constexpr int PCL_MAXC = 16;
+constexpr uint32_t PCL_SPIN_CAP = 1u << 20;
 
 // A pivot candidate as integers that order like the rule "largest value,
 // then lowest position": hi is the value's high word plus one (0: not a
 // candidate, or the diagonal row holding a NaN, whose lo is 1), lo its low word.
-struct PivKey {
+struct alignas(16) PivKey {
     unsigned hi, lo;
     int pos;
-    int pad;
+    int row;  // the candidate's row in its CTA
 };
 
 // the best of a warp's keys, in every lane, by three warp reductions
@@ -378,7 +383,7 @@ __device__ __forceinline__ PivKey best_key(PivKey k) {
     b.hi = __reduce_max_sync(0xffffffffu, k.hi);
     b.lo = __reduce_max_sync(0xffffffffu, k.hi == b.hi ? k.lo : 0u);
     b.pos = __reduce_min_sync(0xffffffffu, k.hi == b.hi && k.lo == b.lo ? k.pos : 0x7fffffff);
-    b.pad = 0;
+    b.row = 0;
     return b;
 }
 
@@ -397,14 +402,55 @@ __device__ __forceinline__ double pivot_rcp(double d) {
 
 template <typename T, bool C>
 struct PanelShared {
-    El<T, C> rec[PCL_SB][PCL_MAXC][PCL_SB];  // mailboxes, per column of the sub-block and sending CTA
-    El<T, C> warp[16][PCL_SB];               // candidate rows of this CTA's warps
+    El<T, C> rec[2][PCL_MAXC][PCL_SB];       // mailboxes per sending CTA, by parity of the column
+    El<T, C> warp[2][16][PCL_SB];            // candidate rows of this CTA's warps, by parity of the column
     El<T, C> U[PCL_SB][LU_NB];               // the sub-block's pivot rows right of it
     El<T, C> L[PCL_SB][PCL_SB];              // their elements inside it
-    PivKey key[PCL_SB][PCL_MAXC];
-    PivKey wkey[16];
-    int owner[PCL_SB];  // local row of pivot q, -1 = another CTA's
+    PivKey key[2][PCL_MAXC];
+    PivKey wkey[2][16];
+    unsigned long long rec_bar[PCL_SB], u_bar;  // mbarriers of the mailboxes and of U
 };
+
+__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ uint32_t peer_addr(const void* p, int rank) {
+    uint32_t r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr(p)), "r"(rank));
+    return r;
+}
+// 8 or 16 bytes into a CTA of the cluster, counted by its mbarrier `bar`
+template <typename V>
+__device__ __forceinline__ void push(uint32_t dst, const V& v, uint32_t bar) {
+    static_assert(sizeof(V) == 8 || sizeof(V) == 16, "8 or 16 bytes");
+    if constexpr (sizeof(V) == 16) {
+        const int4 w = *reinterpret_cast<const int4*>(&v);
+        asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(dst),
+                     "r"(w.x), "r"(w.y), "r"(w.z), "r"(w.w), "r"(bar)
+                     : "memory");
+    } else {
+        const long long w = *reinterpret_cast<const long long*>(&v);
+        asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(dst), "l"(w), "r"(bar)
+                     : "memory");
+    }
+}
+__device__ __forceinline__ void bar_expect(unsigned long long* bar, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)), "r"(bytes) : "memory");
+}
+// waits for the mbarrier's phase; false at the iteration limit
+__device__ __forceinline__ bool bar_wait(unsigned long long* bar, uint32_t parity) {
+    const uint32_t addr = smem_addr(bar);
+    for (uint32_t it = 0; it < PCL_SPIN_CAP; ++it) {
+        uint32_t ok;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}\n"
+            : "=r"(ok)
+            : "r"(addr), "r"(parity)
+            : "memory");
+        if (ok) return true;
+    }
+    return false;
+}
 
 // one element of the panel in shared memory (complex: one 2 sizeof(T) access)
 template <typename T, bool C>
@@ -484,7 +530,7 @@ __device__ __forceinline__ void panel_rank8(T* P, int ldc, int cnt, int jb, int 
 
 template <typename T, bool C, int THREADS>
 __global__ void __launch_bounds__(THREADS) lu_panel_cluster_kernel(T* A, int64_t lda, int n, int k0, int nb, int chunk,
-                                                                   int ldc, int32_t* piv, int32_t* info) {
+                                                                   int ldc, int32_t* piv, int32_t* info, int32_t* flag) {
     using E = El<T, C>;
     constexpr int W = C ? 2 : 1;
     constexpr int NW = THREADS / 32;
@@ -498,20 +544,46 @@ __global__ void __launch_bounds__(THREADS) lu_panel_cluster_kernel(T* A, int64_t
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const int r0 = k0 + rank * chunk;
     const int cnt = max(0, min(chunk, n - r0));
-    for (int e = tid; e < cnt * nb; e += THREADS) {
-        const int r = e / nb, c = e - r * nb;
-        st_p<T, C>(P, c * ldc + r, ld<T, C>(A, (int64_t)(r0 + r) * lda + k0 + c));
-    }
+    // a warp a row, without registers in between: all of the panel in flight.
+    // Complex elements in one copy each where A allows it (16 or 8 bytes).
+    const bool whole = reinterpret_cast<uintptr_t>(A) % (W * sizeof(T)) == 0;
+    for (int r = wid; r < cnt; r += NW)
+        for (int c = lane; c < nb; c += 32) {
+            const uint32_t dst = smem_addr(P + (size_t)W * (c * ldc + r));
+            const T* src = A + W * ((int64_t)(r0 + r) * lda + k0 + c);
+            if (whole) {
+                asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(dst), "l"(src), "n"((int)(W * sizeof(T))));
+            } else {
+                for (int h = 0; h < W; ++h)
+                    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(dst + (uint32_t)(h * sizeof(T))),
+                                 "l"(src + h), "n"((int)sizeof(T)));
+            }
+        }
+    asm volatile("cp.async.wait_all;" ::: "memory");
     const bool mine = tid < cnt;
     int pos = r0 + tid;
     bool done = !mine;
     int bad = 0;  // 1 + first column without a nonzero pivot
+    bool lost = false;  // a wait ran out: the rest runs without waiting, and flag reports it
     if (mine) s_done[tid] = 0;
+    if (tid < 2 * PCL_MAXC) sh.key[tid / PCL_MAXC][tid % PCL_MAXC] = PivKey{0u, 0u, 0x7fffffff, 0};
+    if (tid == 0) {
+        for (int q = 0; q < PCL_SB; ++q)
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&sh.rec_bar[q])) : "memory");
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&sh.u_bar)) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
     __syncthreads();
     cluster.sync();
 
     for (int jb = 0; jb < nb; jb += PCL_SB) {
         const int sw = min(PCL_SB, nb - jb);
+        const int nt = nb - jb - sw;  // columns of the panel right of the sub-block (0 unless sw == PCL_SB)
+        const uint32_t parity = (uint32_t)(jb / PCL_SB) & 1u;
+        if (tid == 0) {
+            for (int q = 0; q < sw; ++q) bar_expect(&sh.rec_bar[q], nc * (uint32_t)(PCL_SB * sizeof(E) + sizeof(PivKey)));
+            if (nt > 0) bar_expect(&sh.u_bar, (uint32_t)(PCL_SB * nt * sizeof(E)));
+        }
         E a[PCL_SB];
         int myq = -1;
 #pragma unroll
@@ -533,36 +605,38 @@ __global__ void __launch_bounds__(THREADS) lu_panel_cluster_kernel(T* A, int64_t
                         key.pos = pos;
                     }
                 }
-                const PivKey wb = best_key(key);
+                PivKey wb = best_key(key);
+                wb.row = tid;
                 if (wb.pos == 0x7fffffff ? lane == 0 : key.pos == wb.pos) {
 #pragma unroll
-                    for (int c = 0; c < PCL_SB; ++c) sh.warp[wid][c] = a[c];
-                    sh.wkey[wid] = wb;
+                    for (int c = 0; c < PCL_SB; ++c) sh.warp[jj & 1][wid][c] = a[c];
+                    sh.wkey[jj & 1][wid] = wb;
                 }
-                if (tid == 0) sh.owner[jj] = -1;
                 __syncthreads();
                 {
                     PivKey k{0u, 0u, 0x7fffffff, 0};
-                    if (lane < NW) k = sh.wkey[lane];
+                    if (lane < NW) k = sh.wkey[jj & 1][lane];
                     const PivKey cb = best_key(k);
                     const unsigned who = __ballot_sync(0xffffffffu, lane < NW && k.pos == cb.pos);
                     const int bw = __ffs((int)who) - 1;
                     // thread (destination, element) pushes one element of the candidate
                     const int dest = tid >> 4, e = tid & 15;
                     if (dest < nc) {
+                        const uint32_t bar = peer_addr(&sh.rec_bar[jj], dest);
                         if (e < PCL_SB)
-                            cluster.map_shared_rank(&sh.rec[jj][rank][0], dest)[e] = sh.warp[bw][e];
+                            push(peer_addr(&sh.rec[jj & 1][rank][e], dest), sh.warp[jj & 1][bw][e], bar);
                         else if (e == PCL_SB)
-                            *cluster.map_shared_rank(&sh.key[jj][rank], dest) = cb;
+                            push(peer_addr(&sh.key[jj & 1][rank], dest), sh.wkey[jj & 1][bw], bar);
                     }
                 }
-                cluster.sync();
+                if (!lost) lost = !bar_wait(&sh.rec_bar[jj], parity);
                 PivKey k{0u, 0u, 0x7fffffff, 0};
-                if (lane < nc) k = sh.key[jj][lane];
+                if (lane < nc) k = sh.key[jj & 1][lane];
                 const PivKey gb = best_key(k);
                 const unsigned who = __ballot_sync(0xffffffffu, lane < nc && k.pos == gb.pos);
-                const E* prow = sh.rec[jj][__ffs((int)who) - 1];
-                const int bp = gb.pos;
+                const int from = max(0, __ffs((int)who) - 1);
+                const E* prow = sh.rec[jj & 1][from];
+                const int bp = gb.pos >= jd && gb.pos < n ? gb.pos : jd;
                 const bool nonzero = gb.hi > 0u && ((gb.hi - 1u) | gb.lo) != 0u;
                 const E pv = prow[jj];
                 E inv{T(0), T(0)};
@@ -584,7 +658,6 @@ __global__ void __launch_bounds__(THREADS) lu_panel_cluster_kernel(T* A, int64_t
                         done = true;
                         s_done[tid] = 1;
                         myq = jj;
-                        sh.owner[jj] = tid;
                     } else {
                         if (pos == jd) pos = bp;
                         E l;
@@ -599,24 +672,24 @@ __global__ void __launch_bounds__(THREADS) lu_panel_cluster_kernel(T* A, int64_t
                         }
                     }
                 }
+                // the rest of the pivot row, to every CTA
+                if (from == rank && nt > 0) {
+                    const int row = min(sh.key[jj & 1][rank].row, ldc - 1);
+                    for (int e = tid; e < nc * nt; e += THREADS) {
+                        const int dest = e / nt, c = e - dest * nt;
+                        push(peer_addr(&sh.U[jj][c], dest), ld_p<T, C>(P, (jb + PCL_SB + c) * ldc + row),
+                             peer_addr(&sh.u_bar, dest));
+                    }
+                }
             }
         }
         if (mine)
 #pragma unroll
             for (int c = 0; c < PCL_SB; ++c)
                 if (c < sw) st_p<T, C>(P, (jb + c) * ldc + tid, a[c]);
-        const int nt = nb - jb - sw;  // columns of the panel right of the sub-block (0 unless sw == PCL_SB)
         if (nt > 0) {
+            if (!lost) lost = !bar_wait(&sh.u_bar, parity);
             __syncthreads();
-            for (int q = 0; q < PCL_SB; ++q) {
-                const int row = sh.owner[q];
-                if (row < 0) continue;  // uniform over the CTA
-                for (int e = tid; e < nc * nt; e += THREADS) {
-                    const int dest = e / nt, c = e - dest * nt;
-                    *cluster.map_shared_rank(&sh.U[q][c], dest) = ld_p<T, C>(P, (jb + PCL_SB + c) * ldc + row);
-                }
-            }
-            cluster.sync();
             if (tid < nt) {
                 E x[PCL_SB];
 #pragma unroll
@@ -639,12 +712,12 @@ __global__ void __launch_bounds__(THREADS) lu_panel_cluster_kernel(T* A, int64_t
         }
     }
     if (rank == 0 && tid == 0 && bad != 0 && *info == 0) *info = bad;
+    if (lost) atomicExch(flag, BEM_ERR_TIMEOUT);
     if (mine) s_pos[tid] = pos;
     __syncthreads();
-    for (int e = tid; e < cnt * nb; e += THREADS) {
-        const int r = e / nb, c = e - r * nb;
-        st<T, C>(A, (int64_t)s_pos[r] * lda + k0 + c, ld_p<T, C>(P, c * ldc + r));
-    }
+    for (int r = wid; r < cnt; r += NW)
+        for (int c = lane; c < nb; c += 32) st<T, C>(A, (int64_t)s_pos[r] * lda + k0 + c, ld_p<T, C>(P, c * ldc + r));
+    cluster.sync();  // no CTA leaves while another may still push to it
 }
 
 // row swaps of one panel applied to the columns outside it
@@ -964,7 +1037,7 @@ int check_flag(bem_ctx* ctx, cudaStream_t s, const char* what) {
 // kernel takes those: more than about 3100 complex or 6200 real FP64 rows).
 template <typename T, bool C>
 int lu_panel_cluster(bem_ctx* ctx, T* A, int64_t lda, int n, int k0, int nb, int32_t* piv, int32_t* info,
-                     cudaStream_t s) {
+                     int32_t* flag, cudaStream_t s) {
     constexpr size_t E = sizeof(T) * (C ? 2 : 1);
     constexpr size_t FIXED = (sizeof(PanelShared<T, C>) + 15) & ~size_t(15);
     constexpr size_t SMEM = 226 * 1024;
@@ -999,7 +1072,7 @@ int lu_panel_cluster(bem_ctx* ctx, T* A, int64_t lda, int n, int k0, int nb, int
             }
         }
         ctx->launches++;
-        return bem_check_cuda(ctx, cudaLaunchKernelEx(&cfg, kernel, A, lda, n, k0, nb, chunk, ldc, piv, info),
+        return bem_check_cuda(ctx, cudaLaunchKernelEx(&cfg, kernel, A, lda, n, k0, nb, chunk, ldc, piv, info, flag),
                               "lu_panel_cluster_kernel");
     };
     return chunk <= 256 ? go(lu_panel_cluster_kernel<T, C, 256>, 256) : go(lu_panel_cluster_kernel<T, C, 512>, 512);
@@ -1047,7 +1120,7 @@ int lu_factor_t(bem_ctx* ctx, T* A, int64_t n, int64_t lda, int32_t* piv, int32_
         int nb = (int)std::min<int64_t>(LU_NB, n - k0);
         int rows = (int)(n - k0);
         int ni = (int)n, k0i = (int)k0;
-        const int rc = lu_panel_cluster<T, C>(ctx, A, lda, ni, k0i, nb, piv, info, s);
+        const int rc = lu_panel_cluster<T, C>(ctx, A, lda, ni, k0i, nb, piv, info, flag, s);
         if (rc < 0) return rc;
         if (rc == 1) {
             // the panel does not fit a cluster's shared memory

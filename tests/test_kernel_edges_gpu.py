@@ -364,6 +364,27 @@ def test_gemm_on_unaligned_complex_operands(engine):
     assert np.abs(C.cpu().numpy() - want).max() < 1e-12 * 10
 
 
+def test_lu_of_an_unaligned_complex_matrix(engine):
+    """A complex128 matrix that starts on an odd multiple of 8 bytes is read
+    half an element at a time: the same pivots, and the same factors to
+    rounding (n eps)."""
+    import ctypes
+    from bem_b200 import _lib
+    n = 129
+    A = torch.as_tensor(_gaussian((n, n), True, 9), device="cuda")
+    raw = torch.zeros(2 * n * n + 1, dtype=torch.float64, device="cuda")
+    raw[1:] = torch.view_as_real(A).reshape(-1)
+    piv2 = torch.empty(n, dtype=torch.int32, device="cuda")
+    info = torch.zeros(1, dtype=torch.int32, device="cuda")
+    rc = engine.lib.bem_lu_factor(engine.ctx, _lib.C128, ctypes.c_void_p(raw.data_ptr() + 8), n, n,
+                                  ctypes.c_void_p(piv2.data_ptr()), ctypes.c_void_p(info.data_ptr()),
+                                  ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+    assert rc == 0 and int(info.item()) == 0
+    piv, _ = engine.lu_factor(A)
+    assert torch.equal(piv, piv2)
+    assert float((raw[1:] - torch.view_as_real(A).reshape(-1)).abs().max()) < n * 2.3e-16 * float(A.abs().max())
+
+
 # ---- both wavenumbers of the Calderon sweep over lane pairs ---------------------------
 @pytest.mark.parametrize("ks", [(0.1, 0.05), (1.2, 0.4), (30.0, 45.0), (0.7, -0.3)])
 @pytest.mark.parametrize("Q", [1, 2, 3])
