@@ -9,11 +9,14 @@
 //             column one grid barrier publishes every CTA's pivot candidate,
 //             after which all CTAs agree on the pivot, swap it in and apply
 //             the rank-1 update to their rows (lu_panel_kernel).
+//   next    : FP64: the three steps below for the next panel's columns in one
+//             launch (lu_next_kernel), so that the next panel starts beside
+//             them for all other columns (look-ahead).
 //   laswp   : the panel's row swaps applied to the columns outside the panel.
 //   trsm    : U12 = L11^-1 A12, L11 staged in shared memory.
-//   update  : A22 -= L21 U12 (bem_gemm.cu: FP64 SIMT tiles for the plain path,
-//             tcgen05 TF32 tensor-core tiles for the FP32 factor).
-// Every device-side wait (grid barriers) is bounded; a timeout sets a flag and
+//   update  : A22 -= L21 U12 (bem_gemm.cuh: FP64 tensor cores for the plain
+//             path, tcgen05 TF32 tensor-core tiles for the FP32 factor).
+// Every device-side wait (grid barriers, mbarriers) is bounded; a timeout sets a flag and
 // the host call returns BEM_ERR_TIMEOUT.
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
@@ -360,12 +363,16 @@ __global__ void __launch_bounds__(256) lu_panel_kernel(T* A, int64_t lda, int n,
 // rows' remaining elements are solved against the sub-block's unit lower
 // triangle and applied as one rank-PCL_SB update, so shared memory is swept once per PCL_SB columns (FP64: on the FP64 tensor
 // cores).  Measured (B200, a column step averaged over a whole factorisation):
-// 2999 complex rows 1.62 us (6.0 us of the cooperative kernel below, a grid
+// 2999 complex rows 1.51 us (6.0 us of the cooperative kernel below, a grid
 // barrier a column; 1.95 with a cluster barrier a column and the panel read
-// through registers), 1280 real rows 1.31 us (5.8; 1.73).
+// through registers), 1280 real rows 1.28 us (5.8; 1.73).  What a step consists
+// of are some twelve dependent shared-memory and warp-reduction latencies of
+// 30 to 200 cycles; a loop over the columns instead of eight copies of the step
+// (registers turned instead of indexed) and half the warps were both slower.
 // ----------------------------------------------------------------------------
 constexpr int PCL_SB = 8;
 constexpr int PCL_MAXC = 16;
+constexpr int PCL_MAXROWS = PCL_MAXC * 512;
 constexpr uint32_t PCL_SPIN_CAP = 1u << 20;
 
 // A pivot candidate as integers that order like the rule "largest value,
@@ -377,14 +384,18 @@ struct alignas(16) PivKey {
     int row;  // the candidate's row in its CTA
 };
 
-// the best of a warp's keys, in every lane, by three warp reductions
-__device__ __forceinline__ PivKey best_key(PivKey k) {
-    PivKey b;
-    b.hi = __reduce_max_sync(0xffffffffu, k.hi);
-    b.lo = __reduce_max_sync(0xffffffffu, k.hi == b.hi ? k.lo : 0u);
-    b.pos = __reduce_min_sync(0xffffffffu, k.hi == b.hi && k.lo == b.lo ? k.pos : 0x7fffffff);
-    b.row = 0;
-    return b;
+// the lane with the best of a warp's keys: usually one lane has the largest
+// high word, and one warp reduction settles it
+__device__ __forceinline__ int best_lane(const PivKey& k) {
+    const unsigned hi = __reduce_max_sync(0xffffffffu, k.hi);
+    unsigned who = __ballot_sync(0xffffffffu, k.hi == hi);
+    if (who & (who - 1)) {
+        const unsigned lo = __reduce_max_sync(0xffffffffu, k.hi == hi ? k.lo : 0u);
+        const bool mine = k.hi == hi && k.lo == lo;
+        const int pos = __reduce_min_sync(0xffffffffu, mine ? k.pos : 0x7fffffff);
+        who = __ballot_sync(0xffffffffu, mine && k.pos == pos);
+    }
+    return __ffs((int)who) - 1;
 }
 
 // 1/d on the pivot chain: in FP64 the approximate reciprocal (about 20 bits)
@@ -402,20 +413,22 @@ __device__ __forceinline__ double pivot_rcp(double d) {
 
 template <typename T, bool C>
 struct PanelShared {
-    El<T, C> rec[2][PCL_MAXC][PCL_SB];       // mailboxes per sending CTA, by parity of the column
+    // mailboxes, per column of the sub-block and sending CTA: the candidate's reciprocal and its elements in the
+    // other columns of the sub-block
+    El<T, C> rec[PCL_SB][PCL_MAXC][PCL_SB];
     El<T, C> warp[2][16][PCL_SB];            // candidate rows of this CTA's warps, by parity of the column
     El<T, C> U[PCL_SB][LU_NB];               // the sub-block's pivot rows right of it
-    El<T, C> L[PCL_SB][PCL_SB];              // their elements inside it
     PivKey key[2][PCL_MAXC];
     PivKey wkey[2][16];
     unsigned long long rec_bar[PCL_SB], u_bar;  // mbarriers of the mailboxes and of U
 };
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ uint32_t peer_addr(const void* p, int rank) {
+// offset from a shared address of this CTA to the same one of another CTA of the cluster
+__device__ __forceinline__ uint32_t peer_offset(const void* p, int rank) {
     uint32_t r;
-    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr(p)), "r"(rank));
-    return r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr(p)), "r"(rank));
+    return r - smem_addr(p);
 }
 // 8 or 16 bytes into a CTA of the cluster, counted by its mbarrier `bar`
 template <typename V>
@@ -489,6 +502,7 @@ __device__ __forceinline__ void panel_rank8(T* P, int ldc, int cnt, int jb, int 
 #pragma unroll
             for (int h = 0; h < 2; ++h)
                 fa[h] = store ? ld_p<T, C>(P, (jb + 4 * h + k4) * ldc + r) : E{T(0), T(0)};
+#pragma unroll 4
             for (int t = 0; t < ct; ++t) {
                 const int cc = t * 8 + 2 * k4;
                 double acc[2][NP];
@@ -530,7 +544,8 @@ __device__ __forceinline__ void panel_rank8(T* P, int ldc, int cnt, int jb, int 
 
 template <typename T, bool C, int THREADS>
 __global__ void __launch_bounds__(THREADS) lu_panel_cluster_kernel(T* A, int64_t lda, int n, int k0, int nb, int chunk,
-                                                                   int ldc, int32_t* piv, int32_t* info, int32_t* flag) {
+                                                                   int ldc, int32_t* piv, int32_t* info, int32_t* flag,
+                                                                   int32_t* src) {
     using E = El<T, C>;
     constexpr int W = C ? 2 : 1;
     constexpr int NW = THREADS / 32;
@@ -564,6 +579,9 @@ __global__ void __launch_bounds__(THREADS) lu_panel_cluster_kernel(T* A, int64_t
     int pos = r0 + tid;
     bool done = !mine;
     int bad = 0;  // 1 + first column without a nonzero pivot
+    // thread (destination, element) of the pushes
+    const int dest = tid >> 4, elem = tid & 15;
+    const uint32_t peer = peer_offset(smem_raw, min(dest, nc - 1));
     bool lost = false;  // a wait ran out: the rest runs without waiting, and flag reports it
     if (mine) s_done[tid] = 0;
     if (tid < 2 * PCL_MAXC) sh.key[tid / PCL_MAXC][tid % PCL_MAXC] = PivKey{0u, 0u, 0x7fffffff, 0};
@@ -588,68 +606,73 @@ __global__ void __launch_bounds__(THREADS) lu_panel_cluster_kernel(T* A, int64_t
         int myq = -1;
 #pragma unroll
         for (int c = 0; c < PCL_SB; ++c) a[c] = mine && c < sw ? ld_p<T, C>(P, (jb + c) * ldc + tid) : E{T(0), T(0)};
+        uint32_t senders = 0;  // 4 bits a column: the CTA its pivot came from
+        int own = -1;          // this CTA's row that became the last pivot
+        // the rest of pivot row q, to every CTA
+        auto push_row = [&](int q) {
+            if (own < 0 || nt <= 0 || dest >= nc) return;
+#pragma unroll 1
+            for (int c = elem; c < nt; c += 16)
+                push(smem_addr(&sh.U[q][c]) + peer, ld_p<T, C>(P, (jb + PCL_SB + c) * ldc + own),
+                     smem_addr(&sh.u_bar) + peer);
+        };
 #pragma unroll
         for (int jj = 0; jj < PCL_SB; ++jj) {
             if (jj < sw) {  // uniform over the cluster
                 const int jd = k0 + jb + jj;
                 // candidate of this row; NaN never wins, but the diagonal row stays as the last resort
-                PivKey key{0u, 0u, 0x7fffffff, 0};
+                PivKey key{0u, 0u, 0x7fffffff, tid};
                 if (!done) {
                     const double v = (double)mag1<T, C>(a[jj]);
-                    if (v >= 0.0) {
-                        key.hi = (unsigned)__double2hiint(v) + 1u;
-                        key.lo = (unsigned)__double2loint(v);
+                    const unsigned hi = (unsigned)__double2hiint(v), lo = (unsigned)__double2loint(v);
+                    if (hi < 0x7ff00000u || (hi == 0x7ff00000u && lo == 0u)) {  // |.| >= 0: not NaN
+                        key.hi = hi + 1u;
+                        key.lo = lo;
                         key.pos = pos;
                     } else if (pos == jd) {
                         key.lo = 1u;
                         key.pos = pos;
                     }
                 }
-                PivKey wb = best_key(key);
-                wb.row = tid;
-                if (wb.pos == 0x7fffffff ? lane == 0 : key.pos == wb.pos) {
+                // every row's reciprocal beside the reductions, so that the pivot's is at hand
+                E rc{T(0), T(0)};
+                if (C) {
+                    const T rd = pivot_rcp(a[jj].re * a[jj].re + a[jj].im * a[jj].im);
+                    rc.re = a[jj].re * rd;
+                    rc.im = -a[jj].im * rd;
+                } else {
+                    rc.re = pivot_rcp(a[jj].re);
+                }
+                if (lane == best_lane(key)) {
 #pragma unroll
-                    for (int c = 0; c < PCL_SB; ++c) sh.warp[jj & 1][wid][c] = a[c];
-                    sh.wkey[jj & 1][wid] = wb;
+                    for (int c = 0; c < PCL_SB; ++c) sh.warp[jj & 1][wid][c] = c == jj ? rc : a[c];
+                    sh.wkey[jj & 1][wid] = key;
                 }
                 __syncthreads();
                 {
                     PivKey k{0u, 0u, 0x7fffffff, 0};
                     if (lane < NW) k = sh.wkey[jj & 1][lane];
-                    const PivKey cb = best_key(k);
-                    const unsigned who = __ballot_sync(0xffffffffu, lane < NW && k.pos == cb.pos);
-                    const int bw = __ffs((int)who) - 1;
+                    const int bw = min(best_lane(k), NW - 1);
                     // thread (destination, element) pushes one element of the candidate
-                    const int dest = tid >> 4, e = tid & 15;
                     if (dest < nc) {
-                        const uint32_t bar = peer_addr(&sh.rec_bar[jj], dest);
-                        if (e < PCL_SB)
-                            push(peer_addr(&sh.rec[jj & 1][rank][e], dest), sh.warp[jj & 1][bw][e], bar);
-                        else if (e == PCL_SB)
-                            push(peer_addr(&sh.key[jj & 1][rank], dest), sh.wkey[jj & 1][bw], bar);
+                        const uint32_t bar = smem_addr(&sh.rec_bar[jj]) + peer;
+                        if (elem < PCL_SB)
+                            push(smem_addr(&sh.rec[jj][rank][elem]) + peer, sh.warp[jj & 1][bw][elem], bar);
+                        else if (elem == PCL_SB)
+                            push(smem_addr(&sh.key[jj & 1][rank]) + peer, sh.wkey[jj & 1][bw], bar);
                     }
                 }
+                if (jj > 0) push_row(jj - 1);
                 if (!lost) lost = !bar_wait(&sh.rec_bar[jj], parity);
                 PivKey k{0u, 0u, 0x7fffffff, 0};
                 if (lane < nc) k = sh.key[jj & 1][lane];
-                const PivKey gb = best_key(k);
-                const unsigned who = __ballot_sync(0xffffffffu, lane < nc && k.pos == gb.pos);
-                const int from = max(0, __ffs((int)who) - 1);
-                const E* prow = sh.rec[jj & 1][from];
+                const int from = min(best_lane(k), nc - 1);
+                const E* prow = sh.rec[jj][from];
+                const PivKey gb = sh.key[jj & 1][from];
                 const int bp = gb.pos >= jd && gb.pos < n ? gb.pos : jd;
                 const bool nonzero = gb.hi > 0u && ((gb.hi - 1u) | gb.lo) != 0u;
-                const E pv = prow[jj];
-                E inv{T(0), T(0)};
-                if (nonzero) {
-                    if (C) {
-                        const T rd = pivot_rcp(pv.re * pv.re + pv.im * pv.im);
-                        inv.re = pv.re * rd;
-                        inv.im = -pv.im * rd;
-                    } else {
-                        inv.re = pivot_rcp(pv.re);
-                    }
-                }
-                if (tid < PCL_SB) sh.L[jj][tid] = prow[tid];
+                const E inv = nonzero ? prow[jj] : E{T(0), T(0)};
+                senders |= (uint32_t)from << (4 * jj);
                 if (!nonzero && bad == 0) bad = jd + 1;
                 if (rank == 0 && tid == 0) piv[jd] = bp;
                 if (!done) {
@@ -672,17 +695,10 @@ __global__ void __launch_bounds__(THREADS) lu_panel_cluster_kernel(T* A, int64_t
                         }
                     }
                 }
-                // the rest of the pivot row, to every CTA
-                if (from == rank && nt > 0) {
-                    const int row = min(sh.key[jj & 1][rank].row, ldc - 1);
-                    for (int e = tid; e < nc * nt; e += THREADS) {
-                        const int dest = e / nt, c = e - dest * nt;
-                        push(peer_addr(&sh.U[jj][c], dest), ld_p<T, C>(P, (jb + PCL_SB + c) * ldc + row),
-                             peer_addr(&sh.u_bar, dest));
-                    }
-                }
+                own = from == rank ? min(gb.row, ldc - 1) : -1;
             }
         }
+        push_row(PCL_SB - 1);
         if (mine)
 #pragma unroll
             for (int c = 0; c < PCL_SB; ++c)
@@ -697,7 +713,7 @@ __global__ void __launch_bounds__(THREADS) lu_panel_cluster_kernel(T* A, int64_t
                     x[q] = sh.U[q][tid];
 #pragma unroll
                     for (int w = 0; w < q; ++w) {
-                        const E l = sh.L[q][w];
+                        const E l = sh.rec[q][(senders >> (4 * q)) & 15u][w];
                         x[q].re -= l.re * x[w].re - (C ? l.im * x[w].im : T(0));
                         if (C) x[q].im -= l.re * x[w].im + l.im * x[w].re;
                     }
@@ -713,18 +729,21 @@ __global__ void __launch_bounds__(THREADS) lu_panel_cluster_kernel(T* A, int64_t
     }
     if (rank == 0 && tid == 0 && bad != 0 && *info == 0) *info = bad;
     if (lost) atomicExch(flag, BEM_ERR_TIMEOUT);
-    if (mine) s_pos[tid] = pos;
+    if (mine) {
+        s_pos[tid] = pos;
+        src[pos - k0] = r0 + tid;
+    }
     __syncthreads();
     for (int r = wid; r < cnt; r += NW)
         for (int c = lane; c < nb; c += 32) st<T, C>(A, (int64_t)s_pos[r] * lda + k0 + c, ld_p<T, C>(P, c * ldc + r));
     cluster.sync();  // no CTA leaves while another may still push to it
 }
 
-// row swaps of one panel applied to the columns outside it
+// row swaps of one panel applied to the columns from c0 (to n) outside [x0, x1)
 template <typename T, bool C>
-__global__ void laswp_kernel(T* A, int64_t lda, int n, int k0, int nb, const int32_t* piv) {
-    int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= n || (c >= k0 && c < k0 + nb)) return;
+__global__ void laswp_kernel(T* A, int64_t lda, int c0, int n, int x0, int x1, int k0, int nb, const int32_t* piv) {
+    int c = c0 + blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= n || (c >= x0 && c < x1)) return;
     for (int j = 0; j < nb; ++j) {
         int r1 = k0 + j, r2 = piv[k0 + j];
         if (r1 == r2) continue;
@@ -748,13 +767,14 @@ constexpr int TRSM_B = 8;
 constexpr int TRSM_ROWS = 8;
 
 template <typename T, bool C>
-__global__ void __launch_bounds__(TRSM_COLS* TRSM_ROWS) trsm_kernel(T* A, int64_t lda, int n, int k0, int nb) {
+__global__ void __launch_bounds__(TRSM_COLS* TRSM_ROWS) trsm_kernel(T* A, int64_t lda, int col0, int n, int k0,
+                                                                              int nb) {
     using E = El<T, C>;
     constexpr int THREADS = TRSM_COLS * TRSM_ROWS;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     E* L = reinterpret_cast<E*>(smem_raw);  // [nb][nb]
     E* X = L + nb * nb;                     // [nb][TRSM_COLS]
-    const int c0 = k0 + nb + blockIdx.x * TRSM_COLS;
+    const int c0 = col0 + blockIdx.x * TRSM_COLS;  // of the columns [col0, n)
     const int ncol = min(TRSM_COLS, n - c0);
     for (int idx = threadIdx.x; idx < nb * nb; idx += THREADS) {
         int r = idx / nb, c = idx - r * nb;
@@ -803,6 +823,131 @@ __global__ void __launch_bounds__(TRSM_COLS* TRSM_ROWS) trsm_kernel(T* A, int64_
     for (int idx = threadIdx.x; idx < nb * TRSM_COLS; idx += THREADS) {
         int r = idx / TRSM_COLS, cc = idx - r * TRSM_COLS;
         if (cc < ncol) st<T, C>(A, (int64_t)(k0 + r) * lda + c0 + cc, X[idx]);
+    }
+}
+
+// The next panel's columns [c0, c1) after the cluster's panel at k0 (LU_NB
+// columns): row swaps, U12 = L11^{-1} A12 and A22 -= L21 U12 in one launch.
+// These columns are the serial chain of the factorisation (panel, its
+// application to the next panel, next panel), so what counts is latency: as
+// separate launches they cost 5 + 15 + 24 us and three launch gaps a step (2999
+// complex), here 21 us.  A
+// cluster takes NX_COLS columns, its CTAs a share of the rows each; every CTA
+// reads the LU_NB rows of A12 and its own rows at their places before the
+// swaps (src, written by the panel), and solves A12 itself.  All reads of A come
+// before the cluster barrier and all writes after it, so the swap needs no copy.
+// The products run from zero on the FP64 tensor cores and are subtracted once.
+constexpr int NX_COLS = 8;
+constexpr int NX_LD = LU_NB + 1;  // odd: conflict-free down a column of L11
+template <bool C>
+__global__ void __launch_bounds__(256) lu_next_kernel(double* A, int64_t lda, int n, int k0, int c0, int c1, int chunk,
+                                                      const int32_t* src) {
+    using E = El<double, C>;
+    constexpr int W = C ? 2 : 1, NP = C ? 2 : 1;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    double* L = reinterpret_cast<double*>(smem_raw);  // [LU_NB][NX_LD]
+    double* X = L + W * LU_NB * NX_LD;                // [LU_NB][NX_COLS]
+    double* Y = X + W * LU_NB * NX_COLS;              // [chunk][NX_COLS]
+    cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const int k1 = k0 + LU_NB, r0 = k1 + (int)blockIdx.x * chunk, cnt = max(0, min(chunk, n - r0));
+    const int cb = c0 + (int)blockIdx.y * NX_COLS, ncol = min(NX_COLS, c1 - cb);
+    const bool whole = reinterpret_cast<uintptr_t>(A) % (W * sizeof(double)) == 0;
+    auto fetch = [&](double* dst, int64_t row, int col) {
+        const double* a = A + W * (row * lda + col);
+        if (whole) {
+            asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(smem_addr(dst)), "l"(a), "n"(8 * W));
+        } else {
+            for (int h = 0; h < W; ++h)
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_addr(dst + h)), "l"(a + h));
+        }
+    };
+    for (int e = tid; e < LU_NB * LU_NB; e += 256) {
+        const int r = e / LU_NB, c = e % LU_NB;
+        if (c < r) fetch(L + W * (r * NX_LD + c), k0 + r, k0 + c);
+    }
+    const int cc = tid & 7;  // column of this thread in the copies and the solve
+    for (int r = tid >> 3; r < LU_NB + cnt; r += 32) {
+        const int row = r < LU_NB ? r : r0 - k1 + r;  // position in the panel
+        double* dst = r < LU_NB ? X + W * (r * NX_COLS + cc) : Y + W * ((r - LU_NB) * NX_COLS + cc);
+        if (cc < ncol)
+            fetch(dst, min(max(src[row], k0), n - 1), cb + cc);
+        else
+            for (int h = 0; h < W; ++h) dst[h] = 0.0;
+    }
+    // a warp per 8 x 8 tile of rows; its part of L21, one tile ahead
+    const int row8 = lane >> 2, k4 = lane & 3;
+    E f[LU_NB / 4];
+    auto rows_of = [&](int rt) {
+        const int r = rt * 8 + row8;
+#pragma unroll
+        for (int h = 0; h < LU_NB / 4; ++h)
+            f[h] = r < cnt ? ld<double, C>(A, (int64_t)(r0 + r) * lda + k0 + 4 * h + k4) : E{0.0, 0.0};
+    };
+    rows_of(wid);
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    cluster.sync();
+    // X = L11^{-1} X in blocks of TRSM_B rows, as in trsm_kernel
+    for (int b = 0; b < LU_NB; b += TRSM_B) {
+        E x[TRSM_B];
+        if (tid < NX_COLS) {
+#pragma unroll
+            for (int q = 0; q < TRSM_B; ++q) {
+                x[q] = ld_p<double, C>(X, (b + q) * NX_COLS + tid);
+#pragma unroll
+                for (int p = 0; p < q; ++p) {
+                    const E l = ld_p<double, C>(L, (b + q) * NX_LD + b + p);
+                    x[q].re -= l.re * x[p].re - (C ? l.im * x[p].im : 0.0);
+                    if (C) x[q].im -= l.re * x[p].im + l.im * x[p].re;
+                }
+                st_p<double, C>(X, (b + q) * NX_COLS + tid, x[q]);
+            }
+        }
+        __syncthreads();
+        if (b + TRSM_B >= LU_NB) break;
+#pragma unroll
+        for (int q = 0; q < TRSM_B; ++q) x[q] = ld_p<double, C>(X, (b + q) * NX_COLS + cc);
+        for (int r = b + TRSM_B + (tid >> 3); r < LU_NB; r += 32) {
+            E acc = ld_p<double, C>(X, r * NX_COLS + cc);
+#pragma unroll
+            for (int q = 0; q < TRSM_B; ++q) {
+                const E l = ld_p<double, C>(L, r * NX_LD + b + q);
+                acc.re -= l.re * x[q].re - (C ? l.im * x[q].im : 0.0);
+                if (C) acc.im -= l.re * x[q].im + l.im * x[q].re;
+            }
+            st_p<double, C>(X, r * NX_COLS + cc, acc);
+        }
+        __syncthreads();
+    }
+    if (blockIdx.x == 0)
+        for (int r = tid >> 3; r < LU_NB; r += 32)
+            if (cc < ncol) st<double, C>(A, (int64_t)(k0 + r) * lda + cb + cc, ld_p<double, C>(X, r * NX_COLS + cc));
+    // the real and imaginary products on separate chains
+    for (int rt = wid; rt * 8 < cnt; rt += 8) {
+        const int r = rt * 8 + row8;
+        const bool ok = r < cnt;
+        double p[NP][2] = {}, q[NP][2] = {};  // re re, re im; im im, im re
+#pragma unroll
+        for (int h = 0; h < LU_NB / 4; ++h) {
+            const E u = ld_p<double, C>(X, (4 * h + k4) * NX_COLS + row8);
+            bem_gemm_detail::dmma_acc(p[0][0], p[0][1], f[h].re, u.re);
+            if (C) {
+                bem_gemm_detail::dmma_acc(q[0][0], q[0][1], f[h].im, u.im);
+                bem_gemm_detail::dmma_acc(p[NP - 1][0], p[NP - 1][1], f[h].re, u.im);
+                bem_gemm_detail::dmma_acc(q[NP - 1][0], q[NP - 1][1], f[h].im, u.re);
+            }
+        }
+        rows_of(rt + 8);
+        if (ok)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int c = 2 * k4 + e;
+                if (c >= ncol) continue;
+                E v = ld_p<double, C>(Y, r * NX_COLS + c);
+                v.re -= C ? p[0][e] - q[0][e] : p[0][e];
+                if (C) v.im -= p[NP - 1][e] + q[NP - 1][e];
+                st<double, C>(A, (int64_t)(r0 + r) * lda + cb + c, v);
+            }
     }
 }
 
@@ -997,18 +1142,21 @@ struct LinWs {
     GridBar* bar;
     PivSlot* slots;  // [2][PANEL_MAXB]
     void* rowbuf;    // [2][PANEL_MAXB+1][LU_NB] panel-row copies (16 B per element)
+    int32_t* src;    // [PCL_MAXROWS] rows of a cluster's panel: where each came from
 };
 
 // at_least: bytes the workspace has to have for a later call too
 int linws(bem_ctx* ctx, size_t at_least, LinWs* w) {
     const size_t off_slots = 256;
     const size_t off_rows = off_slots + sizeof(PivSlot) * 2 * PANEL_MAXB;
-    const size_t total = off_rows + 16 * (size_t)2 * (PANEL_MAXB + 1) * LU_NB;
+    const size_t off_src = off_rows + 16 * (size_t)2 * (PANEL_MAXB + 1) * LU_NB;
+    const size_t total = off_src + sizeof(int32_t) * PCL_MAXROWS;
     if (int rc = bem_ws_reserve(ctx, std::max(total, at_least))) return rc;
     char* base = (char*)ctx->ws;
     w->bar = (GridBar*)base;
     w->slots = (PivSlot*)(base + off_slots);
     w->rowbuf = (void*)(base + off_rows);
+    w->src = (int32_t*)(base + off_src);
     return BEM_OK;
 }
 
@@ -1037,7 +1185,7 @@ int check_flag(bem_ctx* ctx, cudaStream_t s, const char* what) {
 // kernel takes those: more than about 3100 complex or 6200 real FP64 rows).
 template <typename T, bool C>
 int lu_panel_cluster(bem_ctx* ctx, T* A, int64_t lda, int n, int k0, int nb, int32_t* piv, int32_t* info,
-                     int32_t* flag, cudaStream_t s) {
+                     int32_t* flag, int32_t* src, cudaStream_t s) {
     constexpr size_t E = sizeof(T) * (C ? 2 : 1);
     constexpr size_t FIXED = (sizeof(PanelShared<T, C>) + 15) & ~size_t(15);
     constexpr size_t SMEM = 226 * 1024;
@@ -1056,13 +1204,15 @@ int lu_panel_cluster(bem_ctx* ctx, T* A, int64_t lda, int n, int k0, int nb, int
     at[0].val.clusterDim.x = (unsigned)nc;
     at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
     cfg.gridDim = dim3((unsigned)nc);
-    cfg.dynamicSmemBytes = smem;
+    // all of an SM's shared memory: the panel is the factorisation's serial
+    // chain, so no CTA of the update beside it (look-ahead) shares its SMs
+    cfg.dynamicSmemBytes = SMEM;
     cfg.stream = s;
     cfg.attrs = at;
     cfg.numAttrs = 1;
     auto go = [&](auto* kernel, int threads) -> int {
         cfg.blockDim = dim3((unsigned)threads);
-        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM);
         if (nc > 8) {
             cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
             int fit = 0;
@@ -1072,10 +1222,43 @@ int lu_panel_cluster(bem_ctx* ctx, T* A, int64_t lda, int n, int k0, int nb, int
             }
         }
         ctx->launches++;
-        return bem_check_cuda(ctx, cudaLaunchKernelEx(&cfg, kernel, A, lda, n, k0, nb, chunk, ldc, piv, info, flag),
+        return bem_check_cuda(ctx, cudaLaunchKernelEx(&cfg, kernel, A, lda, n, k0, nb, chunk, ldc, piv, info, flag, src),
                               "lu_panel_cluster_kernel");
     };
     return chunk <= 256 ? go(lu_panel_cluster_kernel<T, C, 256>, 256) : go(lu_panel_cluster_kernel<T, C, 512>, 512);
+}
+
+// queues lu_next_kernel for the columns [c0, c1) (rows below k0 + LU_NB exist)
+template <bool C>
+int lu_next(bem_ctx* ctx, double* A, int64_t lda, int n, int k0, int c0, int c1, const int32_t* src, cudaStream_t s) {
+    constexpr size_t E = sizeof(double) * (C ? 2 : 1);
+    const int rows = n - k0 - LU_NB;
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute at[1];
+    cfg.blockDim = dim3(256);
+    cfg.stream = s;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    int nc = 1;
+    while (nc < PCL_MAXC && (rows + nc - 1) / nc > 32) nc *= 2;
+    int chunk = 0;
+    for (;; nc = 8) {
+        chunk = (rows + nc - 1) / nc;
+        at[0].val.clusterDim.x = (unsigned)nc;
+        cfg.gridDim = dim3((unsigned)nc, (unsigned)((c1 - c0 + NX_COLS - 1) / NX_COLS));
+        cfg.dynamicSmemBytes = E * (LU_NB * NX_LD + (LU_NB + (size_t)chunk) * NX_COLS);
+        cudaFuncSetAttribute(lu_next_kernel<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes);
+        if (nc <= 8) break;
+        cudaFuncSetAttribute(lu_next_kernel<C>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        int fit = 0;
+        if (cudaOccupancyMaxActiveClusters(&fit, lu_next_kernel<C>, &cfg) == cudaSuccess && fit >= 1) break;
+        cudaGetLastError();
+    }
+    ctx->launches++;
+    return bem_check_cuda(ctx, cudaLaunchKernelEx(&cfg, lu_next_kernel<C>, A, lda, n, k0, c0, c1, chunk, src),
+                          "lu_next_kernel");
 }
 
 // Workspace of lu_solve: permutation, the inverses of the diagonal tiles,
@@ -1116,41 +1299,80 @@ int lu_factor_t(bem_ctx* ctx, T* A, int64_t n, int64_t lda, int32_t* piv, int32_
     if (nblk < 1) return bem_fail(ctx, BEM_ERR_CUDA, "lu_panel_kernel cannot be made co-resident");
     if (use_smem && sizeof(El<T, C>) * (size_t)std::max<int64_t>(32, (n + nblk - 1) / nblk) * LU_NB > PANEL_SMEM)
         return bem_fail(ctx, BEM_ERR_CUDA, "lu_panel_kernel: fewer co-resident CTAs than SMs");
-    for (int64_t k0 = 0; k0 < n; k0 += LU_NB) {
-        int nb = (int)std::min<int64_t>(LU_NB, n - k0);
-        int rows = (int)(n - k0);
-        int ni = (int)n, k0i = (int)k0;
-        const int rc = lu_panel_cluster<T, C>(ctx, A, lda, ni, k0i, nb, piv, info, flag, s);
-        if (rc < 0) return rc;
-        if (rc == 1) {
-            // the panel does not fit a cluster's shared memory
-            int blocks = std::min(nblk, std::max(1, (rows + 31) / 32));
-            int chunk = (rows + blocks - 1) / blocks;
-            El<T, C>* rb = (El<T, C>*)w.rowbuf;
-            size_t smem = use_smem ? sizeof(El<T, C>) * (size_t)chunk * LU_NB : 0;
-            void* args[] = {&A, &lda, &ni, &k0i, &nb, &chunk, &piv, &info, &w.bar, &w.slots, &rb, &flag};
-            if (int e = bem_check_cuda(ctx, cudaLaunchCooperativeKernel(pk, blocks, threads, args, smem, s),
-                                       "lu_panel_kernel"))
-                return e;
+    // Look-ahead: the panel occupies one cluster, so the next panel's columns are
+    // brought up to date first, on the high-priority side stream, and factored
+    // there while the caller's stream works on all other columns (2999 complex:
+    // 10.5 -> 7.3 ms with the solves).  FP32 stays on one stream (its
+    // tensor-core updates share a scratch).
+    const bool ahead = sizeof(T) == 8;
+    if (ahead)
+        if (int rc = bem_lookahead_stream(ctx)) return rc;
+    const cudaStream_t sp = ahead ? ctx->aux : s;
+    auto order = [&](cudaStream_t first, cudaEvent_t ev, cudaStream_t then) {
+        if (!ahead) return;
+        cudaEventRecord(ev, first);
+        cudaStreamWaitEvent(then, ev, 0);
+    };
+    // panel k0 applied to the columns [c0, c1), and its swaps to the finished ones left of `left`
+    const size_t tsmem_max = sizeof(El<T, C>) * LU_NB * (LU_NB + TRSM_COLS);
+    cudaFuncSetAttribute(trsm_kernel<T, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsmem_max);
+    auto apply = [&](int k0, int nb, int left, int c0, int c1, cudaStream_t st) -> int {
+        const int first = left > 0 ? 0 : c0;
+        if (c1 > first) {
+            laswp_kernel<T, C><<<(unsigned)((c1 - first + 255) / 256), 256, 0, st>>>(A, lda, first, c1, left, c0, k0, nb, piv);
             ctx->launches++;
         }
-        laswp_kernel<T, C><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(A, lda, ni, k0i, nb, piv);
+        const int cols = c1 - c0, k1 = k0 + nb;
+        if (cols <= 0) return BEM_OK;
+        trsm_kernel<T, C><<<(unsigned)((cols + TRSM_COLS - 1) / TRSM_COLS), TRSM_COLS * TRSM_ROWS,
+                            sizeof(El<T, C>) * nb * (nb + TRSM_COLS), st>>>(A, lda, c0, c1, k0, nb);
         ctx->launches++;
-        int64_t rest = n - k0 - nb;
-        if (rest > 0) {
-            size_t tsmem = sizeof(El<T, C>) * nb * (nb + TRSM_COLS);
-            cudaFuncSetAttribute(trsm_kernel<T, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsmem);
-            trsm_kernel<T, C><<<(unsigned)((rest + TRSM_COLS - 1) / TRSM_COLS), TRSM_COLS * TRSM_ROWS, tsmem, s>>>(
-                A, lda, ni, k0i, nb);
-            ctx->launches++;
-            // A22 -= L21 U12
-            T* A22 = A + (C ? 2 : 1) * ((k0 + nb) * lda + k0 + nb);
-            const T* L21 = A + (C ? 2 : 1) * ((k0 + nb) * lda + k0);
-            const T* U12 = A + (C ? 2 : 1) * (k0 * lda + k0 + nb);
-            if (int rc = bem_gemm_update<T, C>(ctx, A22, L21, U12, rest, rest, nb, lda, s)) return rc;
+        // A22 -= L21 U12
+        auto at = [&](int64_t r, int64_t c) { return A + (C ? 2 : 1) * (r * lda + c); };
+        return bem_gemm_update<T, C>(ctx, at(k1, c0), at(k1, k0), at(k0, c0), n - k1, cols, nb, lda, st);
+    };
+    auto steps = [&]() -> int {
+        for (int64_t k0 = 0; k0 < n; k0 += LU_NB) {
+            int nb = (int)std::min<int64_t>(LU_NB, n - k0);
+            int rows = (int)(n - k0);
+            int ni = (int)n, k0i = (int)k0;
+            const int rc = lu_panel_cluster<T, C>(ctx, A, lda, ni, k0i, nb, piv, info, flag, w.src, sp);
+            if (rc < 0) return rc;
+            if (rc == 1) {
+                // the panel does not fit a cluster's shared memory
+                order(sp, ctx->ev_diag, s);
+                int blocks = std::min(nblk, std::max(1, (rows + 31) / 32));
+                int chunk = (rows + blocks - 1) / blocks;
+                El<T, C>* rb = (El<T, C>*)w.rowbuf;
+                size_t smem = use_smem ? sizeof(El<T, C>) * (size_t)chunk * LU_NB : 0;
+                void* args[] = {&A, &lda, &ni, &k0i, &nb, &chunk, &piv, &info, &w.bar, &w.slots, &rb, &flag};
+                if (int e = bem_check_cuda(ctx, cudaLaunchCooperativeKernel(pk, blocks, threads, args, smem, s),
+                                           "lu_panel_kernel"))
+                    return e;
+                ctx->launches++;
+                order(s, ctx->ev_next, sp);
+            }
+            const int k1 = k0i + nb, k2 = ahead ? std::min(ni, k1 + LU_NB) : k1;
+            order(sp, ctx->ev_diag, s);
+            if (k2 > k1) {
+                // the columns' earlier updates ran on s
+                if (ahead) cudaStreamWaitEvent(sp, ctx->ev_next, 0);
+                if constexpr (sizeof(T) == 8) {
+                    if (int e = rc == 1 ? apply(k0i, nb, 0, k1, k2, sp)
+                                        : lu_next<C>(ctx, A, lda, ni, k0i, k1, k2, w.src, sp))
+                        return e;
+                }
+            }
+            if (int e = apply(k0i, nb, k0i, k2, ni, s)) return e;
+            if (ahead) cudaEventRecord(ctx->ev_next, s);
+            if (int e = bem_check_cuda(ctx, cudaGetLastError(), "lu step")) return e;
         }
-        if (int rc = bem_check_cuda(ctx, cudaGetLastError(), "lu step")) return rc;
-    }
+        return BEM_OK;
+    };
+    order(s, ctx->ev_next, sp);
+    const int rc = steps();
+    order(sp, ctx->ev_diag, s);
+    if (rc) return rc;
     return check_flag(ctx, s, "lu_factor");
 }
 

@@ -131,6 +131,30 @@ def test_lu_panel_sizes(engine, n, dtype):
     assert np.abs(_swapped(A, piv) - low @ up).max() < tol
 
 
+@pytest.mark.parametrize("n,dtype", [(129, "float64"), (1000, "complex128"), (2113, "float64"), (3300, "complex128")])
+def test_lu_look_ahead(engine, n, dtype):
+    """The next panel beside the update: the same factors every time, bit for
+    bit (no race), also where the first panels are too large for a cluster
+    (3300 complex rows), and P A = L U as in test_lu_panel_sizes."""
+    torch.manual_seed(n)
+    A = torch.randn(n, n, dtype=getattr(torch, dtype), device="cuda")
+    runs = []
+    for _ in range(3):
+        LU = A.clone()
+        piv, info = engine.lu_factor(LU)
+        assert int(info.item()) == 0
+        runs.append((LU, piv))
+    F, piv = runs[0]
+    for LU, p in runs[1:]:
+        assert torch.equal(p, piv) and torch.equal(LU, F)
+    perm = np.arange(n)
+    for i, p in enumerate(piv.cpu().numpy()):
+        perm[[i, p]] = perm[[p, i]]
+    low, up = torch.tril(F, -1) + torch.eye(n, dtype=F.dtype, device="cuda"), torch.triu(F)
+    err = (A[torch.as_tensor(perm, device="cuda")] - low @ up).abs().max()
+    assert float(err) < 4 * n * 2.3e-16 * float(up.abs().max())
+
+
 def test_lu_pivots_match_the_textbook(engine):
     """The pivot sequence of a matrix with ties and exact zeros: the lowest
     row of the largest |re| + |im|."""
