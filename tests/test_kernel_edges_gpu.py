@@ -409,6 +409,54 @@ def test_lu_of_an_unaligned_complex_matrix(engine):
     assert float((raw[1:] - torch.view_as_real(A).reshape(-1)).abs().max()) < n * 2.3e-16 * float(A.abs().max())
 
 
+# ---- products with dense matrices ------------------------------------------------------
+@pytest.mark.parametrize("dtype", ["float64", "complex128", "float32", "complex64"])
+@pytest.mark.parametrize("m,n", [(1, 1), (9, 31), (8, 128), (65, 129), (70, 256), (3, 517)])
+def test_gemv_remainders(engine, m, n, dtype):
+    """Around the unrolled part of a row (4 or 8 x 32 elements), rows further
+    apart than they are long, complex data at odd multiples of 8 bytes: FP64
+    sums of n terms, n eps times the sum of magnitudes."""
+    import ctypes
+    cplx = dtype.startswith("complex")
+    A = torch.as_tensor(_gaussian((m, n + 3), cplx, n), device="cuda").to(getattr(torch, dtype))[:, :n]
+    x = _gaussian(n, cplx, m + n)
+    y0 = _gaussian(m, cplx, 3)
+    a = A.cpu().numpy().astype(x.dtype)
+    bound = 2 * (n + 4) * 2.3e-16 * (np.abs(a) @ np.abs(x) + np.abs(y0)).max()
+    want = 0.5 * y0 - 2.0 * a @ x
+    y = torch.as_tensor(y0.copy(), device="cuda")
+    engine.gemv(A, torch.as_tensor(x, device="cuda"), y, alpha=-2.0, beta=0.5)
+    assert np.abs(y.cpu().numpy() - want).max() <= bound
+    if dtype == "complex128":
+        raw = torch.zeros(2 * n + 1, dtype=torch.float64, device="cuda")
+        raw[1:] = torch.view_as_real(torch.as_tensor(x, device="cuda")).reshape(-1)
+        y = torch.as_tensor(y0.copy(), device="cuda")
+        rc = engine.lib.bem_gemv(engine.ctx, 1, ctypes.c_void_p(A.data_ptr()), m, n, A.stride(0),
+                                 ctypes.c_void_p(raw.data_ptr() + 8), ctypes.c_void_p(y.data_ptr()), -2.0, 0.5,
+                                 ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+        assert rc == 0 and np.abs(y.cpu().numpy() - want).max() <= bound
+
+
+@pytest.mark.parametrize("cplx", [False, True])
+@pytest.mark.parametrize("n", [1, 3, 31, 33, 100, 257])
+def test_lstsq_products_remainders(engine, n, cplx):
+    """min |[A; P] x - b| at sizes around the row chunks of the adjoint
+    product (32 rows, 4 at a time): A and P well conditioned (3 I + noise of
+    norm about 1), so the refined solution is the least squares one to about
+    1e-10."""
+    A, P = (3.0 * np.eye(n) + _gaussian((n, n), cplx, n + i) / (3 * np.sqrt(n)) for i in (1, 2))
+    b = _gaussian(2 * n, cplx, 7)
+    A_, P_ = (torch.as_tensor(M, device="cuda").to(torch.complex128 if cplx else torch.float64) for M in (A, P))
+    N = torch.empty_like(A_)
+    d = torch.empty(n, dtype=torch.float64, device="cuda")
+    engine.gram(A_, P_, N, d, tensor_cores=False)
+    piv, dinv, _ = engine.chol_factor(N, tensor_cores=False)
+    x = torch.zeros(n, dtype=A_.dtype, device="cuda")
+    engine.lstsq_refine(A_, P_, d, N, piv, dinv, torch.as_tensor(b, device="cuda").to(A_.dtype), x)
+    want = np.linalg.lstsq(np.vstack([A, P]), b, rcond=None)[0]
+    assert np.abs(x.cpu().numpy() - want).max() < 1e-10 * max(1.0, np.abs(want).max())
+
+
 # ---- both wavenumbers of the Calderon sweep over lane pairs ---------------------------
 @pytest.mark.parametrize("ks", [(0.1, 0.05), (1.2, 0.4), (30.0, 45.0), (0.7, -0.3)])
 @pytest.mark.parametrize("Q", [1, 2, 3])
