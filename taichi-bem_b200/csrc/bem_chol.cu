@@ -186,8 +186,8 @@ __global__ void __launch_bounds__(256) chol64_kernel(double* A, int64_t lda, int
 // triangular, tri & 2: op(B) is upper triangular; the K range of a tile then
 // ends at its diagonal.
 //
-// 64 x 64 entries per CTA, eight warps of 32 x 16 (4 x 2 fragments of 8 x 8;
-// complex: four real products per complex one), K in stages of 8 that cp.async
+// BM x 64 entries per CTA (BM = 64 or 32), eight warps of BM / 2 x 16 (4 or 2 x
+// 2 fragments of 8 x 8; complex: four real products per complex one), K in stages of 8 that cp.async
 // brings straight into shared memory, DG_STAGES deep, one CTA barrier a stage.
 // The factorisations call this with K = 64 and 256, so a CTA lives for 8 to 32
 // stages: depth, two CTAs per SM and C on its way into L2 are what keep the
@@ -198,7 +198,7 @@ __global__ void __launch_bounds__(256) chol64_kernel(double* A, int64_t lda, int
 // Measured (B200, against one stage prefetched in registers and two barriers a
 // stage): the trailing updates of a 2999 complex LU (K = 64) 3.3 against 4.0 ms
 // (22 against 18 TFLOP/s), those inside the panels of a 7682 complex Cholesky
-// (K = 64 and 256) 6.0 against 6.9 ms.
+// (K = 64 and 256) 6.0 against 6.9 ms (5.7 with 32-row tiles where few).
 constexpr int DG_BM = 64, DG_BK = 8, DG_STAGES = 4;
 constexpr int DG_OVERWRITE = 4;  // flag beside the triangular ones; C may then be A where n <= 64 (a CTA reads only its rows)
 template <bool CPLX>
@@ -229,7 +229,7 @@ __device__ __forceinline__ void cp_entry(double* dst, const double* src, bool ok
     if (CPLX) asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d + 8), "l"(src + 1), "r"(bytes) : "memory");
 }
 
-template <bool CPLX, bool CONJA, bool CONJT, bool LOWER>
+template <bool CPLX, bool CONJA, bool CONJT, bool LOWER, int BM>
 __global__ void __launch_bounds__(256, 2) dmma_gemm_kernel(double* Cm, int64_t ldc,
                                                             const double* Am, int64_t lda,
                                                             const double* __restrict__ Bm, int64_t ldb, int64_t m,
@@ -237,24 +237,25 @@ __global__ void __launch_bounds__(256, 2) dmma_gemm_kernel(double* Cm, int64_t l
                                                             int tri, int al) {
     using Tile = DgTile<CPLX>;
     constexpr int W = Tile::W, LD = Tile::LD, NP = CPLX ? 2 : 1;
+    constexpr int FA = BM / 16;  // fragments of a warp along the rows
     extern __shared__ __align__(16) double dg_smem[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int64_t m0 = (int64_t)blockIdx.y * DG_BM, n0 = (int64_t)blockIdx.x * DG_BM;
-    if (LOWER && n0 > m0 + DG_BM - 1 + diag) return;
+    const int64_t m0 = (int64_t)blockIdx.y * BM, n0 = (int64_t)blockIdx.x * DG_BM;
+    if (LOWER && n0 > m0 + BM - 1 + diag) return;
     const int wr = warp & 1, wc = warp >> 1;
     const bool overwrite = (tri & DG_OVERWRITE) != 0;  // C = alpha op(A) op(B)
     const bool vec_c = CPLX && (reinterpret_cast<uintptr_t>(Cm) & 15) == 0;
-    double acc[4][2][NP][2];
+    double acc[FA][2][NP][2];
     auto c_entry = [&](int a, int b, int e, bool& ok) -> double* {
-        const int64_t gr = m0 + 32 * wr + 8 * a + (lane >> 2), gc = n0 + 16 * wc + 8 * b + 2 * (lane & 3) + e;
+        const int64_t gr = m0 + BM / 2 * wr + 8 * a + (lane >> 2), gc = n0 + 16 * wc + 8 * b + 2 * (lane & 3) + e;
         ok = gr < m && gc < n;
         return Cm + W * (gr * ldc + gc);
     };
     const int kbeg = (int)blockIdx.z * kchunk;
     int kend = min(k, kbeg + kchunk);
-    if (tri & 1) kend = (int)min((int64_t)kend, m0 + DG_BM);
+    if (tri & 1) kend = (int)min((int64_t)kend, m0 + BM);
     if (tri & 2) kend = (int)min((int64_t)kend, n0 + DG_BM);
-    // an operand's 64 entries x 8 k of a stage, two per thread, along its rows in memory:
+    // an operand's 64 (A: BM) entries x 8 k of a stage, two (one) per thread, along its rows in memory:
     // stored with k contiguous (A, B^H): k = tid % 8, entry tid / 8 + 32 h; otherwise entry tid % 64, k = tid / 64 + 4 h
     auto stage = [&](int slot, int k0) {
         double* sA = dg_smem + (size_t)slot * 2 * Tile::OPERAND;
@@ -263,8 +264,8 @@ __global__ void __launch_bounds__(256, 2) dmma_gemm_kernel(double* Cm, int64_t l
         for (int h = 0; h < 2; ++h) {
             const int kc = tid & 7, ec = (tid >> 3) + 32 * h;  // k contiguous
             const int ks = (tid >> 6) + 4 * h, es = tid & 63;  // entries contiguous
-            {
-                const int kk = CONJA ? ks : kc, e = CONJA ? es : ec;
+            if (32 * h < BM) {
+                const int kk = !CONJA ? kc : (BM == 64 ? ks : tid >> 5), e = !CONJA ? ec : (BM == 64 ? es : tid & 31);
                 const int64_t gr = m0 + e;
                 const int gk = k0 + kk;
                 const bool ok = gr < m && gk < kend;
@@ -288,7 +289,7 @@ __global__ void __launch_bounds__(256, 2) dmma_gemm_kernel(double* Cm, int64_t l
         asm volatile("cp.async.commit_group;" ::: "memory");
     }
 #pragma unroll
-    for (int a = 0; a < 4; ++a)
+    for (int a = 0; a < FA; ++a)
 #pragma unroll
         for (int b = 0; b < 2; ++b) {
 #pragma unroll
@@ -309,10 +310,10 @@ __global__ void __launch_bounds__(256, 2) dmma_gemm_kernel(double* Cm, int64_t l
 #pragma unroll
         for (int k4 = 0; k4 < DG_BK; k4 += 4) {
             const int kr = k4 + (lane & 3);
-            double fa[4][NP], fb[2][NP];
+            double fa[FA][NP], fb[2][NP];
 #pragma unroll
-            for (int a = 0; a < 4; ++a) {
-                const double* e = sA + W * (kr * LD + 32 * wr + 8 * a + (lane >> 2));
+            for (int a = 0; a < FA; ++a) {
+                const double* e = sA + W * (kr * LD + BM / 2 * wr + 8 * a + (lane >> 2));
                 if (CPLX) {
                     const double2 v = *reinterpret_cast<const double2*>(e);
                     fa[a][0] = v.x;
@@ -333,7 +334,7 @@ __global__ void __launch_bounds__(256, 2) dmma_gemm_kernel(double* Cm, int64_t l
                 }
             }
 #pragma unroll
-            for (int a = 0; a < 4; ++a)
+            for (int a = 0; a < FA; ++a)
 #pragma unroll
                 for (int b = 0; b < 2; ++b) {
                     dmma(acc[a][b][0][0], acc[a][b][0][1], fa[a][0], fb[b][0]);
@@ -348,7 +349,7 @@ __global__ void __launch_bounds__(256, 2) dmma_gemm_kernel(double* Cm, int64_t l
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     const bool add = gridDim.z == 1 && !overwrite;
 #pragma unroll
-    for (int a = 0; a < 4; ++a) {
+    for (int a = 0; a < FA; ++a) {
         double old[2][2][NP];  // one row of fragments: its loads together
 #pragma unroll
         for (int b = 0; b < 2; ++b)
@@ -419,31 +420,43 @@ __global__ void iota_kernel(int32_t* piv, int n) {
     if (i < n) piv[i] = i;
 }
 
-// C += alpha op(A) op(B) (see dmma_gemm_kernel); products with fewer tiles
-// than two waves of CTAs split K into ranges of at least 512.
-template <bool C, bool CONJA, bool CONJT, bool LOWER>
-int gemm64x(bem_ctx* ctx, double* Cm, int64_t ldc, const double* A, int64_t lda, const double* B, int64_t ldb,
-            int64_t m, int64_t n, int k, double alpha, int64_t diag, cudaStream_t s, int tri = 0) {
-    if (m <= 0 || n <= 0 || k <= 0) return BEM_OK;
-    dim3 grid((unsigned)((n + DG_BM - 1) / DG_BM), (unsigned)((m + DG_BM - 1) / DG_BM));
-    if (grid.y > 65535) return bem_fail(ctx, BEM_ERR_INVALID, "dmma_gemm_kernel: m too large");
-    const int64_t tiles = (int64_t)grid.x * grid.y;
-    int splits = 1;
-    if (!LOWER && !(tri & DG_OVERWRITE) && tiles < 2 * (int64_t)ctx->num_sms)
-        splits = (int)std::max<int64_t>(1, std::min<int64_t>((2 * ctx->num_sms) / tiles, k / 512));
+// One launch of dmma_gemm_kernel with tiles of BM x 64; `splits` ranges of K.
+template <bool C, bool CONJA, bool CONJT, bool LOWER, int BM>
+int gemm64_launch(bem_ctx* ctx, double* Cm, int64_t ldc, const double* A, int64_t lda, const double* B, int64_t ldb,
+                  int64_t m, int64_t n, int k, double alpha, int64_t diag, int tri, int splits, cudaStream_t s) {
+    dim3 grid((unsigned)((n + DG_BM - 1) / DG_BM), (unsigned)((m + BM - 1) / BM));
     const int kchunk = (int)(((int64_t)k + splits - 1) / splits + DG_BK - 1) / DG_BK * DG_BK;
     grid.z = (unsigned)(((int64_t)k + kchunk - 1) / kchunk);
     constexpr size_t smem = DgTile<C>::SMEM;
-    if (int rc = bem_check_cuda(ctx, cudaFuncSetAttribute(dmma_gemm_kernel<C, CONJA, CONJT, LOWER>,
+    if (int rc = bem_check_cuda(ctx, cudaFuncSetAttribute(dmma_gemm_kernel<C, CONJA, CONJT, LOWER, BM>,
                                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
                                 "dmma_gemm_kernel smem"))
         return rc;
     // 16-byte copies of complex entries need 16-byte aligned operands
     const int al = ((uintptr_t)A | (uintptr_t)B) % 16 == 0 ? 1 : 0;
-    dmma_gemm_kernel<C, CONJA, CONJT, LOWER><<<grid, 256, smem, s>>>(Cm, ldc, A, lda, B, ldb, m, n, k, alpha, diag,
-                                                                       kchunk, tri, al);
+    dmma_gemm_kernel<C, CONJA, CONJT, LOWER, BM><<<grid, 256, smem, s>>>(Cm, ldc, A, lda, B, ldb, m, n, k, alpha, diag,
+                                                                         kchunk, tri, al);
     ctx->launches++;
     return bem_check_cuda(ctx, cudaGetLastError(), "dmma_gemm_kernel");
+}
+
+// C += alpha op(A) op(B) (see dmma_gemm_kernel); products with fewer tiles
+// than two waves of CTAs split K into ranges of at least 512.  Tiles are 64
+// rows, or 32 where the 64-row tiles would not fill the SMs once: such a
+// product takes one tile's time, and half a tile's is shorter (K = 64
+// complex: L21 of the Cholesky 17.0 -> 10.6 us).
+template <bool C, bool CONJA, bool CONJT, bool LOWER>
+int gemm64x(bem_ctx* ctx, double* Cm, int64_t ldc, const double* A, int64_t lda, const double* B, int64_t ldb,
+            int64_t m, int64_t n, int k, double alpha, int64_t diag, cudaStream_t s, int tri = 0) {
+    if (m <= 0 || n <= 0 || k <= 0) return BEM_OK;
+    if ((m + DG_BM - 1) / DG_BM > 65535) return bem_fail(ctx, BEM_ERR_INVALID, "dmma_gemm_kernel: m too large");
+    const int64_t tiles = ((n + DG_BM - 1) / DG_BM) * ((m + DG_BM - 1) / DG_BM);
+    int splits = 1;
+    if (!LOWER && !(tri & DG_OVERWRITE) && tiles < 2 * (int64_t)ctx->num_sms)
+        splits = (int)std::max<int64_t>(1, std::min<int64_t>((2 * ctx->num_sms) / tiles, k / 512));
+    if (tiles <= ctx->num_sms && splits == 1)
+        return gemm64_launch<C, CONJA, CONJT, LOWER, 32>(ctx, Cm, ldc, A, lda, B, ldb, m, n, k, alpha, diag, tri, 1, s);
+    return gemm64_launch<C, CONJA, CONJT, LOWER, 64>(ctx, Cm, ldc, A, lda, B, ldb, m, n, k, alpha, diag, tri, splits, s);
 }
 
 template <bool C, bool CONJT, bool LOWER>

@@ -351,11 +351,12 @@ def test_tile_lu_zero_and_nan_columns(engine, col):
 # ---- FP64 tensor-core products --------------------------------------------------------------
 @pytest.mark.parametrize("cplx", [False, True])
 @pytest.mark.parametrize("conj_a,conj_b", [(False, False), (False, True), (True, False), (True, True)])
-@pytest.mark.parametrize("m,n,k", [(1, 1, 1), (63, 65, 7), (64, 64, 8), (130, 66, 33), (65, 129, 200), (70, 70, 1100)])
+@pytest.mark.parametrize("m,n,k", [(1, 1, 1), (63, 65, 7), (64, 64, 8), (130, 66, 33), (65, 129, 200), (70, 70, 1100),
+                                   (830, 770, 20)])
 def test_gemm_edges(engine, m, n, k, conj_a, conj_b, cplx):
     """C += alpha op(A) op(B) with leading dimensions beyond the widths, tiles
-    and stages partly filled, fewer stages than the ring, split K (k = 1100):
-    k eps max|A| max|B| sqrt-ish sums, 1e-13 k of the result."""
+    and stages partly filled, fewer stages than the ring, split K (k = 1100),
+    tiles of 32 rows and (more tiles than SMs) of 64: k eps max|A| max|B| sqrt-ish sums, 1e-13 k of the result."""
     dt = torch.complex128 if cplx else torch.float64
 
     def padded(r, c, seed):
