@@ -284,6 +284,11 @@ int bem_mass(bem_ctx* ctx, const bem_space* test, const bem_space* trial, int dt
  * field maps as in bem_assemble); nothing is stored by the forward pass. */
 int bem_adjoint_vertices(bem_ctx* ctx, const bem_op_desc* op, const bem_space* test, const bem_space* trial,
                          const double* lam, const double* u, double* grad, void* stream);
+/* The same, and (K only; data may be NULL) the derivative in the nodal data
+ * from the same quadrature points, accumulated (no reference counterpart):
+ *   data[c] += sum_r lam[r] K(r, c). */
+int bem_adjoint_vertices_data(bem_ctx* ctx, const bem_op_desc* op, const bem_space* test, const bem_space* trial,
+                              const double* lam, const double* u, double* grad, double* data, void* stream);
 
 /* ---- dense linear algebra (replaces torch.linalg.solve, BEM_manager.py:1056) --
  * LU with partial pivoting in place (row-major, n x n, lda).  dtype

@@ -37,7 +37,7 @@ EXPORTS = [
     "bem_adjoint_vertices", "bem_mesh_set_2d", "bem_gmres_ir", "bem_compute_color", "bem_set_mesh_instances",
     "bem_lu_factor_status", "bem_binary_version", "bem_ctx_set_tuning", "bem_assemble_calderon", "bem_gram",
     "bem_lstsq_refine", "bem_chol_factor", "bem_gemm", "bem_chol_inverse", "bem_normal_refine", "bem_near_pair_list",
-    "bem_assemble_batch", "bem_cgs2_append",
+    "bem_assemble_batch", "bem_cgs2_append", "bem_adjoint_vertices_data",
 ]
 STATIC_SOLVE_MAX_N = 32768  # BEM_STATIC_SOLVE_MAX_N
 TUNE_CALDERON_GROUP = 0  # BEM_TUNE_CALDERON_GROUP
@@ -133,6 +133,8 @@ def load():
     L.bem_set_mesh_instances.argtypes = [vp, vp, vp, vp, vp]
     L.bem_adjoint_vertices.argtypes = [vp, ctypes.POINTER(OpDesc), ctypes.POINTER(Space), ctypes.POINTER(Space), vp,
                                        vp, vp, vp]
+    L.bem_adjoint_vertices_data.argtypes = [vp, ctypes.POINTER(OpDesc), ctypes.POINTER(Space), ctypes.POINTER(Space),
+                                            vp, vp, vp, vp, vp]
     for name in EXPORTS:
         if name not in ("bem_last_error", "bem_launch_count", "bem_near_pair_count", "bem_lu_dinv_elems"):
             getattr(L, name).restype = ctypes.c_int

@@ -364,14 +364,18 @@ class Engine:
         self._check(self.lib.bem_ctx_set_tuning(self.ctx, int(key), int(value)))
 
     def adjoint_vertices(self, desc: L.OpDesc, test: DeviceSpace, trial: DeviceSpace, lam: torch.Tensor,
-                         u: torch.Tensor, grad: torch.Tensor):
-        """grad [nv, 3] += d/dX sum lam[r] A(r, c) u[c] (Laplace V or K, FP64)."""
+                         u: torch.Tensor, grad: torch.Tensor, data: torch.Tensor | None = None):
+        """grad [nv, 3] += d/dX sum lam[r] A(r, c) u[c] (Laplace V or K, FP64);
+        K: data[c] += sum lam[r] K(r, c), when given."""
         assert lam.dtype == torch.float64 and u.dtype == torch.float64 and grad.dtype == torch.float64
         assert lam.is_contiguous() and u.is_contiguous() and grad.is_contiguous() and grad.numel() == 3 * self.nv
         self._check_spaces(test, trial, lam.numel(), u.numel())
         ts, rs = test.c(), trial.c()
-        self._check(self.lib.bem_adjoint_vertices(self.ctx, ctypes.byref(desc), ctypes.byref(ts), ctypes.byref(rs),
-                                                  _ptr(lam), _ptr(u), _ptr(grad), _stream_ptr()))
+        if data is not None:
+            assert data.dtype == torch.float64 and data.is_contiguous() and data.numel() == u.numel()
+        self._check(self.lib.bem_adjoint_vertices_data(self.ctx, ctypes.byref(desc), ctypes.byref(ts),
+                                                       ctypes.byref(rs), _ptr(lam), _ptr(u), _ptr(grad), _ptr(data),
+                                                       _stream_ptr()))
         return grad
 
     def mass(self, test: DeviceSpace, trial: DeviceSpace, out=None, scale=1.0, out_t=None, scale_t=0.0, x=None,

@@ -113,9 +113,10 @@ class DirichletShape:
         eng = self.engine
         lam = self._solve_Vt(grad_t.to(torch.float64).contiguous())
         grad = torch.zeros(self.nv, 3, dtype=torch.float64, device=self.device)
-        # -d(lam^T V t)/dX and +d(lam^T K g)/dX from the adjoint kernels
+        # -d(lam^T V t)/dX and +d(lam^T K g)/dX from the adjoint kernels, w = K^T lam from the latter's points
+        w = torch.zeros(self.nv, dtype=torch.float64, device=self.device)
         eng.adjoint_vertices(self._desc(L.OP_V, "fp64"), self.P0, self.P0, (-lam).contiguous(), self._t, grad)
-        eng.adjoint_vertices(self._desc(L.OP_K, "fp64"), self.P0, self.P1, lam, self._g, grad)
+        eng.adjoint_vertices(self._desc(L.OP_K, "fp64"), self.P0, self.P1, lam, self._g, grad, w)
         # 1/2 d(lam^T M g)/dX: M_{i,b} = J_i / 6, dJ_i/dP_a = n_i x (P_{a+2} - P_{a+1})
         X = self._X
         P = X[self.tris]                                    # [nt, 3 vertices, 3]
@@ -126,10 +127,6 @@ class DirichletShape:
             e = P[:, (a + 2) % 3] - P[:, (a + 1) % 3]
             grad.index_add_(0, self.tris[:, a], s[:, None] * torch.linalg.cross(n, e))
         # data term: [(1/2 M + K)^T lam]_v grad u(X_v)
-        w = torch.zeros(self.nv, dtype=torch.float64, device=self.device)
-        Kt = torch.zeros(self.nt, self.nv, dtype=torch.float64, device=self.device)
-        eng.assemble(self._desc(L.OP_K, "fp64"), self.P0, self.P1, Kt)
-        w += Kt.transpose(0, 1) @ lam
         area6 = (torch.linalg.norm(nraw, dim=1) / 6.0) * lam  # (1/2 M)^T lam: 1/2 * J_i / 6 per panel vertex
         for a in range(3):
             w.index_add_(0, self.tris[:, a], 0.5 * area6)

@@ -72,12 +72,14 @@ struct PairMoments {
     double S0;        // sum w k
     double SX[3][3];  // sum w beta_a(xi) dk/dd        (test vertex a)
     double SY[3][3];  // sum w beta_b(eta) dk/dd       (trial vertex b, enters with -)
+    double SU[3];     // K: sum w (d_e . n_j)/(4 pi r^3) hat_b, the entries K(i, b)
     double SN[3];     // K: sum (w / J_j) u d_e / (4 pi r^3)   (derivative with respect to N_j)
     __device__ __forceinline__ void zero() {
         S0 = 0.0;
         for (int a = 0; a < 3; ++a)
             for (int c = 0; c < 3; ++c) SX[a][c] = SY[a][c] = 0.0;
         SN[0] = SN[1] = SN[2] = 0.0;
+        SU[0] = SU[1] = SU[2] = 0.0;
     }
     __device__ __forceinline__ void reduce() {
         S0 = warp_sum_d(S0);
@@ -86,16 +88,19 @@ struct PairMoments {
                 SX[a][c] = warp_sum_d(SX[a][c]);
                 SY[a][c] = warp_sum_d(SY[a][c]);
             }
-        for (int c = 0; c < 3; ++c) SN[c] = warp_sum_d(SN[c]);
+        for (int c = 0; c < 3; ++c) {
+            SN[c] = warp_sum_d(SN[c]);
+            SU[c] = warp_sum_d(SU[c]);
+        }
     }
 };
 
 // one point: d = x - y, weight w (with J_i J_j), barycentric weights bx, by,
-// trial density uy (K), argument sign sgn (the swapped coincide term of K),
+// trial hats hy and density uy (K; hy . data), argument sign sgn (the swapped coincide term of K),
 // 1/J_j (K)
 template <int OP>
 __device__ __forceinline__ void adj_point(PairMoments& M, const double d[3], double w, const double bx[3],
-                                          const double by[3], double uy, double sgn, const double nj[3],
+                                          const double by[3], const double hy[3], double uy, double sgn, const double nj[3],
                                           double invJj) {
     const double r2 = d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
     const double rinv = dev_rsqrt(r2);
@@ -112,6 +117,7 @@ __device__ __forceinline__ void adj_point(PairMoments& M, const double d[3], dou
         const double g3 = BEM_INV4PI * rinv * rinv2;  // 1/(4 pi r^3)
         const double wu = w * uy;
         M.S0 += wu * dn * g3;
+        for (int b = 0; b < 3; ++b) M.SU[b] += w * dn * g3 * hy[b];
         // d/dd [(d_e . n) g3(r)] = sgn [n g3 - 3 (d_e . n) d_e / (4 pi r^5)]
         for (int c = 0; c < 3; ++c) g[c] = sgn * wu * (nj[c] * g3 - 3.0 * dn * de[c] * g3 * rinv2);
         for (int c = 0; c < 3; ++c) M.SN[c] += wu * invJj * de[c] * g3;
@@ -149,6 +155,7 @@ struct AdjArgs {
     const double* lam;
     const double* u;
     double* grad;
+    double* data;  // K, optional: data[c] += sum_r lam[r] K(r, c)
 };
 
 __device__ __forceinline__ void load_tri(const AdjArgs& a, int g, double v[3][3], double n[3]) {
@@ -198,9 +205,16 @@ __device__ __forceinline__ void pair_grads(const PairMoments& M, double cw, cons
 // registers (capping K at 168 measured the same).  5120 panels, GaussQR 4
 // (B200): V 8.0 and K 14.3 ms, against 22 and 33 ms per ordered pair with the
 // hats of both sides applied at every point.
-template <int OP>
+//
+// DATA (K): the product K^T lam, the derivative in the nodal data, from the
+// same points.  d.n_i is constant over the test points and sum_q t d.n_j is
+// there already, so it costs nothing per point pair and six multiply-adds a
+// trial point: K 14.3 -> 15.1 ms, in place of a dense FP64 block and its
+// product (7.4 ms at 5120 panels, GaussQR 4).
+template <int OP, bool DATA>
 __global__ void __launch_bounds__(ADJ_THREADS) adj_far_kernel(AdjArgs a) {
     constexpr bool K = OP == BEM_OP_K;
+    static_assert(K || !DATA, "the data derivative is the double layer's");
     extern __shared__ __align__(16) unsigned char smem_raw[];
     double4* sx = reinterpret_cast<double4*>(smem_raw);             // [ti][Q2]
     double2* sp = reinterpret_cast<double2*>(sx + a.ti * a.Q2);    // [Q2] phi_1, phi_2
@@ -266,6 +280,7 @@ __global__ void __launch_bounds__(ADJ_THREADS) adj_far_kernel(AdjArgs a) {
         lamj = row >= 0 ? a.lam[row] : 0.0;
     }
     double gyacc[3][3] = {{0.0}};
+    double kyacc[3] = {0.0};  // DATA: K^T lam at the trial panel's hats
     const double4* ptsj = a.pts + (size_t)gj * Q2;
 
     for (int t = 0; t < a.ti; ++t) {
@@ -275,7 +290,7 @@ __global__ void __launch_bounds__(ADJ_THREADS) adj_far_kernel(AdjArgs a) {
         const double lami = s_lam[t], lamb = both ? lamj : 0.0;
         const bool live = valid_j && !(both && gi > gj) && (lami != 0.0 || lamb != 0.0) &&
                           bem_relation(s_tri[t], tri_j, gi == gj) == REL_SEPARATE;
-        double gx[3][3] = {{0.0}};
+        double gx[3][3] = {{0.0}}, kx[3] = {0.0};
         if (live) {
             double ni[3], D[3];
             for (int c = 0; c < 3; ++c) {
@@ -289,6 +304,7 @@ __global__ void __launch_bounds__(ADJ_THREADS) adj_far_kernel(AdjArgs a) {
             double S0 = 0.0;                                          // V: sum w/r
             double xa[3] = {0.0}, ya[3] = {0.0};                      // K: moments of A t (along n_j)
             double xb[3] = {0.0}, yb3[3] = {0.0};                     // K: moments of B t (along -n_i)
+            double kj[3] = {0.0}, ki[3] = {0.0};                      // DATA: hat moments of K_ij and of -K_ji
             double sij = 0.0, sji = 0.0, Nj[3] = {0.0}, Ni[3] = {0.0};  // K: J_i, J_j, N_j and N_i parts
             const double Dnj = D[0] * nj[0] + D[1] * nj[1] + D[2] * nj[2];
             const double Dni = D[0] * ni[0] + D[1] * ni[1] + D[2] * ni[2];
@@ -372,6 +388,10 @@ __global__ void __launch_bounds__(ADJ_THREADS) adj_far_kernel(AdjArgs a) {
                         yb3[m] = fma(wp[m] * lamb, tb[0], yb3[m]);
                         Nj[m] = fma(wA, td[m], Nj[m]);
                         Ni[m] = fma(-wB, tbd[m], Ni[m]);
+                        if (DATA) {
+                            kj[m] = fma(wp[m], tdn, kj[m]);
+                            ki[m] = fma(w * dni, ta[m], ki[m]);
+                        }
                     }
                 }
             }
@@ -415,6 +435,10 @@ __global__ void __launch_bounds__(ADJ_THREADS) adj_far_kernel(AdjArgs a) {
                     gx[h][c] = cw * (tx[c] + along * hx);
                     gyacc[h][c] += cw * (ty[c] - along * hy);
                 }
+                if (DATA) {
+                    kx[h] = -BEM_INV4PI * lamb * (h == 0 ? ki[0] - ki[1] - ki[2] : ki[h]);
+                    kyacc[h] += BEM_INV4PI * lami * (h == 0 ? kj[0] - kj[1] - kj[2] : kj[h]);
+                }
             }
         }
         // test-vertex gradients: reduce over the warp's trial panels
@@ -424,11 +448,24 @@ __global__ void __launch_bounds__(ADJ_THREADS) adj_far_kernel(AdjArgs a) {
             for (int b = 0; b < 3; ++b)
                 for (int c = 0; c < 3; ++c)
                     if (gx[b][c] != 0.0) atomicAdd(a.grad + 3 * s_tri[t][b] + c, gx[b][c]);
+        if (DATA && s_ri[t] >= 0) {  // uniform across the CTA
+            for (int b = 0; b < 3; ++b) kx[b] = warp_sum_d(kx[b]);
+            if (lane < 3) {
+                const int col = a.trial_dof[3 * s_ri[t] + lane];
+                const double v = lane == 0 ? kx[0] : lane == 1 ? kx[1] : kx[2];
+                if (col >= 0 && v != 0.0) atomicAdd(a.data + col, v);
+            }
+        }
     }
     if (valid_j)
         for (int b = 0; b < 3; ++b)
             for (int c = 0; c < 3; ++c)
                 if (gyacc[b][c] != 0.0) atomicAdd(a.grad + 3 * tri_j[b] + c, gyacc[b][c]);
+    if (DATA && valid_j)
+        for (int b = 0; b < 3; ++b) {
+            const int col = a.trial_dof[3 * lj + b];
+            if (col >= 0 && kyacc[b] != 0.0) atomicAdd(a.data + col, kyacc[b]);
+        }
 }
 
 // ---- near pairs: one warp per ordered pair of the near list ----
@@ -486,15 +523,17 @@ __global__ void __launch_bounds__(128) adj_near_kernel(AdjArgs a) {
         // P1 data at the trial point; the swapped twin of a coincident point has the
         // opposite normal derivative, with the data at the same point (quirk: the two
         // cancel) or at the test point's parameters, and V's same value
-        double ub = 1.0, w = wj;
+        double ub = 1.0, w = wj, hy[3] = {by[0], by[1], by[2]};
         if (OP == BEM_OP_K) {
             ub = by[0] * uj[0] + by[1] * uj[1] + by[2] * uj[2];
-            if (twin)
+            if (twin) {
                 ub -= quirk ? ub : sx_[sloty[0]] * uj[0] + sx_[sloty[1]] * uj[1] + sx_[sloty[2]] * uj[2];
+                for (int b = 0; b < 3; ++b) hy[b] -= quirk ? by[b] : sx_[sloty[b]];
+            }
         } else if (twin) {
             w = wj + wj;
         }
-        adj_point<OP>(M, d, w, bx, by, ub, 1.0, nj, invJj);
+        adj_point<OP>(M, d, w, bx, by, hy, ub, 1.0, nj, invJj);
     };
     NearDigits dg;
     const int Q = a.Q, Q4 = Q * Q * Q * Q;
@@ -515,12 +554,17 @@ __global__ void __launch_bounds__(128) adj_near_kernel(AdjArgs a) {
             atomicAdd(a.grad + 3 * ti[b] + c, gx[b][c]);
             atomicAdd(a.grad + 3 * tj[b] + c, gy[b][c]);
         }
+    if (OP == BEM_OP_K && a.data)
+        for (int b = 0; b < 3; ++b) {
+            const int col = a.trial_dof[3 * lj + b];
+            if (col >= 0) atomicAdd(a.data + col, lam * M.SU[b]);
+        }
 }
 
 }  // namespace
 
 int bem_launch_adjoint(bem_ctx* ctx, const bem_op_desc* op, const bem_space* test, const bem_space* trial,
-                       const double* lam, const double* u, double* grad, cudaStream_t s) {
+                       const double* lam, const double* u, double* grad, double* data, cudaStream_t s) {
     if (int rc = bem_fill_local_map(ctx, test, ctx->test_local, s)) return rc;
     if (int rc = bem_fill_local_map(ctx, trial, ctx->trial_local, s)) return rc;
     AdjArgs a;
@@ -550,6 +594,7 @@ int bem_launch_adjoint(bem_ctx* ctx, const bem_op_desc* op, const bem_space* tes
     a.lam = lam;
     a.u = u;
     a.grad = grad;
+    a.data = data;
     // as in bem_launch_far64: fewer test panels per CTA where the call has too few CTAs for some waves
     a.ti = ADJ_TI;
     const int64_t cols = (a.n_trial + ADJ_THREADS - 1) / ADJ_THREADS;
@@ -559,10 +604,13 @@ int bem_launch_adjoint(bem_ctx* ctx, const bem_op_desc* op, const bem_space* tes
     const unsigned nblocks = (unsigned)((a.n_near + 3) / 4);
     if (a.n_test > 0 && a.n_trial > 0) {
         if (op->op == BEM_OP_V) {
-            adj_far_kernel<BEM_OP_V><<<fgrid, ADJ_THREADS, smem, s>>>(a);
+            adj_far_kernel<BEM_OP_V, false><<<fgrid, ADJ_THREADS, smem, s>>>(a);
             if (nblocks) adj_near_kernel<BEM_OP_V><<<nblocks, 128, 0, s>>>(a);
         } else {
-            adj_far_kernel<BEM_OP_K><<<fgrid, ADJ_THREADS, smem, s>>>(a);
+            if (data)
+                adj_far_kernel<BEM_OP_K, true><<<fgrid, ADJ_THREADS, smem, s>>>(a);
+            else
+                adj_far_kernel<BEM_OP_K, false><<<fgrid, ADJ_THREADS, smem, s>>>(a);
             if (nblocks) adj_near_kernel<BEM_OP_K><<<nblocks, 128, 0, s>>>(a);
         }
         ctx->launches += nblocks ? 2 : 1;

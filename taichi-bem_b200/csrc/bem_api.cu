@@ -493,6 +493,11 @@ int bem_mass(bem_ctx* ctx, const bem_space* test, const bem_space* trial, int dt
 
 int bem_adjoint_vertices(bem_ctx* ctx, const bem_op_desc* op, const bem_space* test, const bem_space* trial,
                          const double* lam, const double* u, double* grad, void* stream) {
+    return bem_adjoint_vertices_data(ctx, op, test, trial, lam, u, grad, nullptr, stream);
+}
+
+int bem_adjoint_vertices_data(bem_ctx* ctx, const bem_op_desc* op, const bem_space* test, const bem_space* trial,
+                              const double* lam, const double* u, double* grad, double* data, void* stream) {
     if (!ctx) return BEM_ERR_INVALID;
     if (ctx->nt == 0) return bem_fail(ctx, BEM_ERR_NOMESH, "no mesh set");
     if (!op || !lam || !u || !grad) return bem_fail(ctx, BEM_ERR_INVALID, "adjoint: null argument");
@@ -503,7 +508,8 @@ int bem_adjoint_vertices(bem_ctx* ctx, const bem_op_desc* op, const bem_space* t
     if (int rc = check_space(ctx, trial, "trial")) return rc;
     if (test->nb != 1 || trial->nb != (op->op == BEM_OP_V ? 1 : 3))
         return bem_fail(ctx, BEM_ERR_INVALID, "adjoint: V needs P0 x P0 spaces, K a P0 test and a P1 trial space");
-    return bem_launch_adjoint(ctx, op, test, trial, lam, u, grad, (cudaStream_t)stream);
+    if (data && op->op != BEM_OP_K) return bem_fail(ctx, BEM_ERR_INVALID, "adjoint: the data derivative is K's");
+    return bem_launch_adjoint(ctx, op, test, trial, lam, u, grad, data, (cudaStream_t)stream);
 }
 
 }  // extern "C"

@@ -101,7 +101,7 @@ int bem_tiled_precond_async(bem_ctx* ctx, int dtype, const void* LU, int64_t n, 
 int bem_launch_geometry(bem_ctx* ctx, cudaStream_t s);
 int bem_fill_local_map(bem_ctx* ctx, const bem_space* sp, int32_t* map, cudaStream_t s);
 int bem_launch_adjoint(bem_ctx* ctx, const bem_op_desc* op, const bem_space* test, const bem_space* trial,
-                       const double* lam, const double* u, double* grad, cudaStream_t s);
+                       const double* lam, const double* u, double* grad, double* data, cudaStream_t s);
 int bem_lookahead_stream(bem_ctx* ctx);
 int bem_launch_assemble(bem_ctx* ctx, const bem_op_desc* op, const bem_space* test, const bem_space* trial,
                         int mode, void* out, int64_t ld, double scale, void* out_t, double scale_t, const void* x,

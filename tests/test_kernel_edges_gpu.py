@@ -266,6 +266,38 @@ def test_adjoint_over_partial_lists(engine, op, nby):
         assert abs(fd - grad[i, c]) < 1e-6 * np.abs(grad).max()
 
 
+@pytest.mark.parametrize("quirk", [True, False])
+@pytest.mark.parametrize("Q", [1, 4, 12])
+def test_adjoint_data_derivative(engine, Q, quirk):
+    """data += K^T lam beside the vertex gradient, over lists that overlap in
+    part with skipped dofs and zeros in lam, against the assembled block: the
+    same points in another order, sums of at most 162 entries: 1e-12 of the
+    largest; the gradient as without it (atomic order: 1e-12)."""
+    from bem_b200 import _lib as L
+    from bem_b200 import icosphere
+    from bem_b200.engine import DeviceSpace
+    v, f = icosphere(1)
+    v = v * (1.0 + 0.05 * np.sin(3.0 * v[:, :1]))
+    engine.set_mesh(v, f, Q)
+    td, rd = (DeviceSpace.from_numpy(*_partial_space(f, len(v), nb, c, s), engine.device)
+              for nb, c, s in ((1, 50, 3), (3, 66, 4)))
+    gen = torch.Generator(device="cuda").manual_seed(8)
+    lam = torch.randn(len(f), dtype=torch.float64, device="cuda", generator=gen)
+    lam[::7] = 0.0
+    u = torch.randn(len(v), dtype=torch.float64, device="cuda", generator=gen)
+    u[::5] = 0.0
+    desc = engine.op_desc(L.OP_K, False, quirk=quirk)
+    K = torch.zeros(len(f), len(v), dtype=torch.float64, device="cuda")
+    engine.assemble(desc, td, rd, K)
+    grads = [torch.zeros(len(v), 3, dtype=torch.float64, device="cuda") for _ in range(2)]
+    data = torch.ones(len(v), dtype=torch.float64, device="cuda")
+    engine.adjoint_vertices(desc, td, rd, lam, u, grads[0], data)
+    engine.adjoint_vertices(desc, td, rd, lam, u, grads[1])
+    ref = 1.0 + (lam[:, None] * K).sum(0)
+    assert float((data - ref).abs().max()) < 1e-12 * float(ref.abs().max())
+    assert float((grads[0] - grads[1]).abs().max()) < 1e-12 * float(grads[1].abs().max())
+
+
 # ---- near pairs ------------------------------------------------------------------------------
 @pytest.mark.parametrize("quirk", [True, False])
 @pytest.mark.parametrize("Q", [1, 2, 3, 6])
