@@ -11,8 +11,8 @@
 // the split phase argument, the basis weights) is formed once and only
 // e^{ikr} and the accumulation run per wavenumber.  The layout follows the
 // single-wavenumber far kernel (bem_assembly.cu): one thread per (test
-// panel, trial panel) pair, 128 trial panels per CTA, FAR_TI test panels'
-// points in shared memory, FP32 sums over the test points and FP64 sums over
+// panel, trial panel) pair, 128 trial panels per CTA, up to FAR_TI test
+// panels' points in shared memory, FP32 sums over the test points and FP64 sums over
 // the trial points in mixed precision (pair frame, bem_farfield.cuh), FP64
 // throughout on the plain path.  Coincident / edge / vertex pairs take the
 // FP64 Sauter-Schwab kernel, two wavenumbers per launch (bem_near.cu).
@@ -41,6 +41,7 @@ struct KbArgs {
     const void* phi;
     const double* phi64;
     int Q2;
+    int ti;  // test panels per CTA
     int dk;  // 1: the kernel's k-derivative at fixed k2 (as bem_assemble's deriv_k)
     int64_t ld;
     double k[KB_MAX], k2[KB_MAX], scale[KB_MAX], scale_t[KB_MAX];
@@ -81,8 +82,8 @@ __global__ void __launch_bounds__(FAR_THREADS) far_kbatch_kernel(KbArgs a) {
     constexpr bool W_OP = (OP == BEM_OP_W);
 
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    V4* sx = reinterpret_cast<V4*>(smem_raw);             // [FAR_TI][Q2]
-    T* sphi = reinterpret_cast<T*>(sx + FAR_TI * a.Q2);  // [Q2*3]
+    V4* sx = reinterpret_cast<V4*>(smem_raw);           // [ti][Q2]
+    T* sphi = reinterpret_cast<T*>(sx + a.ti * a.Q2);  // [Q2*3]
     __shared__ int s_gi[FAR_TI];
     __shared__ int s_tri[FAR_TI][3];
     __shared__ double s_cen[FAR_TI][3];
@@ -90,10 +91,10 @@ __global__ void __launch_bounds__(FAR_THREADS) far_kbatch_kernel(KbArgs a) {
 
     const int Q2 = a.Q2;
     const int lj = blockIdx.x * FAR_THREADS + threadIdx.x;
-    const int li0 = blockIdx.y * FAR_TI;
+    const int li0 = blockIdx.y * a.ti;
     const V4* pts = reinterpret_cast<const V4*>(a.pts);
 
-    for (int idx = threadIdx.x; idx < FAR_TI * Q2; idx += FAR_THREADS) {
+    for (int idx = threadIdx.x; idx < a.ti * Q2; idx += FAR_THREADS) {
         const int t = idx / Q2, q = idx - t * Q2;
         const int li = li0 + t;
         if (li < a.n_test) sx[idx] = pts[(size_t)a.test_panels[li] * Q2 + q];
@@ -102,7 +103,7 @@ __global__ void __launch_bounds__(FAR_THREADS) far_kbatch_kernel(KbArgs a) {
         const T* phi = reinterpret_cast<const T*>(a.phi);
         for (int idx = threadIdx.x; idx < Q2 * 3; idx += FAR_THREADS) sphi[idx] = phi[idx];
     }
-    if (threadIdx.x < FAR_TI) {
+    if (threadIdx.x < a.ti) {
         const int li = li0 + threadIdx.x;
         const int gi = li < a.n_test ? a.test_panels[li] : -1;
         s_gi[threadIdx.x] = gi;
@@ -131,7 +132,7 @@ __global__ void __launch_bounds__(FAR_THREADS) far_kbatch_kernel(KbArgs a) {
     const bool small = a.small_phase != 0;
     const bool dk = a.dk != 0;
 
-    for (int t = 0; t < FAR_TI; ++t) {
+    for (int t = 0; t < a.ti; ++t) {
         const int li = li0 + t;
         if (li >= a.n_test) break;  // uniform across the CTA
         const int gi = s_gi[t];
@@ -297,11 +298,19 @@ __global__ void __launch_bounds__(FAR_THREADS) far_kbatch_kernel(KbArgs a) {
 }
 
 template <int OP, int NBX, int NBY, typename T, int NKB>
-int launch_kb(bem_ctx* ctx, const KbArgs& a, cudaStream_t s) {
+int launch_kb(bem_ctx* ctx, KbArgs a, cudaStream_t s) {
     using V4 = typename V4T<T>::type;
-    dim3 grid((a.n_trial + FAR_THREADS - 1) / FAR_THREADS, (a.n_test + FAR_TI - 1) / FAR_TI);
+    // Fewer test panels per CTA where the call has too few CTAs for some waves
+    // (three fit an SM): with eight, 272 panels are 102 CTAs for 148 SMs.  All
+    // three operators of the sweep, GaussQR 3, FP64: 110 panels 2.60 -> 0.65 ms, 272
+    // panels 2.82 -> 1.45 ms (mixed 1.82 -> 1.07), 858 panels 2.78 -> 2.56 ms;
+    // 1280 panels and more are the same either way.
+    a.ti = FAR_TI;
+    const int64_t cols = (a.n_trial + FAR_THREADS - 1) / FAR_THREADS;
+    while (a.ti > 1 && cols * ((a.n_test + a.ti - 1) / a.ti) < 16 * (int64_t)ctx->num_sms) a.ti /= 2;
+    dim3 grid((unsigned)cols, (unsigned)((a.n_test + a.ti - 1) / a.ti));
     if (grid.y > 65535) return bem_fail(ctx, BEM_ERR_INVALID, "too many test panels for one launch");
-    const size_t smem = FAR_TI * a.Q2 * sizeof(V4) + a.Q2 * 3 * sizeof(T);
+    const size_t smem = a.ti * a.Q2 * sizeof(V4) + a.Q2 * 3 * sizeof(T);
     far_kbatch_kernel<OP, NBX, NBY, T, NKB><<<grid, FAR_THREADS, smem, s>>>(a);
     ctx->launches++;
     return bem_check_cuda(ctx, cudaGetLastError(), "far_kbatch_kernel launch");
