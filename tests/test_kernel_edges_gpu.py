@@ -298,6 +298,30 @@ def test_adjoint_data_derivative(engine, Q, quirk):
     assert float((grads[0] - grads[1]).abs().max()) < 1e-12 * float(grads[1].abs().max())
 
 
+@pytest.mark.parametrize("deriv_k", [False, True])
+@pytest.mark.parametrize("op", ["V", "W"])
+def test_batched_symmetric_blocks_over_partial_lists(engine, op, deriv_k):
+    """P1 x P1 blocks of three wavenumbers, lists that overlap in part with
+    skipped dofs, a transposed copy: against the one-wavenumber kernel, the
+    same FP64 terms in another order (sums of at most ~200): 1e-12."""
+    from bem_b200 import _lib as L
+    from bem_b200 import icosphere
+    from bem_b200.engine import DeviceSpace
+    v, f = icosphere(1)
+    engine.set_mesh(v, f, 3)
+    td, rd = (DeviceSpace.from_numpy(*_partial_space(f, len(v), 3, c, s), engine.device) for c, s in ((50, 3), (66, 4)))
+    ks, k2s, scales, scales_t = [0.7, 2.0, 9.0], [0.3, 4.0, 80.0], [1.0, -0.5, 2.0], [0.25, 1.5, -1.0]
+    desc = lambda k, k2: engine.op_desc(getattr(L, "OP_" + op), True, k, k2, deriv_k=deriv_k)
+    new = lambda: torch.zeros(len(v), len(v), dtype=torch.complex128, device="cuda")
+    outs, outs_t = [new() for _ in ks], [new() for _ in ks]
+    engine.assemble_batch(desc(0.7, 0.3), td, rd, ks, k2s, outs, scales, outs_t, scales_t)
+    for i in range(3):
+        ref, ref_t = new(), new()
+        engine.assemble(desc(ks[i], k2s[i]), td, rd, ref, scale=scales[i], out_t=ref_t, scale_t=scales_t[i])
+        for x, y in ((outs[i], ref), (outs_t[i], ref_t)):
+            assert float((x - y).abs().max()) < 1e-12 * float(y.abs().max())
+
+
 # ---- near pairs ------------------------------------------------------------------------------
 @pytest.mark.parametrize("quirk", [True, False])
 @pytest.mark.parametrize("Q", [1, 2, 3, 6])
