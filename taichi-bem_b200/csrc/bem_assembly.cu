@@ -24,6 +24,8 @@
 #include <cuda_runtime.h>
 
 #include "bem_internal.cuh"
+#include <type_traits>
+
 #include "bem_farfield.cuh"
 
 namespace {
@@ -188,6 +190,7 @@ __device__ __forceinline__ void kval_split(float r2, float s, float dn, float k,
 
 struct FarArgs {
     int n_test, n_trial;
+    int ti;  // test panels per CTA (far_kernel, far_vkg_sym_x2_kernel)
     const int32_t* test_panels;
     const int32_t* test_dof;
     const int32_t* trial_panels;
@@ -217,8 +220,9 @@ struct FarArgs {
 };
 
 
-template <int OP, bool HELM, int NBX, int NBY, typename T>
+template <int OP, bool HELM, int NBX, int NBY, typename T, bool FULL>
 __global__ void __launch_bounds__(FAR_THREADS) far_kernel(FarArgs a) {
+    const int ti = FULL ? FAR_TI : a.ti;
     using V4 = typename V4T<T>::type;
     constexpr bool W_OP = (OP == BEM_OP_W);
     // accumulate phi-weighted moments for every op except Laplace W, whose
@@ -228,8 +232,8 @@ __global__ void __launch_bounds__(FAR_THREADS) far_kernel(FarArgs a) {
     constexpr int AY = NEED_PHI ? NBY : 1;
 
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    V4* sx = reinterpret_cast<V4*>(smem_raw);                 // [FAR_TI][Q2]
-    T* sphi = reinterpret_cast<T*>(sx + FAR_TI * a.Q2);      // [Q2*3]
+    V4* sx = reinterpret_cast<V4*>(smem_raw);                 // [ti][Q2]
+    T* sphi = reinterpret_cast<T*>(sx + ti * a.Q2);      // [Q2*3]
     __shared__ int s_gi[FAR_TI];
     __shared__ int s_tri[FAR_TI][3];
     __shared__ double s_cen[FAR_TI][3];
@@ -237,10 +241,10 @@ __global__ void __launch_bounds__(FAR_THREADS) far_kernel(FarArgs a) {
 
     const int Q2 = a.Q2;
     const int lj = blockIdx.x * FAR_THREADS + threadIdx.x;
-    const int li0 = blockIdx.y * FAR_TI;
+    const int li0 = blockIdx.y * ti;
     const V4* pts = reinterpret_cast<const V4*>(a.pts);
 
-    for (int idx = threadIdx.x; idx < FAR_TI * Q2; idx += FAR_THREADS) {
+    for (int idx = threadIdx.x; idx < ti * Q2; idx += FAR_THREADS) {
         int t = idx / Q2, q = idx - t * Q2;
         int li = li0 + t;
         if (li < a.n_test) sx[idx] = pts[(size_t)a.test_panels[li] * Q2 + q];
@@ -249,7 +253,7 @@ __global__ void __launch_bounds__(FAR_THREADS) far_kernel(FarArgs a) {
         const T* phi = reinterpret_cast<const T*>(a.phi);
         for (int idx = threadIdx.x; idx < Q2 * 3; idx += FAR_THREADS) sphi[idx] = phi[idx];
     }
-    if (threadIdx.x < FAR_TI) {
+    if (threadIdx.x < ti) {
         int li = li0 + threadIdx.x;
         int gi = li < a.n_test ? a.test_panels[li] : -1;
         s_gi[threadIdx.x] = gi;
@@ -275,7 +279,7 @@ __global__ void __launch_bounds__(FAR_THREADS) far_kernel(FarArgs a) {
     const T kk = T(a.k);
     const int lane = threadIdx.x & 31;
 
-    for (int t = 0; t < FAR_TI; ++t) {
+    for (int t = 0; t < ti; ++t) {
         const int li = li0 + t;
         if (li >= a.n_test) break;  // uniform across the CTA
         const int gi = s_gi[t];
@@ -1025,16 +1029,17 @@ __device__ __forceinline__ void x2_trial_point(int P2, const float4* __restrict_
     }
 }
 
-template <bool HELM, int PH>
+template <bool HELM, int PH, bool FULL>
 __global__ void __launch_bounds__(FAR_THREADS, 5) far_vkg_sym_x2_kernel(FarArgs a, VkgArgs v) {
+    const int ti = FULL ? FAR_TI : a.ti;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int Q2 = a.Q2;
     const int P2 = (Q2 + 1) / 2;                                    // point pairs per panel
-    float4* sxy = reinterpret_cast<float4*>(smem_raw);              // [FAR_TI][P2] (x0 x1 y0 y1)
-    float4* szw = sxy + FAR_TI * P2;                                // [FAR_TI][P2] (z0 z1 w0 w1)
-    float4* sg = szw + FAR_TI * P2;                                 // [FAR_TI][P2] (re0 re1 im0 im1)
-    float2* sxx = reinterpret_cast<float2*>(sg + FAR_TI * P2);      // [FAR_TI][P2] (|x0|^2 |x1|^2)
-    float2* sdn = sxx + FAR_TI * P2;                                // [P2][FAR_THREADS] d.n_j of this thread's pair
+    float4* sxy = reinterpret_cast<float4*>(smem_raw);              // [ti][P2] (x0 x1 y0 y1)
+    float4* szw = sxy + ti * P2;                                // [ti][P2] (z0 z1 w0 w1)
+    float4* sg = szw + ti * P2;                                 // [ti][P2] (re0 re1 im0 im1)
+    float2* sxx = reinterpret_cast<float2*>(sg + ti * P2);      // [ti][P2] (|x0|^2 |x1|^2)
+    float2* sdn = sxx + ti * P2;                                // [P2][FAR_THREADS] d.n_j of this thread's pair
     float* sphi = reinterpret_cast<float*>(sdn + P2 * FAR_THREADS);  // [Q2*3]
     __shared__ int s_gi[FAR_TI];
     __shared__ int s_tri[FAR_TI][3];
@@ -1043,7 +1048,7 @@ __global__ void __launch_bounds__(FAR_THREADS, 5) far_vkg_sym_x2_kernel(FarArgs 
 
     const int n = a.n_test;  // == n_trial
     const int j0 = blockIdx.x * FAR_THREADS;
-    const int li0 = blockIdx.y * FAR_TI;
+    const int li0 = blockIdx.y * ti;
     if (j0 + FAR_THREADS - 1 <= li0) return;
     const int lj = j0 + threadIdx.x;
     const float4* pts = reinterpret_cast<const float4*>(a.pts);
@@ -1051,7 +1056,7 @@ __global__ void __launch_bounds__(FAR_THREADS, 5) far_vkg_sym_x2_kernel(FarArgs 
         const float* phi = reinterpret_cast<const float*>(a.phi);
         for (int idx = threadIdx.x; idx < Q2 * 3; idx += FAR_THREADS) sphi[idx] = phi[idx];
     }
-    if (threadIdx.x < FAR_TI) {
+    if (threadIdx.x < ti) {
         int li = li0 + threadIdx.x;
         int gi = li < n ? a.test_panels[li] : -1;
         s_gi[threadIdx.x] = gi;
@@ -1062,7 +1067,7 @@ __global__ void __launch_bounds__(FAR_THREADS, 5) far_vkg_sym_x2_kernel(FarArgs 
         }
     }
     __syncthreads();
-    for (int idx = threadIdx.x; idx < FAR_TI * P2; idx += FAR_THREADS) {
+    for (int idx = threadIdx.x; idx < ti * P2; idx += FAR_THREADS) {
         const int t = idx / P2, p = idx - t * P2;
         const int li = li0 + t;
         const int q0 = 2 * p, q1 = 2 * p + 1 < Q2 ? 2 * p + 1 : Q2 - 1;
@@ -1106,7 +1111,7 @@ __global__ void __launch_bounds__(FAR_THREADS, 5) far_vkg_sym_x2_kernel(FarArgs 
     float2* sdn_me = sdn + threadIdx.x;
     double rj_re = 0.0, rj_im = 0.0;
 
-    for (int t = 0; t < FAR_TI; ++t) {
+    for (int t = 0; t < ti; ++t) {
         const int li = li0 + t;
         if (li >= n) break;
         const int gi = s_gi[t];
@@ -1202,16 +1207,20 @@ __global__ void __launch_bounds__(FAR_THREADS, 5) far_vkg_sym_x2_kernel(FarArgs 
 }
 
 template <int OP, bool HELM, int NBX, int NBY>
-int launch_far(bem_ctx* ctx, const FarArgs& fa, bool fp32, cudaStream_t s) {
-    dim3 grid((fa.n_trial + FAR_THREADS - 1) / FAR_THREADS, (fa.n_test + FAR_TI - 1) / FAR_TI);
+int launch_far(bem_ctx* ctx, FarArgs fa, bool fp32, cudaStream_t s) {
+    fa.ti = fp32 ? bem_far_ti(ctx, fa.n_test, (fa.n_trial + FAR_THREADS - 1) / FAR_THREADS) : FAR_TI;
+    dim3 grid((fa.n_trial + FAR_THREADS - 1) / FAR_THREADS, (fa.n_test + fa.ti - 1) / fa.ti);
     if (grid.y > 65535) return bem_fail(ctx, BEM_ERR_INVALID, "too many test panels for one launch");
     if (fa.n_test <= 0 || fa.n_trial <= 0) return BEM_OK;
     if (fp32) {
-        const size_t smem = FAR_TI * fa.Q2 * sizeof(float4) + fa.Q2 * 3 * sizeof(float);
-        far_kernel<OP, HELM, NBX, NBY, float><<<grid, FAR_THREADS, smem, s>>>(fa);
+        const size_t smem = fa.ti * fa.Q2 * sizeof(float4) + fa.Q2 * 3 * sizeof(float);
+        if (fa.ti == FAR_TI)
+            far_kernel<OP, HELM, NBX, NBY, float, true><<<grid, FAR_THREADS, smem, s>>>(fa);
+        else
+            far_kernel<OP, HELM, NBX, NBY, float, false><<<grid, FAR_THREADS, smem, s>>>(fa);
     } else {
-        const size_t smem = FAR_TI * fa.Q2 * sizeof(double4) + fa.Q2 * 3 * sizeof(double);
-        far_kernel<OP, HELM, NBX, NBY, double><<<grid, FAR_THREADS, smem, s>>>(fa);
+        const size_t smem = fa.ti * fa.Q2 * sizeof(double4) + fa.Q2 * 3 * sizeof(double);
+        far_kernel<OP, HELM, NBX, NBY, double, true><<<grid, FAR_THREADS, smem, s>>>(fa);
     }
     ctx->launches++;
     return bem_check_cuda(ctx, cudaGetLastError(), "far_kernel launch");
@@ -1360,16 +1369,25 @@ int bem_launch_dirichlet(bem_ctx* ctx, const bem_op_desc* op, const bem_space* t
     if (fa.n_test > 0 && fa.n_trial > 0 && sym) {
         if (fp32) {
             const int P2 = (fa.Q2 + 1) / 2;
-            size_t smem = 3 * FAR_TI * P2 * sizeof(float4) + FAR_TI * P2 * sizeof(float2) +
+            fa.ti = bem_far_ti(ctx, fa.n_test, (int)grid.x);
+            grid.y = (fa.n_test + fa.ti - 1) / fa.ti;
+            size_t smem = 3 * fa.ti * P2 * sizeof(float4) + fa.ti * P2 * sizeof(float2) +
                           P2 * FAR_THREADS * sizeof(float2) + fa.Q2 * 3 * sizeof(float);
-            if (!helm)
-                far_vkg_sym_x2_kernel<false, 2><<<grid, FAR_THREADS, smem, s>>>(fa, va);
-            else if (fa.small_phase == 2)
-                far_vkg_sym_x2_kernel<true, 2><<<grid, FAR_THREADS, smem, s>>>(fa, va);
-            else if (fa.small_phase == 1)
-                far_vkg_sym_x2_kernel<true, 1><<<grid, FAR_THREADS, smem, s>>>(fa, va);
+            auto go = [&](auto full) {
+                constexpr bool FULL = decltype(full)::value;
+                if (!helm)
+                    far_vkg_sym_x2_kernel<false, 2, FULL><<<grid, FAR_THREADS, smem, s>>>(fa, va);
+                else if (fa.small_phase == 2)
+                    far_vkg_sym_x2_kernel<true, 2, FULL><<<grid, FAR_THREADS, smem, s>>>(fa, va);
+                else if (fa.small_phase == 1)
+                    far_vkg_sym_x2_kernel<true, 1, FULL><<<grid, FAR_THREADS, smem, s>>>(fa, va);
+                else
+                    far_vkg_sym_x2_kernel<true, 0, FULL><<<grid, FAR_THREADS, smem, s>>>(fa, va);
+            };
+            if (fa.ti == FAR_TI)
+                go(std::true_type{});
             else
-                far_vkg_sym_x2_kernel<true, 0><<<grid, FAR_THREADS, smem, s>>>(fa, va);
+                go(std::false_type{});
         } else {
             size_t smem = FAR_TI * fa.Q2 * (sizeof(double4) + 2 * sizeof(double)) + fa.Q2 * 3 * sizeof(double);
             if (helm)

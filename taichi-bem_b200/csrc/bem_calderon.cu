@@ -50,6 +50,7 @@ struct CalArgs {
     const void* pts;
     const void* phi;      // [Q2*3] P1 hats at the separate-rule points (FP32 or FP64)
     const double* phi64;  // [Q2*3] FP64
+    int ti;               // test panels per CTA (far_calderon_pair_kernel)
     int Q2;
     double k[CAL_MAXK], k2[CAL_MAXK], coef[CAL_MAXK];
     double* out[CAL_MAXK];
@@ -811,15 +812,16 @@ __global__ void __launch_bounds__(FAR_THREADS, SM ? 3 : 1) far_calderon_k2_kerne
 // moments, the exchange and the latency between them.  Four CTAs of the FP32
 // form per SM cost registers (22.3 ms); fetching the next points early did not
 // pay either (24 to 25 ms).
-template <typename T, int PH>
+template <typename T, int PH, bool FULL_TI>
 __global__ void __launch_bounds__(FAR_THREADS, 3) far_calderon_pair_kernel(CalArgs a) {
+    const int ti = FULL_TI ? FAR_TI : a.ti;
     using V4 = typename V4T<T>::type;
     constexpr bool SPLIT = sizeof(T) == 4;
     constexpr unsigned FULL = 0xffffffffu;
     const int Q2 = a.Q2, QP = (Q2 + 1) / 2;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    V4* sx = reinterpret_cast<V4*>(smem_raw);              // [FAR_TI][2 QP] test points
-    V4* sp = reinterpret_cast<V4*>(sx + FAR_TI * 2 * QP);  // [QP] (phi_1, phi_1', phi_2, phi_2') of a point pair
+    V4* sx = reinterpret_cast<V4*>(smem_raw);              // [ti][2 QP] test points
+    V4* sp = reinterpret_cast<V4*>(sx + ti * 2 * QP);  // [QP] (phi_1, phi_1', phi_2, phi_2') of a point pair
     __shared__ int s_gi[FAR_TI];
     __shared__ int s_tri[FAR_TI][3];
     __shared__ double s_cen[FAR_TI][3];
@@ -827,7 +829,7 @@ __global__ void __launch_bounds__(FAR_THREADS, 3) far_calderon_pair_kernel(CalAr
 
     const int n = a.n;
     const int j0 = blockIdx.x * (FAR_THREADS / 2);
-    const int li0 = blockIdx.y * FAR_TI;
+    const int li0 = blockIdx.y * ti;
     if (j0 + FAR_THREADS / 2 - 1 <= li0) return;  // tile strictly below the diagonal
     const int lj = j0 + (threadIdx.x >> 1), w = threadIdx.x & 1;
     const int even = threadIdx.x & 30;  // the pair's first lane
@@ -844,7 +846,7 @@ __global__ void __launch_bounds__(FAR_THREADS, 3) far_calderon_pair_kernel(CalAr
             sp[p] = v;
         }
     }
-    if (threadIdx.x < FAR_TI) {
+    if (threadIdx.x < ti) {
         const int li = li0 + threadIdx.x;
         const int gi = li < n ? a.panels[li] : -1;
         s_gi[threadIdx.x] = gi;
@@ -855,7 +857,7 @@ __global__ void __launch_bounds__(FAR_THREADS, 3) far_calderon_pair_kernel(CalAr
         }
     }
     __syncthreads();
-    for (int idx = threadIdx.x; idx < FAR_TI * 2 * QP; idx += FAR_THREADS) {
+    for (int idx = threadIdx.x; idx < ti * 2 * QP; idx += FAR_THREADS) {
         const int t = idx / (2 * QP), q = idx - t * 2 * QP;
         if (li0 + t >= n) continue;
         V4 v = pts[(size_t)s_gi[t] * Q2 + (q < Q2 ? q : Q2 - 1)];
@@ -877,7 +879,7 @@ __global__ void __launch_bounds__(FAR_THREADS, 3) far_calderon_pair_kernel(CalAr
     const V4* ptsj = pts + (size_t)gj * Q2;
     const T kk = T(w ? a.k[1] : a.k[0]);
 
-    for (int t = 0; t < FAR_TI; ++t) {
+    for (int t = 0; t < ti; ++t) {
         const int li = li0 + t;
         if (li >= n) break;  // uniform across the CTA
         const int gi = s_gi[t];
@@ -1025,12 +1027,17 @@ __global__ void __launch_bounds__(FAR_THREADS, 3) far_calderon_pair_kernel(CalAr
 }
 
 template <typename T, int PH>
-int launch_calderon_pair(bem_ctx* ctx, const CalArgs& a, cudaStream_t s) {
-    dim3 grid((a.n + FAR_THREADS / 2 - 1) / (FAR_THREADS / 2), (a.n + FAR_TI - 1) / FAR_TI);
+int launch_calderon_pair(bem_ctx* ctx, CalArgs a, cudaStream_t s) {
+    const int cols = (a.n + FAR_THREADS / 2 - 1) / (FAR_THREADS / 2);
+    a.ti = bem_far_ti(ctx, a.n, cols);
+    dim3 grid(cols, (a.n + a.ti - 1) / a.ti);
     if (grid.y > 65535) return bem_fail(ctx, BEM_ERR_INVALID, "calderon: too many panels for one launch");
     const int QP = (a.Q2 + 1) / 2;
-    const size_t smem = (size_t)(FAR_TI * 2 * QP + QP) * sizeof(typename V4T<T>::type);
-    far_calderon_pair_kernel<T, PH><<<grid, FAR_THREADS, smem, s>>>(a);
+    const size_t smem = (size_t)(a.ti * 2 * QP + QP) * sizeof(typename V4T<T>::type);
+    if (a.ti == FAR_TI)
+        far_calderon_pair_kernel<T, PH, true><<<grid, FAR_THREADS, smem, s>>>(a);
+    else
+        far_calderon_pair_kernel<T, PH, false><<<grid, FAR_THREADS, smem, s>>>(a);
     ctx->launches++;
     return bem_check_cuda(ctx, cudaGetLastError(), "far_calderon_pair_kernel launch");
 }

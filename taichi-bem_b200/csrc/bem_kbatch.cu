@@ -330,9 +330,8 @@ int launch_kb(bem_ctx* ctx, KbArgs a, cudaStream_t s) {
     // three operators of the sweep, GaussQR 3, FP64: 110 panels 2.60 -> 0.65 ms, 272
     // panels 2.82 -> 1.45 ms (mixed 1.82 -> 1.07), 858 panels 2.78 -> 2.56 ms;
     // 1280 panels and more are the same either way.
-    a.ti = FAR_TI;
     const int64_t cols = (a.n_trial + FAR_THREADS - 1) / FAR_THREADS;
-    while (a.ti > 1 && cols * ((a.n_test + a.ti - 1) / a.ti) < 16 * (int64_t)ctx->num_sms) a.ti /= 2;
+    a.ti = bem_far_ti(ctx, a.n_test, cols);
     dim3 grid((unsigned)cols, (unsigned)((a.n_test + a.ti - 1) / a.ti));
     if (grid.y > 65535) return bem_fail(ctx, BEM_ERR_INVALID, "too many test panels for one launch");
     const size_t smem = a.ti * a.Q2 * sizeof(V4) + a.Q2 * 3 * sizeof(T);
