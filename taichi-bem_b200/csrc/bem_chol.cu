@@ -540,7 +540,7 @@ int chol_t(bem_ctx* ctx, double* A, int64_t n, int64_t lda, bool tensor_cores, i
     iota_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(piv, ni);
     ctx->launches += 3;
     if (int rc = bem_check_cuda(ctx, cudaGetLastError(), "chol_to_lu")) return rc;
-    return bem_tile_inverses(ctx, C ? BEM_C128 : BEM_F64, A, n, lda, dinv, s);
+    return bem_tile_inverses(ctx, C, A, n, lda, dinv, s);
 }
 
 // X = L^{-1} for the lower triangle of L (n x n, lda) whose diagonal tiles'

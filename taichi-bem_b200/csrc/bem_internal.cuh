@@ -85,9 +85,12 @@ int bem_build_near_list(bem_ctx* ctx, int nv, int nt);
 // A device buffer of at least `bytes` owned by the context (grown, never
 // shrunk; freed with it), for scratch that lives within one call.
 int bem_big_ws(bem_ctx* ctx, size_t bytes, void** out);
-// Explicit inverses of the 64 x 64 diagonal tiles of a tile-LU factor into
-// dinv (bem_tilelu.cu); dtype BEM_F64/C128/F32/C64.
-int bem_tile_inverses(bem_ctx* ctx, int dtype, const void* A, int64_t n, int64_t lda, void* dinv, cudaStream_t s);
+// Explicit inverses of the 64 x 64 diagonal tiles of an FP64 tile-LU factor into
+// dinv (bem_tilelu.cu); a zero pivot's reciprocal is 0.
+int bem_tile_inverses(bem_ctx* ctx, bool cplx, const double* A, int64_t n, int64_t lda, void* dinv, cudaStream_t s);
+// The same for bem_lu_tri_solve: dtype BEM_F64/C128/F32/C64, the inverses in FP64
+// (16 bytes an element) whatever the factor's type; NaN where the solve has to substitute.
+int bem_solve_inverses(bem_ctx* ctx, int dtype, const void* A, int64_t n, int64_t lda, void* dinv, cudaStream_t s);
 // x = U^{-1} L^{-1} b for nrhs (already permuted) right-hand sides, vs doubles
 // apart, with a partial-pivoting factor and its tiles' inverses; y is scratch,
 // err (zeroed by the caller) receives BEM_ERR_TIMEOUT (bem_tilelu.cu).

@@ -1295,15 +1295,15 @@ int lu_next(bem_ctx* ctx, double* A, int64_t lda, int n, int k0, int c0, int c1,
                           "lu_next_kernel");
 }
 
-// Workspace of lu_solve: permutation, the inverses of the diagonal tiles,
+// Workspace of lu_solve: permutation, the inverses of the diagonal tiles (FP64),
 // three sets of nrhs vectors vs doubles apart.
 struct SolveLayout {
     size_t off_dinv, off_vec, total;
     int64_t vs;
-    SolveLayout(size_t elem, int W, int64_t n, int64_t nrhs) {
+    SolveLayout(int W, int64_t n, int64_t nrhs) {
         auto up = [](size_t v) { return (v + 255) & ~size_t(255); };
         off_dinv = up(sizeof(int32_t) * (size_t)n);
-        off_vec = off_dinv + up(2 * elem * (size_t)bem_lu_dinv_elems(n));
+        off_vec = off_dinv + up(2 * sizeof(double) * (size_t)bem_lu_dinv_elems(n));
         vs = (int64_t)(up(sizeof(double) * W * (size_t)n) / sizeof(double));
         total = off_vec + 3 * sizeof(double) * (size_t)(nrhs * vs);
     }
@@ -1313,7 +1313,7 @@ template <typename T, bool C>
 int lu_factor_t(bem_ctx* ctx, T* A, int64_t n, int64_t lda, int32_t* piv, int32_t* info, cudaStream_t s) {
     // one growth of the workspace for the factorisation and a solve with it
     LinWs w;
-    if (int rc = linws(ctx, SolveLayout(sizeof(T), C ? 2 : 1, n, 1).total, &w)) return rc;
+    if (int rc = linws(ctx, SolveLayout(C ? 2 : 1, n, 1).total, &w)) return rc;
     cudaMemsetAsync(w.bar, 0, sizeof(GridBar), s);
     cudaMemsetAsync(info, 0, sizeof(int32_t), s);
     cudaMemsetAsync(ctx->flags + 2, 0, sizeof(int32_t), s);
@@ -1416,7 +1416,7 @@ int lu_solve_t(bem_ctx* ctx, const T* LU, int64_t n, int64_t lda, const int32_t*
     if (nrhs < 1 || nrhs > 8) return bem_fail(ctx, BEM_ERR_INVALID, "lu_solve supports 1..8 right-hand sides");
     if ((size_t)n * sizeof(int32_t) > 200 * 1024) return bem_fail(ctx, BEM_ERR_INVALID, "lu_solve: n > 51200");
     const int W = C ? 2 : 1;
-    const SolveLayout lay(sizeof(T), W, n, nrhs);
+    const SolveLayout lay(W, n, nrhs);
     if (int rc = bem_ws_reserve(ctx, lay.total)) return rc;
     const int64_t vs = lay.vs;
     char* base = (char*)ctx->ws;
@@ -1431,7 +1431,7 @@ int lu_solve_t(bem_ctx* ctx, const T* LU, int64_t n, int64_t lda, const int32_t*
     const unsigned blocks = (unsigned)((n * nrhs + 255) / 256);
     gather_rhs_kernel<<<blocks, 256, 0, s>>>(b, ldb, perm, vb, vs, (int)n, (int)nrhs, W);
     ctx->launches += 2;
-    if (int rc = bem_tile_inverses(ctx, dtype, LU, n, lda, dinv, s)) return rc;
+    if (int rc = bem_solve_inverses(ctx, dtype, LU, n, lda, dinv, s)) return rc;
     if (int rc = bem_lu_tri_solve(ctx, dtype, LU, n, lda, dinv, vb, vy, vx, (int)nrhs, vs, flag, s)) return rc;
     scatter_rhs_kernel<<<blocks, 256, 0, s>>>(vx, vs, b, ldb, (int)n, (int)nrhs, W);
     ctx->launches++;

@@ -64,6 +64,16 @@ __device__ __forceinline__ CE<T> cinv(CE<T> a) {
     T d = a.re * a.re + a.im * a.im;
     return d > T(0) ? CE<T>{a.re / d, -a.im / d} : CE<T>{T(0), T(0)};
 }
+// x / a over the whole range: a is scaled by a power of two, so that its
+// square neither overflows nor underflows; a = 0 gives infinities and NaN
+template <bool C>
+__device__ __forceinline__ CE<double> cdiv(CE<double> x, CE<double> a) {
+    if (!C) return CE<double>{x.re / a.re, 0.0};
+    const double m = fmax(fabs(a.re), fabs(a.im));
+    const int e = m > 0.0 && m <= 1.7976931348623157e308 ? ilogb(m) : 0;
+    const double re = scalbn(a.re, -e), im = scalbn(a.im, -e), d = re * re + im * im;
+    return CE<double>{scalbn((x.re * re + x.im * im) / d, -e), scalbn((x.im * re - x.re * im) / d, -e)};
+}
 
 // --------------------------------------------------------------------------
 // diagonal tile: GEPP inside the tile; explicit inverses of the factored tiles
@@ -210,28 +220,49 @@ __global__ void __launch_bounds__(256) tile_diag_kernel(T* A, int64_t lda, int n
 // diagonal block, one CTA per block (blockIdx.x = block), by block
 // substitution over DIAG_PW-row blocks against the identity.  Runs once the
 // factorisation is complete: later row swaps never touch a diagonal block.
-template <typename T, bool C>
-__global__ void __launch_bounds__(256) tile_inv_kernel(const T* A, int64_t lda, int n, CE<T>* dinv) {
+// The inverses are formed and held in D: the factor's own type for the
+// preconditioners (a zero pivot's reciprocal is 0, so that they stay finite),
+// FP64 for bem_lu_solve.  EXACT: an inverse X that one correction of the solve
+// does not bring to the accuracy of substitution is written as NaN, which the
+// solve looks for.  The correction squares the relative residual of the first
+// product, a few eps |T||X|: up to 2^24 that leaves (4 * 1.1e-16 * 2^24)^2 =
+// 5e-17.  A zero pivot, or an inverse that overflows, fails the same test.
+constexpr double INV_COND_MAX = 16777216.0;
+template <typename T, bool C, typename D, bool EXACT>
+__global__ void __launch_bounds__(256) tile_inv_kernel(const T* A, int64_t lda, int n, CE<D>* dinv) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    CE<T>* S = reinterpret_cast<CE<T>*>(smem_raw);  // [LU_T][DIAG_LD] factored block
-    CE<T>* X = S + LU_T * DIAG_LD;                  // [LU_T][LU_T] inverse being built
+    CE<D>* S = reinterpret_cast<CE<D>*>(smem_raw);  // [LU_T][DIAG_LD] factored block
+    CE<D>* X = S + LU_T * DIAG_LD;                  // [LU_T][LU_T] inverse being built
     const int k0 = blockIdx.x * LU_T;
     const int m = min(LU_T, n - k0);
     const int tid = threadIdx.x;
     for (int e = tid; e < LU_T * LU_T; e += blockDim.x) {
         const int r = e / LU_T, c = e - r * LU_T;
-        CE<T> v = CE<T>{T(0), T(0)};
-        if (r < m && c < m) v = ldE<T, C>(A, (int64_t)(k0 + r) * lda + k0 + c);
+        CE<D> v = CE<D>{D(0), D(0)};
+        if (r < m && c < m) {
+            const CE<T> t = ldE<T, C>(A, (int64_t)(k0 + r) * lda + k0 + c);
+            v = CE<D>{(D)t.re, (D)t.im};
+        }
         S[r * DIAG_LD + c] = v;
     }
     __syncthreads();
-    CE<T>* D = dinv + (size_t)blockIdx.x * 2 * LU_T * LU_T;
+    CE<D>* out = dinv + (size_t)blockIdx.x * 2 * LU_T * LU_T;
     // ---- explicit inverses by block substitution against the identity ----
     // Linv: for row block i: X_i = L_ii^{-1} (E_i - sum_{k<i} L_ik X_k)
     // Uinv: for row block i (descending): X_i = U_ii^{-1} (E_i - sum_{k>i} U_ik X_k)
     // thread: column c = tid & 63, rows (tid >> 6) * 2 + {0, 1} of the block
-    __shared__ CE<T> s_rdiag[LU_T];  // 1 / U[r][r], formed in parallel off the substitution chain
-    if (tid < LU_T) s_rdiag[tid] = tid < m ? cinv(S[tid * DIAG_LD + tid]) : CE<T>{T(1), T(0)};
+    __shared__ CE<D> s_rdiag[LU_T];  // 1 / U[r][r], formed in parallel off the substitution chain
+    __shared__ D s_sum[EXACT ? LU_T : 1];
+    if (tid < LU_T) {
+        CE<D> v{D(1), D(0)};
+        if (tid < m) {
+            if constexpr (EXACT)
+                v = cdiv<C>(v, S[tid * DIAG_LD + tid]);
+            else
+                v = cinv(S[tid * DIAG_LD + tid]);
+        }
+        s_rdiag[tid] = v;
+    }
     const int c = tid & 63, rq = (tid >> 6) * 2;
     for (int which = 0; which < 2; ++which) {
         for (int bs = 0; bs < LU_T / DIAG_PW; ++bs) {
@@ -241,17 +272,17 @@ __global__ void __launch_bounds__(256) tile_inv_kernel(const T* A, int64_t lda, 
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const int r = r0 + rq + h;
-                CE<T> v = CE<T>{r == c ? T(1) : T(0), T(0)};
+                CE<D> v = CE<D>{r == c ? D(1) : D(0), D(0)};
                 if (r < m) {
                     if (which == 0) {
                         for (int q = 0; q < r0; ++q) {
-                            const CE<T> l = S[r * DIAG_LD + q], x = X[q * LU_T + c];
+                            const CE<D> l = S[r * DIAG_LD + q], x = X[q * LU_T + c];
                             v.re -= l.re * x.re - l.im * x.im;
                             v.im -= l.re * x.im + l.im * x.re;
                         }
                     } else {
                         for (int q = r0 + DIAG_PW; q < m; ++q) {
-                            const CE<T> uu = S[r * DIAG_LD + q], x = X[q * LU_T + c];
+                            const CE<D> uu = S[r * DIAG_LD + q], x = X[q * LU_T + c];
                             v.re -= uu.re * x.re - uu.im * x.im;
                             v.im -= uu.re * x.im + uu.im * x.re;
                         }
@@ -262,7 +293,7 @@ __global__ void __launch_bounds__(256) tile_inv_kernel(const T* A, int64_t lda, 
             __syncthreads();
             // diagonal block: substitution down (Linv) or up (Uinv) the 8 rows, one thread per column
             if (tid < LU_T) {
-                CE<T> y[DIAG_PW];
+                CE<D> y[DIAG_PW];
 #pragma unroll
                 for (int i = 0; i < DIAG_PW; ++i) y[i] = X[(r0 + i) * LU_T + c];
                 if (which == 0) {
@@ -270,12 +301,12 @@ __global__ void __launch_bounds__(256) tile_inv_kernel(const T* A, int64_t lda, 
                     for (int i = 0; i < DIAG_PW; ++i) {
                         const int r = r0 + i;
                         if (r >= m) {
-                            y[i] = CE<T>{r == c ? T(1) : T(0), T(0)};  // identity padding of a short last tile
+                            y[i] = CE<D>{r == c ? D(1) : D(0), D(0)};  // identity padding of a short last tile
                             continue;
                         }
 #pragma unroll
                         for (int q = 0; q < i; ++q) {
-                            const CE<T> l = S[r * DIAG_LD + r0 + q];
+                            const CE<D> l = S[r * DIAG_LD + r0 + q];
                             y[i].re -= l.re * y[q].re - l.im * y[q].im;
                             y[i].im -= l.re * y[q].im + l.im * y[q].re;
                         }
@@ -285,17 +316,17 @@ __global__ void __launch_bounds__(256) tile_inv_kernel(const T* A, int64_t lda, 
                     for (int i = DIAG_PW - 1; i >= 0; --i) {
                         const int r = r0 + i;
                         if (r >= m) {
-                            y[i] = CE<T>{r == c ? T(1) : T(0), T(0)};
+                            y[i] = CE<D>{r == c ? D(1) : D(0), D(0)};
                             continue;
                         }
                         if (c >= m) {
-                            y[i] = CE<T>{T(0), T(0)};
+                            y[i] = CE<D>{D(0), D(0)};
                             continue;
                         }
 #pragma unroll
                         for (int q = i + 1; q < DIAG_PW; ++q) {
                             if (r0 + q >= m) continue;
-                            const CE<T> uu = S[r * DIAG_LD + r0 + q];
+                            const CE<D> uu = S[r * DIAG_LD + r0 + q];
                             y[i].re -= uu.re * y[q].re - uu.im * y[q].im;
                             y[i].im -= uu.re * y[q].im + uu.im * y[q].re;
                         }
@@ -307,7 +338,27 @@ __global__ void __launch_bounds__(256) tile_inv_kernel(const T* A, int64_t lda, 
             }
             __syncthreads();
         }
-        for (int e = tid; e < LU_T * LU_T; e += blockDim.x) D[which * LU_T * LU_T + e] = X[e];
+        bool good = true;
+        if constexpr (EXACT) {
+            // the largest row sum of |T| |X| (thread: row tid / 4, every fourth column)
+            const int r = tid >> 2, p = tid & 3;
+            D sum = D(0);
+            for (int q = p; q < LU_T; q += 4) sum += fabs(X[r * LU_T + q].re) + fabs(X[r * LU_T + q].im);
+            sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+            sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+            if (p == 0) s_sum[r] = sum;
+            __syncthreads();
+            sum = p == 0 && which == 0 ? s_sum[r] : D(0);  // L's unit diagonal
+            for (int q = p; q < LU_T; q += 4) {
+                const CE<D> t = S[r * DIAG_LD + q];
+                if (which == 0 ? q < r : q >= r) sum += (fabs(t.re) + fabs(t.im)) * s_sum[q];
+            }
+            sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+            sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+            good = !__syncthreads_or(!(sum <= D(INV_COND_MAX)));
+        }
+        for (int e = tid; e < LU_T * LU_T; e += blockDim.x)
+            out[which * LU_T * LU_T + e] = good ? X[e] : CE<D>{D(NAN), D(NAN)};
         __syncthreads();
     }
 }
@@ -475,40 +526,49 @@ __device__ __forceinline__ bool pending(double v) { return __double_as_longlong(
 //
 // Sums over the streamed blocks are held in ACC: the factor's own type for the
 // preconditioners (as the products of an FP32 factor are), FP64 with REF.  REF
-// (the solves of a partial-pivoting factor): the explicit inverse is corrected
-// once against the diagonal block itself, y0 = D a, y = y0 + D (a - T y0) in
-// FP64, which brings its backward error to that of substitution.
+// (the solves of a partial-pivoting factor): the explicit inverse, in FP64
+// whatever the factor's type, is corrected once against the diagonal block
+// itself, y0 = D a, y = y0 + D (a - T y0), which brings its backward error to
+// that of substitution.  Where that is not finite (an inverse that
+// tile_inv_kernel did not accept, infinities and NaN of the right-hand side)
+// the block is solved by substitution instead, so the solve has the range of
+// substitution too.
 constexpr int SOLVE_LD = LU_T + 4;  // padded row stride of the staged blocks
-constexpr size_t solve_smem_bytes(size_t elem, bool ref) { return (ref ? 3 : 2) * elem * LU_T * SOLVE_LD; }
+// elem, inv: bytes of an element of the factor and of the diagonal inverses
+constexpr size_t solve_smem_bytes(size_t elem, size_t inv, bool ref) {
+    return ((ref ? 2 : 1) * elem + inv) * LU_T * SOLVE_LD;
+}
+
+// type of the diagonal inverses of a solve
+template <typename T, bool REF>
+struct SolveInv {
+    using type = typename std::conditional<REF, double, T>::type;
+};
 
 template <typename T, bool C, int NR, bool REF>
-__global__ void __launch_bounds__(256) tri_solve_kernel(const T* LU, int64_t lda, int n, const CE<T>* dinv,
+__global__ void __launch_bounds__(256) tri_solve_kernel(const T* LU, int64_t lda, int n,
+                                                        const CE<typename SolveInv<T, REF>::type>* dinv,
                                                         const double* b, double* y, double* x, int64_t vs,
                                                         int vec, int32_t* err, const int* skip) {
     // skip != NULL: a device word set by the asynchronous refinement once it
     // has converged; the later, already queued solves return at once
     if (skip != nullptr && *skip != 0) return;
-    using ACC = typename std::conditional<REF, double, T>::type;
+    using ACC = typename SolveInv<T, REF>::type;
     constexpr int RW = LU_T / 8;  // rows per warp in the streamed part
     constexpr int W = C ? 2 : 1;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    CE<T>* sB = reinterpret_cast<CE<T>*>(smem_raw);  // [LU_T][SOLVE_LD] last dependency block
-    CE<T>* sD = sB + LU_T * SOLVE_LD;                 // [LU_T][SOLVE_LD] diagonal inverse
-    CE<T>* sT = sD + LU_T * SOLVE_LD;                 // REF: [LU_T][SOLVE_LD] diagonal block
+    CE<ACC>* sD = reinterpret_cast<CE<ACC>*>(smem_raw);              // [LU_T][SOLVE_LD] diagonal inverse
+    CE<T>* sB = reinterpret_cast<CE<T>*>(sD + LU_T * SOLVE_LD);      // [LU_T][SOLVE_LD] last dependency block
+    CE<T>* sT = sB + LU_T * SOLVE_LD;                                // REF: [LU_T][SOLVE_LD] diagonal block
     __shared__ double s_acc[LU_T][NR][2];
     __shared__ double s_x[LU_T][NR][2];
     __shared__ double s_r[REF ? LU_T : 1][NR][2];
     __shared__ int s_abort;
-    __shared__ int s_zero[2];  // REF: last row of the diagonal block with a zero pivot, -1 = none; by row parity
     const int nbk = (n + LU_T - 1) / LU_T;
     const int P = gridDim.x;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const int gr = tid >> 2, gq = tid & 3;  // GEMV mapping: row gr, columns gq + 4i
-    if (tid == 0) {
-        s_abort = 0;
-        s_zero[0] = s_zero[1] = -1;
-    }
-    int par = 0;
+    if (tid == 0) s_abort = 0;
     __syncthreads();
     // element i of the row at p (aligned: one access per complex element)
     auto elem = [&](const T* p, int i) -> CE<T> {
@@ -592,7 +652,7 @@ __global__ void __launch_bounds__(256) tri_solve_kernel(const T* LU, int64_t lda
             };
             if (nstream > 0) load(0);
             // stage the diagonal inverse, the critical block and the diagonal block
-            const CE<T>* Dk = dinv + (size_t)k * 2 * LU_T * LU_T + (fwd ? 0 : LU_T * LU_T);
+            const CE<ACC>* Dk = dinv + (size_t)k * 2 * LU_T * LU_T + (fwd ? 0 : LU_T * LU_T);
             for (int e = tid; e < LU_T * LU_T; e += blockDim.x) {
                 const int r = e / LU_T, c = e - r * LU_T;
                 sD[r * SOLVE_LD + c] = Dk[e];
@@ -605,10 +665,7 @@ __global__ void __launch_bounds__(256) tri_solve_kernel(const T* LU, int64_t lda
                 sB[r * SOLVE_LD + c] = v;
                 if constexpr (REF) {
                     CE<T> d = CE<T>{r == c ? T(1) : T(0), T(0)};
-                    if (r < m && c < m && (fwd ? c < r : c >= r)) {
-                        d = elem(row + (int64_t)W * r0, c);
-                        if (r == c && d.re == T(0) && d.im == T(0)) atomicMax(&s_zero[par], r);
-                    }
+                    if (r < m && c < m && (fwd ? c < r : c >= r)) d = elem(row + (int64_t)W * r0, c);
                     sT[r * SOLVE_LD + c] = d;
                 }
             }
@@ -663,9 +720,8 @@ __global__ void __launch_bounds__(256) tri_solve_kernel(const T* LU, int64_t lda
                 }
             __syncthreads();
             if (s_abort) return;
-            if (REF && tid == 0) s_zero[par ^ 1] = -1;  // the previous row's reads are done, the next row's writes not begun
             // (row gr of S) . v, in A, in all four lanes of the row
-            auto gemv = [&](auto zero, const CE<T>* S, const double (*v)[NR][2], double (*out)[2]) {
+            auto gemv = [&](auto zero, const auto* S, const double (*v)[NR][2], double (*out)[2]) {
                 using A = decltype(zero);
                 A sr[NR], si[NR];
 #pragma unroll
@@ -673,7 +729,7 @@ __global__ void __launch_bounds__(256) tri_solve_kernel(const T* LU, int64_t lda
 #pragma unroll
                 for (int i = 0; i < LU_T / 4; ++i) {
                     const int c = gq + 4 * i;
-                    const CE<T> l = S[gr * SOLVE_LD + c];
+                    const auto l = S[gr * SOLVE_LD + c];
 #pragma unroll
                     for (int r = 0; r < NR; ++r) {
                         const A vr = (A)v[c][r][0], vi = (A)v[c][r][1];
@@ -741,15 +797,38 @@ __global__ void __launch_bounds__(256) tri_solve_kernel(const T* LU, int64_t lda
                     }
                 __syncthreads();
                 gemv(0.0, sD, s_r, q);
+                bool finite = true;
 #pragma unroll
                 for (int r = 0; r < NR; ++r) {
                     o[r][0] += q[r][0];
                     o[r][1] += q[r][1];
-                    // a zero pivot divides by zero, as substitution would, and the rows above
-                    // it depend on that value (the inverse holds 0 there)
-                    if (gr <= s_zero[par]) {
-                        const double zero = (double)sT[s_zero[par] * SOLVE_LD + s_zero[par]].re;
-                        o[r][0] = o[r][1] = (gr == s_zero[par] && !C ? s_r[gr][r][0] : zero) / zero;
+                    if (gr < m) finite = finite && isfinite(o[r][0]) && isfinite(o[r][1]);
+                }
+                if (__syncthreads_or(!finite)) {
+                    // substitution, a warp per right-hand side
+                    if (wid < NR)
+                        for (int q0 = 0; q0 < m; ++q0) {
+                            const int c = fwd ? q0 : m - 1 - q0;
+                            const CE<T> d = sT[c * SOLVE_LD + c];
+                            CE<double> v{s_acc[c][wid][0], s_acc[c][wid][1]};
+                            if (!fwd) v = cdiv<C>(v, CE<double>{(double)d.re, (double)d.im});
+                            for (int i = lane; i < m; i += 32) {
+                                if (fwd ? i <= c : i >= c) continue;
+                                const CE<T> l = sT[i * SOLVE_LD + c];
+                                s_acc[i][wid][0] -= (double)l.re * v.re - (C ? (double)l.im * v.im : 0.0);
+                                if (C) s_acc[i][wid][1] -= (double)l.re * v.im + (double)l.im * v.re;
+                            }
+                            if (lane == 0) {
+                                s_x[c][wid][0] = v.re;
+                                s_x[c][wid][1] = v.im;
+                            }
+                            __syncwarp();
+                        }
+                    __syncthreads();
+#pragma unroll
+                    for (int r = 0; r < NR; ++r) {
+                        o[r][0] = s_x[gr][r][0];
+                        o[r][1] = s_x[gr][r][1];
                     }
                 }
             }
@@ -760,7 +839,6 @@ __global__ void __launch_bounds__(256) tri_solve_kernel(const T* LU, int64_t lda
                     if (C) st_vol(dst + r * vs + (int64_t)W * (r0 + gr) + 1, o[r][1]);
                 }
             __syncthreads();
-            par ^= 1;
         }
     }
 }
@@ -784,12 +862,13 @@ __global__ void pending_kernel(double* y, double* x, int64_t nd, const int* skip
 // Queues the triangular solve of NR permuted right-hand sides b (vs doubles
 // apart) into x; y is scratch.  err receives BEM_ERR_TIMEOUT if a wait runs out.
 template <typename T, bool C, int NR, bool REF>
-cudaError_t queue_tri_solve(int sms, const T* LU, int64_t n, int64_t lda, const CE<T>* dinv, const double* b, double* y,
-                            double* x, int64_t vs, int32_t* err, const int* skip, cudaStream_t s) {
+cudaError_t queue_tri_solve(int sms, const T* LU, int64_t n, int64_t lda, const CE<typename SolveInv<T, REF>::type>* dinv,
+                            const double* b, double* y, double* x, int64_t vs, int32_t* err, const int* skip,
+                            cudaStream_t s) {
     const int nbk = (int)((n + LU_T - 1) / LU_T);
     const int64_t nd = NR == 1 ? (C ? 2 : 1) * n : NR * vs;
     pending_kernel<<<(unsigned)((nd + 255) / 256), 256, 0, s>>>(y, x, nd, skip);
-    const size_t smem = solve_smem_bytes(sizeof(CE<T>), REF);
+    const size_t smem = solve_smem_bytes(sizeof(CE<T>), sizeof(*dinv), REF);
     const void* fn = (const void*)tri_solve_kernel<T, C, NR, REF>;
     if (cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) return e;
     int per_sm = 0;
@@ -827,7 +906,7 @@ int factor_t(bem_ctx* ctx, T* A, int64_t n, int64_t lda, int32_t* piv, CE<T>* di
     cudaMemsetAsync(info, 0, sizeof(int32_t), s);
     const size_t asmem = apply_smem_bytes(sizeof(CE<T>));
     const size_t ismem = inv_smem_bytes(sizeof(CE<T>));
-    cudaFuncSetAttribute(tile_inv_kernel<T, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ismem);
+    cudaFuncSetAttribute(tile_inv_kernel<T, C, T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ismem);
     cudaFuncSetAttribute(tile_apply_kernel<T, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)asmem);
     if (int rc = bem_lookahead_stream(ctx)) return rc;
     const int ni = (int)n;
@@ -889,7 +968,7 @@ int factor_t(bem_ctx* ctx, T* A, int64_t n, int64_t lda, int32_t* piv, CE<T>* di
         if (int rc = bem_check_cuda(ctx, cudaGetLastError(), "tiled lu step")) return rc;
     }
     // explicit inverses of every diagonal block (for the solves)
-    tile_inv_kernel<T, C><<<(unsigned)((n + LU_T - 1) / LU_T), 256, ismem, s>>>(A, lda, ni, dinv);
+    tile_inv_kernel<T, C, T, false><<<(unsigned)((n + LU_T - 1) / LU_T), 256, ismem, s>>>(A, lda, ni, dinv);
     ctx->launches++;
     // No synchronisation: a tensor-core update whose bounded wait ran out
     // records it in flags[4], which the next solve on this context reads
@@ -969,9 +1048,9 @@ int precond_t(bem_ctx* ctx, const T* LU, int64_t n, int64_t lda, const int32_t* 
 }
 
 // x = U^{-1} L^{-1} b for nrhs permuted right-hand sides (vs doubles apart), the
-// diagonal inverses refined against the diagonal blocks; two at a time.
+// FP64 diagonal inverses refined against the diagonal blocks; two at a time.
 template <typename T, bool C>
-int lu_tri_t(bem_ctx* ctx, const T* LU, int64_t n, int64_t lda, const CE<T>* dinv, const double* b, double* y, double* x,
+int lu_tri_t(bem_ctx* ctx, const T* LU, int64_t n, int64_t lda, const CE<double>* dinv, const double* b, double* y, double* x,
              int nrhs, int64_t vs, int32_t* err, cudaStream_t s) {
     for (int c = 0; c < nrhs;) {
         const int m = nrhs - c >= 2 ? 2 : 1;
@@ -1036,22 +1115,29 @@ int bem_lu_solve_tiled(bem_ctx* ctx, int dtype, const void* LU, int64_t n, int64
 
 }  // extern "C"
 
-template <typename T, bool C>
-int tile_inverses_t(bem_ctx* ctx, const T* A, int64_t n, int64_t lda, CE<T>* dinv, cudaStream_t s) {
-    const size_t ismem = inv_smem_bytes(sizeof(CE<T>));
-    cudaFuncSetAttribute(tile_inv_kernel<T, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ismem);
-    tile_inv_kernel<T, C><<<(unsigned)((n + LU_T - 1) / LU_T), 256, ismem, s>>>(A, lda, (int)n, dinv);
+template <typename T, bool C, typename D, bool EXACT>
+int tile_inverses_t(bem_ctx* ctx, const T* A, int64_t n, int64_t lda, CE<D>* dinv, cudaStream_t s) {
+    const size_t ismem = inv_smem_bytes(sizeof(CE<D>));
+    cudaFuncSetAttribute(tile_inv_kernel<T, C, D, EXACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ismem);
+    tile_inv_kernel<T, C, D, EXACT><<<(unsigned)((n + LU_T - 1) / LU_T), 256, ismem, s>>>(A, lda, (int)n, dinv);
     ctx->launches++;
     return bem_check_cuda(ctx, cudaGetLastError(), "tile_inv_kernel");
 }
 
-int bem_tile_inverses(bem_ctx* ctx, int dtype, const void* A, int64_t n, int64_t lda, void* dinv, cudaStream_t s) {
+int bem_tile_inverses(bem_ctx* ctx, bool cplx, const double* A, int64_t n, int64_t lda, void* dinv, cudaStream_t s) {
+    CE<double>* d = (CE<double>*)dinv;
+    return cplx ? tile_inverses_t<double, true, double, false>(ctx, A, n, lda, d, s)
+                : tile_inverses_t<double, false, double, false>(ctx, A, n, lda, d, s);
+}
+
+int bem_solve_inverses(bem_ctx* ctx, int dtype, const void* A, int64_t n, int64_t lda, void* dinv, cudaStream_t s) {
+    CE<double>* d = (CE<double>*)dinv;
     switch (dtype) {
-        case BEM_F64: return tile_inverses_t<double, false>(ctx, (const double*)A, n, lda, (CE<double>*)dinv, s);
-        case BEM_C128: return tile_inverses_t<double, true>(ctx, (const double*)A, n, lda, (CE<double>*)dinv, s);
-        case BEM_F32: return tile_inverses_t<float, false>(ctx, (const float*)A, n, lda, (CE<float>*)dinv, s);
-        case BEM_C64: return tile_inverses_t<float, true>(ctx, (const float*)A, n, lda, (CE<float>*)dinv, s);
-        default: return bem_fail(ctx, BEM_ERR_INVALID, "tile inverses: unknown dtype");
+        case BEM_F64: return tile_inverses_t<double, false, double, true>(ctx, (const double*)A, n, lda, d, s);
+        case BEM_C128: return tile_inverses_t<double, true, double, true>(ctx, (const double*)A, n, lda, d, s);
+        case BEM_F32: return tile_inverses_t<float, false, double, true>(ctx, (const float*)A, n, lda, d, s);
+        case BEM_C64: return tile_inverses_t<float, true, double, true>(ctx, (const float*)A, n, lda, d, s);
+        default: return bem_fail(ctx, BEM_ERR_INVALID, "lu_solve: unknown dtype");
     }
 }
 
@@ -1060,8 +1146,8 @@ int bem_lu_tri_solve(bem_ctx* ctx, int dtype, const void* LU, int64_t n, int64_t
     switch (dtype) {
         case BEM_F64: return lu_tri_t<double, false>(ctx, (const double*)LU, n, lda, (const CE<double>*)dinv, b, y, x, nrhs, vs, err, s);
         case BEM_C128: return lu_tri_t<double, true>(ctx, (const double*)LU, n, lda, (const CE<double>*)dinv, b, y, x, nrhs, vs, err, s);
-        case BEM_F32: return lu_tri_t<float, false>(ctx, (const float*)LU, n, lda, (const CE<float>*)dinv, b, y, x, nrhs, vs, err, s);
-        case BEM_C64: return lu_tri_t<float, true>(ctx, (const float*)LU, n, lda, (const CE<float>*)dinv, b, y, x, nrhs, vs, err, s);
+        case BEM_F32: return lu_tri_t<float, false>(ctx, (const float*)LU, n, lda, (const CE<double>*)dinv, b, y, x, nrhs, vs, err, s);
+        case BEM_C64: return lu_tri_t<float, true>(ctx, (const float*)LU, n, lda, (const CE<double>*)dinv, b, y, x, nrhs, vs, err, s);
         default: return bem_fail(ctx, BEM_ERR_INVALID, "lu_solve: unknown dtype");
     }
 }

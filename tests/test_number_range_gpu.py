@@ -1,0 +1,91 @@
+"""The dense solvers and kernels at the ends of the number range and at the
+last digits, against extended precision (numpy's long double) or CUDA."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def engine():
+    from bem_b200.engine import Engine
+    e = Engine()
+    yield e
+    e.close()
+
+
+def _gaussian(shape, cplx, seed):
+    rng = np.random.default_rng(seed)
+    x = rng.standard_normal(shape)
+    return x + 1j * rng.standard_normal(shape) if cplx else x
+
+
+def _gepp(A):
+    """L U of A with its rows swapped, in A's own type; the permuted A is not kept."""
+    A = A.copy()
+    for j in range(len(A)):
+        p = j + int(np.argmax(np.abs(A[j:, j])))
+        A[[j, p]] = A[[p, j]]
+        A[j + 1:, j] /= A[j, j]
+        A[j + 1:, j + 1:] -= np.outer(A[j + 1:, j], A[j, j + 1:])
+    return A
+
+
+def _backward_error(F, x, b):
+    """Componentwise: max |L U x - b| / (|L||U||x| + |b|), in long double."""
+    wide = np.clongdouble if np.iscomplexobj(F) else np.longdouble
+    F, x, b = F.astype(wide), x.astype(wide), b.astype(wide)
+    low, up = np.tril(F, -1) + np.eye(len(F)), np.triu(F)
+    res = np.abs(low @ (up @ x) - b)
+    return float((res / (np.abs(low) @ (np.abs(up) @ np.abs(x)) + np.abs(b))).max())
+
+
+def _solve(engine, F, b):
+    n = len(F)
+    piv = torch.arange(n, dtype=torch.int32, device="cuda")
+    x = torch.as_tensor(b, device="cuda").clone()
+    engine.lu_solve(torch.as_tensor(F, device="cuda"), piv, x)
+    return x.cpu().numpy()
+
+
+@pytest.mark.parametrize("dtype", ["float32", "complex64", "float64", "complex128"])
+@pytest.mark.parametrize("n", [64, 200])
+def test_lu_solve_is_backward_stable(engine, n, dtype):
+    """The factors of a Gaussian matrix (not dominant), solved in FP64 whatever
+    their type: two triangles of n products, sqrt(n) roundings of 1.1e-16 each
+    against the sum of their magnitudes (substitution in numpy: 2e-17 to 6e-17)."""
+    F = _gepp(_gaussian((n, n), dtype.startswith("complex"), n).astype(dtype))
+    b = _gaussian((n, 3), dtype.startswith("complex"), 1)
+    x = _solve(engine, F, b)
+    assert _backward_error(F, x, b) < np.sqrt(n) * 1.2e-16
+
+
+@pytest.mark.parametrize("dtype,exp", [("float32", -80), ("float32", -100), ("float32", 66), ("complex64", -80),
+                                       ("complex64", 66), ("float64", -550), ("float64", 520), ("complex128", -550),
+                                       ("complex128", 520)])
+def test_lu_solve_where_squares_leave_the_range(engine, dtype, exp):
+    """U scaled by 2^exp: the pivots are ordinary numbers of their type, their
+    squares are not.  Bound as above."""
+    n = 130
+    F = _gepp(_gaussian((n, n), dtype.startswith("complex"), 3).astype(dtype))
+    F = (np.tril(F, -1) + np.triu(F) * np.ldexp(1.0, exp).astype(F.real.dtype)).astype(dtype)
+    b = _gaussian((n, 2), dtype.startswith("complex"), 4)
+    x = _solve(engine, F, b)
+    assert np.isfinite(x).all()
+    assert _backward_error(F, x, b) < np.sqrt(n) * 1.2e-16
+
+
+@pytest.mark.parametrize("dtype", ["float32", "complex64", "float64", "complex128"])
+def test_lu_solve_where_a_tile_inverse_overflows(engine, dtype):
+    """U = I - 2^20 (superdiagonal), x of small integers: the inverse holds
+    2^1260, substitution has integers only and is exact."""
+    n = 100
+    F = (np.eye(n) - 2.0 ** 20 * np.eye(n, k=1)).astype(dtype)
+    cplx = dtype.startswith("complex")
+    if cplx:
+        F = (F.astype(np.complex128) * (1 + 1j)).astype(dtype)
+    F = np.triu(F)
+    x0 = np.rint(4 * _gaussian((n, 2), cplx, 5))
+    b = F.astype(np.complex128 if cplx else np.float64) @ x0
+    assert np.array_equal(_solve(engine, F, b), x0)
