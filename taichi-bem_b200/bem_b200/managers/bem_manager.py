@@ -315,21 +315,32 @@ class BEMManager:
 
     # -- solve --------------------------------------------------------------------------
     def _lu_solve_fp64(self, A: torch.Tensor, b: torch.Tensor, cols) -> torch.Tensor:
-        """Partial-pivoting FP64 LU and solves.  An exact zero pivot raises
-        torch.linalg.LinAlgError, as the reference's torch.linalg.solve does
-        on a singular matrix (BEM_manager.py:1056)."""
+        """Partial-pivoting FP64 LU and solves.  An exact zero pivot, with the
+        unknowns in reverse order too, raises torch.linalg.LinAlgError, as the
+        reference's torch.linalg.solve does on a singular matrix
+        (BEM_manager.py:1056)."""
         LU = A.clone()
         piv, info = self.engine.lu_factor(LU)
         zero_pivot = int(info.item())  # the solves below synchronise the stream anyway
+        reverse = False
         if zero_pivot > 0:
-            raise torch.linalg.LinAlgError(
-                "linalg.solve: The solver failed because the input matrix is singular "
-                f"(zero pivot in column {zero_pivot - 1}).")
+            # A matrix that is singular to rounding only (Laplace Neumann: the
+            # constants) has a last pivot of a few roundings, which the order of
+            # the atomic sums decides and which can come out as exactly 0.  The
+            # unknowns in reverse order round differently; a zero row or column
+            # has a zero pivot in either.
+            reverse = True
+            LU = A.flip(0, 1)
+            piv, info = self.engine.lu_factor(LU)
+            if int(info.item()) > 0:
+                raise torch.linalg.LinAlgError(
+                    "linalg.solve: The solver failed because the input matrix is singular "
+                    f"(zero pivot in column {zero_pivot - 1}).")
         xs = []
         for c in cols:
-            x = c.clone()
+            x = c.flip(0) if reverse else c.clone()
             self.engine.lu_solve(LU, piv, x)
-            xs.append(x)
+            xs.append(x.flip(0) if reverse else x)
         self.solve_info = {"factor": "fp64", "info": info}
         return xs[0] if b.dim() == 1 else torch.stack(xs, 1)
 

@@ -292,12 +292,15 @@ __global__ void __launch_bounds__(FAR_THREADS) far64_kernel(Far64Args a) {
                 fi = fr * sR;
                 fr = fr * cR;
             }
+            auto times_f = [&](double& re, double& im) {
+                const double u = re, v = im;
+                re = HELM ? u * fr - v * fi : u * fr;
+                im = HELM ? u * fi + v * fr : 0.0;
+            };
+            // W: after the curl product (below), as the general kernel does
+            if (KIND != 1)
 #pragma unroll
-            for (int m = 0; m < NM; ++m) {
-                const double u = Mr[m], v = Mi[m];
-                Mr[m] = HELM ? u * fr - v * fi : u * fr;
-                Mi[m] = HELM ? u * fi + v * fr : 0.0;
-            }
+                for (int m = 0; m < NM; ++m) times_f(Mr[m], Mi[m]);
             if constexpr (SYM) {
                 double vr[NB][NB], vi[NB][NB];
                 if constexpr (NB == 1) {
@@ -335,6 +338,7 @@ __global__ void __launch_bounds__(FAR_THREADS) far64_kernel(Far64Args a) {
                                 const double cd = cx[0] * cy[0] + cx[1] * cy[1] + cx[2] * cy[2];
                                 vr[x][y] = PHI ? Mr[0] * cd - k2n * vr[x][y] : Mr[0] * cd;
                                 vi[x][y] = PHI ? Mi[0] * cd - k2n * vi[x][y] : Mi[0] * cd;
+                                times_f(vr[x][y], vi[x][y]);
                             }
                         }
                     }

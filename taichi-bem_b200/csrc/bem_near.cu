@@ -220,20 +220,20 @@ __device__ __forceinline__ void near_integrate(const NearArgs& a, const NearPair
         near_points(P.rel, gp[dg.ix], gp[dg.iy], gp[dg.iz], gp[dg.iw], weight, add);
         dg.next(Q);
     }
-    // the warp's sums in every lane
+    // the warp's sums in every lane, without 1/(4 pi)
 #pragma unroll
     for (int q = 0; q < NK; ++q) {
         if (G)
 #pragma unroll
             for (int m = 0; m < M.NG; ++m) {
-                M.gr[q][m] = warp_sum(M.gr[q][m]) * BEM_INV4PI;
-                if (HELM) M.gi[q][m] = warp_sum(M.gi[q][m]) * BEM_INV4PI;
+                M.gr[q][m] = warp_sum(M.gr[q][m]);
+                if (HELM) M.gi[q][m] = warp_sum(M.gi[q][m]);
             }
         if (with_k)
 #pragma unroll
             for (int m = 0; m < M.ND; ++m) {
-                M.kr[q][m] = warp_sum(M.kr[q][m]) * BEM_INV4PI;
-                if (HELM) M.ki[q][m] = warp_sum(M.ki[q][m]) * BEM_INV4PI;
+                M.kr[q][m] = warp_sum(M.kr[q][m]);
+                if (HELM) M.ki[q][m] = warp_sum(M.ki[q][m]);
             }
     }
 }
@@ -316,6 +316,8 @@ __global__ void __launch_bounds__(128) near_kernel(NearArgs a) {
             vr = near_hat<MX, MY>(mr, P.sx, P.sy, bx, by);
             vi = HELM ? near_hat<MX, MY>(mi, P.sx, P.sy, bx, by) : 0.0;
         }
+        vr *= BEM_INV4PI;
+        vi *= BEM_INV4PI;
         if (row < 0 || col < 0) continue;
         if (a.mode == 0) {
             if (a.out[q] == nullptr) continue;
@@ -346,7 +348,8 @@ __global__ void __launch_bounds__(128) near_vkg_kernel(NearArgs a) {
     if (lane == 0) {
         const int row = a.test_dof[P.li], col = a.trial_dof[P.lj];
         if (row >= 0 && col >= 0)
-            add_entry<HELM>(a.out[0], (int64_t)row * a.ld + col, a.scale[0] * M.gr[0][0], a.scale[0] * M.gi[0][0], true);
+            add_entry<HELM>(a.out[0], (int64_t)row * a.ld + col, a.scale[0] * (BEM_INV4PI * M.gr[0][0]),
+                            a.scale[0] * (BEM_INV4PI * M.gi[0][0]), true);
     } else if (lane == 1) {
         const int row = a.rows[P.li];
         if (row < 0) return;
@@ -366,6 +369,8 @@ __global__ void __launch_bounds__(128) near_vkg_kernel(NearArgs a) {
                 cr += vr * a.x[col];
             }
         }
+        cr *= BEM_INV4PI;
+        ci *= BEM_INV4PI;
         if (HELM) {
             atomicAdd(a.y + 2 * (int64_t)row, a.scale_k * cr);
             atomicAdd(a.y + 2 * (int64_t)row + 1, a.scale_k * ci);
@@ -428,7 +433,8 @@ __global__ void __launch_bounds__(128) near_calderon_kernel(NearArgs a) {
                 vi += a.k2[q] * nd * near_hat<GX, GX>(M.gi[q], P.sx, P.sy, bx, by);
             }
         }
-        add_entry<HELM>(a.out[q], (int64_t)row * a.ld + col, a.scale[q] * vr, a.scale[q] * vi, true);
+        add_entry<HELM>(a.out[q], (int64_t)row * a.ld + col, a.scale[q] * (BEM_INV4PI * vr),
+                        a.scale[q] * (BEM_INV4PI * vi), true);
     }
 }
 

@@ -89,3 +89,42 @@ def test_lu_solve_where_a_tile_inverse_overflows(engine, dtype):
     x0 = np.rint(4 * _gaussian((n, 2), cplx, 5))
     b = F.astype(np.complex128 if cplx else np.float64) @ x0
     assert np.array_equal(_solve(engine, F, b), x0)
+
+
+# ---- zero pivots by rounding -------------------------------------------------------------
+@pytest.fixture(scope="module")
+def manager():
+    from bem_b200.managers import CoreManager
+    from tests._util import load_fixture, torch_callbacks
+    d = load_fixture("cube_lap_neu_q5")
+    params = eval(str(d["params"]))
+    params.update(vertices=d["vertices"], panels=d["panels"])
+    core = CoreManager(params)
+    core.initialization(*torch_callbacks(str(d["data_kind"]), float(params.get("k", 0.0)), d["direction"]))
+    yield core._BEM_manager
+    core.kill()
+
+
+def test_a_pivot_that_rounds_to_zero_does_not_raise(manager):
+    """[[3, 1], [1, fl(1/3)]] is not singular (determinant -2^-54), but its
+    second pivot is fl(1/3) - fl(1/3) = 0; the other way round it is 1 - 3
+    fl(1/3) = 2^-54 in one FMA.  The solution's residual is a few roundings of
+    |A||x|; a matrix with a zero column raises."""
+    A = np.array([[3.0, 1.0], [1.0, 1.0 / 3.0]])
+    b = _gaussian((2, 2), False, 1)
+    Ad, bd = torch.as_tensor(A, device="cuda"), torch.as_tensor(b, device="cuda")
+    assert int(manager.engine.lu_factor(Ad.clone())[1].item()) == 2
+    x = manager._lu_solve_fp64(Ad, bd, [bd[:, 0].contiguous(), bd[:, 1].contiguous()]).cpu().numpy()
+    res = np.abs(A.astype(np.longdouble) @ x.astype(np.longdouble) - b)
+    assert (res <= 4 * 2.3e-16 * (np.abs(A) @ np.abs(x) + np.abs(b))).all()
+    Ad[:, 1] = 0.0
+    with pytest.raises(torch.linalg.LinAlgError, match="singular"):
+        manager._lu_solve_fp64(Ad, bd[:, 0], [bd[:, 0].contiguous()])
+
+
+def test_laplace_neumann_never_raises(manager):
+    """The pure Neumann cube: 500 assemblies, each its own order of the atomic
+    sums, are all solved."""
+    for _ in range(500):
+        manager._mat_A.zero_()
+        manager.run()
