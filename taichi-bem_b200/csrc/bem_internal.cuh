@@ -137,6 +137,17 @@ int bem_launch_assemble_batch(bem_ctx* ctx, const bem_op_desc* op, const bem_spa
 // Class of the bound on the FP32 split phase |k (r - R)| <= k (rho_i + rho_j):
 // 2 when <= 0.3 (short polynomials), 1 when <= 0.78 < pi/4 (no reduction), 0 otherwise
 int bem_phase_class(double bound);
+// The power of two that brings a = re + i im to the size of 1, from the exponent
+// fields: 1/a = conj(a s) / |a s|^2 s has the range of the type, where |a|^2 may
+// overflow or underflow, and the same digits where it does not.
+__device__ __forceinline__ double bem_unit_scale(double re, double im) {
+    const int h = max(__double2hiint(re) & 0x7fffffff, __double2hiint(im) & 0x7fffffff) >> 20;
+    return __hiloint2double(max(2046 - h, 1) << 20, 0);
+}
+__device__ __forceinline__ float bem_unit_scale(float re, float im) {
+    const int h = max(__float_as_int(re) & 0x7fffffff, __float_as_int(im) & 0x7fffffff) >> 23;
+    return __int_as_float(max(254 - h, 1) << 23);
+}
 int bem_launch_dirichlet(bem_ctx* ctx, const bem_op_desc* op, const bem_space* test, const bem_space* trial,
                          void* out, int64_t ld, double scale, const bem_space* rows, const bem_space* data,
                          const void* g, void* y, double scale_k, int conj_g, cudaStream_t s);

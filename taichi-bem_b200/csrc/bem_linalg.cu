@@ -138,6 +138,16 @@ struct PivSlot {
     int pad;
 };
 
+// 1/a of a pivot candidate; not finite for zero
+template <typename T, bool C>
+__device__ __forceinline__ El<T, C> pivot_inverse(El<T, C> a) {
+    if (!C) return El<T, C>{T(1) / a.re, T(0)};
+    const T s = bem_unit_scale(a.re, a.im);
+    a = El<T, C>{a.re * s, a.im * s};
+    const T rd = T(1) / (a.re * a.re + a.im * a.im);
+    return El<T, C>{a.re * rd * s, -a.im * rd * s};
+}
+
 // ----------------------------------------------------------------------------
 // panel factorisation (cooperative)
 //
@@ -306,15 +316,7 @@ __global__ void __launch_bounds__(256) lu_panel_kernel(T* A, int64_t lda, int n,
         // 5. scale column jj below the diagonal, rank-1 update of the panel
         const E pv = s_prow[j];
         const bool nonzero = s_pv > 0.0;
-        E inv;
-        if (C) {
-            T d = pv.re * pv.re + pv.im * pv.im;
-            inv.re = nonzero ? pv.re / d : T(0);
-            inv.im = nonzero ? -pv.im / d : T(0);
-        } else {
-            inv.re = nonzero ? T(1) / pv.re : T(0);
-            inv.im = T(0);
-        }
+        const E inv = nonzero ? pivot_inverse<T, C>(pv) : E{T(0), T(0)};
         for (int r = max(r_begin, jj + 1) + wid; r < r_end; r += nwarps) {
             E a = get(r, j);
             E l;
@@ -396,19 +398,6 @@ __device__ __forceinline__ int best_lane(const PivKey& k) {
         who = __ballot_sync(0xffffffffu, mine && k.pos == pos);
     }
     return __ffs((int)who) - 1;
-}
-
-// 1/d on the pivot chain: in FP64 the approximate reciprocal (about 20 bits)
-// and one third-order step, where d is far from the ends of the range; a
-// division otherwise
-__device__ __forceinline__ float pivot_rcp(float d) { return 1.0f / d; }
-__device__ __forceinline__ double pivot_rcp(double d) {
-    const double m = fabs(d);
-    if (!(m > 1e-290 && m < 1e290)) return 1.0 / d;
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
-    const double e = fma(-d, y, 1.0);
-    return fma(y, fma(e, e, e), y);
 }
 
 template <typename T, bool C>
@@ -635,14 +624,7 @@ __global__ void __launch_bounds__(THREADS) lu_panel_cluster_kernel(T* A, int64_t
                     }
                 }
                 // every row's reciprocal beside the reductions, so that the pivot's is at hand
-                E rc{T(0), T(0)};
-                if (C) {
-                    const T rd = pivot_rcp(a[jj].re * a[jj].re + a[jj].im * a[jj].im);
-                    rc.re = a[jj].re * rd;
-                    rc.im = -a[jj].im * rd;
-                } else {
-                    rc.re = pivot_rcp(a[jj].re);
-                }
+                const E rc = pivot_inverse<T, C>(a[jj]);
                 if (lane == best_lane(key)) {
 #pragma unroll
                     for (int c = 0; c < PCL_SB; ++c) sh.warp[jj & 1][wid][c] = c == jj ? rc : a[c];

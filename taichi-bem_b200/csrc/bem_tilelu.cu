@@ -59,20 +59,25 @@ template <typename T>
 __device__ __forceinline__ CE<T> cmul(CE<T> a, CE<T> b) {
     return CE<T>{a.re * b.re - a.im * b.im, a.re * b.im + a.im * b.re};
 }
-template <typename T>
+// 1 / a; 0 for zero and NaN (a preconditioner's factor stays finite)
+template <bool C, typename T>
 __device__ __forceinline__ CE<T> cinv(CE<T> a) {
+    if (!C) return CE<T>{fabs(a.re) > T(0) ? T(1) / a.re : T(0), T(0)};
     T d = a.re * a.re + a.im * a.im;
-    return d > T(0) ? CE<T>{a.re / d, -a.im / d} : CE<T>{T(0), T(0)};
+    if (d > T(1e-30) && d < T(1e30)) return CE<T>{a.re / d, -a.im / d};  // the scale off the pivot chain
+    const T s = bem_unit_scale(a.re, a.im);
+    a = CE<T>{a.re * s, a.im * s};
+    d = a.re * a.re + a.im * a.im;
+    return d > T(0) ? CE<T>{a.re / d * s, -a.im / d * s} : CE<T>{T(0), T(0)};
 }
-// x / a over the whole range: a is scaled by a power of two, so that its
-// square neither overflows nor underflows; a = 0 gives infinities and NaN
+// x / a over the whole range; a = 0 gives infinities and NaN
 template <bool C>
 __device__ __forceinline__ CE<double> cdiv(CE<double> x, CE<double> a) {
     if (!C) return CE<double>{x.re / a.re, 0.0};
-    const double m = fmax(fabs(a.re), fabs(a.im));
-    const int e = m > 0.0 && m <= 1.7976931348623157e308 ? ilogb(m) : 0;
-    const double re = scalbn(a.re, -e), im = scalbn(a.im, -e), d = re * re + im * im;
-    return CE<double>{scalbn((x.re * re + x.im * im) / d, -e), scalbn((x.im * re - x.re * im) / d, -e)};
+    const double s = bem_unit_scale(a.re, a.im);
+    a = CE<double>{a.re * s, a.im * s};
+    const double d = a.re * a.re + a.im * a.im;
+    return CE<double>{(x.re * a.re + x.im * a.im) / d * s, (x.im * a.re - x.re * a.im) / d * s};
 }
 
 // --------------------------------------------------------------------------
@@ -173,7 +178,7 @@ __global__ void __launch_bounds__(256) tile_diag_kernel(T* A, int64_t lda, int n
             __syncthreads();
             const CE<T> pv = s_row[j];
             if (!(pv.re != T(0) || pv.im != T(0)) && zero == 0) zero = k0 + j + 1;
-            const CE<T> inv = cinv(pv);
+            const CE<T> inv = cinv<C>(pv);
             CE<T> l[4];
 #pragma unroll
             for (int a = 0; a < 4; ++a) {
@@ -259,7 +264,7 @@ __global__ void __launch_bounds__(256) tile_inv_kernel(const T* A, int64_t lda, 
             if constexpr (EXACT)
                 v = cdiv<C>(v, S[tid * DIAG_LD + tid]);
             else
-                v = cinv(S[tid * DIAG_LD + tid]);
+                v = cinv<C>(S[tid * DIAG_LD + tid]);
         }
         s_rdiag[tid] = v;
     }
@@ -418,7 +423,7 @@ __global__ void __launch_bounds__(256) tile_apply_kernel(T* A, int64_t lda, int 
             const int r = ty + 16 * a, c = tx + 16 * b;
             const CE<T> d = r < m && c < m ? ldE<T, C>(A, (int64_t)(k0 + r) * lda + k0 + c) : CE<T>{T(0), T(0)};
             D[r * APPLY_LD + c] = d;
-            if (r == c) s_rdiag[r] = r < m ? cinv(d) : CE<T>{T(0), T(0)};
+            if (r == c) s_rdiag[r] = r < m ? cinv<C>(d) : CE<T>{T(0), T(0)};
         }
     __syncthreads();
     if (mode == 0) {

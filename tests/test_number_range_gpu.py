@@ -128,3 +128,33 @@ def test_laplace_neumann_never_raises(manager):
     for _ in range(500):
         manager._mat_A.zero_()
         manager.run()
+
+
+# ---- pivots whose square leaves the range --------------------------------------------------
+@pytest.mark.parametrize("dtype,exp,tiled", [
+    (t, e, tiled)
+    for t, e in [("float32", -80), ("float32", 66), ("complex64", -66), ("complex64", -80), ("complex64", 66),
+                 ("float64", -550), ("float64", 520), ("complex128", -515), ("complex128", -550), ("complex128", 520)]
+    for tiled in (False, True)
+    if not (tiled and t in ("float64", "complex128"))])  # the tile factor compares its candidates in FP32
+def test_lu_is_equivariant_under_powers_of_two(engine, dtype, exp, tiled):
+    """2^exp A has A's pivots and L, and 2^exp U: all operations but the
+    products that test the pivots' size scale exactly.  FP32 factors above one
+    tile would also use the tensor cores' split, so one tile is taken; rounding
+    of the reciprocal alone may differ (1/a from |a|^2 or from the scaled a),
+    a few eps of a Gaussian factor's growth, 64 eps max|F|."""
+    n = 64
+    A = _gaussian((n, n), dtype.startswith("complex"), 9).astype(dtype)
+    A += 4 * np.eye(n, dtype=dtype)
+    scale = np.ldexp(1.0, exp)
+    out = []
+    for f in (1.0, scale):
+        LU = torch.as_tensor(A * np.asarray(f, A.real.dtype), device="cuda").contiguous()
+        piv, *_, info = (engine.lu_factor_tiled if tiled else engine.lu_factor)(LU)
+        assert int(info.item()) == 0
+        F = LU.cpu().numpy().astype(np.clongdouble if np.iscomplexobj(A) else np.longdouble)
+        out.append((piv.cpu().numpy(), np.tril(F, -1) + np.triu(F) / f))
+    (p0, F0), (p1, F1) = out
+    assert np.array_equal(p0, p1)
+    eps = 2.3e-16 if dtype in ("float64", "complex128") else 1.2e-7
+    assert np.abs(F1 - F0).max() < 64 * eps * np.abs(F0).max()
