@@ -498,6 +498,10 @@ int bem_set_mesh_instances(bem_ctx* ctx, float* solved_vertices, float* exact_ve
  * out[0] = FP32 FMA TFLOP/s, out[1] = FP64 FMA TFLOP/s, out[2] = MUFU (rsqrt)
  * Gop/s.  Synchronous; allocates a small buffer. */
 int bem_measure_peaks(bem_ctx* ctx, double* out, void* stream);
+/* The FP64 functions of the quadrature kernels on n device values x (no
+ * reference counterpart; for tests): which 0: a = sqrt x, b = 1/sqrt x; 1: a =
+ * sin x, b = cos x; 2: the same for |x| <= pi/4; 3: for |x| <= 0.3. */
+int bem_device_math(bem_ctx* ctx, int which, const double* x, double* a, double* b, int64_t n, void* stream);
 /* No reference counterpart.  *version = the binary architecture (major*10 +
  * minor, cudaFuncGetAttributes' binaryVersion) of this library's device code
  * as loaded on the current device: 100 for the sm_100a build.  Needs a GPU. */

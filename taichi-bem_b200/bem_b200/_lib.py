@@ -38,6 +38,7 @@ EXPORTS = [
     "bem_lu_factor_status", "bem_binary_version", "bem_ctx_set_tuning", "bem_assemble_calderon", "bem_gram",
     "bem_lstsq_refine", "bem_chol_factor", "bem_gemm", "bem_chol_inverse", "bem_normal_refine", "bem_near_pair_list",
     "bem_assemble_batch", "bem_cgs2_append", "bem_adjoint_vertices_data",
+    "bem_device_math",
 ]
 STATIC_SOLVE_MAX_N = 32768  # BEM_STATIC_SOLVE_MAX_N
 TUNE_CALDERON_GROUP = 0  # BEM_TUNE_CALDERON_GROUP
@@ -133,6 +134,7 @@ def load():
     L.bem_set_mesh_instances.argtypes = [vp, vp, vp, vp, vp]
     L.bem_adjoint_vertices.argtypes = [vp, ctypes.POINTER(OpDesc), ctypes.POINTER(Space), ctypes.POINTER(Space), vp,
                                        vp, vp, vp]
+    L.bem_device_math.argtypes = [vp, ctypes.c_int, vp, vp, vp, ctypes.c_int64, vp]
     L.bem_adjoint_vertices_data.argtypes = [vp, ctypes.POINTER(OpDesc), ctypes.POINTER(Space), ctypes.POINTER(Space),
                                             vp, vp, vp, vp, vp]
     for name in EXPORTS:

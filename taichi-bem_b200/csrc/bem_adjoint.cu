@@ -103,7 +103,8 @@ __device__ __forceinline__ void adj_point(PairMoments& M, const double d[3], dou
                                           const double by[3], const double hy[3], double uy, double sgn, const double nj[3],
                                           double invJj) {
     const double r2 = d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
-    const double rinv = dev_rsqrt(r2);
+    double r, rinv;
+    dev_r_rinv(r2, r, rinv);
     const double rinv2 = rinv * rinv;
     double g[3];
     if (OP == BEM_OP_V) {
@@ -325,7 +326,8 @@ __global__ void __launch_bounds__(ADJ_THREADS) adj_far_kernel(AdjArgs a) {
                     const double4 xp = sxt[q];
                     const double2 ph = sp[q];
                     const double dx = xp.x + e0, dy = xp.y + e1, dz = xp.z + e2;
-                    const double rinv = dev_rsqrt(fma(dx, dx, fma(dy, dy, dz * dz)));
+                    double r, rinv;
+                    dev_r_rinv(fma(dx, dx, fma(dy, dy, dz * dz)), r, rinv);
                     const double rinv2 = rinv * rinv;
                     const double h = xp.w * rinv;
                     const double w3 = h * rinv2;  // w / r^3

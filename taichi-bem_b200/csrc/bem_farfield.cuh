@@ -32,24 +32,25 @@ __device__ __forceinline__ void dev_r_rinv(float r2, float& r, float& rinv) {
     rinv = fmaf(0.5f * y0, e, y0);
     r = fmaf(0.5f * p, e, p);
 }
-// FP64: the hardware's approximate reciprocal square root (about 20 bits; the
-// low word of its result is zero, so its square is exact) and one step of the
-// third-order iteration y (1 + e/2 + 3 e^2/8), e = 1 - r2 y^2, whose remainder
-// 5 e^3/16 is below 2^-58: five FP64 operations, against about ten and a range
-// check in the library's rsqrt.  0 and infinity keep the approximation's
-// infinity and 0, as the library's do.
-__device__ __forceinline__ double dev_rsqrt(double r2) {
-    double y0;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y0) : "d"(r2));
-    const double e = fma(-r2, y0 * y0, 1.0);
-    const double y = fma(y0 * e, fma(0.375, e, 0.5), y0);
-    // exponent field 0 or all ones: the iteration has no finite value there
-    const bool special = (unsigned)(__double2hiint(y0) - 0x00100000) >= 0x7fe00000u;
-    return special ? y0 : y;
-}
+// FP64: the hardware's approximate reciprocal square root y (about 20 bits) and
+// one step of Goldschmidt's coupled iteration for sqrt x and 1/sqrt x (R. E.
+// Goldschmidt, MIT 1964) in its third-order form (Ercegovac, Imbert, Matula,
+// Muller and Wei, IEEE Trans. Comput. 49(7), 2000).  With p = x y, about sqrt x,
+// and e = 1 - p y: 1/sqrt x = y (1 - e)^(-1/2) and sqrt x = p (1 - e)^(-1/2) up
+// to p's rounding, and the binomial series 1 + e/2 + 3 e^2/8 leaves 5 e^3/16,
+// below 2^-58.  p's rounding enters e once and both results by half: with the last
+// rounding at most 1 ulp each.  For x = 0, infinity and NaN, where e is not
+// finite, 1/sqrt x is the approximation's infinity, 0 and NaN, and sqrt x NaN;
+// a subnormal x counts as 0.
 __device__ __forceinline__ void dev_r_rinv(double r2, double& r, double& rinv) {
-    rinv = dev_rsqrt(r2);
-    r = r2 * rinv;
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(r2));
+    const double p = r2 * y;
+    const double e = fma(-p, y, 1.0);
+    const double q = e * fma(0.375, e, 0.5);
+    r = fma(p, q, p);
+    // |e| < 1, by its exponent (off the FP64 pipe)
+    rinv = (__double2hiint(e) & 0x7fffffff) < 0x3ff00000 ? fma(y, q, y) : y;
 }
 
 // Pair frame of an FP32 separate pair.  With D = c_i - c_j (FP64 centroid
@@ -150,7 +151,7 @@ __device__ __forceinline__ void dev_sincos_phase(float x, bool small, float* s, 
         dev_sincos(x, s, c);
 }
 
-// FP64 sine and cosine on |y| <= 0.3 (SHORT) or |y| <= pi/4: Taylor
+// FP64 sine and cosine on |y| <= 0.3 (SHORT) or |y| <= pi/4: the Taylor
 // polynomials whose first dropped terms are below 2.7e-17 (y^13) and 5.5e-19
 // (y^14), or 4.7e-17 (y^17) and 2.1e-18 (y^18).
 template <bool SHORT>
@@ -180,10 +181,11 @@ __device__ __forceinline__ void dev_sincos_poly64(double y, double* s, double* c
 }
 __device__ __noinline__ void dev_sincos_any(double x, double* s, double* c) { sincos(x, s, c); }
 // Any FP64 phase.  Up to 1e5 (a wavenumber of 1e5 on a unit mesh): reduction
-// by n pi/2 with pi/2 split in two doubles (n pi/2_hi enters by one FMA, the
-// remainder is good to 2^-54), the polynomials above and the quadrant; beyond,
-// and for infinities and NaN, the library's sincos.  About 24 FP64 operations
-// against about 40; the library's large-argument path is kept out of line.
+// by n pi/2 with pi/2 split in two doubles (Cody and Waite, Software Manual for
+// the Elementary Functions, 1980), the first product exact in its FMA; then the
+// polynomials above and the quadrant.  The reduced argument carries two
+// roundings of at most 2^-54, the results at most 2.3e-16.  Beyond, and for
+// infinities and NaN, CUDA's sincos, kept out of line.
 __device__ __forceinline__ void dev_sincos(double x, double* s, double* c) {
     if (!(fabs(x) <= 1e5)) {
         double a, b;

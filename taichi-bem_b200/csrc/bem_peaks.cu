@@ -3,6 +3,7 @@
 // FP64 FMA pipes and the special-function unit, not by HBM or tensor cores).
 #include <cuda_runtime.h>
 
+#include "bem_farfield.cuh"
 #include "bem_internal.cuh"
 
 namespace {
@@ -71,6 +72,33 @@ extern "C" int bem_measure_peaks(bem_ctx* ctx, double* out, void* stream) {
     out[1] = 2.0 * fmas / (ms64 * 1e-3) / 1e12;  // FP64 TFLOP/s
     out[2] = fmas / (msmu * 1e-3) / 1e9;         // MUFU (rsqrt) Gop/s
     return BEM_OK;
+}
+
+namespace {
+
+__global__ void math_kernel(int which, const double* x, double* a, double* b, int64_t n) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    double u, v;
+    switch (which) {
+        case 0: dev_r_rinv(x[i], u, v); break;
+        case 1: dev_sincos(x[i], &u, &v); break;
+        case 2: dev_sincos_poly64<false>(x[i], &u, &v); break;
+        default: dev_sincos_poly64<true>(x[i], &u, &v);
+    }
+    a[i] = u;
+    b[i] = v;
+}
+
+}  // namespace
+
+extern "C" int bem_device_math(bem_ctx* ctx, int which, const double* x, double* a, double* b, int64_t n, void* stream) {
+    if (!ctx) return BEM_ERR_INVALID;
+    if (!x || !a || !b || n <= 0 || n > (int64_t)1 << 30 || which < 0 || which > 3)
+        return bem_fail(ctx, BEM_ERR_INVALID, "device_math: bad arguments");
+    math_kernel<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>(which, x, a, b, n);
+    ctx->launches++;
+    return bem_check_cuda(ctx, cudaGetLastError(), "math_kernel");
 }
 
 // Architecture of the device code this library runs on the current device:

@@ -158,3 +158,63 @@ def test_lu_is_equivariant_under_powers_of_two(engine, dtype, exp, tiled):
     assert np.array_equal(p0, p1)
     eps = 2.3e-16 if dtype in ("float64", "complex128") else 1.2e-7
     assert np.abs(F1 - F0).max() < 64 * eps * np.abs(F0).max()
+
+
+# ---- FP64 root and phase of the quadrature kernels ----------------------------------------
+def _device_math(engine, which, x):
+    x = torch.as_tensor(np.ascontiguousarray(x), device="cuda")
+    a, b = torch.empty_like(x), torch.empty_like(x)
+    engine._check(engine.lib.bem_device_math(engine.ctx, which, x.data_ptr(), a.data_ptr(), b.data_ptr(), x.numel(),
+                                             torch.cuda.current_stream().cuda_stream))
+    torch.cuda.synchronize()
+    return x, a.cpu().numpy(), b.cpu().numpy()
+
+
+def test_root_and_reciprocal_root_to_the_last_digit(engine):
+    """sqrt x and 1/sqrt x within 1 ulp (half an ulp for the last rounding,
+    half for that of p = x y), over the whole range of normal numbers and
+    densely around powers of two; within one more of CUDA's; the ends."""
+    rng = np.random.default_rng(1)
+    m = np.concatenate([rng.uniform(1.0, 4.0, 400000), 1.0 + np.arange(64) * 2.0 ** -52, 4.0 - np.arange(1, 65) * 2.0 ** -51])
+    x = np.concatenate([m, np.ldexp(m, 2 * rng.integers(-510, 511, len(m)))])
+    x = x[(x >= 2.3e-308) & np.isfinite(x)]
+    xd, r, rinv = _device_math(engine, 0, x)
+    root = np.sqrt(x.astype(np.longdouble))
+    assert (np.abs(r - root) <= 1.01 * np.spacing(r)).all()
+    assert (np.abs(rinv - 1 / root) <= 1.01 * np.spacing(rinv)).all()
+    assert (np.abs(rinv - torch.rsqrt(xd).cpu().numpy()) <= 2 * np.spacing(rinv)).all()
+    _, _, rinv = _device_math(engine, 0, np.array([0.0, np.inf, np.nan, -1.0]))
+    assert rinv[0] == np.inf and rinv[1] == 0.0 and np.isnan(rinv[2:]).all()
+
+
+@pytest.mark.parametrize("which,bound", [(2, np.pi / 4), (3, 0.3)])
+def test_short_sine_and_cosine(engine, which, bound):
+    """Half an ulp for the last rounding, half for the first dropped term, the
+    rest of Horner's scheme enters with y^2 / 2: 1.5 ulp."""
+    rng = np.random.default_rng(2)
+    x = np.concatenate([rng.uniform(-bound, bound, 400000), bound * 2.0 ** -rng.uniform(0, 60, 100000), [0.0, bound]])
+    xd, s, c = _device_math(engine, which, x)
+    wide = x.astype(np.longdouble)
+    assert (np.abs(s - np.sin(wide)) <= 1.5 * np.spacing(np.abs(s))).all()
+    assert (np.abs(c - np.cos(wide)) <= 1.5 * np.spacing(c)).all()
+
+
+def test_sine_and_cosine_of_any_phase(engine):
+    """2.3e-16 absolute (two roundings of the reduced argument, one ulp of the
+    polynomials) up to the switch at 1e5, next to multiples of pi/2 and on
+    both sides of the switch; beyond it CUDA's own; infinities and NaN."""
+    rng = np.random.default_rng(3)
+    near = np.rint(rng.uniform(0, 63661, 100000)) * (np.pi / 2)
+    near = np.nextafter(near, near * (1 + rng.choice([-1, 1], len(near)) * 1e-3))
+    x = np.concatenate([rng.uniform(-1e5, 1e5, 400000), rng.uniform(-7, 7, 100000), near, 10.0 ** rng.uniform(-300, 5, 50000),
+                        1e5 + np.arange(-64, 65) * np.spacing(1e5), [0.0]])
+    xd, s, c = _device_math(engine, 1, x)
+    wide = x.astype(np.longdouble)
+    assert np.abs(s - np.sin(wide)).max() < 2.3e-16 and np.abs(c - np.cos(wide)).max() < 2.3e-16
+    assert np.abs(s - torch.sin(xd).cpu().numpy()).max() < 4.6e-16
+    assert np.abs(c - torch.cos(xd).cpu().numpy()).max() < 4.6e-16
+    x = np.concatenate([rng.uniform(1e5, 1e9, 1000), 2.0 ** rng.uniform(17, 1000, 1000)])
+    xd, s, c = _device_math(engine, 1, x)
+    assert np.abs(s - torch.sin(xd).cpu().numpy()).max() < 2.3e-16
+    _, s, c = _device_math(engine, 1, np.array([np.inf, -np.inf, np.nan]))
+    assert np.isnan(s).all() and np.isnan(c).all()
