@@ -24,6 +24,7 @@
 #include <cuda_runtime.h>
 
 #include "bem_internal.cuh"
+#include <cmath>
 #include <type_traits>
 
 #include "bem_farfield.cuh"
@@ -1253,8 +1254,12 @@ int bem_launch_geometry(bem_ctx* ctx, cudaStream_t s) {
 }
 
 // Class of the bound on the FP32 split phase |k (r - R)| <= k (rho_i + rho_j):
-// 2 when <= 0.3 (short polynomials), 1 when <= 0.78 < pi/4 (no reduction), 0 otherwise
-int bem_phase_class(double bound) { return bound <= 0.3 ? 2 : (bound <= 0.78 ? 1 : 0); }
+// 2 when <= 0.3 (short polynomials), 1 when <= 0.78 < pi/4 (no reduction), 0
+// otherwise.  A negative wavenumber has the bound of its magnitude.
+int bem_phase_class(double bound) {
+    bound = std::fabs(bound);
+    return bound <= 0.3 ? 2 : (bound <= 0.78 ? 1 : 0);
+}
 
 int bem_fill_local_map(bem_ctx* ctx, const bem_space* sp, int32_t* map, cudaStream_t s) {
     if (int rc = bem_check_cuda(ctx, cudaMemsetAsync(map, 0xff, sizeof(int32_t) * ctx->nt, s), "memset")) return rc;

@@ -218,3 +218,40 @@ def test_sine_and_cosine_of_any_phase(engine):
     assert np.abs(s - torch.sin(xd).cpu().numpy()).max() < 2.3e-16
     _, s, c = _device_math(engine, 1, np.array([np.inf, -np.inf, np.nan]))
     assert np.isnan(s).all() and np.isnan(c).all()
+
+
+# ---- negative wavenumbers ------------------------------------------------------------------
+def _spaces(engine, v, f):
+    from bem_b200.engine import DeviceSpace
+    p = np.arange(len(f), dtype=np.int32)
+    return (DeviceSpace.from_numpy(p, 1, p, engine.device), DeviceSpace.from_numpy(p, 3, f.reshape(-1).copy(), engine.device))
+
+
+@pytest.mark.parametrize("k", [-40.0, -0.2])
+def test_mixed_precision_at_negative_wavenumbers(engine, k):
+    """Blocks, products and the Dirichlet pass against FP64: the FP32 phase k (r
+    - R), up to 40 * 2 * 0.35 = 28, carries 6e-8 of itself: 28 * 6e-8 =
+    1.7e-6 of an entry, 5e-6 of the largest."""
+    from bem_b200 import _lib as L
+    from bem_b200 import icosphere
+    v, f = icosphere(1)
+    engine.set_mesh(v, f, 3)
+    p0, p1 = _spaces(engine, v, f)
+    g = torch.as_tensor(_gaussian(len(v), True, 6), device="cuda")
+    x0 = torch.as_tensor(_gaussian(len(f), True, 7), device="cuda")
+    res = []
+    for prec in (L.PREC_FP64, L.PREC_MIXED):
+        new = lambda *s: torch.zeros(*s, dtype=torch.complex128, device="cuda")
+        out = []
+        for op, t, r in ((L.OP_V, p0, p0), (L.OP_K, p0, p1), (L.OP_KP, p1, p0), (L.OP_W, p1, p1)):
+            nt, nr = (len(f) if s is p0 else len(v) for s in (t, r))
+            desc = engine.op_desc(op, True, k, k * k, precision=prec)
+            out.append(new(nt, nr))
+            engine.assemble(desc, t, r, out[-1])
+            out.append(new(nt))
+            engine.apply(desc, t, r, x0 if r is p0 else g, out[-1])
+        out += [new(len(f), len(f)), new(len(f))]
+        engine.assemble_dirichlet(engine.op_desc(L.OP_V, True, k, k * k, precision=prec), p0, p0, out[-2], p0, p1, g, out[-1])
+        res.append(out)
+    for want, got in zip(*res):
+        assert float((got - want).abs().max()) < 5e-6 * float(want.abs().max())
