@@ -243,7 +243,7 @@ __global__ void __launch_bounds__(ADJ_THREADS) adj_far_kernel(AdjArgs a) {
         const int t = threadIdx.x, li = li0 + t;
         const int gi = li < a.n_test ? a.test_panels[li] : -1;
         s_gi[t] = gi;
-        s_ri[t] = gi >= 0 ? a.trial_local[gi] : -1;
+        s_ri[t] = gi >= 0 && a.test_local[gi] == li ? a.trial_local[gi] : -1;
         const int row = li < a.n_test ? a.test_dof[li] : -1;
         s_lam[t] = row >= 0 ? a.lam[row] : 0.0;
         double u[3];
@@ -268,7 +268,8 @@ __global__ void __launch_bounds__(ADJ_THREADS) adj_far_kernel(AdjArgs a) {
 
     const bool valid_j = lj < a.n_trial;
     const int gj = valid_j ? a.trial_panels[lj] : 0;
-    const int rj = valid_j ? a.test_local[gj] : -1;  // index of the trial panel in the test list
+    // index of the trial panel in the test list; -1 also for a list's further entries of one panel
+    const int rj = valid_j && a.trial_local[gj] == lj ? a.test_local[gj] : -1;
     int tri_j[3];
     for (int c = 0; c < 3; ++c) tri_j[c] = a.tris[3 * gj + c];
     const double nj[3] = {a.normal[3 * gj], a.normal[3 * gj + 1], a.normal[3 * gj + 2]};

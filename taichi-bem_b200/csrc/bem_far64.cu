@@ -11,7 +11,8 @@
 //          sum w phi_a(x) (-d.n_i) F / r^3   (K: row j, hats of i; K': hats of i, column j)
 // with F = (1 - ikr) e^{ikr}.  The lists may differ (a Mix partition): a pair
 // whose reversed order is in the call too is evaluated by the order with the
-// smaller test panel and added for both, any other one for its own.
+// smaller test panel and added for both, any other one for its own (so is every
+// further entry of a panel that a list names twice: the maps hold one of them).
 //
 // Bound: FP64 issue.  What a point pair costs is therefore its count of FP64
 // instructions (V Helmholtz: 3 differences, 3 for r^2, 5 for 1/r, r, the
@@ -130,7 +131,7 @@ __global__ void __launch_bounds__(FAR_THREADS) far64_kernel(Far64Args a) {
         const int li = li0 + threadIdx.x;
         const int gi = li < a.n_test ? a.test_panels[li] : -1;
         s_gi[threadIdx.x] = gi;
-        s_ri[threadIdx.x] = gi >= 0 ? a.trial_local[gi] : -1;
+        s_ri[threadIdx.x] = gi >= 0 && a.test_local[gi] == li ? a.trial_local[gi] : -1;
         for (int c = 0; c < 3; ++c) {
             s_tri[threadIdx.x][c] = gi >= 0 ? a.tris[3 * gi + c] : -1;
             s_cen[threadIdx.x][c] = gi >= 0 ? a.centroid[3 * gi + c] : 0.0;
@@ -147,7 +148,7 @@ __global__ void __launch_bounds__(FAR_THREADS) far64_kernel(Far64Args a) {
 
     const bool valid_j = lj < a.n_trial;
     const int gj = valid_j ? a.trial_panels[lj] : 0;
-    const int rj = valid_j ? a.test_local[gj] : -1;  // index of the trial panel in the test list
+    const int rj = valid_j && a.trial_local[gj] == lj ? a.test_local[gj] : -1;  // index of the trial panel in the test list
     int tri_j[3];
     double cj[3], nj[3];
 #pragma unroll

@@ -255,3 +255,51 @@ def test_mixed_precision_at_negative_wavenumbers(engine, k):
         res.append(out)
     for want, got in zip(*res):
         assert float((got - want).abs().max()) < 5e-6 * float(want.abs().max())
+
+
+# ---- lists that name a panel twice -----------------------------------------------------------
+@pytest.mark.parametrize("op,nbx,nby", [("V", 3, 3), ("W", 3, 3), ("K", 1, 3), ("KP", 3, 1)])
+def test_panels_named_twice(engine, op, nbx, nby):
+    """Separate pairs count once per entry of either list, touching ones once
+    per panel: against the sum of calls without repeats, at FP64's last digits
+    (sums of up to ~300 terms in another order: 1e-12 of the largest)."""
+    from bem_b200 import _lib as L
+    from bem_b200 import icosphere
+    from bem_b200.engine import DeviceSpace
+    v, f = icosphere(1)
+    engine.set_mesh(v, f, 3)
+    touch = (f[:, None, :, None] == f[None, :, None, :]).any((2, 3))
+    rng = np.random.default_rng(11)
+    ts, rs = rng.permutation(len(f))[:50], rng.permutation(len(f))[:60]
+    te = rng.choice(np.intersect1d(ts, rs), 6, replace=False)
+    re = rng.choice(np.intersect1d(ts, rs), 5, replace=False)
+
+    def space(p, nb):  # as a C caller can pass it; from_numpy refuses repeats
+        p = torch.as_tensor(np.asarray(p, np.int32), device="cuda")
+        dof = p if nb == 1 else torch.as_tensor(f.astype(np.int32), device="cuda")[p.long()].reshape(-1).contiguous()
+        return DeviceSpace(p, nb, dof)
+
+    rows, cols = (len(f) if nb == 1 else len(v) for nb in (nbx, nby))
+    desc = engine.op_desc(getattr(L, "OP_" + op), False)
+    x = torch.as_tensor(_gaussian(cols, False, 12), device="cuda")
+    lam = torch.as_tensor(_gaussian(rows, False, 13), device="cuda")
+
+    def call(t, r, acc):
+        td, rd = space(t, nbx), space(r, nby)
+        engine.assemble(desc, td, rd, acc[0])
+        engine.apply(desc, td, rd, x, acc[1])
+        if op == "K":
+            engine.adjoint_vertices(desc, td, rd, lam, x, acc[2], acc[3])
+
+    new = lambda: [torch.zeros(s, dtype=torch.float64, device="cuda") for s in ((rows, cols), (rows,), (len(v), 3), (cols,))]
+    want, got = new(), new()
+    call(ts, rs, want)
+    for e in te:
+        call([e], rs[~touch[e, rs]], want)
+        for g in re[~touch[e, re]]:
+            call([e], [g], want)
+    for g in re:
+        call(ts[~touch[ts, g]], [g], want)
+    call(np.concatenate([ts, te]), np.concatenate([rs, re]), got)
+    for w, g in zip(want, got):
+        assert float((w - g).abs().max()) <= 1e-12 * float(w.abs().max())
