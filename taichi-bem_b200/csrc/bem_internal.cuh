@@ -137,6 +137,15 @@ int bem_launch_assemble_batch(bem_ctx* ctx, const bem_op_desc* op, const bem_spa
 // Class of the bound on the FP32 split phase |k (r - R)| <= k (rho_i + rho_j):
 // 2 when <= 0.3 (short polynomials), 1 when <= 0.78 < pi/4 (no reduction), 0 otherwise
 int bem_phase_class(double bound);
+// "Not written yet" in the solution vectors of the triangular solves
+// (bem_tilelu.cu): a signalling NaN, which no arithmetic produces (results that
+// are NaN are quiet).  A right-hand side that holds these bits is passed on as a
+// quiet NaN.
+constexpr unsigned long long BEM_PENDING = 0x7ff4deadbeef0001ull;
+__device__ __forceinline__ bool bem_pending(double v) { return __double_as_longlong(v) == (long long)BEM_PENDING; }
+__device__ __forceinline__ double bem_not_pending(double v) {
+    return bem_pending(v) ? __longlong_as_double(0x7ff8000000000000ll) : v;
+}
 // The power of two that brings a = re + i im to the size of 1, from the exponent
 // fields: 1/a = conj(a s) / |a s|^2 s has the range of the type, where |a|^2 may
 // overflow or underflow, and the same digits where it does not.

@@ -966,7 +966,7 @@ __global__ void gather_rhs_kernel(const double* b, int64_t ldb, const int32_t* p
     if (id >= (int64_t)n * nrhs) return;
     const int i = (int)(id / nrhs), c = (int)(id % nrhs);
     const int64_t src = W * ((int64_t)perm[i] * ldb + c);
-    for (int w = 0; w < W; ++w) out[c * vs + (int64_t)W * i + w] = b[src + w];
+    for (int w = 0; w < W; ++w) out[c * vs + (int64_t)W * i + w] = bem_not_pending(b[src + w]);
 }
 __global__ void scatter_rhs_kernel(const double* x, int64_t vs, double* b, int64_t ldb, int n, int nrhs, int W) {
     const int64_t id = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;

@@ -494,11 +494,8 @@ __global__ void __launch_bounds__(256) tile_apply_kernel(T* A, int64_t lda, int 
 // --------------------------------------------------------------------------
 // barrier-free triangular solves
 // --------------------------------------------------------------------------
-// "Not written yet": a signalling NaN, which no arithmetic produces (results
-// that are NaN are quiet) and which the permutation kernels below fill the
-// solution vectors with.  A value is its own ready flag.
-constexpr unsigned long long PENDING = 0x7ff4deadbeef0001ull;
-
+// The solution vectors start out as BEM_PENDING (pending_kernel); a value is its
+// own ready flag.
 __device__ __forceinline__ double ld_vol(const double* p) {
     double v;
     asm volatile("ld.volatile.global.f64 %0, [%1];" : "=d"(v) : "l"(p) : "memory");
@@ -507,11 +504,10 @@ __device__ __forceinline__ double ld_vol(const double* p) {
 __device__ __forceinline__ void st_vol(double* p, double v) {
     asm volatile("st.volatile.global.f64 [%0], %1;" ::"l"(p), "d"(v) : "memory");
 }
-__device__ __forceinline__ bool pending(double v) { return __double_as_longlong(v) == (long long)PENDING; }
 
 // x = U^{-1} L^{-1} b for NR right-hand sides (FP64, real or complex
 // interleaved, vs doubles apart; b already permuted), y the intermediate;
-// y and x are PENDING on entry.  Persistent: CTA b owns block rows b, b + P,
+// y and x are BEM_PENDING on entry.  Persistent: CTA b owns block rows b, b + P,
 // ... of each pass (forward with L into y, backward with U into x), all CTAs
 // are co-resident (cooperative launch) and wait only for rows earlier in the
 // pass's order, so every wait ends; the waits are bounded all the same.
@@ -602,7 +598,7 @@ __global__ void __launch_bounds__(256) tri_solve_kernel(const T* LU, int64_t lda
                     if (c < lim) {
                         a = ld_vol(v + r * vs + (int64_t)W * (base + c));
                         if (C) d = ld_vol(v + r * vs + (int64_t)W * (base + c) + 1);
-                        ready = ready && !pending(a) && !pending(d);
+                        ready = ready && !bem_pending(a) && !bem_pending(d);
                     }
                     re[h][r] = a;
                     im[h][r] = d;
@@ -612,7 +608,7 @@ __global__ void __launch_bounds__(256) tri_solve_kernel(const T* LU, int64_t lda
             // lane 0 polls one value; the others wait for it
             int ok = 1;
             if (lane == 0) {
-                while (pending(ld_vol(v + (int64_t)W * base))) {
+                while (bem_pending(ld_vol(v + (int64_t)W * base))) {
                     if (++it > FLAG_SPIN_CAP) {
                         atomicExch(err, BEM_ERR_TIMEOUT);
                         ok = 0;
@@ -853,7 +849,7 @@ __global__ void permute_kernel(const double* b, const int32_t* perm, double* out
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     int s = perm[i];
-    for (int w = 0; w < W; ++w) out[W * i + w] = b[W * s + w];
+    for (int w = 0; w < W; ++w) out[W * i + w] = bem_not_pending(b[W * s + w]);
 }
 
 // y and x start out not written
@@ -861,7 +857,7 @@ __global__ void pending_kernel(double* y, double* x, int64_t nd, const int* skip
     if (skip != nullptr && *skip != 0) return;
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= nd) return;
-    y[i] = x[i] = __longlong_as_double((long long)PENDING);
+    y[i] = x[i] = __longlong_as_double((long long)BEM_PENDING);
 }
 
 // Queues the triangular solve of NR permuted right-hand sides b (vs doubles

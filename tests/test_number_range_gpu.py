@@ -303,3 +303,21 @@ def test_panels_named_twice(engine, op, nbx, nby):
     call(np.concatenate([ts, te]), np.concatenate([rs, re]), got)
     for w, g in zip(want, got):
         assert float((w - g).abs().max()) <= 1e-12 * float(w.abs().max())
+
+
+def test_solve_with_any_bits_in_the_right_hand_side(engine):
+    """A right-hand side that holds the very NaN that marks an unwritten value
+    of the sweep is a NaN like any other: no wait runs out."""
+    n = 200
+    b = torch.ones(n, dtype=torch.float64, device="cuda")
+    b.view(torch.int64)[70] = 0x7FF4DEADBEEF0001
+    F = torch.eye(n, dtype=torch.float64, device="cuda")
+    piv = torch.arange(n, dtype=torch.int32, device="cuda")
+    x = b.clone()
+    engine.lu_solve(F, piv, x)
+    assert bool(x[70].isnan())
+    LU = torch.eye(n, dtype=torch.float32, device="cuda")
+    tpiv, dinv, _ = engine.lu_factor_tiled(LU)
+    y = b.clone()
+    engine.lu_solve_tiled(LU, tpiv, dinv, y)
+    assert bool(y[70].isnan())
