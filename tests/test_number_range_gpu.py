@@ -321,3 +321,49 @@ def test_solve_with_any_bits_in_the_right_hand_side(engine):
     y = b.clone()
     engine.lu_solve_tiled(LU, tpiv, dinv, y)
     assert bool(y[70].isnan())
+
+
+# ---- pivot sequence --------------------------------------------------------------------------
+def _exact_elimination(n, cplx, seed):
+    """Rows in random order of L U with L in {0, 1/2 (unit)} and U of integers
+    with powers of two (times a unit) on its diagonal, and n / 4 planted ties: a
+    row r that repeats the pivot row j up to column j (times a unit) has |l| = 1
+    there, and whichever of the two becomes the pivot, the other goes on as row r.
+    Every value of the elimination is a small dyadic number."""
+    rng = np.random.default_rng(seed)
+    units = np.array([1, -1, 1j, -1j]) if cplx else np.array([1.0, -1.0])
+    pick = lambda *s: units[rng.integers(0, len(units), s)]
+    low = np.tril(0.5 * pick(n, n) * (rng.random((n, n)) < 0.5), -1)
+    up = np.triu(rng.integers(-3, 4, (n, n)) * pick(n, n), 1) + np.diag(2.0 ** rng.integers(0, 3, n) * pick(n))
+    pairs = np.sort(rng.permutation(n)[:n // 4 * 2].reshape(-1, 2), 1)
+    low[:, pairs[:, 0]] = 0.0
+    for j, r in pairs:
+        s = pick(1)[0]
+        low[r, :j] = s * low[j, :j]
+        low[r, j] = s
+    return ((low + np.eye(n)) @ up)[rng.permutation(n)]
+
+
+@pytest.mark.parametrize("cplx", [False, True])
+@pytest.mark.parametrize("n", [40, 150, 700])
+def test_every_pivot_matches_the_textbook(engine, n, cplx):
+    """The whole pivot sequence, ties included (the lowest row of the largest
+    |re| + |im|), over several sub-blocks, panels and CTAs: exact arithmetic,
+    so the sequence and the factors are equal."""
+    A = _exact_elimination(n, cplx, n)
+    assert np.array_equal(A * 2, np.rint(A.real * 2) + (1j * np.rint(A.imag * 2) if cplx else 0.0))
+    ref, want, ties = A.copy(), [], 0
+    for j in range(n):
+        size = np.abs(ref[j:, j].real) + np.abs(ref[j:, j].imag)
+        p = j + int(np.argmax(size))
+        ties += int((size == size.max()).sum() > 1)
+        want.append(p)
+        ref[[j, p]] = ref[[p, j]]
+        ref[j + 1:, j] *= 1.0 / ref[j, j]
+        ref[j + 1:, j + 1:] -= np.outer(ref[j + 1:, j], ref[j, j + 1:])
+    assert ties >= n // 8
+    LU = torch.as_tensor(A, device="cuda")
+    piv, info = engine.lu_factor(LU)
+    assert int(info.item()) == 0
+    assert list(piv.cpu().numpy()) == want
+    assert np.array_equal(LU.cpu().numpy(), ref)
