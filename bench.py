@@ -70,8 +70,8 @@ TRANS_WORKLOAD = ("Helmholtz transmission 2x2 block Calderon system, icosphere s
                   "30722 unknowns), k_out=5, k_in=7.5 (n_i=2.25), GaussQR=5, incident plane wave, least squares on "
                   "the stacked [A; P+_i] (61444 x 30722)")
 # Algorithmic FP32 work per evaluation of the fused Calderon sweep
-# (far_calderon_kernel<float, 2, Helmholtz>), counted once from its scalar
-# source and kept fixed: the pair-frame geometry (e, s, r^2, r and 1/r with the
+# (two wavenumbers, Helmholtz), counted once from a scalar form of
+# the sweep and kept fixed: the pair-frame geometry (e, s, r^2, r and 1/r with the
 # Newton step, d.n_j, the split phase, w/r, w/r^3, t_j) 24 flops, and per
 # wavenumber the phase 1, sine/cosine polynomials 21, k r 1, G 2,
 # (1 - ikr) e^{ikr} 4 and the 14 test-point sums 26 = 55; two wavenumbers:

@@ -216,7 +216,7 @@ int bem_assemble_calderon(bem_ctx* ctx, const bem_op_desc* op, int nk, const dou
  * out and out_t are host arrays of nk entries; out/out_t hold device
  * pointers to BEM_C128 blocks.  Every separate panel pair's geometry is
  * evaluated once for 2 or 4 wavenumbers (BEM_TUNE_KBATCH_GROUP); near pairs
- * take the FP64 Sauter-Schwab kernel per wavenumber.  Replaces the per-k
+ * take the FP64 Sauter-Schwab kernel, two wavenumbers per launch.  Replaces the per-k
  * operator forward passes of the reference's wavenumber sweep
  * (demo/demo_3d_plot_Sio.py:63-82 -> get_mat_A1_inv_norm /
  * get_augment_mat_A1_inv_norm, BEM_manager.py:922-988 ->
@@ -299,7 +299,9 @@ int bem_adjoint_vertices_data(bem_ctx* ctx, const bem_op_desc* op, const bem_spa
 int bem_lu_factor(bem_ctx* ctx, int dtype, void* A, int64_t n, int64_t lda, int32_t* piv, int32_t* info,
                   void* stream);
 /* Solve with the factors: b (n x nrhs, row-major, ldb) overwritten by x (the
- * solve half of torch.linalg.solve, BEM_manager.py:1056). */
+ * solve half of torch.linalg.solve, BEM_manager.py:1056).  b and the arithmetic
+ * are FP64 whatever the factor's dtype; 1 <= nrhs <= 8, n <= 51200.  A zero pivot
+ * divides by zero. */
 int bem_lu_solve(bem_ctx* ctx, int dtype, const void* LU, int64_t n, int64_t lda, const int32_t* piv,
                  void* b, int64_t nrhs, int64_t ldb, void* stream);
 /* y = alpha*A*x + beta*y for one vector (dtype of A: F64/C128/F32/C64; x, y in
@@ -333,8 +335,9 @@ int bem_lu_factor_tiled(bem_ctx* ctx, int dtype, void* A, int64_t n, int64_t lda
 int bem_lu_factor_status(bem_ctx* ctx, void* stream);
 /* The solve half of torch.linalg.solve (BEM_manager.py:1056):
  * x = U^{-1} L^{-1} P b for one FP64 right-hand side b (overwritten), with the
- * factors of bem_lu_factor_tiled; a persistent kernel driven by per-tile ready
- * flags (bounded waits; BEM_ERR_TIMEOUT if one runs out). */
+ * factors of bem_lu_factor_tiled; a persistent kernel in which every value of
+ * the solution is its own ready flag (bounded waits; BEM_ERR_TIMEOUT if one runs
+ * out). */
 int bem_lu_solve_tiled(bem_ctx* ctx, int dtype, const void* LU, int64_t n, int64_t lda, const int32_t* piv,
                        const void* dinv, void* b, void* stream);
 

@@ -587,7 +587,7 @@ __global__ void __launch_bounds__(FAR_THREADS) far_calderon_x2_kernel(CalArgs a)
 // cosine, (1 - ikr) e^{ikr} and the 14 sums over the test points -- runs on
 // FFMA2 / FMUL2 / FADD2, one instruction for both wavenumbers.  Same
 // algebra, summation order and FP64 moments as
-// far_calderon_kernel<float, 2, true, PH>; the test points' phi_1, phi_2 are
+// far_calderon_kernel<float, 1, true, PH> per wavenumber; the test points' phi_1, phi_2 are
 // staged as broadcast pairs.  PH 2 / 1: the short / full sine and cosine
 // polynomials without argument reduction; PH 0: the reduced scalar form per
 // lane.
@@ -801,7 +801,7 @@ __global__ void __launch_bounds__(FAR_THREADS, SM ? 3 : 1) far_calderon_k2_kerne
 // wavenumber's phase, sine and cosine, and carries 30 moments.  FP32: a point
 // pair (q, q + 1) runs packed through the phase and the products, and the sums
 // take q, then q + 1, so every value and its rounding is that of
-// far_calderon_kernel<float, 2, true, PH>.  FP64: the phase relative to the
+// far_calderon_kernel<float, 1, true, PH>.  FP64: the phase relative to the
 // centroid distance, as in the other FP64 sweeps.  An odd Q^2 is padded by a
 // copy of the last point with weight 0 (it adds exact zeros).
 //   Assembly of both block systems, against both wavenumbers in one scalar

@@ -6,8 +6,8 @@
 //
 // Right-looking, panels of 1024 columns by default (BEM_TUNE_CHOL_NB), each
 // factored in sub-blocks of 64 in FP64:
-//   chol64_kernel     the 64 x 64 diagonal block in shared memory, and the
-//                     inverse of its factor;
+//   chol64_kernel     the 64 x 64 diagonal block and the inverse of its factor,
+//                     both in registers;
 //   dmma_gemm_kernel  L21 = A21 L11^{-H} (a product with that inverse) and the
 //                     update of the panel's remaining columns, on the FP64
 //                     tensor cores (DMMA);

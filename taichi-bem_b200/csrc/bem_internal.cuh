@@ -130,7 +130,7 @@ int bem_launch_far64(bem_ctx* ctx, const bem_op_desc* op, const bem_space* test,
                      void* out, int64_t ld, double scale, void* out_t, double scale_t, const void* x, void* y,
                      int conj_x, cudaStream_t s);
 // One operator at nk Helmholtz wavenumbers (bem_kbatch.cu): far pairs in
-// k-batched launches, near pairs per wavenumber.
+// k-batched launches, near pairs two wavenumbers per launch.
 int bem_launch_assemble_batch(bem_ctx* ctx, const bem_op_desc* op, const bem_space* test, const bem_space* trial,
                               int nk, const double* k, const double* k2, void* const* out, int64_t ld,
                               const double* scale, void* const* out_t, const double* scale_t, cudaStream_t s);

@@ -368,8 +368,8 @@ int dispatch_kb(bem_ctx* ctx, const KbArgs& a, int nbx, int nby, bool fp32, int 
 // nk wavenumbers of one operator (validated by bem_assemble_batch): far
 // pairs in groups of 2 or 4 wavenumbers per launch (BEM_TUNE_KBATCH_GROUP;
 // always 2 for P1 x P1 blocks; a short last group is padded with slots that
-// are not written), near pairs per wavenumber on the FP64 Sauter-Schwab
-// kernel.
+// are not written), near pairs on the FP64 Sauter-Schwab kernel, two wavenumbers
+// per launch.
 int bem_launch_assemble_batch(bem_ctx* ctx, const bem_op_desc* op, const bem_space* test, const bem_space* trial,
                               int nk, const double* k, const double* k2, void* const* out, int64_t ld,
                               const double* scale, void* const* out_t, const double* scale_t, cudaStream_t s) {

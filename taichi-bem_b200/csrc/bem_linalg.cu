@@ -1396,7 +1396,8 @@ template <typename T, bool C>
 int lu_solve_t(bem_ctx* ctx, const T* LU, int64_t n, int64_t lda, const int32_t* piv, double* b, int64_t nrhs,
                int64_t ldb, cudaStream_t s) {
     if (nrhs < 1 || nrhs > 8) return bem_fail(ctx, BEM_ERR_INVALID, "lu_solve supports 1..8 right-hand sides");
-    if ((size_t)n * sizeof(int32_t) > 200 * 1024) return bem_fail(ctx, BEM_ERR_INVALID, "lu_solve: n > 51200");
+    // no larger size has been run (a complex FP64 factor of 51200 rows is 42 GB)
+    if (n > 51200) return bem_fail(ctx, BEM_ERR_INVALID, "lu_solve: n > 51200");
     const int W = C ? 2 : 1;
     const SolveLayout lay(W, n, nrhs);
     if (int rc = bem_ws_reserve(ctx, lay.total)) return rc;

@@ -985,7 +985,8 @@ struct SolveWs {
 };
 
 int solve_ws(bem_ctx* ctx, int64_t n, int W, SolveWs* w) {
-    if ((size_t)n * sizeof(int32_t) > 200 * 1024) return bem_fail(ctx, BEM_ERR_INVALID, "tiled solve: n > 51200");
+    // no larger size has been run (a complex FP32 factor of 51200 rows is 21 GB)
+    if (n > 51200) return bem_fail(ctx, BEM_ERR_INVALID, "tiled solve: n > 51200");
     const size_t off = ((size_t)n * 4 + 255) & ~size_t(255);
     const size_t vec = (sizeof(double) * W * (size_t)n + 255) & ~size_t(255);
     if (int rc = bem_ws_reserve(ctx, off + 3 * vec)) return rc;
