@@ -204,13 +204,13 @@ __device__ __forceinline__ void pair_grads(const PairMoments& M, double cw, cons
 // once per trial point.  Bound: FP64 issue, 27 (V) and 50 (K) instructions a
 // point pair for both orders, two thirds of the FP64 pipe at 168 and 252
 // registers (capping K at 168 measured the same).  5120 panels, GaussQR 4
-// (B200): V 8.0 and K 14.3 ms, against 22 and 33 ms per ordered pair with the
+// (B200): V 7.8 and K 14.3 ms, against 22 and 33 ms per ordered pair with the
 // hats of both sides applied at every point.
 //
 // DATA (K): the product K^T lam, the derivative in the nodal data, from the
 // same points.  d.n_i is constant over the test points and sum_q t d.n_j is
 // there already, so it costs nothing per point pair and six multiply-adds a
-// trial point: K 14.3 -> 15.1 ms, in place of a dense FP64 block and its
+// trial point: K 14.3 -> 15.4 ms, in place of a dense FP64 block and its
 // product (7.4 ms at 5120 panels, GaussQR 4).
 template <int OP, bool DATA>
 __global__ void __launch_bounds__(ADJ_THREADS) adj_far_kernel(AdjArgs a) {

@@ -15,7 +15,7 @@
 // further entry of a panel that a list names twice: the maps hold one of them).
 //
 // Bound: FP64 issue.  What a point pair costs is therefore its count of FP64
-// instructions (V Helmholtz: 3 differences, 3 for r^2, 5 for 1/r, r, the
+// instructions (V Helmholtz: 3 differences, 3 for r^2, 6 for r and 1/r, the
 // phase, 13 for sine and cosine, 3 to accumulate), and everything that does
 // not depend on both points is taken out: e^{ikr} = e^{ikR} e^{ik(r - R)} with
 // R the centroid distance leaves a phase of a few panel diameters, which the
@@ -25,8 +25,8 @@
 // Measured (B200, this kernel against the general one per ordered pair with
 // the library's rsqrt and sincos): V Helmholtz, 5120 panels, GaussQR 5: 16.9
 // against 58.4 ms (FP64 pipe 78 % busy, 29 FP64 instructions a point pair);
-// K Laplace product, 2970 panels: 5.1 against 7.9 ms (66 %); V and K of 1280
-// panels: 0.63 and 1.00 against 1.19 and 1.57 ms.
+// K Laplace product, 2970 panels: 5.0 against 7.9 ms; V and K of 1280 panels:
+// 0.63 and 0.97 against 1.19 and 1.57 ms.
 #include <algorithm>
 #include <cmath>
 

@@ -365,9 +365,9 @@ __global__ void __launch_bounds__(256) lu_panel_kernel(T* A, int64_t lda, int n,
 // rows' remaining elements are solved against the sub-block's unit lower
 // triangle and applied as one rank-PCL_SB update, so shared memory is swept once per PCL_SB columns (FP64: on the FP64 tensor
 // cores).  Measured (B200, a column step averaged over a whole factorisation):
-// 2999 complex rows 1.51 us (6.0 us of the cooperative kernel below, a grid
+// 2999 complex rows 1.44 us (6.0 us of the cooperative kernel below, a grid
 // barrier a column; 1.95 with a cluster barrier a column and the panel read
-// through registers), 1280 real rows 1.28 us (5.8; 1.73).  What a step consists
+// through registers), 1280 real rows 1.19 us (5.8; 1.73).  What a step consists
 // of are some twelve dependent shared-memory and warp-reduction latencies of
 // 30 to 200 cycles; a loop over the columns instead of eight copies of the step
 // (registers turned instead of indexed) and half the warps were both slower.
