@@ -169,6 +169,7 @@ int bem_ctx_create(bem_ctx** out_ctx) {
         return BEM_ERR_CUDA;
     }
     cudaDeviceGetAttribute(&ctx->num_sms, cudaDevAttrMultiProcessorCount, ctx->device);
+    cudaDeviceGetAttribute(&ctx->l2_bytes, cudaDevAttrL2CacheSize, ctx->device);
     if (cudaMalloc((void**)&ctx->flags, 16 * sizeof(int32_t)) != cudaSuccess) {
         delete ctx;
         return BEM_ERR_CUDA;

@@ -20,6 +20,7 @@ struct bem_ctx {
     int64_t launches = 0;
     int device = 0;
     int num_sms = 148;
+    int l2_bytes = 0;  // of the L2 cache
     int tune[BEM_TUNE_KEYS] = {0};  // launch-shape choices (bem_ctx_set_tuning); 0 = built-in default
 
     // ---- mesh (device) ----

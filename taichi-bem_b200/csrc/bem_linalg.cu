@@ -23,6 +23,7 @@
 
 #include <complex>
 #include <functional>
+#include <type_traits>
 #include <vector>
 
 #include <cmath>
@@ -975,35 +976,45 @@ __global__ void scatter_rhs_kernel(const double* x, int64_t vs, double* b, int64
     for (int w = 0; w < W; ++w) b[W * ((int64_t)i * ldb + c) + w] = x[c * vs + (int64_t)W * i + w];
 }
 
-// sum_q A[q] x[q] of one row over a warp.  The row comes from memory once and is
-// not wanted again (streaming loads: x keeps its place in the caches), so what
-// counts is bytes in flight: U elements a lane are loaded before the first is
-// used, complex FP64 ones by one 16-byte load where `al` (A and x aligned)
-// allows it.  Measured, complex FP64: 2999 x 2999 41 -> 28 us, 7682 x 7682
-// 220 -> 164 us (5.8 TB/s); U = 8 27 and 172 us, without the streaming hint 36
-// and 187 us.
-template <typename T, bool C>
-__device__ __forceinline__ void row_dot(const T* a, const double* x, int64_t n, bool al, double& sr, double& si) {
-    constexpr int U = C ? 4 : 8;
+// sum_q A[q] x[q] of one row over a warp.  What counts is bytes in flight: U
+// elements a lane are loaded before the first is used, complex ones by one load
+// where `al` (A and x aligned) allows it.  Streaming loads leave the caches to x
+// and other operands; a real matrix that fits the L2 cache is read without the
+// hint (stream false), so that a repeated product finds it there.  Complex rows
+// start at different chunks, since rows a multiple of a few KB apart otherwise keep
+// asking the same memory channels.  Measured, a product repeated / after the cache
+// was flushed, against one element in flight a lane: complex FP64 2999 x 2999 51 ->
+// 33 / 55 -> 33 us, 6000 x 6000 108 -> 109 / 121 -> 114 us (without the rotation
+// 116 / 131), 8000 x 8000 231 -> 171 / 242 -> 178 us; real FP64 3000 x 3000 19 ->
+// 19 / 32 -> 30 us (with the hint 27 / 25), 6000 x 6000 62 -> 57 / 73 -> 58 us;
+// complex FP32 8000 x 8000 125 -> 108 / 130 -> 107 us.
+template <typename T, bool C, bool STREAM>
+__device__ __forceinline__ void row_dot_as(const T* a, const double* x, int64_t n, int64_t row, bool al, double& sr,
+                                           double& si) {
+    constexpr int U = C && sizeof(T) == 4 ? 4 : 8;
+    using V2 = typename std::conditional<sizeof(T) == 8, double2, float2>::type;
     const int lane = threadIdx.x & 31;
     double r[2] = {0.0, 0.0}, m[2] = {0.0, 0.0};
     auto add = [&](int u, El<T, C> e, double xr, double xi) {
         r[u & 1] += (double)e.re * xr - (C ? (double)e.im * xi : 0.0);
         if (C) m[u & 1] += (double)e.re * xi + (double)e.im * xr;
     };
-    int64_t q = lane;
-    for (; q + (U - 1) * 32 < n; q += U * 32) {
+    const int64_t chunks = n / (U * 32);
+    int64_t c = C && chunks ? row % chunks : 0;
+    for (int64_t k = 0; k < chunks; ++k) {
+        const int64_t q = c * (U * 32) + lane;
         El<T, C> e[U];
-        if (C && sizeof(T) == 8 && al) {
 #pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const double2 v = __ldcs(reinterpret_cast<const double2*>(a) + q + 32 * u);
-                e[u].re = (T)v.x;
-                e[u].im = (T)v.y;
+        for (int u = 0; u < U; ++u) {
+            if (!C) {
+                e[u] = El<T, C>{STREAM ? __ldcs(a + q + 32 * u) : a[q + 32 * u], T(0)};
+            } else if (al) {
+                const V2 v = __ldcs(reinterpret_cast<const V2*>(a) + q + 32 * u);
+                e[u].re = v.x;
+                e[u].im = v.y;
+            } else {
+                e[u] = ld<T, C>(a, q + 32 * u);
             }
-        } else {
-#pragma unroll
-            for (int u = 0; u < U; ++u) e[u] = C ? ld<T, C>(a, q + 32 * u) : El<T, C>{__ldcs(a + q + 32 * u), T(0)};
         }
 #pragma unroll
         for (int u = 0; u < U; ++u) {
@@ -1015,14 +1026,24 @@ __device__ __forceinline__ void row_dot(const T* a, const double* x, int64_t n, 
                 add(u, e[u], C ? x[2 * i] : x[i], C ? x[2 * i + 1] : 0.0);
             }
         }
+        if (++c == chunks) c = 0;
     }
-    for (; q < n; q += 32) add(0, ld<T, C>(a, q), C ? x[2 * q] : x[q], C ? x[2 * q + 1] : 0.0);
+    for (int64_t q = chunks * (U * 32) + lane; q < n; q += 32)
+        add(0, ld<T, C>(a, q), C ? x[2 * q] : x[q], C ? x[2 * q + 1] : 0.0);
     sr = r[0] + r[1];
     si = m[0] + m[1];
     for (int o = 16; o > 0; o >>= 1) {
         sr += __shfl_xor_sync(0xffffffffu, sr, o);
         if (C) si += __shfl_xor_sync(0xffffffffu, si, o);
     }
+}
+template <typename T, bool C>
+__device__ __forceinline__ void row_dot(const T* a, const double* x, int64_t n, int64_t row, bool al, bool stream,
+                                        double& sr, double& si) {
+    if (C || stream)
+        row_dot_as<T, C, true>(a, x, n, row, al, sr, si);
+    else
+        row_dot_as<T, C, false>(a, x, n, row, al, sr, si);
 }
 // complex elements of A and x can be read 16 bytes at a time (rows of A too: lda counts elements)
 __device__ __forceinline__ bool aligned16(const void* a, const void* x) {
@@ -1032,12 +1053,12 @@ __device__ __forceinline__ bool aligned16(const void* a, const void* x) {
 // y = alpha A x + beta y, A stored as T (real/complex), x/y FP64
 template <typename T, bool C>
 __global__ void __launch_bounds__(256) gemv_kernel(const T* A, int64_t m, int64_t n, int64_t lda, const double* x,
-                                                    double* y, double alpha, double beta) {
+                                                    double* y, double alpha, double beta, int stream) {
     const int lane = threadIdx.x & 31;
     const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (row >= m) return;
     double sr, si;
-    row_dot<T, C>(A + (C ? 2 : 1) * row * lda, x, n, aligned16(A, x), sr, si);
+    row_dot<T, C>(A + (C ? 2 : 1) * row * lda, x, n, row, aligned16(A, x), stream != 0, sr, si);
     if (lane == 0) {
         if (C) {
             double yr = beta == 0.0 ? 0.0 : beta * y[2 * row];
@@ -1119,13 +1140,14 @@ __global__ void ref_sumsq_kernel(const double* v, int64_t n, RefState* st) {
 // r = b - A x, one warp per row (the FP64 residual of the refinement)
 template <typename T, bool C>
 __global__ void __launch_bounds__(256) ref_residual_kernel(const T* A, int64_t n, int64_t lda, const double* x,
-                                                            const double* b, double* r, const RefState* st) {
+                                                            const double* b, double* r, const RefState* st,
+                                                            int stream) {
     if (st->done) return;
     const int lane = threadIdx.x & 31;
     const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (row >= n) return;
     double sr, si;
-    row_dot<T, C>(A + (C ? 2 : 1) * row * lda, x, n, aligned16(A, x), sr, si);
+    row_dot<T, C>(A + (C ? 2 : 1) * row * lda, x, n, row, aligned16(A, x), stream != 0, sr, si);
     if (lane == 0) {
         if (C) {
             r[2 * row] = b[2 * row] - sr;
@@ -1152,6 +1174,12 @@ __global__ void ref_decide_kernel(RefState* st, double tol2, int maxit) {
     else if (st->it >= maxit)
         st->done = 3;
     st->prev2 = rn2;
+}
+
+// row_dot's stream: m x n elements do not fit the L2 cache
+template <typename T, bool C>
+int beyond_l2(const bem_ctx* ctx, int64_t m, int64_t n) {
+    return (double)m * (double)n * sizeof(T) * (C ? 2 : 1) > (double)ctx->l2_bytes ? 1 : 0;
 }
 
 struct LinWs {
@@ -1460,9 +1488,11 @@ int refine_async(bem_ctx* ctx, bool C, const void* A_hi, const void* LU_lo, cons
             ref_axpy_kernel<<<vblocks, 256, 0, s>>>(x, d, nd, st);
             const unsigned rblocks = (unsigned)((n + 7) / 8);
             if (C)
-                ref_residual_kernel<double, true><<<rblocks, 256, 0, s>>>((const double*)A_hi, n, lda, x, b, r, st);
+                ref_residual_kernel<double, true><<<rblocks, 256, 0, s>>>((const double*)A_hi, n, lda, x, b, r, st,
+                                                                         beyond_l2<double, true>(ctx, n, n));
             else
-                ref_residual_kernel<double, false><<<rblocks, 256, 0, s>>>((const double*)A_hi, n, lda, x, b, r, st);
+                ref_residual_kernel<double, false><<<rblocks, 256, 0, s>>>((const double*)A_hi, n, lda, x, b, r, st,
+                                                                          beyond_l2<double, false>(ctx, n, n));
             ref_sumsq_kernel<<<sblocks, 256, 0, s>>>(r, nd, st);
             ref_decide_kernel<<<1, 1, 0, s>>>(st, tol * tol, maxit);
             ctx->launches += 4;
@@ -1966,7 +1996,7 @@ template <typename T, bool C>
 int gemv_t(bem_ctx* ctx, const T* A, int64_t m, int64_t n, int64_t lda, const double* x, double* y, double alpha,
            double beta, cudaStream_t s) {
     unsigned blocks = (unsigned)((m + 7) / 8);
-    gemv_kernel<T, C><<<blocks, 256, 0, s>>>(A, m, n, lda, x, y, alpha, beta);
+    gemv_kernel<T, C><<<blocks, 256, 0, s>>>(A, m, n, lda, x, y, alpha, beta, beyond_l2<T, C>(ctx, m, n));
     ctx->launches++;
     return bem_check_cuda(ctx, cudaGetLastError(), "gemv_kernel");
 }
