@@ -97,6 +97,10 @@ int bem_solve_inverses(bem_ctx* ctx, int dtype, const void* A, int64_t n, int64_
 // err (zeroed by the caller) receives BEM_ERR_TIMEOUT (bem_tilelu.cu).
 int bem_lu_tri_solve(bem_ctx* ctx, int dtype, const void* LU, int64_t n, int64_t lda, const void* dinv, const double* b,
                      double* y, double* x, int nrhs, int64_t vs, int32_t* err, cudaStream_t s);
+// The same for n <= BEM_SMALL_SOLVE by substitution, without the inverses.
+constexpr int BEM_SMALL_SOLVE = 128;
+int bem_lu_small_solve(bem_ctx* ctx, int dtype, const void* LU, int64_t n, int64_t lda, const double* b, double* x,
+                       int nrhs, int64_t vs, cudaStream_t s);
 // Asynchronous preconditioner step of the refinement (bem_tilelu.cu).
 int bem_tiled_precond_async(bem_ctx* ctx, int dtype, const void* LU, int64_t n, int64_t lda, const int32_t* piv,
                             const void* dinv, const double* r, double** out, const int* skip, cudaStream_t s);

@@ -1442,8 +1442,12 @@ int lu_solve_t(bem_ctx* ctx, const T* LU, int64_t n, int64_t lda, const int32_t*
     const unsigned blocks = (unsigned)((n * nrhs + 255) / 256);
     gather_rhs_kernel<<<blocks, 256, 0, s>>>(b, ldb, perm, vb, vs, (int)n, (int)nrhs, W);
     ctx->launches += 2;
-    if (int rc = bem_solve_inverses(ctx, dtype, LU, n, lda, dinv, s)) return rc;
-    if (int rc = bem_lu_tri_solve(ctx, dtype, LU, n, lda, dinv, vb, vy, vx, (int)nrhs, vs, flag, s)) return rc;
+    if (n <= BEM_SMALL_SOLVE) {
+        if (int rc = bem_lu_small_solve(ctx, dtype, LU, n, lda, vb, vx, (int)nrhs, vs, s)) return rc;
+    } else {
+        if (int rc = bem_solve_inverses(ctx, dtype, LU, n, lda, dinv, s)) return rc;
+        if (int rc = bem_lu_tri_solve(ctx, dtype, LU, n, lda, dinv, vb, vy, vx, (int)nrhs, vs, flag, s)) return rc;
+    }
     scatter_rhs_kernel<<<blocks, 256, 0, s>>>(vx, vs, b, ldb, (int)n, (int)nrhs, W);
     ctx->launches++;
     if (int rc = bem_check_cuda(ctx, cudaGetLastError(), "lu_solve")) return rc;

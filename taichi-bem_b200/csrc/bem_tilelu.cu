@@ -535,6 +535,7 @@ __device__ __forceinline__ void st_vol(double* p, double v) {
 // the block is solved by substitution instead, so the solve has the range of
 // substitution too.
 constexpr int SOLVE_LD = LU_T + 4;  // padded row stride of the staged blocks
+constexpr int SMALL_LD = LU_T + 1;  // of small_solve_kernel's tile
 // elem, inv: bytes of an element of the factor and of the diagonal inverses
 constexpr size_t solve_smem_bytes(size_t elem, size_t inv, bool ref) {
     return ((ref ? 2 : 1) * elem + inv) * LU_T * SOLVE_LD;
@@ -844,6 +845,110 @@ __global__ void __launch_bounds__(256) tri_solve_kernel(const T* LU, int64_t lda
     }
 }
 
+// The same solve for a small matrix (b permuted, x; vs doubles apart): a CTA per
+// right-hand side substitutes, tile by tile, with the vector in shared memory.
+// There the inverses of the diagonal tiles (49 us, one CTA's chain whatever n)
+// and the sweep's hops between CTAs cost more than substitution does, and the
+// sweep takes two right-hand sides at a time.  Measured (a whole bem_lu_solve,
+// complex FP64, one and eight right-hand sides, the sweep in brackets): 16 rows 53
+// and 53 us (82, 147), 80 rows 90 and 89 us (120, 232), 128 rows 115 and 116 us
+// (123, 240); 192 rows 164 and 164 us (131, 271), so the sweep goes on from there.
+template <typename T, bool C>
+__global__ void __launch_bounds__(256) small_solve_kernel(const T* LU, int64_t lda, int n, const double* b, double* x,
+                                                          int64_t vs) {
+    constexpr int W = C ? 2 : 1;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    CE<double>* sx = reinterpret_cast<CE<double>*>(smem_raw);        // [n]
+    CE<T>* sT = reinterpret_cast<CE<T>*>(sx + n);                    // [LU_T][SMALL_LD] diagonal tile
+    __shared__ CE<double> s_rd[LU_T];                                // reciprocals of its pivots
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    b += (int64_t)blockIdx.x * vs;
+    x += (int64_t)blockIdx.x * vs;
+    for (int i = tid; i < n; i += 256) sx[i] = CE<double>{b[W * i], C ? b[W * i + 1] : 0.0};
+    const int nbk = (n + LU_T - 1) / LU_T;
+    for (int pass = 0; pass < 2; ++pass) {
+        const bool fwd = pass == 0;
+        for (int t = 0; t < nbk; ++t) {
+            const int k0 = (fwd ? t : nbk - 1 - t) * LU_T, m = min(LU_T, n - k0);
+            for (int e = tid; e < LU_T * LU_T; e += 256) {
+                const int r = e / LU_T, c = e % LU_T;
+                if (r < m && c < m) sT[r * SMALL_LD + c] = ldE<T, C>(LU, (int64_t)(k0 + r) * lda + k0 + c);
+            }
+            __syncthreads();
+            if (!fwd) {
+                if (tid < m) {
+                    const CE<T> u = sT[tid * SMALL_LD + tid];
+                    s_rd[tid] = cdiv<C>(CE<double>{1.0, 0.0}, CE<double>{(double)u.re, (double)u.im});
+                }
+                __syncthreads();
+            }
+            if (wid == 0) {
+                // rows lane and lane + 32 of the tile
+                CE<double> v0 = lane < m ? sx[k0 + lane] : CE<double>{0.0, 0.0};
+                CE<double> v1 = lane + 32 < m ? sx[k0 + lane + 32] : CE<double>{0.0, 0.0};
+                for (int q = 0; q < m; ++q) {
+                    const int c = fwd ? q : m - 1 - q;
+                    CE<double> p = c < 32 ? v0 : v1;
+                    p.re = __shfl_sync(0xffffffffu, p.re, c & 31);
+                    if (C) p.im = __shfl_sync(0xffffffffu, p.im, c & 31);
+                    if (!fwd) {
+                        const CE<double> rd = s_rd[c];
+                        if (isfinite(rd.re) && isfinite(rd.im)) {
+                            p = CE<double>{p.re * rd.re - (C ? p.im * rd.im : 0.0), C ? p.re * rd.im + p.im * rd.re : 0.0};
+                        } else {
+                            const CE<T> u = sT[c * SMALL_LD + c];
+                            p = cdiv<C>(p, CE<double>{(double)u.re, (double)u.im});
+                        }
+                        if (lane == (c & 31)) (c < 32 ? v0 : v1) = p;
+                    }
+                    if (lane < m && (fwd ? lane > c : lane < c)) {
+                        const CE<T> l = sT[lane * SMALL_LD + c];
+                        v0.re -= (double)l.re * p.re - (C ? (double)l.im * p.im : 0.0);
+                        if (C) v0.im -= (double)l.re * p.im + (double)l.im * p.re;
+                    }
+                    if (lane + 32 < m && (fwd ? lane + 32 > c : lane + 32 < c)) {
+                        const CE<T> l = sT[(lane + 32) * SMALL_LD + c];
+                        v1.re -= (double)l.re * p.re - (C ? (double)l.im * p.im : 0.0);
+                        if (C) v1.im -= (double)l.re * p.im + (double)l.im * p.re;
+                    }
+                }
+                if (lane < m) sx[k0 + lane] = v0;
+                if (lane + 32 < m) sx[k0 + lane + 32] = v1;
+            }
+            __syncthreads();
+            // the tile's columns off the rows still to come, a warp per row
+            const int r0 = fwd ? k0 + m : 0, r1 = fwd ? n : k0;
+            for (int r = r0 + wid; r < r1; r += 8) {
+                const T* row = LU + W * ((int64_t)r * lda + k0);
+                double sr = 0.0, si = 0.0;
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int c = lane + 32 * h;
+                    if (c >= m) continue;
+                    const CE<T> l = ldE<T, C>(row, c);
+                    const CE<double> v = sx[k0 + c];
+                    sr += (double)l.re * v.re - (C ? (double)l.im * v.im : 0.0);
+                    if (C) si += (double)l.re * v.im + (double)l.im * v.re;
+                }
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) {
+                    sr += __shfl_xor_sync(0xffffffffu, sr, o);
+                    if (C) si += __shfl_xor_sync(0xffffffffu, si, o);
+                }
+                if (lane == 0) {
+                    sx[r].re -= sr;
+                    if (C) sx[r].im -= si;
+                }
+            }
+            __syncthreads();
+        }
+    }
+    for (int i = tid; i < n; i += 256) {
+        x[W * i] = sx[i].re;
+        if (C) x[W * i + 1] = sx[i].im;
+    }
+}
+
 __global__ void permute_kernel(const double* b, const int32_t* perm, double* out, int n, int W, const int* skip) {
     if (skip != nullptr && *skip != 0) return;
     int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1139,6 +1244,30 @@ int bem_solve_inverses(bem_ctx* ctx, int dtype, const void* A, int64_t n, int64_
         case BEM_C128: return tile_inverses_t<double, true, double, true>(ctx, (const double*)A, n, lda, d, s);
         case BEM_F32: return tile_inverses_t<float, false, double, true>(ctx, (const float*)A, n, lda, d, s);
         case BEM_C64: return tile_inverses_t<float, true, double, true>(ctx, (const float*)A, n, lda, d, s);
+        default: return bem_fail(ctx, BEM_ERR_INVALID, "lu_solve: unknown dtype");
+    }
+}
+
+template <typename T, bool C>
+int small_solve_t(bem_ctx* ctx, const T* LU, int64_t n, int64_t lda, const double* b, double* x, int nrhs, int64_t vs,
+                  cudaStream_t s) {
+    const size_t smem = sizeof(CE<double>) * (size_t)n + sizeof(CE<T>) * LU_T * SMALL_LD;
+    if (int rc = bem_check_cuda(ctx, cudaFuncSetAttribute(small_solve_kernel<T, C>,
+                                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+                                "small_solve_kernel smem"))
+        return rc;
+    small_solve_kernel<T, C><<<(unsigned)nrhs, 256, smem, s>>>(LU, lda, (int)n, b, x, vs);
+    ctx->launches++;
+    return bem_check_cuda(ctx, cudaGetLastError(), "small_solve_kernel");
+}
+
+int bem_lu_small_solve(bem_ctx* ctx, int dtype, const void* LU, int64_t n, int64_t lda, const double* b, double* x,
+                       int nrhs, int64_t vs, cudaStream_t s) {
+    switch (dtype) {
+        case BEM_F64: return small_solve_t<double, false>(ctx, (const double*)LU, n, lda, b, x, nrhs, vs, s);
+        case BEM_C128: return small_solve_t<double, true>(ctx, (const double*)LU, n, lda, b, x, nrhs, vs, s);
+        case BEM_F32: return small_solve_t<float, false>(ctx, (const float*)LU, n, lda, b, x, nrhs, vs, s);
+        case BEM_C64: return small_solve_t<float, true>(ctx, (const float*)LU, n, lda, b, x, nrhs, vs, s);
         default: return bem_fail(ctx, BEM_ERR_INVALID, "lu_solve: unknown dtype");
     }
 }

@@ -51,3 +51,45 @@ def test_product_beyond_the_l2_cache(engine, dtype):
     y = torch.zeros(n, dtype=dtype, device="cuda")
     engine.gemv(A, x, y)
     assert bool(((y - A @ x).abs() <= 4 * n ** 0.5 * 1.2e-16 * (A.abs() @ x.abs())).all())
+
+
+@pytest.mark.parametrize("dtype", _DTYPES)
+@pytest.mark.parametrize("n,nrhs", [(1, 8), (31, 3), (64, 8), (65, 1), (127, 5), (128, 8), (129, 8)])
+def test_lu_solve_at_the_small_line(engine, n, nrhs, dtype):
+    """Substitution for small matrices and the sweep beyond: the solution of a
+    dominant system, n eps cond = 129 * 1.1e-16 * ~30 < 1e-12, and the same
+    whether the right-hand sides are solved together or alone."""
+    hi = torch.complex128 if dtype.is_complex else torch.float64
+    LU = (_gaussian((n, n), dtype, n) / n ** 0.5 + 3.0 * torch.eye(n, dtype=dtype, device="cuda")).contiguous()
+    piv, _ = engine.lu_factor(LU)
+    F = LU.to(hi)
+    M = (torch.tril(F, -1) + torch.eye(n, dtype=hi, device="cuda")) @ torch.triu(F)
+    b = _gaussian((n, nrhs), hi, 8)
+    x = b.clone()
+    engine.lu_solve(LU, piv, x)
+    pb = b.clone()
+    for i, p in enumerate(piv.tolist()):
+        pb[[i, p]] = pb[[p, i]]
+    ref = torch.linalg.solve(M, pb)
+    assert float((x - ref).abs().max()) < 1e-12 * max(1.0, float(ref.abs().max()))
+    for c in range(nrhs):
+        xc = b[:, c].contiguous()
+        engine.lu_solve(LU, piv, xc)
+        assert float((xc - x[:, c]).abs().max()) <= 1e-14 * float(x.abs().max())
+
+
+@pytest.mark.parametrize("cplx", [False, True])
+def test_small_solve_with_a_zero_pivot_is_not_finite(engine, cplx):
+    """As beyond the line: rows that depend on the zero pivot are infinite or
+    NaN, the others are solved."""
+    n, z = 90, 70
+    dtype = torch.complex128 if cplx else torch.float64
+    A = torch.triu(_gaussian((n, n), dtype, 1)) + 9.0 * torch.eye(n, dtype=dtype, device="cuda")
+    A[z, z] = 0.0
+    b = _gaussian((n, 1), dtype, 2)
+    x = b.clone()
+    engine.lu_solve(A, torch.arange(n, dtype=torch.int32, device="cuda"), x)
+    ref = torch.linalg.solve(A[z + 1:, z + 1:], b[z + 1:])
+    assert float((x[z + 1:] - ref).abs().max()) < 1e-12 * float(ref.abs().max())
+    x = x.cpu().numpy()
+    assert not np.isfinite(x[:z + 1]).any()
