@@ -1111,9 +1111,21 @@ extern "C" int bem_assemble_calderon(bem_ctx* ctx, const bem_op_desc* op, int nk
     if (int rc = bem_check_cuda(ctx, cudaEventRecord(ctx->ev_next, s), "calderon fork")) return rc;
     if (int rc = bem_check_cuda(ctx, cudaStreamWaitEvent(ctx->aux, ctx->ev_next, 0), "calderon fork")) return rc;
     const cudaStream_t sn = ctx->aux;
-    if (int rc = bem_fill_local_map(ctx, neu, ctx->test_local, sn)) return rc;
-    if (int rc = bem_fill_local_map(ctx, neu, ctx->trial_local, sn)) return rc;
-    if (int rc = bem_launch_near_calderon(ctx, op, nk, k, k2, neu, dir, out, coef, ld, sn)) return rc;
+    auto near = [&]() -> int {
+        if (int rc = bem_fill_local_map(ctx, neu, ctx->test_local, sn)) return rc;
+        if (int rc = bem_fill_local_map(ctx, neu, ctx->trial_local, sn)) return rc;
+        return bem_launch_near_calderon(ctx, op, nk, k, k2, neu, dir, out, coef, ld, sn);
+    };
+    // The near pairs' CTAs fill the SMs' registers.  Launched first, they run beside
+    // the first waves of a large sweep; a sweep whose CTAs (half of the grid, the
+    // rest lies below the diagonal) fit the SMs at once would wait for all of them,
+    // so it goes first.  One wavenumber, mixed, Laplace, GaussQR 5, near pairs first
+    // and sweep first: 80 panels 558 and 305 us, 320 panels 716 and 319, 960 panels 813
+    // and 686, 1280 panels 1088 and 1285 us.
+    const int64_t grid_ctas = (int64_t)((neu->n_panels + FAR_THREADS - 1) / FAR_THREADS) * ((neu->n_panels + FAR_TI - 1) / FAR_TI);
+    const bool near_first = grid_ctas >= 8 * (int64_t)ctx->num_sms;
+    if (near_first)
+        if (int rc = near()) return rc;
     CalArgs a{};
     a.n = neu->n_panels;
     a.panels = neu->panels;
@@ -1190,6 +1202,7 @@ extern "C" int bem_assemble_calderon(bem_ctx* ctx, const bem_op_desc* op, int nk
             rc = launch_calderon_one(ctx, b, fp32, helm, s);
         }
     }
+    if (!near_first && !rc) rc = near();
     // join: the caller's stream waits for the near-pair kernels
     if (int e = bem_check_cuda(ctx, cudaEventRecord(ctx->ev_diag, sn), "calderon join")) return e;
     if (int e = bem_check_cuda(ctx, cudaStreamWaitEvent(s, ctx->ev_diag, 0), "calderon join")) return e;
