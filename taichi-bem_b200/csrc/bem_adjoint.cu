@@ -598,10 +598,14 @@ int bem_launch_adjoint(bem_ctx* ctx, const bem_op_desc* op, const bem_space* tes
     a.u = u;
     a.grad = grad;
     a.data = data;
-    // as in bem_launch_far64: fewer test panels per CTA where the call has too few CTAs for some waves
+    // as in bem_launch_far64: fewer test panels per CTA where the call has too few
+    // CTAs for some waves.  With few points a pair the trial vertices' atomics, one
+    // set per CTA, weigh more than idle SMs (K, 320 panels, GaussQR 2: 118, 106, 98
+    // and 117 us with 1, 2, 4 and 8; GaussQR 5: 416, 491, 549 and 656 us)
     a.ti = ADJ_TI;
     const int64_t cols = (a.n_trial + ADJ_THREADS - 1) / ADJ_THREADS;
-    while (a.ti > 1 && cols * ((a.n_test + a.ti - 1) / a.ti) < 16 * (int64_t)ctx->num_sms) a.ti /= 2;
+    const int64_t want = (int64_t)ctx->num_sms * (ctx->Q2 <= 4 ? 1 : (ctx->Q2 <= 9 ? 3 : 16));
+    while (a.ti > 1 && cols * ((a.n_test + a.ti - 1) / a.ti) < want) a.ti /= 2;
     const size_t smem = ((sizeof(double4) + sizeof(double)) * a.ti + sizeof(double2)) * ctx->Q2;
     const dim3 fgrid((unsigned)cols, (unsigned)((a.n_test + a.ti - 1) / a.ti));
     const unsigned nblocks = (unsigned)((a.n_near + 3) / 4);
