@@ -1209,7 +1209,7 @@ __global__ void __launch_bounds__(FAR_THREADS, 5) far_vkg_sym_x2_kernel(FarArgs 
 
 template <int OP, bool HELM, int NBX, int NBY>
 int launch_far(bem_ctx* ctx, FarArgs fa, bool fp32, cudaStream_t s) {
-    fa.ti = fp32 ? bem_far_ti(ctx, fa.n_test, (fa.n_trial + FAR_THREADS - 1) / FAR_THREADS) : FAR_TI;
+    fa.ti = bem_far_ti(ctx, fa.n_test, (fa.n_trial + FAR_THREADS - 1) / FAR_THREADS);
     dim3 grid((fa.n_trial + FAR_THREADS - 1) / FAR_THREADS, (fa.n_test + fa.ti - 1) / fa.ti);
     if (grid.y > 65535) return bem_fail(ctx, BEM_ERR_INVALID, "too many test panels for one launch");
     if (fa.n_test <= 0 || fa.n_trial <= 0) return BEM_OK;
@@ -1221,7 +1221,10 @@ int launch_far(bem_ctx* ctx, FarArgs fa, bool fp32, cudaStream_t s) {
             far_kernel<OP, HELM, NBX, NBY, float, false><<<grid, FAR_THREADS, smem, s>>>(fa);
     } else {
         const size_t smem = fa.ti * fa.Q2 * sizeof(double4) + fa.Q2 * 3 * sizeof(double);
-        far_kernel<OP, HELM, NBX, NBY, double, true><<<grid, FAR_THREADS, smem, s>>>(fa);
+        if (fa.ti == FAR_TI)
+            far_kernel<OP, HELM, NBX, NBY, double, true><<<grid, FAR_THREADS, smem, s>>>(fa);
+        else
+            far_kernel<OP, HELM, NBX, NBY, double, false><<<grid, FAR_THREADS, smem, s>>>(fa);
     }
     ctx->launches++;
     return bem_check_cuda(ctx, cudaGetLastError(), "far_kernel launch");
