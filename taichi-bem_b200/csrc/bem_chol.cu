@@ -187,11 +187,11 @@ __global__ void __launch_bounds__(256) chol64_kernel(double* A, int64_t lda, int
 // ends at its diagonal.
 //
 // BM x 64 entries per CTA (BM = 64 or 32), eight warps of BM / 2 x 16 (4 or 2 x
-// 2 fragments of 8 x 8; complex: four real products per complex one), K in stages of 8 that cp.async
-// brings straight into shared memory, DG_STAGES deep, one CTA barrier a stage.
+// 2 fragments of 8 x 8; complex: four real products per complex one), K in stages of DG_BK that cp.async
+// brings straight into shared memory, four (DG_BK = 8) or three (16) deep, one CTA barrier a stage.
 // The factorisations call this with K = 64 and 256, so a CTA lives for 8 to 32
 // stages: depth, two CTAs per SM and C on its way into L2 are what keep the
-// tensor pipe fed.  Shared rows are k, entries interleaved; the row strides put the
+// tensor pipe fed.  Long products have half the barriers with DG_BK = 16.  Shared rows are k, entries interleaved; the row strides put the
 // fragments' 8-lane (16-byte) or 16-lane (8-byte) phases on distinct banks.
 // The fragment layouts of m8n8k4: A[row = lane / 4][k = lane % 4], B[k = lane %
 // 4][col = lane / 4], C[row = lane / 4][col = 2 (lane % 4) + {0, 1}].
@@ -199,14 +199,18 @@ __global__ void __launch_bounds__(256) chol64_kernel(double* A, int64_t lda, int
 // stage): the trailing updates of a 2999 complex LU (K = 64) 3.3 against 4.0 ms
 // (22 against 18 TFLOP/s), those inside the panels of a 7682 complex Cholesky
 // (K = 64 and 256) 6.0 against 6.9 ms (5.7 with 32-row tiles where few).
-constexpr int DG_BM = 64, DG_BK = 8, DG_STAGES = 4;
+// Long products, against that form: A B of 1500 complex 930 and 932 us (958 in
+// stages of 8), A^H B 874 and 1006, A B^H 1015 and 985 us; A^H B of 2500 real 1122 and
+// 1149 us (1248 in stages of 8).
+constexpr int DG_BM = 64;
 constexpr int DG_OVERWRITE = 4;  // flag beside the triangular ones; C may then be A where n <= 64 (a CTA reads only its rows)
-template <bool CPLX>
+template <bool CPLX, int BK>
 struct DgTile {
     static constexpr int W = CPLX ? 2 : 1;
+    static constexpr int STAGES = BK == 8 ? 4 : 3;
     static constexpr int LD = CPLX ? DG_BM + 2 : DG_BM + 4;  // entries per k row
-    static constexpr int OPERAND = DG_BK * LD * W;           // doubles per operand and stage
-    static constexpr size_t SMEM = sizeof(double) * 2 * OPERAND * DG_STAGES;
+    static constexpr int OPERAND = BK * LD * W;              // doubles per operand and stage
+    static constexpr size_t SMEM = sizeof(double) * 2 * OPERAND * STAGES;
 };
 
 __device__ __forceinline__ void dmma(double& d0, double& d1, double a, double b) {
@@ -229,13 +233,14 @@ __device__ __forceinline__ void cp_entry(double* dst, const double* src, bool ok
     if (CPLX) asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d + 8), "l"(src + 1), "r"(bytes) : "memory");
 }
 
-template <bool CPLX, bool CONJA, bool CONJT, bool LOWER, int BM>
+template <bool CPLX, bool CONJA, bool CONJT, bool LOWER, int BM, int DG_BK>
 __global__ void __launch_bounds__(256, 2) dmma_gemm_kernel(double* Cm, int64_t ldc,
                                                             const double* Am, int64_t lda,
                                                             const double* __restrict__ Bm, int64_t ldb, int64_t m,
                                                             int64_t n, int k, double alpha, int64_t diag, int kchunk,
                                                             int tri, int al) {
-    using Tile = DgTile<CPLX>;
+    using Tile = DgTile<CPLX, DG_BK>;
+    constexpr int DG_STAGES = Tile::STAGES;
     constexpr int W = Tile::W, LD = Tile::LD, NP = CPLX ? 2 : 1;
     constexpr int FA = BM / 16;  // fragments of a warp along the rows
     extern __shared__ __align__(16) double dg_smem[];
@@ -255,37 +260,46 @@ __global__ void __launch_bounds__(256, 2) dmma_gemm_kernel(double* Cm, int64_t l
     int kend = min(k, kbeg + kchunk);
     if (tri & 1) kend = (int)min((int64_t)kend, m0 + BM);
     if (tri & 2) kend = (int)min((int64_t)kend, n0 + DG_BM);
-    // an operand's 64 (A: BM) entries x 8 k of a stage, two (one) per thread, along its rows in memory:
-    // stored with k contiguous (A, B^H): k = tid % 8, entry tid / 8 + 32 h; otherwise entry tid % 64, k = tid / 64 + 4 h
-    auto stage = [&](int slot, int k0) {
+    // an operand's 64 (A: BM) entries x 8 k, two (one) copies per thread, along its rows in memory:
+    // stored with k contiguous (A, B^H): eight k of an entry side by side (real: 4 k of 4 entries in 16 lanes,
+    // which the row stride puts on distinct banks), and the entry 32 further; otherwise 64 entries of a k, and k + 4
+    const int kc = CPLX ? tid & 7 : (tid & 3) | ((tid >> 2) & 4), ec = CPLX ? tid >> 3 : ((tid >> 2) & 3) | ((tid >> 5) << 2);
+    const int ks = tid >> 6, es = tid & 63;  // entries contiguous
+    const int ka = !CONJA ? kc : (BM == 64 ? ks : tid >> 5), ea = !CONJA ? ec : (BM == 64 ? es : tid & 31);
+    const int kb = CONJT ? kc : ks, eb = CONJT ? ec : es;
+    // this thread's first entry of the next stage, and the steps to the other ones and along K
+    const double* pa = Am + W * (CONJA ? (int64_t)(kbeg + ka) * lda + m0 + ea : (m0 + ea) * lda + kbeg + ka);
+    const double* pb = Bm + W * (CONJT ? (n0 + eb) * ldb + kbeg + kb : (int64_t)(kbeg + kb) * ldb + n0 + eb);
+    const int64_t ha = W * (CONJA ? 4 : 32) * lda, hb = W * (CONJT ? 32 : 4) * ldb;
+    const int64_t ga = CONJA ? 8 * W * lda : 8 * W, gb = CONJT ? 8 * W : 8 * W * ldb;
+    int kleft = kend - kbeg;
+    auto stage = [&](int slot) {
         double* sA = dg_smem + (size_t)slot * 2 * Tile::OPERAND;
         double* sB = sA + Tile::OPERAND;
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int kc = tid & 7, ec = (tid >> 3) + 32 * h;  // k contiguous
-            const int ks = (tid >> 6) + 4 * h, es = tid & 63;  // entries contiguous
-            if (32 * h < BM) {
-                const int kk = !CONJA ? kc : (BM == 64 ? ks : tid >> 5), e = !CONJA ? ec : (BM == 64 ? es : tid & 31);
-                const int64_t gr = m0 + e;
-                const int gk = k0 + kk;
-                const bool ok = gr < m && gk < kend;
-                const double* src = Am + W * (CONJA ? (int64_t)gk * lda + gr : gr * lda + gk);
-                cp_entry<CPLX>(sA + W * (kk * LD + e), ok ? src : Am, ok, al != 0);
+        for (int g = 0; g < DG_BK; g += 8) {
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                if (32 * h < BM) {
+                    const int kk = ka + g + (CONJA ? 4 * h : 0), e = ea + (CONJA ? 0 : 32 * h);
+                    const bool ok = m0 + e < m && kk < kleft;
+                    cp_entry<CPLX>(sA + W * (kk * LD + e), ok ? pa + h * ha : Am, ok, al != 0);
+                }
+                {
+                    const int kk = kb + g + (CONJT ? 0 : 4 * h), e = eb + (CONJT ? 32 * h : 0);
+                    const bool ok = n0 + e < n && kk < kleft;
+                    cp_entry<CPLX>(sB + W * (kk * LD + e), ok ? pb + h * hb : Bm, ok, al != 0);
+                }
             }
-            {
-                const int kk = CONJT ? kc : ks, e = CONJT ? ec : es;
-                const int64_t gc = n0 + e;
-                const int gk = k0 + kk;
-                const bool ok = gc < n && gk < kend;
-                const double* src = Bm + W * (CONJT ? gc * ldb + gk : (int64_t)gk * ldb + gc);
-                cp_entry<CPLX>(sB + W * (kk * LD + e), ok ? src : Bm, ok, al != 0);
-            }
+            pa += ga;
+            pb += gb;
         }
+        kleft -= DG_BK;
     };
     const int nk = kend > kbeg ? (kend - kbeg + DG_BK - 1) / DG_BK : 0;
 #pragma unroll
     for (int s = 0; s < DG_STAGES - 1; ++s) {
-        if (s < nk) stage(s, kbeg + s * DG_BK);
+        if (s < nk) stage(s);
         asm volatile("cp.async.commit_group;" ::: "memory");
     }
 #pragma unroll
@@ -303,7 +317,7 @@ __global__ void __launch_bounds__(256, 2) dmma_gemm_kernel(double* Cm, int64_t l
     for (int kt = 0; kt < nk; ++kt) {
         asm volatile("cp.async.wait_group %0;" ::"n"(DG_STAGES - 2) : "memory");
         __syncthreads();  // stage kt is in; the slot of stage kt - 1 is free
-        if (kt + DG_STAGES - 1 < nk) stage((kt + DG_STAGES - 1) % DG_STAGES, kbeg + (kt + DG_STAGES - 1) * DG_BK);
+        if (kt + DG_STAGES - 1 < nk) stage((kt + DG_STAGES - 1) % DG_STAGES);
         asm volatile("cp.async.commit_group;" ::: "memory");
         const double* sA = dg_smem + (size_t)(kt % DG_STAGES) * 2 * Tile::OPERAND;
         const double* sB = sA + Tile::OPERAND;
@@ -421,21 +435,21 @@ __global__ void iota_kernel(int32_t* piv, int n) {
 }
 
 // One launch of dmma_gemm_kernel with tiles of BM x 64; `splits` ranges of K.
-template <bool C, bool CONJA, bool CONJT, bool LOWER, int BM>
+template <bool C, bool CONJA, bool CONJT, bool LOWER, int BM, int DG_BK>
 int gemm64_launch(bem_ctx* ctx, double* Cm, int64_t ldc, const double* A, int64_t lda, const double* B, int64_t ldb,
                   int64_t m, int64_t n, int k, double alpha, int64_t diag, int tri, int splits, cudaStream_t s) {
     dim3 grid((unsigned)((n + DG_BM - 1) / DG_BM), (unsigned)((m + BM - 1) / BM));
     const int kchunk = (int)(((int64_t)k + splits - 1) / splits + DG_BK - 1) / DG_BK * DG_BK;
     grid.z = (unsigned)(((int64_t)k + kchunk - 1) / kchunk);
-    constexpr size_t smem = DgTile<C>::SMEM;
-    if (int rc = bem_check_cuda(ctx, cudaFuncSetAttribute(dmma_gemm_kernel<C, CONJA, CONJT, LOWER, BM>,
+    constexpr size_t smem = DgTile<C, DG_BK>::SMEM;
+    if (int rc = bem_check_cuda(ctx, cudaFuncSetAttribute(dmma_gemm_kernel<C, CONJA, CONJT, LOWER, BM, DG_BK>,
                                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
                                 "dmma_gemm_kernel smem"))
         return rc;
     // 16-byte copies of complex entries need 16-byte aligned operands
     const int al = ((uintptr_t)A | (uintptr_t)B) % 16 == 0 ? 1 : 0;
-    dmma_gemm_kernel<C, CONJA, CONJT, LOWER, BM><<<grid, 256, smem, s>>>(Cm, ldc, A, lda, B, ldb, m, n, k, alpha, diag,
-                                                                         kchunk, tri, al);
+    dmma_gemm_kernel<C, CONJA, CONJT, LOWER, BM, DG_BK>
+        <<<grid, 256, smem, s>>>(Cm, ldc, A, lda, B, ldb, m, n, k, alpha, diag, kchunk, tri, al);
     ctx->launches++;
     return bem_check_cuda(ctx, cudaGetLastError(), "dmma_gemm_kernel");
 }
@@ -455,8 +469,13 @@ int gemm64x(bem_ctx* ctx, double* Cm, int64_t ldc, const double* A, int64_t lda,
     if (!LOWER && !(tri & DG_OVERWRITE) && tiles < 2 * (int64_t)ctx->num_sms)
         splits = (int)std::max<int64_t>(1, std::min<int64_t>((2 * ctx->num_sms) / tiles, k / 512));
     if (tiles <= ctx->num_sms && splits == 1)
-        return gemm64_launch<C, CONJA, CONJT, LOWER, 32>(ctx, Cm, ldc, A, lda, B, ldb, m, n, k, alpha, diag, tri, 1, s);
-    return gemm64_launch<C, CONJA, CONJT, LOWER, 64>(ctx, Cm, ldc, A, lda, B, ldb, m, n, k, alpha, diag, tri, splits, s);
+        return gemm64_launch<C, CONJA, CONJT, LOWER, 32, 8>(ctx, Cm, ldc, A, lda, B, ldb, m, n, k, alpha, diag, tri, 1, s);
+    // stages of 16 where the ranges of K are long and B comes in rows (with B^H, 8 is the faster)
+    if constexpr (!CONJT && !LOWER)
+        if (k / splits >= 512)
+            return gemm64_launch<C, CONJA, CONJT, LOWER, 64, 16>(ctx, Cm, ldc, A, lda, B, ldb, m, n, k, alpha, diag, tri,
+                                                                 splits, s);
+    return gemm64_launch<C, CONJA, CONJT, LOWER, 64, 8>(ctx, Cm, ldc, A, lda, B, ldb, m, n, k, alpha, diag, tri, splits, s);
 }
 
 template <bool C, bool CONJT, bool LOWER>

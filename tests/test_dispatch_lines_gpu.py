@@ -53,6 +53,22 @@ def test_product_beyond_the_l2_cache(engine, dtype):
     assert bool(((y - A @ x).abs() <= 4 * n ** 0.5 * 1.2e-16 * (A.abs() @ x.abs())).all())
 
 
+@pytest.mark.parametrize("dtype", [torch.float64, torch.complex128])
+@pytest.mark.parametrize("conj_a,conj_b", [(False, False), (False, True), (True, False), (True, True)])
+@pytest.mark.parametrize("m,n,k", [(1290, 1283, 511), (1290, 1283, 512), (1283, 1290, 529), (33, 70, 2087)])
+def test_gemm_long_products(engine, m, n, k, conj_a, conj_b, dtype):
+    """K below, at and beyond the line of the longer stages, with remainders of
+    a stage and a tile, whole and split K; k eps of the magnitudes."""
+    A = _gaussian((k, m + 3) if conj_a else (m, k + 3), dtype, 5)[:, :m if conj_a else k]
+    B = _gaussian((n, k + 1) if conj_b else (k, n + 1), dtype, 6)[:, :k if conj_b else n]
+    C0 = _gaussian((m, n), dtype, 7)
+    C = C0.clone()
+    engine.gemm(A, B, C, alpha=0.3, conj_a=conj_a, conj_b=conj_b)
+    a, b = A.mH if conj_a else A, B.mH if conj_b else B
+    mag = 0.3 * (a.abs() @ b.abs()) + C0.abs()
+    assert bool(((C - (C0 + 0.3 * (a @ b))).abs() <= 4 * (k ** 0.5 + 2) * 1.2e-16 * mag).all())
+
+
 @pytest.mark.parametrize("dtype", _DTYPES)
 @pytest.mark.parametrize("n,nrhs", [(1, 8), (31, 3), (64, 8), (65, 1), (127, 5), (128, 8), (129, 8)])
 def test_lu_solve_at_the_small_line(engine, n, nrhs, dtype):
