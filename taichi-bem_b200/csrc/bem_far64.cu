@@ -442,6 +442,11 @@ int bem_launch_far64(bem_ctx* ctx, const bem_op_desc* op, const bem_space* test,
                      void* out, int64_t ld, double scale, void* out_t, double scale_t, const void* x, void* y,
                      int conj_x, cudaStream_t s) {
     if (op->precision != BEM_PREC_FP64 || op->deriv_k) return 1;
+    // one point a panel (GaussQR 1): what is left is the writing of both orders, which
+    // costs more than the second evaluation.  One order against both, k = 2: K block of
+    // 1280 panels 81 against 103 us, V block of 5120 panels 578 against 685 us, K'
+    // product of 320 panels 42 against 89 us.
+    if (ctx->Q2 == 1) return 1;
     const int nx = test->nb, ny = trial->nb;
     const bool v1 = op->op == BEM_OP_V && nx == 1 && ny == 1, v3 = op->op == BEM_OP_V && nx == 3 && ny == 3;
     const bool w3 = op->op == BEM_OP_W && nx == 3 && ny == 3;

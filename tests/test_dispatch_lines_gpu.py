@@ -109,3 +109,48 @@ def test_small_solve_with_a_zero_pivot_is_not_finite(engine, cplx):
     assert float((x[z + 1:] - ref).abs().max()) < 1e-12 * float(ref.abs().max())
     x = x.cpu().numpy()
     assert not np.isfinite(x[:z + 1]).any()
+
+
+def _sphere(engine, sub, Q):
+    from bem_b200 import icosphere
+    from bem_b200.engine import DeviceSpace
+    v, f = icosphere(sub)
+    engine.set_mesh(v, f, Q)
+    p = np.arange(len(f), dtype=np.int32)
+    return v, f, DeviceSpace.from_numpy(p, 1, p, engine.device), DeviceSpace.from_numpy(p, 3, f.reshape(-1).copy(), engine.device)
+
+
+@pytest.mark.parametrize("cplx", [False, True])
+def test_one_point_rule(engine, cplx):
+    """GaussQR 1 in FP64: on panels that share no vertex V, K and K' (its second
+    block) are the kernels at the rule's points, 1e-13 of the largest entry
+    for a dozen roundings and the sine; products against the blocks."""
+    from bem_b200 import _lib as L
+    v, f, p0, _ = _sphere(engine, 2, 1)
+    nt, k = len(f), 2.0 if cplx else 0.0
+    dtype = torch.complex128 if cplx else torch.float64
+    new = lambda: torch.zeros(nt, nt, dtype=dtype, device="cuda")
+    V, K, Kt, KP = new(), new(), new(), new()
+    desc = lambda op: engine.op_desc(getattr(L, "OP_" + op), cplx, k, k * k)
+    engine.assemble(desc("V"), p0, p0, V)
+    engine.assemble(desc("K"), p0, p0, K, 1.0, Kt, -0.5)
+    engine.assemble(desc("KP"), p0, p0, KP)
+    t = v[f]
+    cross = np.cross(t[:, 1] - t[:, 0], t[:, 2] - t[:, 0])
+    area2 = np.linalg.norm(cross, axis=1)  # twice the area
+    nrm = cross / area2[:, None]
+    # the one-point Duffy rule: y = v0 + (v1 - v0) / 2 + (v2 - v1) / 4, weight 1/2
+    y = t[:, 0] + 0.5 * (t[:, 1] - t[:, 0]) + 0.25 * (t[:, 2] - t[:, 1])
+    d = y[:, None] - y[None]  # x - y
+    far = ~np.array([[len(set(a) & set(b)) > 0 for b in f] for a in f])
+    r = np.sqrt((d * d).sum(-1)) + ~far
+    G = area2[:, None] * area2[None] * 0.25 * (np.exp(1j * k * r) if cplx else 1.0) / (4 * np.pi * r)
+    dn = (G * (1 - 1j * k * r if cplx else 1.0) / r ** 2)
+    Kref, KPref = dn * np.einsum("ijc,jc->ij", d, nrm), -dn * np.einsum("ijc,ic->ij", d, nrm)
+    for got, ref in ((V, G), (K, Kref), (Kt, -0.5 * Kref.T), (KP, KPref)):
+        assert np.abs((got.cpu().numpy() - ref)[far]).max() < 1e-13 * np.abs(ref[far]).max()
+    x = _gaussian((nt,), dtype, 9)
+    for op, A in (("V", V), ("K", K), ("KP", KP)):
+        z = torch.zeros(nt, dtype=dtype, device="cuda")
+        engine.apply(desc(op), p0, p0, x, z)
+        assert float((z - A @ x).abs().max()) < 1e-13 * float((A.abs() @ x.abs()).max())
