@@ -289,7 +289,7 @@ __global__ void __launch_bounds__(FAR_THREADS) far64_kernel(Far64Args a) {
             double fr = BEM_INV4PI, fi = 0.0;
             if (HELM) {
                 double sR, cR;
-                dev_sincos(phR, &sR, &cR);
+                dev_sincos_frame(phR, &sR, &cR);
                 fi = fr * sR;
                 fr = fr * cR;
             }

@@ -179,14 +179,21 @@ __device__ __forceinline__ void dev_sincos_poly64(double y, double* s, double* c
     pc = fma(y2, pc, -0.5);
     *c = fma(y2, pc, 1.0);
 }
+// Any FP64 phase: CUDA's.  The reduction of dev_sincos_frame in its place, at every
+// point of a pair, costs the sweeps registers: FP64 at 5120 panels, GaussQR 3, the
+// Dirichlet sweep 6.14 -> 6.68 ms, the batched K 15.2 -> 16.3 ms, V 8.07 -> 8.30 ms.
+__device__ __forceinline__ void dev_sincos(double x, double* s, double* c) { sincos(x, s, c); }
 __device__ __noinline__ void dev_sincos_any(double x, double* s, double* c) { sincos(x, s, c); }
-// Any FP64 phase.  Up to 1e5 (a wavenumber of 1e5 on a unit mesh): reduction
+// e^{ikR} of a pair frame, once per pair.  Up to 1e5 (a wavenumber of 1e5 on a unit mesh): reduction
 // by n pi/2 with pi/2 split in two doubles (Cody and Waite, Software Manual for
 // the Elementary Functions, 1980), the first product exact in its FMA; then the
 // polynomials above and the quadrant.  The reduced argument carries two
 // roundings of at most 2^-54, the results at most 2.3e-16.  Beyond, and for
-// infinities and NaN, CUDA's sincos, kept out of line.
-__device__ __forceinline__ void dev_sincos(double x, double* s, double* c) {
+// infinities and NaN, CUDA's sincos, kept out of line: its registers beside the
+// pair kernels' moments cost them more than its arithmetic.  5120 panels, phases of
+// the pairs <= 0.3, against CUDA's sincos in its place: V 2.93 -> 2.84, W 4.58 ->
+// 4.51 ms at GaussQR 3; V 1.18 -> 1.09 ms at 2.
+__device__ __forceinline__ void dev_sincos_frame(double x, double* s, double* c) {
     if (!(fabs(x) <= 1e5)) {
         double a, b;
         dev_sincos_any(x, &a, &b);

@@ -82,7 +82,7 @@ __global__ void math_kernel(int which, const double* x, double* a, double* b, in
     double u, v;
     switch (which) {
         case 0: dev_r_rinv(x[i], u, v); break;
-        case 1: dev_sincos(x[i], &u, &v); break;
+        case 1: dev_sincos_frame(x[i], &u, &v); break;
         case 2: dev_sincos_poly64<false>(x[i], &u, &v); break;
         default: dev_sincos_poly64<true>(x[i], &u, &v);
     }
