@@ -740,13 +740,14 @@ __global__ void __launch_bounds__(FAR_THREADS) far_vkg_kernel(FarArgs a, VkgArgs
 // above the diagonal are launched; rows i are reduced across the warp, rows j
 // accumulate per thread over the CTA's test panels.
 // ----------------------------------------------------------------------------
-template <bool HELM, typename T>
+template <bool HELM, typename T, bool FULL>
 __global__ void __launch_bounds__(FAR_THREADS) far_vkg_sym_kernel(FarArgs a, VkgArgs v) {
     using V4 = typename V4T<T>::type;
+    const int ti = FULL ? FAR_TI : a.ti;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    V4* sx = reinterpret_cast<V4*>(smem_raw);                        // [FAR_TI][Q2] test points
-    T* sgx = reinterpret_cast<T*>(sx + FAR_TI * a.Q2);                // [FAR_TI][Q2][2] g at test points
-    T* sphi = sgx + FAR_TI * a.Q2 * 2;                                // [Q2*3]
+    V4* sx = reinterpret_cast<V4*>(smem_raw);       // [ti][Q2] test points
+    T* sgx = reinterpret_cast<T*>(sx + ti * a.Q2);  // [ti][Q2][2] g at test points
+    T* sphi = sgx + ti * a.Q2 * 2;                  // [Q2*3]
     __shared__ int s_gi[FAR_TI];
     __shared__ int s_tri[FAR_TI][3];
     __shared__ double s_cen[FAR_TI][3];
@@ -754,10 +755,10 @@ __global__ void __launch_bounds__(FAR_THREADS) far_vkg_sym_kernel(FarArgs a, Vkg
 
     const int Q2 = a.Q2;
     const int n = a.n_test;  // == n_trial
-    // tile (bx = trial tile of FAR_THREADS panels, by = test tile of FAR_TI panels);
+    // tile (bx = trial tile of FAR_THREADS panels, by = test tile of ti panels);
     // skip tiles strictly below the diagonal
     const int j0 = blockIdx.x * FAR_THREADS;
-    const int li0 = blockIdx.y * FAR_TI;
+    const int li0 = blockIdx.y * ti;
     if (j0 + FAR_THREADS - 1 <= li0) return;
     const int lj = j0 + threadIdx.x;
     const V4* pts = reinterpret_cast<const V4*>(a.pts);
@@ -765,7 +766,7 @@ __global__ void __launch_bounds__(FAR_THREADS) far_vkg_sym_kernel(FarArgs a, Vkg
         const T* phi = reinterpret_cast<const T*>(a.phi);
         for (int idx = threadIdx.x; idx < Q2 * 3; idx += FAR_THREADS) sphi[idx] = phi[idx];
     }
-    if (threadIdx.x < FAR_TI) {
+    if (threadIdx.x < ti) {
         int li = li0 + threadIdx.x;
         int gi = li < n ? a.test_panels[li] : -1;
         s_gi[threadIdx.x] = gi;
@@ -776,7 +777,7 @@ __global__ void __launch_bounds__(FAR_THREADS) far_vkg_sym_kernel(FarArgs a, Vkg
         }
     }
     __syncthreads();
-    for (int idx = threadIdx.x; idx < FAR_TI * Q2; idx += FAR_THREADS) {
+    for (int idx = threadIdx.x; idx < ti * Q2; idx += FAR_THREADS) {
         int t = idx / Q2, q = idx - t * Q2;
         int li = li0 + t;
         T gre = T(0), gim = T(0);
@@ -809,7 +810,7 @@ __global__ void __launch_bounds__(FAR_THREADS) far_vkg_sym_kernel(FarArgs a, Vkg
     const int lane = threadIdx.x & 31;
     double rj_re = 0.0, rj_im = 0.0;  // this thread's contribution to row j
 
-    for (int t = 0; t < FAR_TI; ++t) {
+    for (int t = 0; t < ti; ++t) {
         const int li = li0 + t;
         if (li >= n) break;
         const int gi = s_gi[t];
@@ -1375,10 +1376,10 @@ int bem_launch_dirichlet(bem_ctx* ctx, const bem_op_desc* op, const bem_space* t
     const bool sym = test->n_panels == trial->n_panels && test->panels == trial->panels &&
                      test->dof == trial->dof && rows->n_panels == test->n_panels;
     if (fa.n_test > 0 && fa.n_trial > 0 && sym) {
+        fa.ti = bem_far_ti(ctx, fa.n_test, (int)grid.x);
+        grid.y = (fa.n_test + fa.ti - 1) / fa.ti;
         if (fp32) {
             const int P2 = (fa.Q2 + 1) / 2;
-            fa.ti = bem_far_ti(ctx, fa.n_test, (int)grid.x);
-            grid.y = (fa.n_test + fa.ti - 1) / fa.ti;
             size_t smem = 3 * fa.ti * P2 * sizeof(float4) + fa.ti * P2 * sizeof(float2) +
                           P2 * FAR_THREADS * sizeof(float2) + fa.Q2 * 3 * sizeof(float);
             auto go = [&](auto full) {
@@ -1397,11 +1398,18 @@ int bem_launch_dirichlet(bem_ctx* ctx, const bem_op_desc* op, const bem_space* t
             else
                 go(std::false_type{});
         } else {
-            size_t smem = FAR_TI * fa.Q2 * (sizeof(double4) + 2 * sizeof(double)) + fa.Q2 * 3 * sizeof(double);
-            if (helm)
-                far_vkg_sym_kernel<true, double><<<grid, FAR_THREADS, smem, s>>>(fa, va);
+            size_t smem = fa.ti * fa.Q2 * (sizeof(double4) + 2 * sizeof(double)) + fa.Q2 * 3 * sizeof(double);
+            auto go = [&](auto full) {
+                constexpr bool FULL = decltype(full)::value;
+                if (helm)
+                    far_vkg_sym_kernel<true, double, FULL><<<grid, FAR_THREADS, smem, s>>>(fa, va);
+                else
+                    far_vkg_sym_kernel<false, double, FULL><<<grid, FAR_THREADS, smem, s>>>(fa, va);
+            };
+            if (fa.ti == FAR_TI)
+                go(std::true_type{});
             else
-                far_vkg_sym_kernel<false, double><<<grid, FAR_THREADS, smem, s>>>(fa, va);
+                go(std::false_type{});
         }
         ctx->launches++;
         if (int rc = bem_check_cuda(ctx, cudaGetLastError(), "far_vkg_sym_kernel launch")) return rc;

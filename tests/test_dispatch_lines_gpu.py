@@ -154,3 +154,22 @@ def test_one_point_rule(engine, cplx):
         z = torch.zeros(nt, dtype=dtype, device="cuda")
         engine.apply(desc(op), p0, p0, x, z)
         assert float((z - A @ x).abs().max()) < 1e-13 * float((A.abs() @ x.abs()).max())
+
+
+@pytest.mark.parametrize("cplx", [False, True])
+@pytest.mark.parametrize("sub,Q", [(0, 3), (2, 3), (3, 2), (4, 1)])
+def test_fp64_dirichlet_pass_over_test_panel_counts(engine, sub, Q, cplx):
+    """One test panel per CTA, four and eight: the block and the right-hand side
+    of the one pass against those of the two calls, both FP64."""
+    from bem_b200 import _lib as L
+    v, f, p0, p1 = _sphere(engine, sub, Q)
+    nt, k = len(f), 2.0 if cplx else 0.0
+    dtype = torch.complex128 if cplx else torch.float64
+    g = _gaussian((len(v),), dtype, 10)
+    A, B = (torch.zeros(nt, nt, dtype=dtype, device="cuda") for _ in range(2))
+    a, b = (torch.zeros(nt, dtype=dtype, device="cuda") for _ in range(2))
+    engine.assemble_dirichlet(engine.op_desc(L.OP_V, cplx, k, k * k), p0, p0, A, p0, p1, g, a)
+    engine.assemble(engine.op_desc(L.OP_V, cplx, k, k * k), p0, p0, B)
+    engine.apply(engine.op_desc(L.OP_K, cplx, k, k * k), p0, p1, g, b)
+    assert float((A - B).abs().max()) < 1e-13 * float(B.abs().max())
+    assert float((a - b).abs().max()) < 1e-12 * float(b.abs().max())
