@@ -240,9 +240,10 @@ constexpr int FAR_TI = 8;
 // Test panels per CTA of a far sweep: fewer than FAR_TI where the call has too
 // few CTAs for some waves of the three to five that fit an SM.
 // Mixed precision, GaussQR 5, k = 2: K block of 110 panels 0.82 -> 0.17 ms, of
-// 550 panels 0.98 -> 0.65 ms; W product 0.47 -> 0.14 and 0.86 -> 0.69 ms.  The full
-// count is a constant of the kernels where the call has enough CTAs (as a
-// variable it cost them 1 to 2 %).
+// 550 panels 0.98 -> 0.65 ms; W product 0.47 -> 0.14 and 0.86 -> 0.69 ms.  FP64,
+// GaussQR 3, k = 2: Dirichlet pass of 320 panels 0.186 -> 0.108 ms, of 1280 panels
+// 0.64 -> 0.51 ms.  The full count is a constant of the kernels where the call has
+// enough CTAs (as a variable it cost them 1 to 2 %).
 inline int bem_far_ti(const bem_ctx* ctx, int n_test, int64_t cols) {
     int ti = FAR_TI;
     while (ti > 1 && cols * ((n_test + ti - 1) / ti) < 16 * (int64_t)ctx->num_sms) ti /= 2;
