@@ -204,14 +204,14 @@ __device__ __forceinline__ void pair_grads(const PairMoments& M, double cw, cons
 // once per trial point.  Bound: FP64 issue, 27 (V) and 50 (K) instructions a
 // point pair for both orders, two thirds of the FP64 pipe at 168 and 252
 // registers (capping K at 168 measured the same).  5120 panels, GaussQR 4
-// (B200): V 7.8 and K 14.3 ms, against 22 and 33 ms per ordered pair with the
-// hats of both sides applied at every point.
+// (B200), whole calls: V 8.3 and K 14.8 ms, against 22.6 and 36.4 ms per ordered
+// pair with the hats of both sides applied at every point.
 //
 // DATA (K): the product K^T lam, the derivative in the nodal data, from the
 // same points.  d.n_i is constant over the test points and sum_q t d.n_j is
 // there already, so it costs nothing per point pair and six multiply-adds a
-// trial point: K 14.3 -> 15.4 ms, in place of a dense FP64 block and its
-// product (7.4 ms at 5120 panels, GaussQR 4).
+// trial point: 1 ms at 5120 panels, GaussQR 4, in place of a dense FP64 block
+// and its product (7.4 ms).
 template <int OP, bool DATA>
 __global__ void __launch_bounds__(ADJ_THREADS) adj_far_kernel(AdjArgs a) {
     constexpr bool K = OP == BEM_OP_K;
@@ -402,7 +402,10 @@ __global__ void __launch_bounds__(ADJ_THREADS) adj_far_kernel(AdjArgs a) {
             double vi[3][3], vj[3][3], n_[3];
             load_tri(a, gi, vi, n_);
             load_tri(a, gj, vj, n_);
-            const double Ji = 2.0 * a.area[gi], Jj = 2.0 * a.area[gj];
+            // one division a panel instead of one a component of a vertex, which at few points
+            // cost as much as the points.  K, 5120 panels: GaussQR 1 2.48 -> 1.59 ms, 2 3.43 ->
+            // 2.53 ms, 4 15.6 -> 14.8 ms; V 1.43 -> 1.24, 1.94 -> 1.70 and 8.54 -> 8.30 ms
+            const double iJi = 0.5 / a.area[gi], iJj = 0.5 / a.area[gj];
             double cw = BEM_INV4PI;
             if (!K) cw *= lami * uj[0] + lamb * s_u[t][0];
             const double along = K ? -3.0 : -1.0;
@@ -413,16 +416,16 @@ __global__ void __launch_bounds__(ADJ_THREADS) adj_far_kernel(AdjArgs a) {
                 jac_grad(vj, nj, h, hj);
                 if (!K) {
                     for (int c = 0; c < 3; ++c) {
-                        tx[c] = jg[c] / Ji * S0;
-                        ty[c] = hj[c] / Jj * S0;
+                        tx[c] = jg[c] * iJi * S0;
+                        ty[c] = hj[c] * iJj * S0;
                     }
                 } else {
                     double g1[3], g2[3];
                     normal_grad(vi, Ni, h, g1);
                     normal_grad(vj, Nj, h, g2);
                     for (int c = 0; c < 3; ++c) {
-                        tx[c] = jg[c] / Ji * sij + g1[c] / Ji;
-                        ty[c] = hj[c] / Jj * sji + g2[c] / Jj;
+                        tx[c] = fma(jg[c], sij, g1[c]) * iJi;
+                        ty[c] = fma(hj[c], sji, g2[c]) * iJj;
                     }
                     const double hxa = h == 0 ? xa[0] - xa[1] - xa[2] : xa[h], hya = h == 0 ? ya[0] - ya[1] - ya[2] : ya[h];
                     const double hxb = h == 0 ? xb[0] - xb[1] - xb[2] : xb[h],
@@ -600,8 +603,8 @@ int bem_launch_adjoint(bem_ctx* ctx, const bem_op_desc* op, const bem_space* tes
     a.data = data;
     // as in bem_launch_far64: fewer test panels per CTA where the call has too few
     // CTAs for some waves.  With few points a pair the trial vertices' atomics, one
-    // set per CTA, weigh more than idle SMs (K, 320 panels, GaussQR 2: 118, 106, 98
-    // and 117 us with 1, 2, 4 and 8; GaussQR 5: 416, 491, 549 and 656 us)
+    // set per CTA, weigh more than idle SMs (K, 320 panels, GaussQR 2: 114, 97, 86
+    // and 93 us with 1, 2, 4 and 8; GaussQR 5: 403, 475, 528 and 622 us)
     a.ti = ADJ_TI;
     const int64_t cols = (a.n_trial + ADJ_THREADS - 1) / ADJ_THREADS;
     const int64_t want = (int64_t)ctx->num_sms * (ctx->Q2 <= 4 ? 1 : (ctx->Q2 <= 9 ? 3 : 16));

@@ -173,3 +173,38 @@ def test_fp64_dirichlet_pass_over_test_panel_counts(engine, sub, Q, cplx):
     engine.apply(engine.op_desc(L.OP_K, cplx, k, k * k), p0, p1, g, b)
     assert float((A - B).abs().max()) < 1e-13 * float(B.abs().max())
     assert float((a - b).abs().max()) < 1e-12 * float(b.abs().max())
+
+
+@pytest.mark.parametrize("op", ["V", "K"])
+@pytest.mark.parametrize("Q", [1, 2])
+def test_shape_adjoint_with_few_points(engine, op, Q):
+    """Panels of unequal size, where the vertices' share of a pair outweighs its
+    points: central differences of lam . A u, h = 1e-5: truncation h^2 / edge^2
+    ~ 1e-8, rounding eps |F| / (h |grad|) ~ 1e-10 of the largest, so 1e-6."""
+    from bem_b200 import _lib as L
+    v, f, _, _ = _sphere(engine, 1, Q)
+    v = v * (1.0 + 0.4 * v[:, :1])
+    desc = engine.op_desc(getattr(L, "OP_" + op), False)
+    lam, u = (_gaussian((n,), torch.float64, 11) for n in (len(f), len(f) if op == "V" else len(v)))
+
+    def spaces(x):
+        from bem_b200.engine import DeviceSpace
+        engine.set_mesh(x, f, Q)
+        p = np.arange(len(f), dtype=np.int32)
+        p0 = DeviceSpace.from_numpy(p, 1, p, engine.device)
+        return p0, p0 if op == "V" else DeviceSpace.from_numpy(p, 3, f.reshape(-1).copy(), engine.device)
+
+    def form(x):
+        y = torch.zeros(len(f), dtype=torch.float64, device="cuda")
+        engine.apply(desc, *spaces(x), u, y)
+        return float(lam @ y)
+
+    grad = torch.zeros(len(v), 3, dtype=torch.float64, device="cuda")
+    engine.adjoint_vertices(desc, *spaces(v), lam, u, grad)
+    grad = grad.cpu().numpy()
+    rng = np.random.default_rng(12)
+    for _ in range(8):
+        d = np.zeros_like(v)
+        d[rng.integers(len(v)), rng.integers(3)] = 1e-5
+        fd = (form(v + d) - form(v - d)) / 2e-5
+        assert abs(fd - (grad * d).sum() / 1e-5) < 1e-6 * np.abs(grad).max()
